@@ -142,7 +142,14 @@ int mark_done(Context &c, cudaStream_t st, int rc)
 
 uint32_t shoup32_companion(uint64_t w, uint64_t Q) { return (uint32_t)((w << 32) / Q); }
 
-uint64_t shoup64_companion(uint64_t w, uint64_t Q) { return (uint64_t)(((unsigned __int128)w << 64) / Q); }
+// The constant pair of w < Q that mul64 takes (ntt64.cuh); nc64.pm_c / pm_s set.
+ulonglong2 const_pair64(const Context &c, uint64_t w)
+{
+    const uint64_t Q = c.p.Q;
+    if (c.nc64.pm_c)
+        return make_ulonglong2(w << c.nc64.pm_s, (uint64_t)(((unsigned __int128)w << 30) % Q) << c.nc64.pm_s);
+    return make_ulonglong2(w, (uint64_t)(((unsigned __int128)w << 64) / Q));
+}
 
 int build_tables64(Context &c)
 {
@@ -150,24 +157,35 @@ int build_tables64(Context &c)
     T.build(c.p);
     const int N = c.p.N;
     const uint64_t Q = c.p.Q;
+    dev::Ntt64Consts &k = c.nc64;
+    k.Q = Q;
+    k.twoQ = 2 * Q;
+    k.mu64 = c.dp.mu64;
+    k.pm_s = (uint32_t)dev::pm64_shift(Q);
+    k.pm_c = k.pm_s ? (uint32_t)(((uint64_t)1 << (64 - k.pm_s)) - Q) : 0;
+    auto put = [&](uint64_t w, uint64_t &x, uint64_t &xs) {
+        const ulonglong2 v = const_pair64(c, w);
+        x = v.x;
+        xs = v.y;
+    };
+    put(c.p.iN, k.iN, k.iNs);
+    put(host::mulmod(T.irou[1], c.p.iN, Q), k.iw1N, k.iw1Ns);
+    put(((uint64_t)1 << 30) % Q, k.p30, k.p30s);
+    k.dw1 = T.rou[1] << k.pm_s;
+    k.dw2 = T.rou[2] << k.pm_s;
+    k.dw3 = T.rou[3] << k.pm_s;
+    k.dw21 = host::mulmod(T.rou[2], T.rou[1], Q) << k.pm_s;
+    k.dw31 = (Q - host::mulmod(T.rou[3], T.rou[1], Q)) << k.pm_s;
     std::vector<ulonglong2> fw(N), iw(N);
     for (int i = 0; i < N; i++) {
-        fw[i] = make_ulonglong2(T.rou[i], shoup64_companion(T.rou[i], Q));
-        iw[i] = make_ulonglong2(T.irou[i], shoup64_companion(T.irou[i], Q));
+        fw[i] = const_pair64(c, T.rou[i]);
+        iw[i] = const_pair64(c, T.irou[i]);
     }
     cudaError_t e = cudaMalloc(&c.d_tw64, N * sizeof(ulonglong2));
     if (e == cudaSuccess) e = cudaMalloc(&c.d_itw64, N * sizeof(ulonglong2));
     if (e == cudaSuccess) e = cudaMemcpy(c.d_tw64, fw.data(), N * sizeof(ulonglong2), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(c.d_itw64, iw.data(), N * sizeof(ulonglong2), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return c.cuda_fail(e, "twiddle upload");
-    dev::Ntt64Consts &k = c.nc64;
-    k.Q = Q;
-    k.twoQ = 2 * Q;
-    k.iN = c.p.iN;
-    k.iNs = shoup64_companion(c.p.iN, Q);
-    k.iw1N = host::mulmod(T.irou[1], c.p.iN, Q);
-    k.iw1Ns = shoup64_companion(k.iw1N, Q);
-    k.mu64 = c.dp.mu64;
     // factors of the last-digit identity (DevParams::last_digit_from_acc), for
     // the bootstrap key and for every RGSW a RLWE x RGSW product takes:
     // BG^(h - digitG + 1) for h < digitG - 1, BG^-(digitG - 1) for the last row
@@ -176,7 +194,7 @@ int build_tables64(Context &c)
     std::vector<ulonglong2> cf(dG);
     for (uint64_t h = 0; h < dG; h++) {
         const uint64_t f = host::powmod(bg_inv, h + 1 < dG ? dG - 1 - h : dG - 1, Q);
-        cf[h] = make_ulonglong2(f, shoup64_companion(f, Q));
+        cf[h] = const_pair64(c, f);
     }
     e = cudaMalloc(&c.d_cf64, dG * sizeof(ulonglong2));
     if (e == cudaSuccess) e = cudaMemcpy(c.d_cf64, cf.data(), dG * sizeof(ulonglong2), cudaMemcpyHostToDevice);
@@ -243,6 +261,18 @@ int build_rotations(Context &c)
         uint64_t *w = fwd.data() + (size_t)j * N;   // rotate_vector_gen(true): NTT(X^(2^j))
         w[1 << j] = 1;
         T.ntt(w);
+    }
+    if (c.wide) {
+        std::vector<ulonglong2> pairs(2 * rot.size());
+        for (size_t i = 0; i < rot.size(); i++) {
+            pairs[i] = const_pair64(c, rot[i]);
+            pairs[rot.size() + i] = const_pair64(c, fwd[i]);
+        }
+        cudaError_t e = cudaMalloc(&c.d_rot64, pairs.size() * sizeof(ulonglong2));
+        if (e == cudaSuccess)
+            e = cudaMemcpy(c.d_rot64, pairs.data(), pairs.size() * sizeof(ulonglong2), cudaMemcpyHostToDevice);
+        c.d_rot_fwd64 = c.d_rot64 + rot.size();
+        return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "rotation tables");
     }
     cudaError_t e = cudaMalloc(&c.d_rot, rot.size() * sizeof(uint64_t));
     if (e == cudaSuccess) e = cudaMemcpy(c.d_rot, rot.data(), rot.size() * sizeof(uint64_t), cudaMemcpyHostToDevice);
@@ -368,6 +398,7 @@ int fheacc_destroy(fheacc_ctx *ctx)
     cudaFree(c->d_cf64);
     cudaFree(c->d_kskey64);
     cudaFree(c->d_subs64);
+    cudaFree(c->d_rot64);
     cudaFree(c->d_rot);
     cudaFree(c->d_rot_fwd);
     cudaFree(c->d_btkey);
@@ -417,7 +448,7 @@ static int bootstrap_key_pass(Context &c, const uint64_t *btkey, size_t words, b
     if (verify && !(c.wide ? (void *)c.d_btkey64 : (void *)c.d_btkey))
         return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
     if (c.wide) {
-        // device order, one step (all residues) per chunk, Shoup pairs made on the GPU
+        // device order, one step (all residues) per chunk, constant pairs (mul64) made on the GPU
         if (!verify && !c.d_btkey64) {
             cudaError_t e = cudaMalloc(&c.d_btkey64, words * sizeof(ulonglong2));
             if (e != cudaSuccess) {
@@ -451,7 +482,7 @@ static int bootstrap_key_pass(Context &c, const uint64_t *btkey, size_t words, b
                 if (e != cudaSuccess) rc = c.cuda_fail(e, "key upload");
                 else if (derive) rc = launch_derive_keys64(c, d_stage, Br, c.d_cf64, c.stream);
                 ulonglong2 *chunk = c.d_btkey64 + (i * dR + j) * Br * rw;
-                if (!rc) rc = launch_shoup_pairs64(c, d_stage, verify ? d_check : chunk, Br * rw, c.stream);
+                if (!rc) rc = launch_const_pairs64(c, d_stage, verify ? d_check : chunk, Br * rw, c.stream);
                 if (!rc && cudaStreamSynchronize(c.stream) != cudaSuccess) rc = c.cuda_fail(cudaGetLastError(), "key pairs");
                 if (!rc && verify) {
                     e = cudaMemcpy(made.data(), d_check, Br * rw * sizeof(ulonglong2), cudaMemcpyDeviceToHost);
@@ -626,7 +657,7 @@ static int subs_key_pass(Context &c, const uint64_t *subs_key, size_t words, boo
             cudaFree(d_check);
             return c.cuda_fail(e, "substitute key upload");
         }
-        int rc = launch_shoup_pairs64(c, d_stage, verify ? d_check : c.d_subs64, words, c.stream);
+        int rc = launch_const_pairs64(c, d_stage, verify ? d_check : c.d_subs64, words, c.stream);
         if (!rc && cudaStreamSynchronize(c.stream) != cudaSuccess) rc = c.cuda_fail(cudaGetLastError(), "key pairs");
         if (!rc && verify) {
             std::vector<ulonglong2> made(words), held(words);
@@ -908,7 +939,7 @@ int fheacc_rlwe_substitute_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t c
     Context &c = *reinterpret_cast<Context *>(ctx);
     DeviceGuard g(c.device);
     cudaStream_t st = pick_stream(&c, stream);
-    return mark_done(c, st, launch_expand(c, 0, d_in, d_out, count, f, nullptr, nullptr, st));
+    return mark_done(c, st, launch_expand(c, 0, d_in, d_out, count, f, nullptr, st));
 }
 
 int fheacc_rlwe_keyswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t count, const uint64_t *d_ksk,
@@ -922,10 +953,10 @@ int fheacc_rlwe_keyswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t co
     const size_t words = (size_t)c.p.digitKS_R * 2 * c.p.N;
     int rc = ensure_scratch(c, c.io, words * (c.wide ? sizeof(ulonglong2) : sizeof(uint32_t)));
     if (rc) return rc;
-    rc = c.wide ? launch_shoup_pairs64(c, d_ksk, (ulonglong2 *)c.io.ptr, words, st)
+    rc = c.wide ? launch_const_pairs64(c, d_ksk, (ulonglong2 *)c.io.ptr, words, st)
                 : launch_to_u32(c, d_ksk, (uint32_t *)c.io.ptr, words, st);
     if (rc) return rc;
-    return mark_done(c, st, launch_expand(c, 1, d_in, d_out, count, 0, c.io.ptr, nullptr, st));
+    return mark_done(c, st, launch_expand(c, 1, d_in, d_out, count, 0, c.io.ptr, st));
 }
 
 int fheacc_subs_keyswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t count, int f, uint64_t *d_out,
@@ -939,7 +970,7 @@ int fheacc_subs_keyswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t co
     if (!key) return c.fail(FHEACC_ENOKEY, "substitute key not uploaded");
     DeviceGuard g(c.device);
     cudaStream_t st = pick_stream(&c, stream);
-    return mark_done(c, st, launch_expand(c, 2, d_in, d_out, count, f, key, nullptr, st));
+    return mark_done(c, st, launch_expand(c, 2, d_in, d_out, count, f, key, st));
 }
 
 }  // extern "C"
@@ -957,8 +988,7 @@ int expand_device(Context &c, const uint64_t *d_in, uint64_t *d_out, cudaStream_
                                       rw * sizeof(uint64_t), count, cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) return c.cuda_fail(e, "expand copy");
     for (int f = 0; f < logN; f++) {
-        int rc = launch_expand(c, 3, d_out, d_out, 0, f, subs_key_level(c, f), c.d_rot + (size_t)f * N, st, count,
-                               stride);
+        int rc = launch_expand(c, 3, d_out, d_out, 0, f, subs_key_level(c, f), st, count, stride);
         if (rc) return rc;
     }
     return FHEACC_OK;

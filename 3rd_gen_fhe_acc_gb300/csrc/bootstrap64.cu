@@ -10,12 +10,12 @@
 // One RLWE x RGSW step runs on a CTA of 256 threads in two 128-thread groups,
 // group p owning poly p of the accumulator: inverse NTT in shared memory, then
 // for each digit h both groups transform digit h of their poly and all 256
-// threads multiply-accumulate it with the key rows. Keys are stored with their
-// Shoup companions (K, floor(K 2^64 / Q)), so every MAC product is one 64-bit
-// Shoup multiply; the 2 * digitG products of an output stay below 24Q and are
-// reduced once. As in the 32-bit kernel, steps are the outer loop over a
+// threads multiply-accumulate it with the key rows. Keys are stored as constant
+// pairs (mul64 in ntt64.cuh: 16 bytes a word); the two products of a digit and
+// an output are folded together (mul64_2), and the digitG sums are reduced
+// once. As in the 32-bit kernel, steps are the outer loop over a
 // group of ciphertexts per CTA, so the CTAs stream each step's 23 RGSW keys
-// (18 MB with companions) through L2 together; accumulators live in global
+// (18 MB) through L2 together; accumulators live in global
 // memory (32 KB per gate).
 #include "ctx.hpp"
 #include "l2hint.cuh"
@@ -28,68 +28,45 @@ namespace dev {
 constexpr int kMaxGroup64 = 8;   // ciphertexts per worker and claim
 constexpr int kT64 = 256;   // threads per CTA
 
-// One worker's polys in shared memory, layout pi<P> (ntt64.cuh): padded in the
-// blind rotation, plain in the RLWE x RGSW kernel (whose L1 the padding costs).
+// One worker's polys in shared memory, layout pi<P> (ntt64.cuh).
+//
+// What the step costs (2048 gates, blind rotation of the n = 630 set): the L1 /
+// shared-memory data pipe was the busiest unit (72 %, 27 % of all cycles in bank
+// conflicts: the digit tables' gathers and a padding of one word in 8), the
+// multiply pipe 60 %. Folded multiplications alone: 582 -> 523 ms; digits
+// extracted inside the first pass, its first two stages from small products
+// instead of tables, one padding word in 16: 464 ms.
 template <bool P>
 struct Step64SmemT {
     uint64_t acc[2][poly_words64<P>()];   // accumulator; time domain inside a step
     uint64_t buf[2][poly_words64<P>()];   // digit NTTs
 };
 
-constexpr int kMaxTableBG64 = 512;   // largest gadget base with digit tables (40 BG bytes of shared memory)
-
-__device__ __forceinline__ uint64_t mulmod64(uint64_t a, uint64_t b, uint64_t Q)
-{
-    return (uint64_t)((unsigned __int128)a * b % Q);
-}
-
-// Builds the digit tables (DigitTables64) for y < BG in `mem` (40 BG bytes,
-// 16-byte aligned) from the twiddles tw[1..3]; all threads of the CTA take part.
-__device__ __forceinline__ DigitTables64 build_digit_tables64(unsigned char *mem, int BG,
-                                                             const ulonglong2 *__restrict__ tw, uint64_t Q)
-{
-    ulonglong2 *t23 = reinterpret_cast<ulonglong2 *>(mem), *t123 = t23 + BG;
-    uint64_t *t1 = reinterpret_cast<uint64_t *>(t123 + BG);
-    const uint64_t w1 = tw[1].x, w2 = tw[2].x, w3 = tw[3].x;
-    const uint64_t w21 = mulmod64(w2, w1, Q), w31 = mulmod64(w3, w1, Q);
-    for (int y = threadIdx.x; y < BG; y += blockDim.x) {
-        t1[y] = mulmod64((uint64_t)y, w1, Q);
-        t23[y] = make_ulonglong2(mulmod64((uint64_t)y, w2, Q), mulmod64((uint64_t)y, w3, Q));
-        t123[y] = make_ulonglong2(mulmod64((uint64_t)y, w21, Q), mulmod64((uint64_t)y, w31, Q));
-    }
-    return DigitTables64{t1, t23, t123};
-}
-
 // One RLWE x RGSW step on s.acc (NTT domain, values < 2Q) with the key
-// `key` (Shoup pairs, [digitG][2][2][2048]), run by the 256 threads tid of a
+// `key` (constant pairs, [digitG][2][2][2048]), run by the 256 threads tid of a
 // worker that synchronises on named barrier `bar` (its two 128-thread groups
 // on bar + 1 and bar + 2).
 // With acc_nd (the step's NTT-domain accumulator in global memory, read before
 // it is overwritten) the last digit's NTT is replaced by the accumulator: the
 // keys were uploaded with K'_h = K_h - BG^(h-DG+1) K_last, K'_last =
 // BG^-(DG-1) K_last (Q < BG^DG, so sum_h BG^h NTT(digit_h) = acc).
-// With dt the digit transforms start from the digit tables (BG <= kMaxTableBG64).
 // KEEP: acc_nd is read with the L2 evict-last policy (l2hint.cuh).
-template <bool P, bool KEEP = false>
+template <bool PM, bool P, bool KEEP = false>
 __device__ __forceinline__ void step64(Step64SmemT<P> &s, const ulonglong2 *__restrict__ key, int DG, uint32_t bg_bits,
                                        const ulonglong2 *__restrict__ tw, const ulonglong2 *__restrict__ itw,
-                                       const Ntt64Consts &c, const uint64_t *acc_nd, int tid, int bar,
-                                       const DigitTables64 *dt = nullptr)
+                                       const Ntt64Consts &c, const uint64_t *acc_nd, int tid, int bar)
 {
     const int grp = tid >> 7, gtid = tid & 127;
-    ntt64_inv_2048<128, P>(s.acc[grp], itw, c, gtid, bar + 1 + grp);
+    ntt64_inv_2048<PM, 128, P>(s.acc[grp], itw, c, gtid, bar + 1 + grp);
     group_sync(bar, kT64);
     uint64_t sa[8], sb[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) sa[i] = sb[i] = 0;
-    const uint64_t mask = (1ULL << bg_bits) - 1;
+    const uint32_t mask = (1u << bg_bits) - 1;
     const int DH = acc_nd ? DG - 1 : DG;   // digits transformed
     for (int h = 0; h < DH; h++) {
-        const uint32_t sh = bg_bits * h;
-        for (int e = gtid; e < 2048; e += 128) s.buf[grp][pi<P>(e)] = (s.acc[grp][pi<P>(e)] >> sh) & mask;
-        group_sync(bar + 1 + grp, 128);
-        if (dt) ntt64_fwd_2048_digit<128, P>(s.buf[grp], tw, c, gtid, bar + 1 + grp, *dt);
-        else ntt64_fwd_2048<128, P>(s.buf[grp], tw, c, gtid, bar + 1 + grp);
+        ntt64_fwd_2048_load<PM, 128, P, true>(s.buf[grp], LoadDigit64<P>{s.acc[grp], bg_bits * h, mask}, tw, c, gtid,
+                                              bar + 1 + grp);
         group_sync(bar, kT64);
         const ulonglong2 *k0 = key + (size_t)(h * 2 + 0) * 2 * 2048;   // row c_text[h][0]: times digit of a
         const ulonglong2 *k1 = key + (size_t)(h * 2 + 1) * 2 * 2048;   // row c_text[h][1]: times digit of b
@@ -99,8 +76,8 @@ __device__ __forceinline__ void step64(Step64SmemT<P> &s, const ulonglong2 *__re
             const uint64_t da = s.buf[0][pi<P>(k)], db = s.buf[1][pi<P>(k)];
             const ulonglong2 a0 = __ldg(k0 + k), b0 = __ldg(k0 + 2048 + k);
             const ulonglong2 a1 = __ldg(k1 + k), b1 = __ldg(k1 + 2048 + k);
-            sa[i] += shoup64(da, a0.x, a0.y, c.Q) + shoup64(db, a1.x, a1.y, c.Q);
-            sb[i] += shoup64(da, b0.x, b0.y, c.Q) + shoup64(db, b1.x, b1.y, c.Q);
+            sa[i] += mul64_2<PM>(da, a0, db, a1, c);
+            sb[i] += mul64_2<PM>(da, b0, db, b1, c);
         }
         group_sync(bar, kT64);
     }
@@ -121,22 +98,22 @@ __device__ __forceinline__ void step64(Step64SmemT<P> &s, const ulonglong2 *__re
             }
             const ulonglong2 a0 = __ldg(k0 + k), b0 = __ldg(k0 + 2048 + k);
             const ulonglong2 a1 = __ldg(k1 + k), b1 = __ldg(k1 + 2048 + k);
-            sa[i] += shoup64(da, a0.x, a0.y, c.Q) + shoup64(db, a1.x, a1.y, c.Q);
-            sb[i] += shoup64(da, b0.x, b0.y, c.Q) + shoup64(db, b1.x, b1.y, c.Q);
+            sa[i] += mul64_2<PM>(da, a0, db, a1, c);
+            sb[i] += mul64_2<PM>(da, b0, db, b1, c);
         }
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int k = tid + 256 * i;
-        s.acc[0][pi<P>(k)] = barrett64_2q(sa[i], c.mu64, c.Q);
-        s.acc[1][pi<P>(k)] = barrett64_2q(sb[i], c.mu64, c.Q);
+        s.acc[0][pi<P>(k)] = reduce64<PM>(sa[i], c);
+        s.acc[1][pi<P>(k)] = reduce64<PM>(sb[i], c);
     }
     group_sync(bar, kT64);
 }
 
 // Forward / inverse NTT of count polys (u64, canonical in and out), one
 // 128-thread group per poly.
-template <bool INV>
+template <bool PM, bool INV>
 __global__ void __launch_bounds__(kT64) ntt64_kernel(uint64_t *polys, size_t count, const ulonglong2 *__restrict__ tw,
                                                     const __grid_constant__ Ntt64Consts c)
 {
@@ -148,14 +125,13 @@ __global__ void __launch_bounds__(kT64) ntt64_kernel(uint64_t *polys, size_t cou
         uint64_t *poly = polys + pi * 2048;
         for (int e = gtid; e < 2048; e += 128) buf[grp][e] = live ? poly[e] : 0;
         group_sync(1 + grp, 128);
-        if (INV) ntt64_inv_2048<128, false>(buf[grp], tw, c, gtid, 1 + grp);
-        else ntt64_fwd_2048<128, false>(buf[grp], tw, c, gtid, 1 + grp);
+        if (INV) ntt64_inv_2048<PM, 128, false>(buf[grp], tw, c, gtid, 1 + grp);
+        else ntt64_fwd_2048<PM, 128, false>(buf[grp], tw, c, gtid, 1 + grp);
         if (live) {
             for (int e = gtid; e < 2048; e += 128) {
                 uint64_t v = buf[grp][e];
                 if (!INV) {
-                    v = barrett64_2q(v, c.mu64, c.Q);
-                    v = v >= c.Q ? v - c.Q : v;
+                    v = canonical64<PM>(v, c);
                 }
                 poly[e] = v;
             }
@@ -166,10 +142,12 @@ __global__ void __launch_bounds__(kT64) ntt64_kernel(uint64_t *polys, size_t cou
 
 // The last-digit identity on `count` RGSWs [DG][4][N] (u64, reduced in
 // place): row h < DG-1 becomes K_h - cf[h] K_last, row DG-1 becomes
-// cf[DG-1] K_last, mod Q; (cf, cfs) Shoup pairs of the factors.
+// cf[DG-1] K_last, mod Q; cf: constant pairs of the factors (mul64).
+template <bool PM>
 __global__ void derive_keys64_kernel(uint64_t *__restrict__ keys, size_t count, int DG, int N,
-                                     const ulonglong2 *__restrict__ cf, uint64_t Q)
+                                     const ulonglong2 *__restrict__ cf, const __grid_constant__ Ntt64Consts c)
 {
+    const uint64_t Q = c.Q;
     const size_t plane = 4 * (size_t)N;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count * plane;
          i += (size_t)gridDim.x * blockDim.x) {
@@ -178,28 +156,36 @@ __global__ void derive_keys64_kernel(uint64_t *__restrict__ keys, size_t count, 
         const uint64_t last = rg[(size_t)(DG - 1) * plane + x] % Q;
         for (int h = 0; h + 1 < DG; h++) {
             const uint64_t k = rg[(size_t)h * plane + x] % Q;
-            uint64_t m = shoup64(last, cf[h].x, cf[h].y, Q);
+            uint64_t m = mul64<PM>(last, cf[h], c);
             m = m >= Q ? m - Q : m;
             rg[(size_t)h * plane + x] = k >= m ? k - m : k + Q - m;
         }
-        uint64_t m = shoup64(last, cf[DG - 1].x, cf[DG - 1].y, Q);
+        uint64_t m = mul64<PM>(last, cf[DG - 1], c);
         rg[(size_t)(DG - 1) * plane + x] = m >= Q ? m - Q : m;
     }
 }
 
-// (K, floor(K 2^64 / Q)) pairs of key words (reduced mod Q first).
-__global__ void shoup_pairs64_kernel(const uint64_t *__restrict__ in, ulonglong2 *__restrict__ out, size_t n,
-                                     uint64_t Q)
+// Constant pairs (mul64) of key words (reduced mod Q first).
+template <bool PM>
+__global__ void const_pairs64_kernel(const uint64_t *__restrict__ in, ulonglong2 *__restrict__ out, size_t n,
+                                     const __grid_constant__ Ntt64Consts c)
 {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const uint64_t w = in[i] % Q;
-        out[i] = make_ulonglong2(w, (uint64_t)(((unsigned __int128)w << 64) / Q));
+        const uint64_t w = in[i] % c.Q;
+        if (PM) {
+            uint64_t v = mul64<PM>(w, make_ulonglong2(c.p30, c.p30s), c);
+            v = v >= c.Q ? v - c.Q : v;
+            out[i] = make_ulonglong2(w << c.pm_s, v << c.pm_s);
+        } else {
+            out[i] = make_ulonglong2(w, (uint64_t)(((unsigned __int128)w << 64) / c.Q));
+        }
     }
 }
 
 // RLWE_mult_RGSW of count (acc, RGSW-pairs) in reference order; acc canonical.
 // derive: the RGSWs carry the last-digit identity (derive_keys64_kernel) and the
 // last digit's NTT is the input accumulator itself.
+template <bool PM>
 __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_kernel(const uint64_t *__restrict__ acc_in,
                                                                const ulonglong2 *__restrict__ rgsw, uint64_t *acc_out,
                                                                size_t count, size_t rgsw_stride, int DG, uint32_t bg_bits,
@@ -208,14 +194,14 @@ __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_kernel(const uint64_t *
                                                                const __grid_constant__ Ntt64Consts c, int derive)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Step64SmemT<false> &s = *reinterpret_cast<Step64SmemT<false> *>(smem_raw);
+    Step64SmemT<true> &s = *reinterpret_cast<Step64SmemT<true> *>(smem_raw);
     for (size_t ci = blockIdx.x; ci < count; ci += gridDim.x) {
-        for (int e = threadIdx.x; e < 4096; e += kT64) s.acc[e >> 11][e & 2047] = acc_in[ci * 4096 + e];
+        for (int e = threadIdx.x; e < 4096; e += kT64) s.acc[e >> 11][px(e & 2047)] = acc_in[ci * 4096 + e];
         __syncthreads();
-        step64(s, rgsw + ci * rgsw_stride, DG, bg_bits, tw, itw, c, derive ? acc_in + ci * 4096 : nullptr,
+        step64<PM>(s, rgsw + ci * rgsw_stride, DG, bg_bits, tw, itw, c, derive ? acc_in + ci * 4096 : nullptr,
                threadIdx.x, 1);
         for (int e = threadIdx.x; e < 4096; e += kT64) {
-            const uint64_t v = s.acc[e >> 11][e & 2047];
+            const uint64_t v = s.acc[e >> 11][px(e & 2047)];
             acc_out[ci * 4096 + e] = v >= c.Q ? v - c.Q : v;
         }
         __syncthreads();
@@ -228,6 +214,7 @@ __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_kernel(const uint64_t *
 // the multiply-accumulate to partial[ci][h] (two Shoup products per word, < 4Q);
 // rlwe_split_sum64_kernel adds the digitG shares. A lone product's inverse and
 // digit NTTs then take two rounds instead of 1 + digitG.
+template <bool PM>
 __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_split_kernel(const uint64_t *__restrict__ acc_in,
                                                                      const ulonglong2 *__restrict__ rgsw,
                                                                      uint64_t *__restrict__ partial, size_t rgsw_stride,
@@ -237,18 +224,15 @@ __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_split_kernel(const uint
                                                                      const __grid_constant__ Ntt64Consts c)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Step64SmemT<false> &s = *reinterpret_cast<Step64SmemT<false> *>(smem_raw);
+    Step64SmemT<true> &s = *reinterpret_cast<Step64SmemT<true> *>(smem_raw);
     const size_t ci = blockIdx.x / (unsigned)DG;
     const int h = (int)(blockIdx.x - ci * (unsigned)DG);
     const int tid = threadIdx.x, grp = tid >> 7, gtid = tid & 127;
-    for (int e = tid; e < 4096; e += kT64) s.acc[e >> 11][e & 2047] = acc_in[ci * 4096 + e];
+    for (int e = tid; e < 4096; e += kT64) s.acc[e >> 11][px(e & 2047)] = acc_in[ci * 4096 + e];
     __syncthreads();
-    ntt64_inv_2048<128, false>(s.acc[grp], itw, c, gtid, 2 + grp);   // ends with the group's barrier
-    const uint64_t mask = (1ULL << bg_bits) - 1;
-    const uint32_t sh = bg_bits * (uint32_t)h;
-    for (int e = gtid; e < 2048; e += 128) s.buf[grp][e] = (s.acc[grp][e] >> sh) & mask;
-    group_sync(2 + grp, 128);
-    ntt64_fwd_2048<128, false>(s.buf[grp], tw, c, gtid, 2 + grp);
+    ntt64_inv_2048<PM, 128, true>(s.acc[grp], itw, c, gtid, 2 + grp);   // ends with the group's barrier
+    ntt64_fwd_2048_load<PM, 128, true, true>(
+        s.buf[grp], LoadDigit64<true>{s.acc[grp], bg_bits * (uint32_t)h, (1u << bg_bits) - 1}, tw, c, gtid, 2 + grp);
     __syncthreads();
     const ulonglong2 *key = rgsw + ci * rgsw_stride;
     const ulonglong2 *k0 = key + (size_t)(h * 2 + 0) * 2 * 2048;   // row c_text[h][0]: times digit of a
@@ -257,16 +241,17 @@ __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_split_kernel(const uint
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int k = tid + 256 * i;
-        const uint64_t da = s.buf[0][k], db = s.buf[1][k];
+        const uint64_t da = s.buf[0][px(k)], db = s.buf[1][px(k)];
         const ulonglong2 a0 = __ldg(k0 + k), b0 = __ldg(k0 + 2048 + k);
         const ulonglong2 a1 = __ldg(k1 + k), b1 = __ldg(k1 + 2048 + k);
-        out[k] = shoup64(da, a0.x, a0.y, c.Q) + shoup64(db, a1.x, a1.y, c.Q);
-        out[2048 + k] = shoup64(da, b0.x, b0.y, c.Q) + shoup64(db, b1.x, b1.y, c.Q);
+        out[k] = mul64_2<PM>(da, a0, db, a1, c);
+        out[2048 + k] = mul64_2<PM>(da, b0, db, b1, c);
     }
 }
 
 // acc_out[ci] = sum over h of partial[ci][h] mod Q (canonical); the sum of
 // digitG shares < 4Q stays below 2^64 (checked by the launcher).
+template <bool PM>
 __global__ void rlwe_split_sum64_kernel(const uint64_t *__restrict__ partial, uint64_t *__restrict__ acc_out,
                                         size_t count, int DG, const __grid_constant__ Ntt64Consts c)
 {
@@ -276,8 +261,7 @@ __global__ void rlwe_split_sum64_kernel(const uint64_t *__restrict__ partial, ui
         const uint64_t *p = partial + ci * (unsigned)DG * 4096 + e;
         uint64_t sum = 0;
         for (int h = 0; h < DG; h++) sum += p[(size_t)h * 4096];
-        const uint64_t v = barrett64_2q(sum, c.mu64, c.Q);
-        acc_out[w] = v >= c.Q ? v - c.Q : v;
+        acc_out[w] = canonical64<PM>(sum, c);
     }
 }
 
@@ -286,7 +270,7 @@ struct Br64Args {
     const uint32_t *idx1, *idx2;   // optional: gate g reads c1 + idx1[g] * (n+1) (else g)
     const int32_t *gates;
     size_t count;
-    const ulonglong2 *btkey;   // [(i*digitR + j)*Br + r][digitG][2][2][2048] Shoup pairs
+    const ulonglong2 *btkey;   // [(i*digitR + j)*Br + r][digitG][2][2][2048] constant pairs
     uint64_t *accs;            // scratch [count][2][2048], NTT domain, values < 2Q
     uint64_t *acc_out;         // optional canonical NTT accumulators [count][4096]
     uint64_t *extract;         // optional [count][kExtract64]
@@ -299,7 +283,6 @@ struct Br64Args {
     unsigned long long *claim_next;   // next unclaimed ciphertext (zeroed before the launch)
     unsigned *status;          // set to kStatusWaitLimit if a worker gave up waiting
     unsigned wait_limit;       // polls before such a wait gives up (kWorkerWaitLimit)
-    int digit_tables;          // digit NTTs start from tables (DigitTables64) after the residues
     size_t claim_limit;        // ciphertexts [0, claim_limit) are claimed in groups
     // remainder pool: ciphertexts [pool_first, pool_first + pool_count) that all
     // CTAs share item by item (0: none); their state after the claim words
@@ -345,7 +328,7 @@ __device__ __forceinline__ void br64_residues(const Br64Args &A, size_t gid, uin
 // a = 0, b = the test vector, forward NTT. buf: a shared poly (layout pi<P>)
 // that the worker's second 128-thread group transforms; bar: the worker's
 // barrier (its groups on bar + 1 and bar + 2).
-template <bool P>
+template <bool PM, bool P>
 __device__ __forceinline__ void br64_acc_init(const Br64Args &A, const Ntt64Consts &c, const ulonglong2 *tw,
                                               size_t gid, uint32_t val, uint32_t b1, uint32_t b2, uint64_t *buf,
                                               int tid, int bar)
@@ -362,14 +345,13 @@ __device__ __forceinline__ void br64_acc_init(const Br64Args &A, const Ntt64Cons
         buf[pi<P>(e)] = v;
     }
     group_sync(bar, kT64);
-    if (tid >= 128) ntt64_fwd_2048<128, P>(buf, tw, c, tid - 128, bar + 2);
+    if (tid >= 128) ntt64_fwd_2048<PM, 128, P>(buf, tw, c, tid - 128, bar + 2);
     group_sync(bar, kT64);
     uint64_t *acc = A.accs + gid * 4096;
     const uint64_t pol = l2_keep_policy();
     for (int e = tid; e < 2048; e += kT64) {
         st_keep64(acc + e, 0, pol);
-        const uint64_t v = barrett64_2q(buf[pi<P>(e)], c.mu64, c.Q);
-        st_keep64(acc + 2048 + e, v >= c.Q ? v - c.Q : v, pol);
+        st_keep64(acc + 2048 + e, canonical64<PM>(buf[pi<P>(e)], c), pol);
     }
     group_sync(bar, kT64);
 }
@@ -377,7 +359,7 @@ __device__ __forceinline__ void br64_acc_init(const Br64Args &A, const Ntt64Cons
 // Output of ciphertext gid from its accumulator: the extracted RLWE
 // (NTT_a_transpose, RLWE.cpp:218-226, then the inverse NTT of both polys) or
 // the canonical NTT accumulator. a0, a1: shared polys (layout pi<P>).
-template <bool P>
+template <bool PM, bool P>
 __device__ __noinline__ void br64_output(const Br64Args &A, const Ntt64Consts &c, const ulonglong2 *itw,
                                             size_t gid, uint64_t *a0, uint64_t *a1, int tid, int bar)
 {
@@ -388,7 +370,7 @@ __device__ __noinline__ void br64_output(const Br64Args &A, const Ntt64Consts &c
             a1[pi<P>(e)] = __ldcg(acc + 2048 + e);
         }
         group_sync(bar, kT64);
-        ntt64_inv_2048<128, P>(tid < 128 ? a0 : a1, itw, c, tid & 127, bar + 1 + (tid >> 7));
+        ntt64_inv_2048<PM, 128, P>(tid < 128 ? a0 : a1, itw, c, tid & 127, bar + 1 + (tid >> 7));
         group_sync(bar, kT64);
         uint64_t *ext = A.extract + gid * kExtract64;
         for (int e = tid; e < 2048; e += kT64) ext[e] = a0[pi<P>(e)];
@@ -405,6 +387,7 @@ __device__ __noinline__ void br64_output(const Br64Args &A, const Ntt64Consts &c
 // Remainder pool set-up, one 256-thread CTA per pool ciphertext, before the
 // blind rotation on the same stream: residues, last non-zero step, the
 // initialised accumulator, and the output of a ciphertext without steps.
+template <bool PM>
 __global__ void __launch_bounds__(kT64) br64_pool_init_kernel(const __grid_constant__ Br64Args A,
                                                              const ulonglong2 *__restrict__ tw,
                                                              const ulonglong2 *__restrict__ itw,
@@ -431,9 +414,9 @@ __global__ void __launch_bounds__(kT64) br64_pool_init_kernel(const __grid_const
         A.pool_last[p] = l;
         A.pool_done[p] = -1;
     }
-    br64_acc_init<false>(A, c, tw, gid, bv[0], bv[1], bv[2], buf[1], tid, 1);
+    br64_acc_init<PM, false>(A, c, tw, gid, bv[0], bv[1], bv[2], buf[1], tid, 1);
     __syncthreads();
-    if (last < 0) br64_output<false>(A, c, itw, gid, buf[0], buf[1], tid, 1);
+    if (last < 0) br64_output<PM, false>(A, c, itw, gid, buf[0], buf[1], tid, 1);
 }
 
 // Polls of a worker waiting for another worker's step of the same ciphertext
@@ -476,9 +459,8 @@ __device__ __forceinline__ bool pool_take(const Br64Args &A, int S, int mode, un
     }
 }
 
-// W workers of 256 threads per CTA (W = 1: 3 CTAs per SM, 80 registers; the
-// extra resident warps hide the latency of the key stream better than the
-// spill-free 2-CTA register allocation, 862 vs 1028 ms for 2048 gates). Each
+// W workers of 256 threads per CTA (W = 1: a lone gate per SM, 128 registers
+// without spills; 49 ms for one gate where 80 registers took 95 ms). Each
 // CTA claims groups of consecutive ciphertexts; its workers share the group's
 // (step, ciphertext) items through a cursor that walks them step-major, and a
 // worker issues an item once the previous item of its ciphertext (its last
@@ -489,7 +471,7 @@ __device__ __forceinline__ bool pool_take(const Br64Args &A, int S, int mode, un
 // ciphertexts form a pool that all CTAs share item by item (pool_take), their
 // steps ordered by done words in global memory. An XOR swizzle of the shared-memory passes removed their bank
 // conflicts but cost more in index arithmetic than it saved.
-template <int W, int MINB>
+template <bool PM, int W, int MINB>
 __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_constant__ Br64Args A,
                                                           const ulonglong2 *__restrict__ tw,
                                                           const ulonglong2 *__restrict__ itw,
@@ -515,9 +497,6 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
         won = 1;
         pool_seen = 0;
     }
-    // digit tables after the residue table of the largest group
-    const DigitTables64 dt = build_digit_tables64(res + ((size_t)A.group * S + 15) / 16 * 16,
-                                                  A.digit_tables ? 1 << A.bg_bits : 0, tw, c.Q);
     for (;;) {
         if (threadIdx.x == 0) {
             const unsigned long long f = atomicAdd(A.claim_next, (unsigned long long)A.group);
@@ -537,7 +516,7 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
         // acc_initialization, one ciphertext per worker: a = 0, b = test vector,
         // forward NTT (the worker's group 1 transforms b)
         for (int k = wk; k < m; k += W)
-            br64_acc_init<true>(A, c, tw, first + (size_t)k, bvals[k], b1s[k], b2s[k], s.buf[1], tid, bar);
+            br64_acc_init<PM, true>(A, c, tw, first + (size_t)k, bvals[k], b1s[k], b2s[k], s.buf[1], tid, bar);
         __syncthreads();
         // blind rotation: the workers take the group's items from the cursor
         for (;;) {
@@ -606,8 +585,8 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
                 const uint64_t pol = l2_keep_policy();
                 for (int e = tid; e < 4096; e += kT64) s.acc[e >> 11][px(e & 2047)] = ld_keep64(acc + e, pol);
                 group_sync(bar, kT64);
-                step64<true, true>(s, A.btkey + ((size_t)st * A.Br + r) * rgsw_pairs, A.DG, A.bg_bits, tw, itw, c,
-                       A.derive_last ? acc : nullptr, tid, bar, A.digit_tables ? &dt : nullptr);
+                step64<PM, true, true>(s, A.btkey + ((size_t)st * A.Br + r) * rgsw_pairs, A.DG, A.bg_bits, tw, itw, c,
+                       A.derive_last ? acc : nullptr, tid, bar);
             }
             // the item again from the plan (not held in registers across the step;
             // the plan changes only after the barrier below)
@@ -630,11 +609,11 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
                 }
             }
             // a pool ciphertext's output right after its last step
-            if (pool && st == A.pool_last[k]) br64_output<true>(A, c, itw, gid, s.acc[0], s.acc[1], tid, bar);
+            if (pool && st == A.pool_last[k]) br64_output<PM, true>(A, c, itw, gid, s.acc[0], s.acc[1], tid, bar);
         }
         __syncthreads();
         // output, one ciphertext per worker
-        for (int k = wk; k < m; k += W) br64_output<true>(A, c, itw, first + (size_t)k, s.acc[0], s.acc[1], tid, bar);
+        for (int k = wk; k < m; k += W) br64_output<PM, true>(A, c, itw, first + (size_t)k, s.acc[0], s.acc[1], tid, bar);
         __syncthreads();
     }
     // a CTA counts into every bucket it has not counted into yet
@@ -645,6 +624,7 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
 }
 
 // Extraction of canonical NTT RLWEs (u64) for the key-switch entry point.
+template <bool PM>
 __global__ void __launch_bounds__(kT64) extract64_kernel(const uint64_t *__restrict__ rlwe, size_t count,
                                                         uint64_t *__restrict__ extract,
                                                         const ulonglong2 *__restrict__ itw,
@@ -659,7 +639,7 @@ __global__ void __launch_bounds__(kT64) extract64_kernel(const uint64_t *__restr
             buf[1][e] = in[2048 + e];
         }
         __syncthreads();
-        ntt64_inv_2048<128, false>(buf[tid >> 7], itw, c, tid & 127, 1 + (tid >> 7));
+        ntt64_inv_2048<PM, 128, false>(buf[tid >> 7], itw, c, tid & 127, 1 + (tid >> 7));
         __syncthreads();
         uint64_t *ext = extract + ci * kExtract64;
         for (int e = tid; e < 2048; e += kT64) ext[e] = buf[0][e];
@@ -817,34 +797,33 @@ static int sms_of(Context &c)
 int launch_derive_keys64(Context &c, uint64_t *d_keys, size_t count, const ulonglong2 *d_cf, cudaStream_t st)
 {
     if (!count) return FHEACC_OK;
-    dev::derive_keys64_kernel<<<(unsigned)std::min<size_t>((count * 4 * c.p.N + 255) / 256, 8192), 256, 0, st>>>(
-        d_keys, count, (int)c.p.digitG, c.p.N, d_cf, c.p.Q);
+    auto kern = c.nc64.pm_c ? dev::derive_keys64_kernel<true> : dev::derive_keys64_kernel<false>;
+    kern<<<(unsigned)std::min<size_t>((count * 4 * c.p.N + 255) / 256, 8192), 256, 0, st>>>(
+        d_keys, count, (int)c.p.digitG, c.p.N, d_cf, c.nc64);
     c.launches++;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "derive keys launch");
 }
 
-int launch_shoup_pairs64(Context &c, const uint64_t *d_in, ulonglong2 *d_out, size_t n, cudaStream_t st)
+int launch_const_pairs64(Context &c, const uint64_t *d_in, ulonglong2 *d_out, size_t n, cudaStream_t st)
 {
     if (!n) return FHEACC_OK;
     unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)sms_of(c) * 32);
-    dev::shoup_pairs64_kernel<<<blocks, 256, 0, st>>>(d_in, d_out, n, c.p.Q);
+    auto kern = c.nc64.pm_c ? dev::const_pairs64_kernel<true> : dev::const_pairs64_kernel<false>;
+    kern<<<blocks, 256, 0, st>>>(d_in, d_out, n, c.nc64);
     c.launches++;
     cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "shoup pairs launch");
+    return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "constant pairs launch");
 }
 
 int launch_ntt64(Context &c, uint64_t *d_polys, size_t count, bool inverse, cudaStream_t st)
 {
     if (!count) return FHEACC_OK;
     size_t blocks = std::min<size_t>((count + 1) / 2, (size_t)sms_of(c) * 8);
-    if (inverse) {
-        dev::ntt64_kernel<true><<<(unsigned)blocks, dev::kT64, 0, st>>>(d_polys, count, c.d_itw64, c.nc64);
-        c.launches++;
-    } else {
-        dev::ntt64_kernel<false><<<(unsigned)blocks, dev::kT64, 0, st>>>(d_polys, count, c.d_tw64, c.nc64);
-        c.launches++;
-    }
+    auto kern = c.nc64.pm_c ? (inverse ? dev::ntt64_kernel<true, true> : dev::ntt64_kernel<true, false>)
+                            : (inverse ? dev::ntt64_kernel<false, true> : dev::ntt64_kernel<false, false>);
+    kern<<<(unsigned)blocks, dev::kT64, 0, st>>>(d_polys, count, inverse ? c.d_itw64 : c.d_tw64, c.nc64);
+    c.launches++;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "ntt64 launch");
 }
@@ -856,7 +835,7 @@ int launch_rlwe_mult_rgsw64(Context &c, const uint64_t *d_acc, const uint64_t *d
     const size_t rw = (size_t)c.p.digitG * 4 * 2048;
     if (stride != 0 && stride != rw) return c.fail(FHEACC_EINVAL, "RGSW stride: 0 or one RGSW");
     const size_t words = (stride ? count : 1) * rw;
-    // Shoup pairs of the RGSWs, after the last-digit identity when it applies
+    // constant pairs of the RGSWs, after the last-digit identity when it applies
     // (2 of the 2 digitG digit NTTs of a product saved); a call of a few
     // products keeps the plain RGSWs, whose derivation would cost it more
     // (PSI query: homo_expand 7.87 -> 7.51 ms, its 1-item CMUXes 0.79 -> 0.90 ms)
@@ -880,29 +859,30 @@ int launch_rlwe_mult_rgsw64(Context &c, const uint64_t *d_acc, const uint64_t *d
         if (rc) return rc;
         src = staged;
     }
-    rc = launch_shoup_pairs64(c, src, pairs, words, st);
+    rc = launch_const_pairs64(c, src, pairs, words, st);
     if (rc) return rc;
     if (split) {
         uint64_t *partial = reinterpret_cast<uint64_t *>(pairs + words);
-        const size_t smem = sizeof(dev::Step64SmemT<false>);
-        cudaFuncSetAttribute(dev::rlwe_mult_rgsw64_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        dev::rlwe_mult_rgsw64_split_kernel<<<(unsigned)(count * DG), dev::kT64, smem, st>>>(
+        const size_t smem = sizeof(dev::Step64SmemT<true>);
+        auto kern = c.nc64.pm_c ? dev::rlwe_mult_rgsw64_split_kernel<true> : dev::rlwe_mult_rgsw64_split_kernel<false>;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kern<<<(unsigned)(count * DG), dev::kT64, smem, st>>>(
             d_acc, pairs, partial, stride, (int)DG, c.p.BG_bits, c.d_tw64, c.d_itw64, c.nc64);
         c.launches++;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return c.cuda_fail(e, "rlwe_mult_rgsw64 split launch");
         const unsigned blocks = (unsigned)std::min<size_t>((count * 4096 + 255) / 256, (size_t)sms_of(c) * 4);
-        dev::rlwe_split_sum64_kernel<<<blocks, 256, 0, st>>>(partial, d_out, count, (int)DG, c.nc64);
+        auto sum = c.nc64.pm_c ? dev::rlwe_split_sum64_kernel<true> : dev::rlwe_split_sum64_kernel<false>;
+        sum<<<blocks, 256, 0, st>>>(partial, d_out, count, (int)DG, c.nc64);
         c.launches++;
         e = cudaGetLastError();
         return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "rlwe_mult_rgsw64 split sum launch");
     }
-    // no digit tables here: their 20 KB of shared memory cost this kernel more
-    // L1 (twiddles, the shared RGSW) than they saved (homo_expand 7.9 -> 8.4 ms)
-    const size_t smem = sizeof(dev::Step64SmemT<false>);
-    cudaFuncSetAttribute(dev::rlwe_mult_rgsw64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = sizeof(dev::Step64SmemT<true>);
+    auto kern = c.nc64.pm_c ? dev::rlwe_mult_rgsw64_kernel<true> : dev::rlwe_mult_rgsw64_kernel<false>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     size_t blocks = std::min<size_t>(count, (size_t)sms_of(c) * 2);
-    dev::rlwe_mult_rgsw64_kernel<<<(unsigned)blocks, dev::kT64, smem, st>>>(
+    kern<<<(unsigned)blocks, dev::kT64, smem, st>>>(
         d_acc, pairs, d_out, count, stride, (int)c.p.digitG, c.p.BG_bits, c.d_tw64, c.d_itw64, c.nc64, derive ? 1 : 0);
     c.launches++;
     cudaError_t e = cudaGetLastError();
@@ -921,24 +901,19 @@ int launch_blind_rotate64(Context &c, const uint64_t *d_c1, const uint64_t *d_c2
                                       d_extract, max_ctas, st);
 }
 
-template <int W, int MINB>
+template <bool PM, int W, int MINB>
 static int launch_br64_shape(Context &c, dev::Br64Args A, int max_ctas, cudaStream_t st)
 {
-    auto kern = dev::br64_kernel<W, MINB>;
+    auto kern = dev::br64_kernel<PM, W, MINB>;
     const size_t steps = (size_t)c.p.n * c.p.digitR;
     // group cap: kMaxGroup64 (or the tuned cap) per worker, within the shared memory of one CTA
     int cap = W * (c.tune.br_group > 0 ? std::min(c.tune.br_group, dev::kMaxGroup64) : dev::kMaxGroup64);
-    // digit tables when the gadget base allows and shared memory holds them
-    // beside a group of at least kMaxGroup64 per worker (else the group first)
-    const size_t tbytes = 40 * ((size_t)1 << c.p.BG_bits);
-    A.digit_tables = (1 << c.p.BG_bits) <= dev::kMaxTableBG64 &&
-                     W * sizeof(dev::Step64SmemT<true>) + 32 + tbytes + (size_t)cap * steps <= kPipeSmemBudget;
-    const size_t fixed = W * sizeof(dev::Step64SmemT<true>) + 32 + (A.digit_tables ? tbytes : 0);
+    const size_t fixed = W * sizeof(dev::Step64SmemT<true>) + 32;
     if (fixed + (size_t)cap * steps > kPipeSmemBudget)
         cap = fixed < kPipeSmemBudget ? (int)((kPipeSmemBudget - fixed) / steps) : 0;
     if (cap < 1) return c.fail(FHEACC_EINVAL, "n * digitR too large for the blind rotation's residue table");
     auto smem_of = [&](int group) {
-        return W * sizeof(dev::Step64SmemT<true>) + ((size_t)group * steps + 15) / 16 * 16 + (A.digit_tables ? tbytes : 0);
+        return W * sizeof(dev::Step64SmemT<true>) + ((size_t)group * steps + 15) / 16 * 16;
     };
     size_t smem = smem_of(cap);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -976,7 +951,7 @@ static int launch_br64_shape(Context &c, dev::Br64Args A, int max_ctas, cudaStre
     e = cudaMemsetAsync(A.claim_next, 0, kClaimWords * sizeof(uint32_t), st);
     if (e != cudaSuccess) return c.cuda_fail(e, "br64 claim reset");
     if (A.pool_count) {
-        dev::br64_pool_init_kernel<<<(unsigned)A.pool_count, dev::kT64, 0, st>>>(A, c.d_tw64, c.d_itw64, c.nc64);
+        dev::br64_pool_init_kernel<PM><<<(unsigned)A.pool_count, dev::kT64, 0, st>>>(A, c.d_tw64, c.d_itw64, c.nc64);
         c.launches++;
         e = cudaGetLastError();
         if (e != cudaSuccess) return c.cuda_fail(e, "br64 pool launch");
@@ -1032,23 +1007,27 @@ int launch_blind_rotate64_indexed(Context &c, const uint64_t *d_c1, const uint64
     A.status = c.d_status;
     A.wait_limit = c.tune.debug_wait_limit >= 0 ? (unsigned)c.tune.debug_wait_limit : dev::kWorkerWaitLimit;
     for (int i = 0; i < 8; i++) A.gate_constant[i] = c.dp.gate_constant[i];
-    // workers per CTA, by default from the gates per SM (one GB300): up to 1
-    // one worker per CTA (3 CTAs per SM), beyond that two, whose shared memory
-    // leaves room for the digit tables that three workers' does not (2048
-    // gates: 658 ms with two workers and tables, 698 ms with three; 700 gates:
-    // 240 ms either way; 304 gates: 98 / 109 / 146 ms with 2 / 1 / 3)
+    // workers per CTA, by default from the gates per SM: up to 1 one worker,
+    // beyond that two (128 registers a thread without spills; three workers' 80
+    // spill)
     const size_t sms = (size_t)sms_of(c);
     const int w = c.tune.br_pipes > 0 ? c.tune.br_pipes : count <= sms ? 1 : 2;
-    if (w == 3) return launch_br64_shape<3, 1>(c, A, max_ctas, st);
-    if (w == 2) return launch_br64_shape<2, 1>(c, A, max_ctas, st);
-    return launch_br64_shape<1, 3>(c, A, max_ctas, st);
+    if (c.nc64.pm_c) {
+        if (w == 3) return launch_br64_shape<true, 3, 1>(c, A, max_ctas, st);
+        if (w == 2) return launch_br64_shape<true, 2, 1>(c, A, max_ctas, st);
+        return launch_br64_shape<true, 1, 2>(c, A, max_ctas, st);
+    }
+    if (w == 3) return launch_br64_shape<false, 3, 1>(c, A, max_ctas, st);
+    if (w == 2) return launch_br64_shape<false, 2, 1>(c, A, max_ctas, st);
+    return launch_br64_shape<false, 1, 2>(c, A, max_ctas, st);
 }
 
 int launch_extract64(Context &c, const uint64_t *d_rlwe, size_t count, uint64_t *d_extract, cudaStream_t st)
 {
     if (!count) return FHEACC_OK;
     size_t blocks = std::min<size_t>(count, (size_t)sms_of(c) * 4);
-    dev::extract64_kernel<<<(unsigned)blocks, dev::kT64, 0, st>>>(d_rlwe, count, d_extract, c.d_itw64, c.nc64);
+    auto kern = c.nc64.pm_c ? dev::extract64_kernel<true> : dev::extract64_kernel<false>;
+    kern<<<(unsigned)blocks, dev::kT64, 0, st>>>(d_rlwe, count, d_extract, c.d_itw64, c.nc64);
     c.launches++;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "extract64 launch");

@@ -120,14 +120,16 @@ struct Context {
     uint2 *d_fwd_tw = nullptr, *d_inv_tw = nullptr;
     dev::Ntt32Consts nc{};
 
-    // 64-bit path: twiddles as (w, floor(w 2^64 / Q)) pairs in reference order
+    // 64-bit path: twiddles as constant pairs (mul64 in ntt64.cuh) in reference order
     ulonglong2 *d_tw64 = nullptr, *d_itw64 = nullptr;
     dev::Ntt64Consts nc64{};
-    ulonglong2 *d_btkey64 = nullptr;   // Shoup pairs, [(i*digitR + j)*Br + r][digitG][2][2][N]
-    ulonglong2 *d_cf64 = nullptr;      // factors of the last-digit identity, digitG Shoup pairs
-    ulonglong2 *d_subs64 = nullptr;    // Shoup pairs, [logN][digitKS_R][2][N]
-    uint64_t *d_rot = nullptr;         // [logN][N]: NTT(-X^(N - 2^j)), rotate_vector_gen(false)
-    uint64_t *d_rot_fwd = nullptr;     // [logN][N]: NTT(X^(2^j)), rotate_vector_gen(true)
+    ulonglong2 *d_btkey64 = nullptr;   // constant pairs, [(i*digitR + j)*Br + r][digitG][2][2][N]
+    ulonglong2 *d_cf64 = nullptr;      // factors of the last-digit identity, digitG constant pairs
+    ulonglong2 *d_subs64 = nullptr;    // constant pairs, [logN][digitKS_R][2][N]
+    // rotations, [logN][N]: NTT(-X^(N - 2^j)), rotate_vector_gen(false), and
+    // NTT(X^(2^j)), rotate_vector_gen(true); wide: constant pairs
+    uint64_t *d_rot = nullptr, *d_rot_fwd = nullptr;
+    ulonglong2 *d_rot64 = nullptr, *d_rot_fwd64 = nullptr;
     uint64_t *d_kskey64 = nullptr;     // [(d*digitKS + j)*N + i][ks_row]
 
     // keys, device layouts
@@ -212,8 +214,8 @@ int launch_extract_from_ntt32(Context &c, const uint64_t *d_rlwe, size_t count, 
                               cudaStream_t st);
 int launch_modswitch(Context &c, const uint64_t *d_in, size_t count, uint64_t *d_out, cudaStream_t st);
 // 64-bit path (bootstrap64.cu)
-int launch_shoup_pairs64(Context &c, const uint64_t *d_in, ulonglong2 *d_out, size_t n, cudaStream_t st);
-// The last-digit identity applied in place to count RGSWs (d_cf: digitG Shoup pairs).
+int launch_const_pairs64(Context &c, const uint64_t *d_in, ulonglong2 *d_out, size_t n, cudaStream_t st);
+// The last-digit identity applied in place to count RGSWs (d_cf: digitG constant pairs).
 int launch_derive_keys64(Context &c, uint64_t *d_keys, size_t count, const ulonglong2 *d_cf, cudaStream_t st);
 int launch_ntt64(Context &c, uint64_t *d_polys, size_t count, bool inverse, cudaStream_t st);
 int launch_rlwe_mult_rgsw64(Context &c, const uint64_t *d_acc, const uint64_t *d_rgsw, uint64_t *d_out,
@@ -253,7 +255,7 @@ int launch_blind_rotate64_indexed(Context &c, const uint64_t *d_c1, const uint64
 // 2 SUBS_KS, 3 EXPAND (one level f, in place on d_out, for `batches` r
 // arrays bstride words apart)
 int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, size_t count, int f,
-                  const void *ksk, const uint64_t *d_rot, cudaStream_t st, size_t batches = 1, size_t bstride = 0);
+                  const void *ksk, cudaStream_t st, size_t batches = 1, size_t bstride = 0);
 int launch_to_u32(Context &c, const uint64_t *d_in, uint32_t *d_out, size_t n, cudaStream_t st);
 // IMAD throughput probe (probe.cu)
 int measure_imad_rate(Context &c, double *imad_per_s);

@@ -38,14 +38,15 @@ struct ExpArgs {
     uint32_t bits;           // Bks_R_bits
     uint32_t ipow;           // (N / 2^f + 1)^-1 mod 2N
     const uint32_t *ksk32;   // [L][2][N] u32 (narrow)
-    const ulonglong2 *ksk64; // [L][2][N] Shoup pairs (wide)
-    const uint64_t *rot;     // [N] NTT(-X^(N - 2^f)) (EXPAND)
+    const ulonglong2 *ksk64; // [L][2][N] constant pairs (wide)
+    const uint64_t *rot;     // [N] NTT(-X^(N - 2^f)) (EXPAND, narrow)
+    const ulonglong2 *rot64; // the same as constant pairs (wide)
     uint64_t Q, mu64;
 };
 
 __device__ __forceinline__ uint32_t subs_src(uint32_t e, uint32_t ipow, uint32_t N, bool &neg)
 {
-    const uint32_t ip = (uint32_t)(((uint64_t)e * ipow) & (2 * N - 1));
+    const uint32_t ip = (e * ipow) & (2 * N - 1);   // 2 N a power of two: the low word is enough
     neg = ip >= N;
     return neg ? ip - N : ip;
 }
@@ -142,27 +143,43 @@ __global__ void __launch_bounds__(256) expand32_kernel(const __grid_constant__ E
 }
 
 // ------------------------------------------------------------------- wide
+// Word e = j + 128 k of the substituted polynomial (subs_src) for
+// ntt64_fwd_2048_load, or its digit (v >> sh) & mask (mask = 0: the word).
+struct LoadSubs64 {
+    const uint64_t *t;
+    uint64_t Q;
+    uint32_t ipow, sh, mask;
+    __device__ __forceinline__ uint64_t operator()(int j, int k) const
+    {
+        bool neg;
+        const uint32_t s = subs_src((uint32_t)(j + 128 * k), ipow, 2048, neg);
+        uint64_t v = t[px(s)];
+        if (neg && v) v = Q - v;
+        return mask ? (uint64_t)((uint32_t)(v >> sh) & mask) : v;
+    }
+};
+
 // 256 threads in two 128-thread groups; group g transforms poly g.
-__global__ void __launch_bounds__(256) expand64_kernel(const __grid_constant__ ExpArgs A,
+template <bool PM>
+__global__ void __launch_bounds__(256, 2) expand64_kernel(const __grid_constant__ ExpArgs A,
                                                       const ulonglong2 *__restrict__ tw,
                                                       const ulonglong2 *__restrict__ itw,
                                                       const __grid_constant__ Ntt64Consts c)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint64_t(*t)[2048] = reinterpret_cast<uint64_t(*)[2048]>(smem_raw);                 // [2][2048]
-    uint64_t(*buf)[2048] = reinterpret_cast<uint64_t(*)[2048]>(smem_raw + 2 * 2048 * 8);  // [2][2048]
+    uint64_t(*t)[kPoly64] = reinterpret_cast<uint64_t(*)[kPoly64]>(smem_raw);   // [2], layout px
+    uint64_t(*buf)[kPoly64] = t + 2;                                            // [2]
     const int tid = threadIdx.x, grp = tid >> 7, gtid = tid & 127;
     const uint64_t Q = c.Q;
     const int L = A.L;
-    const bool subs = A.mode != kKs;
     const size_t per = A.mode == kExpand ? ((size_t)1 << A.f) : A.count;
     const size_t items = per * A.batches;
     for (size_t it = blockIdx.x; it < items; it += gridDim.x) {
         const size_t bo = it / per * A.bstride, jt = it % per;   // batch offset, item within the batch
         const uint64_t *in = A.in + bo + jt * 4096;
-        for (int e = gtid; e < 2048; e += 128) t[grp][e] = in[grp * 2048 + e];
+        for (int e = gtid; e < 2048; e += 128) t[grp][px(e)] = in[grp * 2048 + e];
         group_sync(1 + grp, 128);
-        ntt64_inv_2048<128, false>(t[grp], itw, c, gtid, 1 + grp);
+        ntt64_inv_2048<PM, 128, true>(t[grp], itw, c, gtid, 1 + grp);
         __syncthreads();
         // transforms: L digits of sigma(a) and sigma(b) (SUBS: sigma(a), sigma(b)),
         // two at a time; MAC after each pair
@@ -174,23 +191,15 @@ __global__ void __launch_bounds__(256) expand64_kernel(const __grid_constant__ E
             const int tr = base + grp;   // transform index of this group
             if (tr < nt) {
                 const int poly = A.mode == kSubs ? tr : (tr == L ? 1 : 0);
-                const bool digit = A.mode != kSubs && tr < L;
-                const uint32_t sh = A.bits * (uint32_t)tr;
-                const uint64_t mask = (1ULL << A.bits) - 1;
-                for (int e = gtid; e < 2048; e += 128) {
-                    uint64_t v;
-                    if (subs) {
-                        bool neg;
-                        const uint32_t s = subs_src((uint32_t)e, A.ipow, 2048, neg);
-                        v = t[poly][s];
-                        if (neg && v) v = Q - v;
-                    } else {
-                        v = t[poly][e];
-                    }
-                    buf[grp][e] = digit ? (v >> sh) & mask : v;
+                // A.ipow = 1 is the identity (kKs)
+                if (A.mode != kSubs && tr < L) {
+                    ntt64_fwd_2048_load<PM, 128, true, true>(
+                        buf[grp], LoadSubs64{t[poly], Q, A.ipow, A.bits * (uint32_t)tr, (1u << A.bits) - 1}, tw, c, gtid,
+                        1 + grp);
+                } else {
+                    ntt64_fwd_2048_load<PM, 128, true, false>(buf[grp], LoadSubs64{t[poly], Q, A.ipow, 0, 0}, tw, c,
+                                                               gtid, 1 + grp);
                 }
-                group_sync(1 + grp, 128);
-                ntt64_fwd_2048<128, false>(buf[grp], tw, c, gtid, 1 + grp);
             }
             __syncthreads();
 #pragma unroll
@@ -200,16 +209,16 @@ __global__ void __launch_bounds__(256) expand64_kernel(const __grid_constant__ E
                 for (int g2 = 0; g2 < 2; g2++) {
                     const int tr = base + g2;
                     if (tr >= nt) continue;
-                    const uint64_t dv = buf[g2][k];
+                    const uint64_t dv = buf[g2][px(k)];
                     if (A.mode == kSubs || tr == L) {
-                        const uint64_t v = barrett64_2q(dv, c.mu64, Q);
+                        const uint64_t v = reduce64<PM>(dv, c);
                         if (A.mode == kSubs && tr == 0) sa[i] = v;
                         else fb[i] = v;
                     } else {
                         const ulonglong2 ka = __ldg(A.ksk64 + (size_t)(tr * 2 + 0) * 2048 + k);
                         const ulonglong2 kb = __ldg(A.ksk64 + (size_t)(tr * 2 + 1) * 2048 + k);
-                        sa[i] += shoup64(dv, ka.x, ka.y, Q);
-                        sb[i] += shoup64(dv, kb.x, kb.y, Q);
+                        sa[i] += mul64<PM>(dv, ka, c);
+                        sb[i] += mul64<PM>(dv, kb, c);
                     }
                 }
             }
@@ -224,7 +233,7 @@ __global__ void __launch_bounds__(256) expand64_kernel(const __grid_constant__ E
                 oa = sa[i] >= Q ? sa[i] - Q : sa[i];
                 ob = fb[i] >= Q ? fb[i] - Q : fb[i];
             } else {
-                uint64_t ra = barrett64_2q(sa[i], c.mu64, Q), rb = barrett64_2q(sb[i], c.mu64, Q);
+                uint64_t ra = reduce64<PM>(sa[i], c), rb = reduce64<PM>(sb[i], c);
                 ra = ra >= Q ? ra - Q : ra;
                 rb = rb >= Q ? rb - Q : rb;
                 const uint64_t nb = fb[i] >= Q ? fb[i] - Q : fb[i];
@@ -233,14 +242,15 @@ __global__ void __launch_bounds__(256) expand64_kernel(const __grid_constant__ E
             }
             if (A.mode == kExpand) {
                 const uint64_t ta = in[k], tb = in[2048 + k];
-                const uint64_t rot = A.rot[k];
+                const ulonglong2 rot = __ldg(A.rot64 + k);
                 uint64_t *hi = A.out + bo + (jt + per) * 4096;
                 const uint64_t s1 = ta + oa, s2 = tb + ob;
                 out[k] = s1 >= Q ? s1 - Q : s1;
                 out[2048 + k] = s2 >= Q ? s2 - Q : s2;
                 const uint64_t d1 = ta >= oa ? ta - oa : ta + Q - oa, d2 = tb >= ob ? tb - ob : tb + Q - ob;
-                hi[k] = (uint64_t)((unsigned __int128)d1 * rot % Q);
-                hi[2048 + k] = (uint64_t)((unsigned __int128)d2 * rot % Q);
+                const uint64_t h1 = mul64<PM>(d1, rot, c), h2 = mul64<PM>(d2, rot, c);
+                hi[k] = h1 >= Q ? h1 - Q : h1;
+                hi[2048 + k] = h2 >= Q ? h2 - Q : h2;
             } else {
                 out[k] = oa;
                 out[2048 + k] = ob;
@@ -257,6 +267,7 @@ __global__ void __launch_bounds__(256) expand64_kernel(const __grid_constant__ E
 // part[item][p] as [sa | sb | fb][2048], each word < 4Q. expand64_combine_kernel
 // adds the shares and applies the level's epilogue. One RLWE's transforms then
 // take two rounds instead of 1 + ceil((L + 1) / 2).
+template <bool PM>
 __global__ void __launch_bounds__(256) expand64_split_kernel(const __grid_constant__ ExpArgs A,
                                                             uint64_t *__restrict__ part, int P,
                                                             const ulonglong2 *__restrict__ tw,
@@ -264,8 +275,8 @@ __global__ void __launch_bounds__(256) expand64_split_kernel(const __grid_consta
                                                             const __grid_constant__ Ntt64Consts c)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint64_t(*t)[2048] = reinterpret_cast<uint64_t(*)[2048]>(smem_raw);                 // [2][2048]
-    uint64_t(*buf)[2048] = reinterpret_cast<uint64_t(*)[2048]>(smem_raw + 2 * 2048 * 8);  // [2][2048]
+    uint64_t(*t)[kPoly64] = reinterpret_cast<uint64_t(*)[kPoly64]>(smem_raw);   // [2], layout px
+    uint64_t(*buf)[kPoly64] = t + 2;                                            // [2]
     const int tid = threadIdx.x, grp = tid >> 7, gtid = tid & 127;
     const uint64_t Q = c.Q;
     const int L = A.L, nt = L + 1;
@@ -274,25 +285,18 @@ __global__ void __launch_bounds__(256) expand64_split_kernel(const __grid_consta
     const int p = (int)(blockIdx.x - it * (unsigned)P);
     const size_t bo = it / per * A.bstride, jt = it % per;
     const uint64_t *in = A.in + bo + jt * 4096;
-    for (int e = gtid; e < 2048; e += 128) t[grp][e] = in[grp * 2048 + e];
+    for (int e = gtid; e < 2048; e += 128) t[grp][px(e)] = in[grp * 2048 + e];
     group_sync(1 + grp, 128);
-    ntt64_inv_2048<128, false>(t[grp], itw, c, gtid, 1 + grp);
+    ntt64_inv_2048<PM, 128, true>(t[grp], itw, c, gtid, 1 + grp);
     __syncthreads();
     const int tr = 2 * p + grp;
     if (tr < nt) {
-        const int poly = tr == L ? 1 : 0;
-        const bool digit = tr < L;
-        const uint32_t sh = A.bits * (uint32_t)tr;
-        const uint64_t mask = (1ULL << A.bits) - 1;
-        for (int e = gtid; e < 2048; e += 128) {
-            bool neg;
-            const uint32_t s = subs_src((uint32_t)e, A.ipow, 2048, neg);
-            uint64_t v = t[poly][s];
-            if (neg && v) v = Q - v;
-            buf[grp][e] = digit ? (v >> sh) & mask : v;
-        }
-        group_sync(1 + grp, 128);
-        ntt64_fwd_2048<128, false>(buf[grp], tw, c, gtid, 1 + grp);
+        if (tr < L)
+            ntt64_fwd_2048_load<PM, 128, true, true>(
+                buf[grp], LoadSubs64{t[0], Q, A.ipow, A.bits * (uint32_t)tr, (1u << A.bits) - 1}, tw, c, gtid, 1 + grp);
+        else
+            ntt64_fwd_2048_load<PM, 128, true, false>(buf[grp], LoadSubs64{t[1], Q, A.ipow, 0, 0}, tw, c, gtid,
+                                                       1 + grp);
     }
     __syncthreads();
     uint64_t *o = part + (it * (unsigned)P + (unsigned)p) * 3 * 2048;
@@ -304,14 +308,14 @@ __global__ void __launch_bounds__(256) expand64_split_kernel(const __grid_consta
         for (int g2 = 0; g2 < 2; g2++) {
             const int tq = 2 * p + g2;
             if (tq >= nt) continue;
-            const uint64_t dv = buf[g2][k];
+            const uint64_t dv = buf[g2][px(k)];
             if (tq == L) {
-                fb = barrett64_2q(dv, c.mu64, Q);
+                fb = reduce64<PM>(dv, c);
             } else {
                 const ulonglong2 ka = __ldg(A.ksk64 + (size_t)(tq * 2 + 0) * 2048 + k);
                 const ulonglong2 kb = __ldg(A.ksk64 + (size_t)(tq * 2 + 1) * 2048 + k);
-                sa += shoup64(dv, ka.x, ka.y, Q);
-                sb += shoup64(dv, kb.x, kb.y, Q);
+                sa += mul64<PM>(dv, ka, c);
+                sb += mul64<PM>(dv, kb, c);
             }
         }
         o[k] = sa;
@@ -323,6 +327,7 @@ __global__ void __launch_bounds__(256) expand64_split_kernel(const __grid_consta
 // The shares of expand64_split_kernel added (P of them, < 4PQ < 2^64, checked
 // by the launcher) and the expand level's epilogue, one thread per item word:
 // s = (-sa, sigma(b) - sb), r[j] <- r[j] + s, r[j + 2^f] <- (r[j] - s) * rot.
+template <bool PM>
 __global__ void expand64_combine_kernel(const __grid_constant__ ExpArgs A, const uint64_t *__restrict__ part, int P,
                                         size_t items, const __grid_constant__ Ntt64Consts c)
 {
@@ -340,7 +345,7 @@ __global__ void expand64_combine_kernel(const __grid_constant__ ExpArgs A, const
             sb += pp[(size_t)(p * 3 + 1) * 2048];
             fb += pp[(size_t)(p * 3 + 2) * 2048];
         }
-        uint64_t ra = barrett64_2q(sa, c.mu64, Q), rb = barrett64_2q(sb, c.mu64, Q);
+        uint64_t ra = reduce64<PM>(sa, c), rb = reduce64<PM>(sb, c);
         ra = ra >= Q ? ra - Q : ra;
         rb = rb >= Q ? rb - Q : rb;
         const uint64_t nb = fb >= Q ? fb - Q : fb;
@@ -350,13 +355,14 @@ __global__ void expand64_combine_kernel(const __grid_constant__ ExpArgs A, const
         uint64_t *out = A.out + bo + jt * 4096;
         uint64_t *hi = A.out + bo + (jt + per) * 4096;
         const uint64_t ta = in[k], tb = in[2048 + k];
-        const uint64_t rot = A.rot[k];
+        const ulonglong2 rot = __ldg(A.rot64 + k);
         const uint64_t s1 = ta + oa, s2 = tb + ob;
         out[k] = s1 >= Q ? s1 - Q : s1;
         out[2048 + k] = s2 >= Q ? s2 - Q : s2;
         const uint64_t d1 = ta >= oa ? ta - oa : ta + Q - oa, d2 = tb >= ob ? tb - ob : tb + Q - ob;
-        hi[k] = (uint64_t)((unsigned __int128)d1 * rot % Q);
-        hi[2048 + k] = (uint64_t)((unsigned __int128)d2 * rot % Q);
+        const uint64_t h1 = mul64<PM>(d1, rot, c), h2 = mul64<PM>(d2, rot, c);
+        hi[k] = h1 >= Q ? h1 - Q : h1;
+        hi[2048 + k] = h2 >= Q ? h2 - Q : h2;
     }
 }
 
@@ -383,9 +389,9 @@ static uint32_t inv_power(int N, int f)
     return 1;
 }
 
-// ksk: narrow, u32 [L][2][N] device words; wide, Shoup pairs.
+// ksk: narrow, u32 [L][2][N] device words; wide, constant pairs (mul64).
 int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, size_t count, int f,
-                  const void *ksk, const uint64_t *d_rot, cudaStream_t st, size_t batches, size_t bstride)
+                  const void *ksk, cudaStream_t st, size_t batches, size_t bstride)
 {
     const int logN = c.wide ? 11 : 10;
     if (f < 0 || f >= logN) return c.fail(FHEACC_EINVAL, "substitution factor out of range");
@@ -394,8 +400,12 @@ int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, s
     A.batches = mode == dev::kExpand ? batches : 1;
     A.bstride = bstride;
     A.L = (int)c.p.digitKS_R; A.bits = c.p.Bks_R_bits; A.ipow = inv_power(c.p.N, mode == dev::kKs ? 0 : f);
-    A.rot = d_rot; A.Q = c.p.Q; A.mu64 = c.dp.mu64;
+    A.Q = c.p.Q; A.mu64 = c.dp.mu64;
     if (mode == dev::kKs) A.ipow = 1;
+    if (mode == dev::kExpand) {
+        if (c.wide) A.rot64 = c.d_rot64 + (size_t)f * c.p.N;
+        else A.rot = c.d_rot + (size_t)f * c.p.N;
+    }
     const size_t items = (mode == dev::kExpand ? ((size_t)1 << f) : count) * A.batches;
     if (!items) return FHEACC_OK;
     size_t blocks = std::min<size_t>(items, (size_t)sms(c) * 4);
@@ -403,7 +413,7 @@ int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, s
     if (c.wide) {
         if (A.L > 8) return c.fail(FHEACC_EINVAL, "digitKS_R too large");
         A.ksk64 = (const ulonglong2 *)ksk;
-        const size_t smem = 4 * 2048 * sizeof(uint64_t);
+        const size_t smem = 4 * dev::kPoly64 * sizeof(uint64_t);
         // an expand level of at most two CTAs per SM of (item, transform pair)
         // splits each item over its transform pairs, for latency
         const int P = (A.L + 2) / 2;
@@ -412,20 +422,22 @@ int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, s
             int rc = ensure_scratch(c, c.expand, words * sizeof(uint64_t));
             if (rc) return rc;
             uint64_t *part = (uint64_t *)c.expand.ptr;
-            cudaFuncSetAttribute(dev::expand64_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            dev::expand64_split_kernel<<<(unsigned)(items * P), 256, smem, st>>>(A, part, P, c.d_tw64, c.d_itw64,
-                                                                                 c.nc64);
+            auto split = c.nc64.pm_c ? dev::expand64_split_kernel<true> : dev::expand64_split_kernel<false>;
+            cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            split<<<(unsigned)(items * P), 256, smem, st>>>(A, part, P, c.d_tw64, c.d_itw64, c.nc64);
             c.launches++;
             e = cudaGetLastError();
             if (e != cudaSuccess) return c.cuda_fail(e, "expand split launch");
             const unsigned cb = (unsigned)std::min<size_t>((items * 2048 + 255) / 256, (size_t)sms(c) * 4);
-            dev::expand64_combine_kernel<<<cb, 256, 0, st>>>(A, part, P, items, c.nc64);
+            auto combine = c.nc64.pm_c ? dev::expand64_combine_kernel<true> : dev::expand64_combine_kernel<false>;
+            combine<<<cb, 256, 0, st>>>(A, part, P, items, c.nc64);
             c.launches++;
             e = cudaGetLastError();
             return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "expand combine launch");
         }
-        cudaFuncSetAttribute(dev::expand64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        dev::expand64_kernel<<<(unsigned)blocks, 256, smem, st>>>(A, c.d_tw64, c.d_itw64, c.nc64);
+        auto kern = c.nc64.pm_c ? dev::expand64_kernel<true> : dev::expand64_kernel<false>;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kern<<<(unsigned)blocks, 256, smem, st>>>(A, c.d_tw64, c.d_itw64, c.nc64);
         c.launches++;
     } else {
         if (A.L > 4) return c.fail(FHEACC_EINVAL, "digitKS_R too large for the 32-bit path");

@@ -12,7 +12,19 @@
 // group barrier per pass.
 // Forward butterflies leave the upper input unreduced
 // (bound grows by 2Q a stage: inputs < Q end below 23Q < 2^59 for Q < 2^54);
-// the inverse keeps Harvey's [0, 2Q) invariant and ends canonical.
+// the inverse ends canonical.
+//
+// The transforms are bound by the 32-bit multiply pipe, so the modular
+// multiplication decides their time. Two forms, chosen by the modulus
+// (template parameter PM):
+//   PM = true: Q = 2^b - c with 48 <= b <= 54 and c <= 2^(b-36), which every Q
+//     picked as the largest prime below a power of two satisfies (pm64_shift).
+//     A constant w is kept as (w, w 2^30 mod Q); x = x1 2^30 + x0 gives
+//     x w = x0 w + x1 (w 2^30) below 2^(b+32), and the bits above 2^b fold
+//     back times c: five 32 x 32 -> 64 multiplies (20 issue slots of the
+//     multiply pipe's 16 lanes) where Shoup's form takes 33. A register-only
+//     butterfly loop: 34 cycles per warp against 42 with Shoup's.
+//   PM = false: Shoup's multiplication, any Q < 2^58.
 #pragma once
 #include <cstdint>
 
@@ -21,51 +33,119 @@ namespace dev {
 
 // Shared-memory layouts of a 2048-word polynomial, chosen by the template
 // parameter P of the transforms: P = false, word e at e; P = true, one padding
-// word after every 8, word e at px(e). Padded, the passes whose threads walk 8
-// consecutive words (the last forward and the first inverse pass) spread a
-// warp over all banks instead of two bank pairs; the offsets of a pass's tuple
-// stay linear in the tuple index (strides 1 within an octet, or multiples of
-// 8). The padding costs shared memory, hence L1, which only some kernels spare.
-constexpr int kPoly64 = 2048 + 256;
-__host__ __device__ __forceinline__ int px(int e) { return e + (e >> 3); }
+// word after every 16, word e at px(e). A 64-bit shared access takes a half
+// warp at a time: padded, its 16 words fall on 16 different bank pairs in
+// every pass (consecutive words; 8 consecutive words of two tuples 136 words
+// apart; the first words of 16 octets), and a tuple's offsets stay
+// compile-time constants.
+constexpr int kPoly64 = 2048 + 128;
+__host__ __device__ __forceinline__ constexpr int px(int e) { return e + (e >> 4); }
 template <bool P>
-__host__ __device__ __forceinline__ int pi(int e) { return P ? px(e) : e; }
+__host__ __device__ __forceinline__ constexpr int pi(int e) { return P ? px(e) : e; }
 template <bool P>
 __host__ __device__ constexpr int poly_words64() { return P ? kPoly64 : 2048; }
 
 struct Ntt64Consts {
     uint64_t Q, twoQ;
-    uint64_t iN, iNs;       // N^-1 and its Shoup companion
+    uint64_t iN, iNs;       // N^-1 as a constant pair (w, companion)
     uint64_t iw1N, iw1Ns;   // irou[1] * N^-1
     uint64_t mu64;          // floor(2^64 / Q)
+    uint64_t p30, p30s;     // PM: 2^30 mod Q as a constant pair
+    // PM: twiddles of a digit's first two stages times 2^pm_s (digit_radix4):
+    // w1, w2, w3, w2 w1, -w3 w1 mod Q
+    uint64_t dw1, dw2, dw3, dw21, dw31;
+    uint32_t pm_c;          // 2^b - Q where the PM form applies (else 0)
+    uint32_t pm_s;          // 64 - b
 };
 
-__device__ __forceinline__ uint64_t shoup64(uint64_t x, uint64_t w, uint64_t ws, uint64_t Q)
+// 64 - b if Q = 2^b - c with 48 <= b <= 54 and c <= 2^(b-36), else 0. The
+// bounds make every product of mul64<true> less than (1 + 2^-4) 2^b < 2Q, and
+// b <= 54 leaves the forward transform's 23Q below the 2^59 of mul64_2<true>.
+inline int pm64_shift(uint64_t Q)
 {
-    const uint64_t t = __umul64hi(x, ws);
-    return x * w - t * Q;   // in [0, 2Q)
+    for (int b = 48; b <= 54; b++) {
+        const uint64_t p = (uint64_t)1 << b;
+        if (Q < p && Q > p / 2) return p - Q <= (uint64_t)1 << (b - 36) ? 64 - b : 0;
+    }
+    return 0;
 }
 
-__device__ __forceinline__ void ct64(uint64_t &x, uint64_t &y, ulonglong2 w, uint64_t Q, uint64_t twoQ)
+__device__ __forceinline__ uint64_t mul_wide64(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+
+// x w mod Q for a constant pair w, in [0, 2Q).
+// PM: w = (w << s, (w 2^30 mod Q) << s), s = 64 - b; x < 2^61. With U and V the
+// sums of the low and high word products, 2^s x w = U + 2^32 V; the word above
+// 2^64 is the part of x w above 2^b. Bounds: x0 < 2^30 and x1 < 2^31 keep both
+// sums below 2^62 + 2^63 + 2^32.
+// Shoup: w = (w, floor(w 2^64 / Q)), any x.
+template <bool PM>
+__device__ __forceinline__ uint64_t mul64(uint64_t x, ulonglong2 w, const Ntt64Consts &c)
 {
-    const uint64_t t = shoup64(y, w.x, w.y, Q);
-    y = x + twoQ - t;
+    if (PM) {
+        const uint32_t x0 = (uint32_t)x & 0x3fffffffu, x1 = (uint32_t)(x >> 30);
+        const uint64_t U = mul_wide64(x0, (uint32_t)w.x) + mul_wide64(x1, (uint32_t)w.y);
+        const uint64_t V = mul_wide64(x0, (uint32_t)(w.x >> 32)) + mul_wide64(x1, (uint32_t)(w.y >> 32)) + (U >> 32);
+        const uint64_t low = (V << 32) | (uint32_t)U;
+        return mul_wide64((uint32_t)(V >> 32), c.pm_c) + (low >> c.pm_s);
+    }
+    const uint64_t t = __umul64hi(x, w.y);
+    return x * w.x - t * c.Q;
+}
+
+// x v + y w mod Q for constant pairs v, w: below 2Q (PM: one fold for both
+// products, x and y < 2^59, sums below 2 (2^62 + 2^61) + 2^32) or 4Q (Shoup).
+template <bool PM>
+__device__ __forceinline__ uint64_t mul64_2(uint64_t x, ulonglong2 v, uint64_t y, ulonglong2 w, const Ntt64Consts &c)
+{
+    if (PM) {
+        const uint32_t x0 = (uint32_t)x & 0x3fffffffu, x1 = (uint32_t)(x >> 30);
+        const uint32_t y0 = (uint32_t)y & 0x3fffffffu, y1 = (uint32_t)(y >> 30);
+        const uint64_t U = mul_wide64(x0, (uint32_t)v.x) + mul_wide64(x1, (uint32_t)v.y) +
+                           mul_wide64(y0, (uint32_t)w.x) + mul_wide64(y1, (uint32_t)w.y);
+        const uint64_t V = mul_wide64(x0, (uint32_t)(v.x >> 32)) + mul_wide64(x1, (uint32_t)(v.y >> 32)) +
+                           mul_wide64(y0, (uint32_t)(w.x >> 32)) + mul_wide64(y1, (uint32_t)(w.y >> 32)) + (U >> 32);
+        const uint64_t low = (V << 32) | (uint32_t)U;
+        return mul_wide64((uint32_t)(V >> 32), c.pm_c) + (low >> c.pm_s);
+    }
+    return mul64<PM>(x, v, c) + mul64<PM>(y, w, c);
+}
+
+// Any 64-bit x to [0, 2Q). PM: x = x1 2^b + x0 folds to x0 + c x1 < 2^b + 2^34.
+template <bool PM>
+__device__ __forceinline__ uint64_t reduce64(uint64_t x, const Ntt64Consts &c)
+{
+    if (PM) {
+        const uint32_t b = 64 - c.pm_s;
+        return (x & (~0ull >> c.pm_s)) + mul_wide64((uint32_t)(x >> b), c.pm_c);
+    }
+    return x - __umul64hi(x, c.mu64) * c.Q;
+}
+
+template <bool PM>
+__device__ __forceinline__ uint64_t canonical64(uint64_t x, const Ntt64Consts &c)
+{
+    const uint64_t v = reduce64<PM>(x, c);
+    return v >= c.Q ? v - c.Q : v;
+}
+
+template <bool PM>
+__device__ __forceinline__ void ct64(uint64_t &x, uint64_t &y, ulonglong2 w, const Ntt64Consts &c)
+{
+    const uint64_t t = mul64<PM>(y, w, c);
+    y = x + c.twoQ - t;
     x = x + t;
 }
 
-__device__ __forceinline__ void gs64(uint64_t &x, uint64_t &y, ulonglong2 w, uint64_t Q, uint64_t twoQ)
+// Gentleman-Sande butterfly of inputs below 2^K Q. Shoup: K = 1, the sum is
+// brought back below 2Q. PM: the sum is left at 2^(K+1) Q.
+template <bool PM, int K>
+__device__ __forceinline__ void gs64(uint64_t &x, uint64_t &y, ulonglong2 w, const Ntt64Consts &c)
 {
     uint64_t u = x + y;
-    u = u >= twoQ ? u - twoQ : u;
-    const uint64_t v = shoup64(x - y + twoQ, w.x, w.y, Q);
+    if (!PM) u = u >= c.twoQ ? u - c.twoQ : u;
+    const uint64_t v = mul64<PM>(x - y + (PM ? c.Q << K : c.twoQ), w, c);
     x = u;
     y = v;
-}
-
-// x < 2^64 -> [0, 2Q)
-__device__ __forceinline__ uint64_t barrett64_2q(uint64_t x, uint64_t mu64, uint64_t Q)
-{
-    return x - __umul64hi(x, mu64) * Q;
 }
 
 __device__ __forceinline__ void group_sync(int bar_id, int threads)
@@ -75,7 +155,7 @@ __device__ __forceinline__ void group_sync(int bar_id, int threads)
 
 // One radix-2^R forward pass: stages t, t/2, ..., t/2^(R-1) (m = N / 2t) on
 // the tuples e0 + k t/2^(R-1) (k < 2^R) of every 2t-block.
-template <int G, int R, bool P>
+template <bool PM, int G, int R, bool P>
 __device__ __forceinline__ void fwd_passR(uint64_t *a, const ulonglong2 *__restrict__ tw, const Ntt64Consts &c,
                                           int tid, int t, int m)
 {
@@ -83,21 +163,22 @@ __device__ __forceinline__ void fwd_passR(uint64_t *a, const ulonglong2 *__restr
     const int h = t >> (R - 1);
     for (int oc = tid; oc < 2048 / K; oc += G) {
         const int grp = oc / h, j = oc - grp * h;
-        const int e0 = grp * 2 * t + j;
+        // e0 + k h in the layout: base + pi(k h), as j < h and h divides 16 or 16 divides h
+        uint64_t *const b = a + pi<P>(grp * 2 * t + j);
         uint64_t x[K];
 #pragma unroll
-        for (int k = 0; k < K; k++) x[k] = a[pi<P>(e0 + k * h)];
+        for (int k = 0; k < K; k++) x[k] = b[pi<P>(k * h)];
 #pragma unroll
         for (int st = 0; st < R; st++) {
             const int d = K >> (st + 1);
 #pragma unroll
             for (int k = 0; k < K; k++) {
                 if (k & d) continue;
-                ct64(x[k], x[k + d], __ldg(tw + (m << st) + (grp << st) + (k >> (R - st))), c.Q, c.twoQ);
+                ct64<PM>(x[k], x[k + d], __ldg(tw + (m << st) + (grp << st) + (k >> (R - st))), c);
             }
         }
 #pragma unroll
-        for (int k = 0; k < K; k++) a[pi<P>(e0 + k * h)] = x[k];
+        for (int k = 0; k < K; k++) b[pi<P>(k * h)] = x[k];
     }
 }
 
@@ -105,106 +186,149 @@ __device__ __forceinline__ void fwd_passR(uint64_t *a, const ulonglong2 *__restr
 // the named barrier `bar`. tw[k] = (psi^bitrev(k), companion). Input < Q,
 // output < 23Q, bit-reversed order as the reference's. Two radix-16 passes
 // (stages t = 1024..128, 64..8) and one radix-8 pass (t = 4, 2, 1).
-template <int G, bool P>
+template <bool PM, int G, bool P>
 __device__ __forceinline__ void ntt64_fwd_2048(uint64_t *a, const ulonglong2 *__restrict__ tw, const Ntt64Consts &c,
                                                int tid, int bar)
 {
-    fwd_passR<G, 4, P>(a, tw, c, tid, 1024, 1);   // t = 1024 .. 128
+    fwd_passR<PM, G, 4, P>(a, tw, c, tid, 1024, 1);   // t = 1024 .. 128
     group_sync(bar, G);
-    fwd_passR<G, 4, P>(a, tw, c, tid, 64, 16);    // t = 64 .. 8
+    fwd_passR<PM, G, 4, P>(a, tw, c, tid, 64, 16);    // t = 64 .. 8
     group_sync(bar, G);
-    fwd_passR<G, 3, P>(a, tw, c, tid, 4, 256);    // t = 4, 2, 1
+    fwd_passR<PM, G, 3, P>(a, tw, c, tid, 4, 256);    // t = 4, 2, 1
     group_sync(bar, G);
 }
 
-// Products of a gadget digit (y < BG) with the three twiddles of the first two
-// forward stages, w1 = psi^bitrev(1) (stage t = 1024), w2 and w3 (t = 512):
-// t1[y] = y w1, t23[y] = (y w2, y w3), t123[y] = (y w2 w1, y w3 w1), mod Q.
-struct DigitTables64 {
-    const uint64_t *t1;
-    const ulonglong2 *t23, *t123;
-};
+// Stages t = 1024 and 512 of four digits (x0, x1, x2, x3) = words e, e + 512,
+// e + 1024, e + 1536 below 2^30, with w1 = psi^bitrev(1) (t = 1024), w2 and w3
+// (t = 512):
+//   x0 + w1 x2 + (w2 x1 + w2 w1 x3)     x0 + w1 x2 - (w2 x1 + w2 w1 x3)
+//   x0 - w1 x2 + (w3 x1 - w3 w1 x3)     x0 - w1 x2 - (w3 x1 - w3 w1 x3)
+// each below 4Q + BG. PM: a product with a digit takes two 32 x 32 -> 64
+// multiplies, so the four outputs take 10 and three folds where butterflies take
+// 20 and four. (Tables of the products in shared memory cost more: their
+// gathers at random digits conflict, and the shared-memory pipe was the busiest
+// unit of the blind rotation.)
+template <bool PM>
+__device__ __forceinline__ void digit_radix4(uint64_t &x0, uint64_t &x1, uint64_t &x2, uint64_t &x3,
+                                             const ulonglong2 *__restrict__ tw, const Ntt64Consts &c)
+{
+    if (PM) {
+        auto fold = [&](uint64_t U, uint64_t V) {
+            V += U >> 32;
+            return mul_wide64((uint32_t)(V >> 32), c.pm_c) + (((V << 32) | (uint32_t)U) >> c.pm_s);
+        };
+        auto lo = [](uint64_t w) { return (uint32_t)w; };
+        auto hi = [](uint64_t w) { return (uint32_t)(w >> 32); };
+        const uint32_t d1 = (uint32_t)x1, d2 = (uint32_t)x2, d3 = (uint32_t)x3;
+        const uint64_t A = fold(mul_wide64(d2, lo(c.dw1)), mul_wide64(d2, hi(c.dw1)));
+        const uint64_t B = fold(mul_wide64(d1, lo(c.dw2)) + mul_wide64(d3, lo(c.dw21)),
+                                mul_wide64(d1, hi(c.dw2)) + mul_wide64(d3, hi(c.dw21)));
+        const uint64_t D = fold(mul_wide64(d1, lo(c.dw3)) + mul_wide64(d3, lo(c.dw31)),
+                                mul_wide64(d1, hi(c.dw3)) + mul_wide64(d3, hi(c.dw31)));
+        const uint64_t u = x0 + A, v = x0 + c.twoQ - A;
+        x0 = u + B;
+        x1 = u + c.twoQ - B;
+        x2 = v + D;
+        x3 = v + c.twoQ - D;
+        return;
+    }
+    const ulonglong2 w1 = __ldg(tw + 1);
+    ct64<PM>(x0, x2, w1, c);
+    ct64<PM>(x1, x3, w1, c);
+    ct64<PM>(x0, x1, __ldg(tw + 2), c);
+    ct64<PM>(x2, x3, __ldg(tw + 3), c);
+}
 
-// First forward pass (stages t = 1024 .. 128) of a digit polynomial (values
-// < BG): the first two stages of each radix-4 group (x0, x1, x2, x3) =
-// x[r, r+4, r+8, r+12] of a 16-tuple come from the tables,
-//   x[r]      = x0 + w1 x2 + w2 x1 + w2 w1 x3
-//   x[r + 4]  = x0 + w1 x2 - w2 x1 - w2 w1 x3
-//   x[r + 8]  = x0 - w1 x2 + w3 x1 - w3 w1 x3
-//   x[r + 12] = x0 - w1 x2 - w3 x1 + w3 w1 x3
-// (each below 3Q + BG), the other two stages are Cooley-Tukey butterflies.
-template <int G, bool P>
-__device__ __forceinline__ void fwd_pass16_digit(uint64_t *a, const ulonglong2 *__restrict__ tw, const Ntt64Consts &c,
-                                                 int tid, const DigitTables64 &T)
+// First forward pass (stages t = 1024 .. 128) of the polynomial whose word e is
+// load(j, k), e = j + 128 k, into a (layout pi<P>): no pass of its own to write
+// the words first. DIGIT: words below 2^30 (digit_radix4).
+template <bool PM, int G, bool P, bool DIGIT, class Load>
+__device__ __forceinline__ void fwd_pass16_load(uint64_t *a, Load load, const ulonglong2 *__restrict__ tw,
+                                                const Ntt64Consts &c, int tid)
 {
     for (int j = tid; j < 128; j += G) {
         uint64_t x[16];
 #pragma unroll
-        for (int k = 0; k < 16; k++) x[k] = a[pi<P>(j + k * 128)];
+        for (int k = 0; k < 16; k++) x[k] = load(j, k);
+        if (DIGIT) {
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const uint64_t x0 = x[r];
-            const uint64_t av = T.t1[x[r + 8]];
-            const ulonglong2 bd = T.t23[x[r + 4]], ce = T.t123[x[r + 12]];
-            x[r] = x0 + av + bd.x + ce.x;
-            x[r + 4] = x0 + av + (c.twoQ - bd.x - ce.x);
-            x[r + 8] = x0 + (c.twoQ - av - ce.y) + bd.y;
-            x[r + 12] = x0 + (c.twoQ - av - bd.y) + ce.y;
+            for (int r = 0; r < 4; r++) digit_radix4<PM>(x[r], x[r + 4], x[r + 8], x[r + 12], tw, c);
         }
 #pragma unroll
-        for (int st = 2; st < 4; st++) {
+        for (int st = DIGIT ? 2 : 0; st < 4; st++) {
             const int d = 16 >> (st + 1);
 #pragma unroll
             for (int k = 0; k < 16; k++) {
                 if (k & d) continue;
-                ct64(x[k], x[k + d], __ldg(tw + (1 << st) + (k >> (4 - st))), c.Q, c.twoQ);
+                ct64<PM>(x[k], x[k + d], __ldg(tw + (1 << st) + (k >> (4 - st))), c);
             }
         }
+        uint64_t *const b = a + pi<P>(j);
 #pragma unroll
-        for (int k = 0; k < 16; k++) a[pi<P>(j + k * 128)] = x[k];
+        for (int k = 0; k < 16; k++) b[pi<P>(k * 128)] = x[k];
     }
 }
 
-// Forward NTT of a digit polynomial (values < BG) as ntt64_fwd_2048, the
-// first two stages from the digit tables; output < 21Q + BG.
-template <int G, bool P>
-__device__ __forceinline__ void ntt64_fwd_2048_digit(uint64_t *a, const ulonglong2 *__restrict__ tw,
-                                                     const Ntt64Consts &c, int tid, int bar, const DigitTables64 &T)
+// Forward NTT of such a polynomial as ntt64_fwd_2048; output < 23Q.
+template <bool PM, int G, bool P, bool DIGIT, class Load>
+__device__ __forceinline__ void ntt64_fwd_2048_load(uint64_t *a, Load load, const ulonglong2 *__restrict__ tw,
+                                                    const Ntt64Consts &c, int tid, int bar)
 {
-    fwd_pass16_digit<G, P>(a, tw, c, tid, T);      // t = 1024 .. 128
+    fwd_pass16_load<PM, G, P, DIGIT>(a, load, tw, c, tid);   // t = 1024 .. 128
     group_sync(bar, G);
-    fwd_passR<G, 4, P>(a, tw, c, tid, 64, 16);    // t = 64 .. 8
+    fwd_passR<PM, G, 4, P>(a, tw, c, tid, 64, 16);    // t = 64 .. 8
     group_sync(bar, G);
-    fwd_passR<G, 3, P>(a, tw, c, tid, 4, 256);    // t = 4, 2, 1
+    fwd_passR<PM, G, 3, P>(a, tw, c, tid, 4, 256);    // t = 4, 2, 1
     group_sync(bar, G);
 }
 
+// The gadget digit (src >> sh) & mask of a canonical time-domain polynomial src
+// (layout pi<P>), for ntt64_fwd_2048_load.
+template <bool P>
+struct LoadDigit64 {
+    const uint64_t *src;
+    uint32_t sh, mask;
+    __device__ __forceinline__ uint64_t operator()(int j, int k) const
+    {
+        return (uint32_t)(src[pi<P>(j) + pi<P>(k * 128)] >> sh) & mask;
+    }
+};
+
 // One radix-8 inverse pass: stages t, 2t, 4t (m = N / 2t) on the octets
-// e0 + k t (k < 8) of every 8t-block.
-template <int G, bool P>
+// e0 + k t (k < 8) of every 8t-block. Inputs below 2^K Q (PM; else 2Q); PM
+// outputs below 2^(K+3) Q, or below 2Q with FOLD (the products, x[4..7], are).
+template <bool PM, int G, bool P, int K, bool FOLD>
 __device__ __forceinline__ void inv_pass8(uint64_t *a, const ulonglong2 *__restrict__ itw, const Ntt64Consts &c,
                                           int tid, int t, int m)
 {
     for (int oc = tid; oc < 256; oc += G) {
-        const int grp = oc / t, j = oc - grp * t;
-        const int e0 = grp * 8 * t + j;
+        int grp = oc / t;
+        const int j = oc - grp * t;
+        // t = 8, padded: a half warp takes blocks two apart (136 words, the other
+        // eight bank pairs) rather than neighbours (68 words)
+        if (P && t == 8) grp = (grp & ~3) | ((grp & 1) << 1) | ((grp >> 1) & 1);
+        uint64_t *const b = a + pi<P>(grp * 8 * t + j);
         uint64_t x[8];
 #pragma unroll
-        for (int k = 0; k < 8; k++) x[k] = a[pi<P>(e0 + k * t)];
+        for (int k = 0; k < 8; k++) x[k] = b[pi<P>(k * t)];
 #pragma unroll
-        for (int k = 0; k < 4; k++) gs64(x[2 * k], x[2 * k + 1], __ldg(itw + m + 4 * grp + k), c.Q, c.twoQ);
+        for (int k = 0; k < 4; k++) gs64<PM, K>(x[2 * k], x[2 * k + 1], __ldg(itw + m + 4 * grp + k), c);
         const ulonglong2 w2a = __ldg(itw + (m >> 1) + 2 * grp), w2b = __ldg(itw + (m >> 1) + 2 * grp + 1);
-        gs64(x[0], x[2], w2a, c.Q, c.twoQ);
-        gs64(x[1], x[3], w2a, c.Q, c.twoQ);
-        gs64(x[4], x[6], w2b, c.Q, c.twoQ);
-        gs64(x[5], x[7], w2b, c.Q, c.twoQ);
+        gs64<PM, K + 1>(x[0], x[2], w2a, c);
+        gs64<PM, K + 1>(x[1], x[3], w2a, c);
+        gs64<PM, K + 1>(x[4], x[6], w2b, c);
+        gs64<PM, K + 1>(x[5], x[7], w2b, c);
         const ulonglong2 w4 = __ldg(itw + (m >> 2) + grp);
-        gs64(x[0], x[4], w4, c.Q, c.twoQ);
-        gs64(x[1], x[5], w4, c.Q, c.twoQ);
-        gs64(x[2], x[6], w4, c.Q, c.twoQ);
-        gs64(x[3], x[7], w4, c.Q, c.twoQ);
+        gs64<PM, K + 2>(x[0], x[4], w4, c);
+        gs64<PM, K + 2>(x[1], x[5], w4, c);
+        gs64<PM, K + 2>(x[2], x[6], w4, c);
+        gs64<PM, K + 2>(x[3], x[7], w4, c);
+        if (PM && FOLD) {
 #pragma unroll
-        for (int k = 0; k < 8; k++) a[pi<P>(e0 + k * t)] = x[k];
+            for (int k = 0; k < 4; k++) x[k] = reduce64<PM>(x[k], c);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) b[pi<P>(k * t)] = x[k];
     }
 }
 
@@ -212,27 +336,29 @@ __device__ __forceinline__ void inv_pass8(uint64_t *a, const ulonglong2 *__restr
 // -> canonical coefficients times N^-1. itw[k] = (psi^-bitrev(k), companion).
 // Three radix-8 passes (stages t = 1..4, 8..32, 64..256) and one radix-4 pass
 // (t = 512 and the last stage, t = 1024, with N^-1 folded into both outputs).
-template <int G, bool P>
+template <bool PM, int G, bool P>
 __device__ __forceinline__ void ntt64_inv_2048(uint64_t *a, const ulonglong2 *__restrict__ itw, const Ntt64Consts &c,
                                                int tid, int bar)
 {
-    inv_pass8<G, P>(a, itw, c, tid, 1, 1024);
+    inv_pass8<PM, G, P, 1, false>(a, itw, c, tid, 1, 1024);   // 2Q -> 16Q
     group_sync(bar, G);
-    inv_pass8<G, P>(a, itw, c, tid, 8, 128);
+    inv_pass8<PM, G, P, 4, true>(a, itw, c, tid, 8, 128);     // 16Q -> 2Q
     group_sync(bar, G);
-    inv_pass8<G, P>(a, itw, c, tid, 64, 16);
+    inv_pass8<PM, G, P, 1, false>(a, itw, c, tid, 64, 16);    // 2Q -> 16Q
     group_sync(bar, G);
     for (int b = tid; b < 512; b += G) {
         uint64_t x0 = a[pi<P>(b)], x1 = a[pi<P>(b + 512)], x2 = a[pi<P>(b + 1024)], x3 = a[pi<P>(b + 1536)];
-        gs64(x0, x1, __ldg(itw + 2), c.Q, c.twoQ);   // t = 512, m = 2, block 0
-        gs64(x2, x3, __ldg(itw + 3), c.Q, c.twoQ);   // block 1
+        gs64<PM, 4>(x0, x1, __ldg(itw + 2), c);   // t = 512, m = 2, block 0
+        gs64<PM, 4>(x2, x3, __ldg(itw + 3), c);   // block 1
         // t = 1024, m = 1, with N^-1 folded into both outputs
-        uint64_t u = shoup64(x0 + x2, c.iN, c.iNs, c.Q);
-        uint64_t v = shoup64(x0 - x2 + c.twoQ, c.iw1N, c.iw1Ns, c.Q);
+        const uint64_t bias = PM ? c.Q << 5 : c.twoQ;
+        const ulonglong2 wu = make_ulonglong2(c.iN, c.iNs), wv = make_ulonglong2(c.iw1N, c.iw1Ns);
+        uint64_t u = mul64<PM>(x0 + x2, wu, c);
+        uint64_t v = mul64<PM>(x0 - x2 + bias, wv, c);
         a[pi<P>(b)] = u >= c.Q ? u - c.Q : u;
         a[pi<P>(b + 1024)] = v >= c.Q ? v - c.Q : v;
-        u = shoup64(x1 + x3, c.iN, c.iNs, c.Q);
-        v = shoup64(x1 - x3 + c.twoQ, c.iw1N, c.iw1Ns, c.Q);
+        u = mul64<PM>(x1 + x3, wu, c);
+        v = mul64<PM>(x1 - x3 + bias, wv, c);
         a[pi<P>(b + 512)] = u >= c.Q ? u - c.Q : u;
         a[pi<P>(b + 1536)] = v >= c.Q ? v - c.Q : v;
     }

@@ -21,6 +21,18 @@ namespace dev {
 
 enum { kEwSub = 0, kEwAdd = 1, kEwRot = 2 };
 
+// out[i] = a[i] * rot[e] mod Q (e = coefficient) for `words` words of N = 2048
+// RLWEs, canonical; rot: constant pairs (mul64).
+template <bool PM>
+__global__ void rlwe_rotate64_kernel(const uint64_t *__restrict__ a, const ulonglong2 *__restrict__ rot,
+                                     uint64_t *__restrict__ out, size_t words, const __grid_constant__ Ntt64Consts c)
+{
+    for (size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x; x < words; x += (size_t)gridDim.x * blockDim.x) {
+        const uint64_t v = mul64<PM>(a[x], __ldg(rot + (x & 2047)), c);
+        out[x] = v >= c.Q ? v - c.Q : v;
+    }
+}
+
 // out[i] = a[i] - b[i], a[i] + b[i], or a[i] * rot[e] (e = coefficient) mod Q
 // for `count` RLWEs of 2N words; a and b step by a_stride / b_stride words per
 // RLWE, out by 2N. Inputs canonical (< Q < 2^62).
@@ -61,6 +73,20 @@ static int launch_elementwise(Context &c, int mode, const uint64_t *a, size_t a_
     c.launches++;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "elementwise launch");
+}
+
+static int launch_rotate64(Context &c, const uint64_t *a, const ulonglong2 *rot, uint64_t *out, size_t count,
+                           cudaStream_t st)
+{
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    const size_t words = count * 4096;
+    const unsigned blocks = (unsigned)std::min<size_t>((words + 255) / 256, (size_t)std::max(sms, 1) * 8);
+    auto kern = c.nc64.pm_c ? dev::rlwe_rotate64_kernel<true> : dev::rlwe_rotate64_kernel<false>;
+    kern<<<blocks, 256, 0, st>>>(a, rot, out, words, c.nc64);
+    c.launches++;
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "rotation launch");
 }
 
 static int mult_rgsw(Context &c, const uint64_t *acc, const uint64_t *rgsw, size_t stride, uint64_t *out,
@@ -128,7 +154,8 @@ int fheacc_rlwe_blind_rotate_async(fheacc_ctx *ctx, const uint64_t *d_in, const 
     const uint64_t *rot = forward ? c.d_rot_fwd : c.d_rot;
     for (int i = 0; i < logN && !rc; i++) {
         // tmp = RLWE_rotate_freq(acc, i, forward); acc = CMUX(acc, tmp, C[i])
-        rc = launch_elementwise(c, dev::kEwRot, d_out, rw, nullptr, 0, rot + (size_t)i * N, tmp, count, st);
+        rc = c.wide ? launch_rotate64(c, d_out, (forward ? c.d_rot_fwd64 : c.d_rot64) + (size_t)i * N, tmp, count, st)
+                    : launch_elementwise(c, dev::kEwRot, d_out, rw, nullptr, 0, rot + (size_t)i * N, tmp, count, st);
         if (!rc) rc = cmux_device(c, d_out, tmp, rw, d_rgsws + (size_t)i * gw, 0, d_out, count, cm, st);
     }
     return rc;
