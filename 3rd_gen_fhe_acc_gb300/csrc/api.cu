@@ -2,6 +2,7 @@
 // context, key upload with the one-time device re-layout, and the bootstrap
 // entry points. Replaces the FPGA backend's configuration, DMA and issue loop
 // (FHE_ACC_runtime/src/myfpga.cpp:82-1660).
+#include "br64.cuh"
 #include "ctx.hpp"
 #include "host/host_math.hpp"
 #include <algorithm>
@@ -75,7 +76,7 @@ int bootstrap_device_with(Context &c, const uint64_t *d_c1, const uint64_t *d_c2
 {
     flags &= ~(uint32_t)FHEACC_FLAG_PROFILE;
     if (c.wide) {
-        if (!c.d_btkey64) return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
+        if (!c.has_btkey()) return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
         if (!c.d_kskey64) return c.fail(FHEACC_ENOKEY, "LWE key-switch key not uploaded");
         int rc = launch_blind_rotate64_with(c, d_c1, d_c2, d_gates, count, flags, (uint64_t *)accs, nullptr,
                                             (uint64_t *)extract, 0, st);
@@ -95,7 +96,7 @@ int bootstrap_device(Context &c, const uint64_t *d_c1, const uint64_t *d_c2, con
                      size_t count, uint64_t *d_out, uint32_t flags, cudaStream_t st, int max_ctas)
 {
     if (c.wide) {
-        if (!c.d_btkey64) return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
+        if (!c.has_btkey()) return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
         if (!c.d_kskey64) return c.fail(FHEACC_ENOKEY, "LWE key-switch key not uploaded");
         int rc = ensure_scratch(c, c.extract, count * kExtract64 * sizeof(uint64_t));
         if (rc) return rc;
@@ -395,6 +396,7 @@ int fheacc_destroy(fheacc_ctx *ctx)
     cudaFree(c->d_tw64);
     cudaFree(c->d_itw64);
     cudaFree(c->d_btkey64);
+    cudaFree(c->d_btkey64_limbs);
     cudaFree(c->d_cf64);
     cudaFree(c->d_kskey64);
     cudaFree(c->d_subs64);
@@ -445,28 +447,34 @@ static int bootstrap_key_pass(Context &c, const uint64_t *btkey, size_t words, b
     const size_t n = c.p.n, dR = c.p.digitR, Br = c.p.Br;
     const size_t rw = (size_t)c.p.digitG * 4 * c.p.N;
     const uint64_t Q = c.p.Q;
-    if (verify && !(c.wide ? (void *)c.d_btkey64 : (void *)c.d_btkey))
+    if (verify && !c.has_btkey())
         return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
     if (c.wide) {
-        // device order, one step (all residues) per chunk, constant pairs (mul64) made on the GPU
-        if (!verify && !c.d_btkey64) {
-            cudaError_t e = cudaMalloc(&c.d_btkey64, words * sizeof(ulonglong2));
+        // device order, one step (all residues) per chunk, device words made on the GPU
+        const bool limbs = c.nc64.pm_c && c.dp.last_digit_from_acc;
+        const size_t wb = limbs ? sizeof(uint2) : sizeof(ulonglong2);   // bytes of a device word
+        if (!verify && !c.has_btkey()) {
+            void *ptr = nullptr;
+            cudaError_t e = cudaMalloc(&ptr, words * wb);
             if (e != cudaSuccess) {
                 cudaGetLastError();
-                c.d_btkey64 = nullptr;
                 return c.fail(FHEACC_ENOMEM, "device memory for the bootstrap key");
             }
-            c.btkey_bytes = words * sizeof(ulonglong2);
+            if (limbs) c.d_btkey64_limbs = (uint2 *)ptr;
+            else c.d_btkey64 = (ulonglong2 *)ptr;
+            c.btkey_bytes = words * wb;
         }
+        char *const base = limbs ? (char *)c.d_btkey64_limbs : (char *)c.d_btkey64;
         std::vector<uint64_t> stage(Br * rw);
         uint64_t *d_stage = nullptr;
-        ulonglong2 *d_check = nullptr;   // verify: the chunk as the upload makes it
-        std::vector<ulonglong2> made, held;
+        char *d_check = nullptr;   // verify: the chunk as the upload makes it
+        std::vector<char> made, held;
+        const size_t cb = Br * rw * wb;
         cudaError_t e = cudaMalloc(&d_stage, Br * rw * sizeof(uint64_t));
         if (e == cudaSuccess && verify) {
-            e = cudaMalloc(&d_check, Br * rw * sizeof(ulonglong2));
-            made.resize(Br * rw);
-            held.resize(Br * rw);
+            e = cudaMalloc(&d_check, cb);
+            made.resize(cb);
+            held.resize(cb);
         }
         if (e != cudaSuccess) {
             cudaFree(d_stage);
@@ -481,14 +489,17 @@ static int bootstrap_key_pass(Context &c, const uint64_t *btkey, size_t words, b
                 e = cudaMemcpy(d_stage, stage.data(), Br * rw * sizeof(uint64_t), cudaMemcpyHostToDevice);
                 if (e != cudaSuccess) rc = c.cuda_fail(e, "key upload");
                 else if (derive) rc = launch_derive_keys64(c, d_stage, Br, c.d_cf64, c.stream);
-                ulonglong2 *chunk = c.d_btkey64 + (i * dR + j) * Br * rw;
-                if (!rc) rc = launch_const_pairs64(c, d_stage, verify ? d_check : chunk, Br * rw, c.stream);
-                if (!rc && cudaStreamSynchronize(c.stream) != cudaSuccess) rc = c.cuda_fail(cudaGetLastError(), "key pairs");
+                char *chunk = base + (i * dR + j) * cb;
+                char *to = verify ? d_check : chunk;
+                if (!rc)
+                    rc = limbs ? launch_limb_words64(c, d_stage, (uint2 *)to, Br * rw, c.stream)
+                               : launch_const_pairs64(c, d_stage, (ulonglong2 *)to, Br * rw, c.stream);
+                if (!rc && cudaStreamSynchronize(c.stream) != cudaSuccess) rc = c.cuda_fail(cudaGetLastError(), "key words");
                 if (!rc && verify) {
-                    e = cudaMemcpy(made.data(), d_check, Br * rw * sizeof(ulonglong2), cudaMemcpyDeviceToHost);
-                    if (e == cudaSuccess) e = cudaMemcpy(held.data(), chunk, Br * rw * sizeof(ulonglong2), cudaMemcpyDeviceToHost);
+                    e = cudaMemcpy(made.data(), d_check, cb, cudaMemcpyDeviceToHost);
+                    if (e == cudaSuccess) e = cudaMemcpy(held.data(), chunk, cb, cudaMemcpyDeviceToHost);
                     if (e != cudaSuccess) rc = c.cuda_fail(e, "key read-back");
-                    else if (std::memcmp(made.data(), held.data(), Br * rw * sizeof(ulonglong2)) != 0)
+                    else if (std::memcmp(made.data(), held.data(), cb) != 0)
                         rc = c.fail(FHEACC_EMISMATCH, "device bootstrap key differs from the given key");
                 }
             }

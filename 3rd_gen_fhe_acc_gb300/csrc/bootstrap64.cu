@@ -18,6 +18,7 @@
 // (18 MB) through L2 together; accumulators live in global
 // memory (32 KB per gate).
 #include "ctx.hpp"
+#include "br64.cuh"
 #include "l2hint.cuh"
 #include "ntt64.cuh"
 #include <algorithm>
@@ -26,7 +27,6 @@ namespace fheacc {
 namespace dev {
 
 constexpr int kMaxGroup64 = 8;   // ciphertexts per worker and claim
-constexpr int kT64 = 256;   // threads per CTA
 
 // One worker's polys in shared memory, layout pi<P> (ntt64.cuh).
 //
@@ -265,129 +265,9 @@ __global__ void rlwe_split_sum64_kernel(const uint64_t *__restrict__ partial, ui
     }
 }
 
-struct Br64Args {
-    const uint64_t *c1, *c2;
-    const uint32_t *idx1, *idx2;   // optional: gate g reads c1 + idx1[g] * (n+1) (else g)
-    const int32_t *gates;
-    size_t count;
-    const ulonglong2 *btkey;   // [(i*digitR + j)*Br + r][digitG][2][2][2048] constant pairs
-    uint64_t *accs;            // scratch [count][2][2048], NTT domain, values < 2Q
-    uint64_t *acc_out;         // optional canonical NTT accumulators [count][4096]
-    uint64_t *extract;         // optional [count][kExtract64]
-    int group;                 // ciphertexts per claim (<= kMaxGroup64 per worker)
-    int derive_last;           // last digit's NTT from the accumulator (DevParams::last_digit_from_acc)
-    int n, DG;
-    uint32_t q, embed, Br, digitR, bg_bits, flags;
-    uint64_t gate_constant[8];
-    StepWindow win;            // keeps the CTAs within a few steps of each other (window.cuh)
-    unsigned long long *claim_next;   // next unclaimed ciphertext (zeroed before the launch)
-    unsigned *status;          // set to kStatusWaitLimit if a worker gave up waiting
-    unsigned wait_limit;       // polls before such a wait gives up (kWorkerWaitLimit)
-    size_t claim_limit;        // ciphertexts [0, claim_limit) are claimed in groups
-    // remainder pool: ciphertexts [pool_first, pool_first + pool_count) that all
-    // CTAs share item by item (0: none); their state after the claim words
-    int pool_count;
-    size_t pool_first;
-    unsigned long long *pool_cursor;   // next (step, pool ciphertext) item, step-major (zeroed)
-    int *pool_done;            // [pool_count] last finished step (-1: none yet)
-    int *pool_last;            // [pool_count] last step with a non-zero residue (-1: none)
-    uint8_t *pool_res;         // [pool_count][n * digitR] residues
-};
-
-// LWE_evaluate (LWE.cpp:203-222) of ciphertext gid and the residues of its
-// refresh steps, the base-Br digits of (q - a_i) mod q (RLWE.cpp:740-760), into
-// res[n * digitR]; the thread that takes i = n writes the b value and the gate's
-// two test-vector bounds. Threads t0, t0 + nt, ... take part.
-__device__ __forceinline__ void br64_residues(const Br64Args &A, size_t gid, uint8_t *res, uint32_t *bval,
-                                              uint32_t *b1, uint32_t *b2, int t0, int nt)
-{
-    const int n = A.n;
-    const uint32_t q = A.q, qmask = q - 1;
-    const int g = A.gates[gid];
-    const bool x2 = (g == 4 || g == 5);
-    const uint64_t *c1 = A.c1 + (A.idx1 ? (size_t)A.idx1[gid] : gid) * (size_t)(n + 1);
-    const uint64_t *c2 = A.c2 + (A.idx2 ? (size_t)A.idx2[gid] : gid) * (size_t)(n + 1);
-    for (int i = t0; i <= n; i += nt) {
-        const uint64_t v = x2 ? 2 * (c1[i] - c2[i]) : c1[i] + c2[i];
-        if (i < n) {
-            uint32_t nega = (q - (uint32_t)(v & qmask)) & qmask;
-            for (uint32_t j = 0; j < A.digitR; j++) {
-                res[i * (int)A.digitR + (int)j] = (uint8_t)(nega % A.Br);
-                nega /= A.Br;
-            }
-        } else {
-            const uint64_t gc = A.gate_constant[(unsigned)g < 6u ? g : 6];
-            *bval = (uint32_t)(v & qmask);
-            *b1 = (uint32_t)(gc & qmask);
-            *b2 = (*b1 + q / 2) & qmask;
-        }
-    }
-}
-
-// acc_initialization (RLWE.cpp:706-724) of ciphertext gid into its accumulator:
-// a = 0, b = the test vector, forward NTT. buf: a shared poly (layout pi<P>)
-// that the worker's second 128-thread group transforms; bar: the worker's
-// barrier (its groups on bar + 1 and bar + 2).
-template <bool PM, bool P>
-__device__ __forceinline__ void br64_acc_init(const Br64Args &A, const Ntt64Consts &c, const ulonglong2 *tw,
-                                              size_t gid, uint32_t val, uint32_t b1, uint32_t b2, uint64_t *buf,
-                                              int tid, int bar)
-{
-    const uint32_t q = A.q, qmask = q - 1;
-    const uint64_t Q8 = c.Q / 8 + 1, negQ8 = c.Q - Q8;
-    for (int e = tid; e < 2048; e += kT64) {
-        uint64_t v = 0;
-        if (e % A.embed == 0 && (uint32_t)e / A.embed < q / 2) {
-            const uint32_t tmp = (val - (uint32_t)e / A.embed) & qmask;
-            if (b1 < b2) v = (tmp >= b1 && tmp < b2) ? negQ8 : Q8;
-            else v = (tmp >= b2 && tmp < b1) ? Q8 : negQ8;
-        }
-        buf[pi<P>(e)] = v;
-    }
-    group_sync(bar, kT64);
-    if (tid >= 128) ntt64_fwd_2048<PM, 128, P>(buf, tw, c, tid - 128, bar + 2);
-    group_sync(bar, kT64);
-    uint64_t *acc = A.accs + gid * 4096;
-    const uint64_t pol = l2_keep_policy();
-    for (int e = tid; e < 2048; e += kT64) {
-        st_keep64(acc + e, 0, pol);
-        st_keep64(acc + 2048 + e, canonical64<PM>(buf[pi<P>(e)], c), pol);
-    }
-    group_sync(bar, kT64);
-}
-
-// Output of ciphertext gid from its accumulator: the extracted RLWE
-// (NTT_a_transpose, RLWE.cpp:218-226, then the inverse NTT of both polys) or
-// the canonical NTT accumulator. a0, a1: shared polys (layout pi<P>).
-template <bool PM, bool P>
-__device__ __noinline__ void br64_output(const Br64Args &A, const Ntt64Consts &c, const ulonglong2 *itw,
-                                            size_t gid, uint64_t *a0, uint64_t *a1, int tid, int bar)
-{
-    const uint64_t *acc = A.accs + gid * 4096;
-    if (A.extract) {
-        for (int e = tid; e < 2048; e += kT64) {
-            a0[pi<P>(e)] = __ldcg(acc + 2047 - e);
-            a1[pi<P>(e)] = __ldcg(acc + 2048 + e);
-        }
-        group_sync(bar, kT64);
-        ntt64_inv_2048<PM, 128, P>(tid < 128 ? a0 : a1, itw, c, tid & 127, bar + 1 + (tid >> 7));
-        group_sync(bar, kT64);
-        uint64_t *ext = A.extract + gid * kExtract64;
-        for (int e = tid; e < 2048; e += kT64) ext[e] = a0[pi<P>(e)];
-        if (tid == 0) ext[2048] = a1[pi<P>(0)];
-    } else {
-        for (int e = tid; e < 4096; e += kT64) {
-            const uint64_t v = __ldcg(acc + e);
-            A.acc_out[gid * 4096 + e] = v >= c.Q ? v - c.Q : v;
-        }
-    }
-    group_sync(bar, kT64);
-}
-
 // Remainder pool set-up, one 256-thread CTA per pool ciphertext, before the
 // blind rotation on the same stream: residues, last non-zero step, the
 // initialised accumulator, and the output of a ciphertext without steps.
-template <bool PM>
 __global__ void __launch_bounds__(kT64) br64_pool_init_kernel(const __grid_constant__ Br64Args A,
                                                              const ulonglong2 *__restrict__ tw,
                                                              const ulonglong2 *__restrict__ itw,
@@ -414,9 +294,9 @@ __global__ void __launch_bounds__(kT64) br64_pool_init_kernel(const __grid_const
         A.pool_last[p] = l;
         A.pool_done[p] = -1;
     }
-    br64_acc_init<PM, false>(A, c, tw, gid, bv[0], bv[1], bv[2], buf[1], tid, 1);
+    br64_acc_init<false, false>(A, c, tw, gid, bv[0], bv[1], bv[2], buf[1], tid, 1);
     __syncthreads();
-    if (last < 0) br64_output<PM, false>(A, c, itw, gid, buf[0], buf[1], tid, 1);
+    if (last < 0) br64_output<false, false>(A, c, itw, gid, buf[0], buf[1], tid, 1);
 }
 
 // Polls of a worker waiting for another worker's step of the same ciphertext
@@ -471,7 +351,7 @@ __device__ __forceinline__ bool pool_take(const Br64Args &A, int S, int mode, un
 // ciphertexts form a pool that all CTAs share item by item (pool_take), their
 // steps ordered by done words in global memory. An XOR swizzle of the shared-memory passes removed their bank
 // conflicts but cost more in index arithmetic than it saved.
-template <bool PM, int W, int MINB>
+template <int W, int MINB>
 __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_constant__ Br64Args A,
                                                           const ulonglong2 *__restrict__ tw,
                                                           const ulonglong2 *__restrict__ itw,
@@ -516,7 +396,7 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
         // acc_initialization, one ciphertext per worker: a = 0, b = test vector,
         // forward NTT (the worker's group 1 transforms b)
         for (int k = wk; k < m; k += W)
-            br64_acc_init<PM, true>(A, c, tw, first + (size_t)k, bvals[k], b1s[k], b2s[k], s.buf[1], tid, bar);
+            br64_acc_init<false, true>(A, c, tw, first + (size_t)k, bvals[k], b1s[k], b2s[k], s.buf[1], tid, bar);
         __syncthreads();
         // blind rotation: the workers take the group's items from the cursor
         for (;;) {
@@ -585,7 +465,7 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
                 const uint64_t pol = l2_keep_policy();
                 for (int e = tid; e < 4096; e += kT64) s.acc[e >> 11][px(e & 2047)] = ld_keep64(acc + e, pol);
                 group_sync(bar, kT64);
-                step64<PM, true, true>(s, A.btkey + ((size_t)st * A.Br + r) * rgsw_pairs, A.DG, A.bg_bits, tw, itw, c,
+                step64<false, true, true>(s, A.btkey + ((size_t)st * A.Br + r) * rgsw_pairs, A.DG, A.bg_bits, tw, itw, c,
                        A.derive_last ? acc : nullptr, tid, bar);
             }
             // the item again from the plan (not held in registers across the step;
@@ -609,11 +489,11 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
                 }
             }
             // a pool ciphertext's output right after its last step
-            if (pool && st == A.pool_last[k]) br64_output<PM, true>(A, c, itw, gid, s.acc[0], s.acc[1], tid, bar);
+            if (pool && st == A.pool_last[k]) br64_output<false, true>(A, c, itw, gid, s.acc[0], s.acc[1], tid, bar);
         }
         __syncthreads();
         // output, one ciphertext per worker
-        for (int k = wk; k < m; k += W) br64_output<PM, true>(A, c, itw, first + (size_t)k, s.acc[0], s.acc[1], tid, bar);
+        for (int k = wk; k < m; k += W) br64_output<false, true>(A, c, itw, first + (size_t)k, s.acc[0], s.acc[1], tid, bar);
         __syncthreads();
     }
     // a CTA counts into every bucket it has not counted into yet
@@ -894,17 +774,17 @@ int launch_blind_rotate64(Context &c, const uint64_t *d_c1, const uint64_t *d_c2
                           cudaStream_t st)
 {
     if (!count) return FHEACC_OK;
-    if (!c.d_btkey64) return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
+    if (!c.has_btkey()) return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
     int rc = ensure_scratch(c, c.accs, bootstrap_accs_bytes(c, count));
     if (rc) return rc;
     return launch_blind_rotate64_with(c, d_c1, d_c2, d_gates, count, flags, (uint64_t *)c.accs.ptr, d_acc_out,
                                       d_extract, max_ctas, st);
 }
 
-template <bool PM, int W, int MINB>
+template <int W, int MINB>
 static int launch_br64_shape(Context &c, dev::Br64Args A, int max_ctas, cudaStream_t st)
 {
-    auto kern = dev::br64_kernel<PM, W, MINB>;
+    auto kern = dev::br64_kernel<W, MINB>;
     const size_t steps = (size_t)c.p.n * c.p.digitR;
     // group cap: kMaxGroup64 (or the tuned cap) per worker, within the shared memory of one CTA
     int cap = W * (c.tune.br_group > 0 ? std::min(c.tune.br_group, dev::kMaxGroup64) : dev::kMaxGroup64);
@@ -951,7 +831,7 @@ static int launch_br64_shape(Context &c, dev::Br64Args A, int max_ctas, cudaStre
     e = cudaMemsetAsync(A.claim_next, 0, kClaimWords * sizeof(uint32_t), st);
     if (e != cudaSuccess) return c.cuda_fail(e, "br64 claim reset");
     if (A.pool_count) {
-        dev::br64_pool_init_kernel<PM><<<(unsigned)A.pool_count, dev::kT64, 0, st>>>(A, c.d_tw64, c.d_itw64, c.nc64);
+        dev::br64_pool_init_kernel<<<(unsigned)A.pool_count, dev::kT64, 0, st>>>(A, c.d_tw64, c.d_itw64, c.nc64);
         c.launches++;
         e = cudaGetLastError();
         if (e != cudaSuccess) return c.cuda_fail(e, "br64 pool launch");
@@ -997,7 +877,7 @@ int launch_blind_rotate64_indexed(Context &c, const uint64_t *d_c1, const uint64
                                   bool window, cudaStream_t st)
 {
     if (!count) return FHEACC_OK;
-    if (!c.d_btkey64) return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
+    if (!c.has_btkey()) return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
     dev::Br64Args A{};
     A.c1 = d_c1; A.c2 = d_c2; A.idx1 = d_idx1; A.idx2 = d_idx2; A.gates = d_gates; A.count = count;
     A.win.steps = window ? 0 : -1;
@@ -1007,19 +887,15 @@ int launch_blind_rotate64_indexed(Context &c, const uint64_t *d_c1, const uint64
     A.status = c.d_status;
     A.wait_limit = c.tune.debug_wait_limit >= 0 ? (unsigned)c.tune.debug_wait_limit : dev::kWorkerWaitLimit;
     for (int i = 0; i < 8; i++) A.gate_constant[i] = c.dp.gate_constant[i];
+    if (c.d_btkey64_limbs) return launch_blind_rotate64_blocks(c, A, max_ctas, st);
     // workers per CTA, by default from the gates per SM: up to 1 one worker,
     // beyond that two (128 registers a thread without spills; three workers' 80
     // spill)
     const size_t sms = (size_t)sms_of(c);
     const int w = c.tune.br_pipes > 0 ? c.tune.br_pipes : count <= sms ? 1 : 2;
-    if (c.nc64.pm_c) {
-        if (w == 3) return launch_br64_shape<true, 3, 1>(c, A, max_ctas, st);
-        if (w == 2) return launch_br64_shape<true, 2, 1>(c, A, max_ctas, st);
-        return launch_br64_shape<true, 1, 2>(c, A, max_ctas, st);
-    }
-    if (w == 3) return launch_br64_shape<false, 3, 1>(c, A, max_ctas, st);
-    if (w == 2) return launch_br64_shape<false, 2, 1>(c, A, max_ctas, st);
-    return launch_br64_shape<false, 1, 2>(c, A, max_ctas, st);
+    if (w == 3) return launch_br64_shape<3, 1>(c, A, max_ctas, st);
+    if (w == 2) return launch_br64_shape<2, 1>(c, A, max_ctas, st);
+    return launch_br64_shape<1, 2>(c, A, max_ctas, st);
 }
 
 int launch_extract64(Context &c, const uint64_t *d_rlwe, size_t count, uint64_t *d_extract, cudaStream_t st)

@@ -2,6 +2,7 @@
 // the kernel translation units. Internal to libfheacc.so.
 #pragma once
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <string>
@@ -123,6 +124,9 @@ struct Context {
     // 64-bit path: twiddles as constant pairs (mul64 in ntt64.cuh) in reference order
     ulonglong2 *d_tw64 = nullptr, *d_itw64 = nullptr;
     dev::Ntt64Consts nc64{};
+    // the bootstrap key of a Q = 2^b - c in limb words (blind_rotate64.cu), or of
+    // any other Q in constant pairs (bootstrap64.cu), same order
+    uint2 *d_btkey64_limbs = nullptr;
     ulonglong2 *d_btkey64 = nullptr;   // constant pairs, [(i*digitR + j)*Br + r][digitG][2][2][N]
     ulonglong2 *d_cf64 = nullptr;      // factors of the last-digit identity, digitG constant pairs
     ulonglong2 *d_subs64 = nullptr;    // constant pairs, [logN][digitKS_R][2][N]
@@ -151,6 +155,7 @@ struct Context {
     std::atomic<uint64_t> launches{0};   // kernels launched (or captured into a graph) so far;
                                          // atomic: a server's worker thread launches while others read
 
+    bool has_btkey() const { return d_btkey || d_btkey64 || d_btkey64_limbs; }
     size_t device_bytes() const
     {
         return btkey_bytes + kskey_bytes + subs_bytes + accs.bytes + extract.bytes + io.bytes + psi.bytes +
@@ -269,8 +274,9 @@ constexpr size_t kExtract64 = 2048 + 8;        // u64 words per extracted RLWE (
 // accumulators and extracted RLWEs (bytes of each).
 inline size_t bootstrap_accs_bytes(const Context &c, size_t count)
 {
+    const size_t S = (size_t)c.p.n * c.p.digitR;   // residues: of every gate (block form) or of the pool's
     return c.wide ? count * 4096 * sizeof(uint64_t) + kClaimWords * sizeof(uint32_t) +
-                        kPool64 * (2 * sizeof(int) + (size_t)c.p.n * c.p.digitR)
+                        std::max(count * (sizeof(int) + S), kPool64 * (2 * sizeof(int) + S))
                   : (count * 2048 + kClaimWords) * sizeof(uint32_t);
 }
 inline size_t bootstrap_extract_bytes(const Context &c, size_t count)

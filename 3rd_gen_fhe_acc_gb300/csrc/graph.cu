@@ -180,7 +180,7 @@ int fheacc_graph_add_bootstrap(fheacc_graph *g, fheacc_ctx *ctx, const uint64_t 
     if (count && (!d_c1 || !d_c2 || !d_gates || !d_out)) return g->fail(FHEACC_EINVAL, "null buffer");
     Context &c = *reinterpret_cast<Context *>(ctx);
     if (g->device >= 0 && g->device != c.device) return g->fail(FHEACC_EINVAL, "contexts of one graph share a device");
-    if (c.wide ? !c.d_btkey64 || !c.d_kskey64 : !c.d_btkey || !c.d_kskey)
+    if (c.wide ? !c.has_btkey() || !c.d_kskey64 : !c.d_btkey || !c.d_kskey)
         return g->fail(FHEACC_ENOKEY, "keys must be uploaded before the context joins a graph");
     g->device = c.device;
     if (!count) return FHEACC_OK;
@@ -223,7 +223,7 @@ int fheacc_autotune(fheacc_ctx *ctx, size_t count, fheacc_tune_trial *trials, in
     if (!ctx) return FHEACC_EINVAL;
     Context &c = *reinterpret_cast<Context *>(ctx);
     if (count == 0 || count > ((size_t)1 << 22)) return c.fail(FHEACC_EINVAL, "autotune: count must be 1..4M");
-    if (c.wide ? !c.d_btkey64 || !c.d_kskey64 : !c.d_btkey || !c.d_kskey)
+    if (c.wide ? !c.has_btkey() || !c.d_kskey64 : !c.d_btkey || !c.d_kskey)
         return c.fail(FHEACC_ENOKEY, "autotune: keys must be uploaded");
     DeviceGuard dg(c.device);
     // synthetic batch: uniform LWE ciphertexts mod q, the six gates in turn

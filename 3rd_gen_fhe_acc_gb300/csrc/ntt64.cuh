@@ -70,7 +70,30 @@ inline int pm64_shift(uint64_t Q)
     return 0;
 }
 
-__device__ __forceinline__ uint64_t mul_wide64(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+// a b, and a b + s as one instruction: from (uint64_t)a * b + s the compiler often
+// makes a multiply and a 64-bit add, both on the multiply pipe (a step of the blind
+// rotation: 70 k instructions of that pipe, 50 k with the chains written out).
+__device__ __forceinline__ uint64_t mul_wide64(uint32_t a, uint32_t b)
+{
+    uint64_t d;
+    asm("mul.wide.u32 %0, %1, %2;" : "=l"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t mad_wide64(uint32_t a, uint32_t b, uint64_t s)
+{
+    uint64_t d;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(s));
+    return d;
+}
+
+// 2^-s (U + 2^32 V) mod Q of products with constants times 2^s (PM): the part
+// above 2^b is the word above 2^64.
+__device__ __forceinline__ uint64_t fold64(uint64_t U, uint64_t V, const Ntt64Consts &c)
+{
+    V += U >> 32;
+    const uint64_t low = (V << 32) | (uint32_t)U;
+    return mad_wide64((uint32_t)(V >> 32), c.pm_c, low >> c.pm_s);
+}
 
 // x w mod Q for a constant pair w, in [0, 2Q).
 // PM: w = (w << s, (w 2^30 mod Q) << s), s = 64 - b; x < 2^61. With U and V the
@@ -83,10 +106,9 @@ __device__ __forceinline__ uint64_t mul64(uint64_t x, ulonglong2 w, const Ntt64C
 {
     if (PM) {
         const uint32_t x0 = (uint32_t)x & 0x3fffffffu, x1 = (uint32_t)(x >> 30);
-        const uint64_t U = mul_wide64(x0, (uint32_t)w.x) + mul_wide64(x1, (uint32_t)w.y);
-        const uint64_t V = mul_wide64(x0, (uint32_t)(w.x >> 32)) + mul_wide64(x1, (uint32_t)(w.y >> 32)) + (U >> 32);
-        const uint64_t low = (V << 32) | (uint32_t)U;
-        return mul_wide64((uint32_t)(V >> 32), c.pm_c) + (low >> c.pm_s);
+        const uint64_t U = mad_wide64(x1, (uint32_t)w.y, mul_wide64(x0, (uint32_t)w.x));
+        const uint64_t V = mad_wide64(x1, (uint32_t)(w.y >> 32), mul_wide64(x0, (uint32_t)(w.x >> 32)));
+        return fold64(U, V, c);
     }
     const uint64_t t = __umul64hi(x, w.y);
     return x * w.x - t * c.Q;
@@ -100,12 +122,14 @@ __device__ __forceinline__ uint64_t mul64_2(uint64_t x, ulonglong2 v, uint64_t y
     if (PM) {
         const uint32_t x0 = (uint32_t)x & 0x3fffffffu, x1 = (uint32_t)(x >> 30);
         const uint32_t y0 = (uint32_t)y & 0x3fffffffu, y1 = (uint32_t)(y >> 30);
-        const uint64_t U = mul_wide64(x0, (uint32_t)v.x) + mul_wide64(x1, (uint32_t)v.y) +
-                           mul_wide64(y0, (uint32_t)w.x) + mul_wide64(y1, (uint32_t)w.y);
-        const uint64_t V = mul_wide64(x0, (uint32_t)(v.x >> 32)) + mul_wide64(x1, (uint32_t)(v.y >> 32)) +
-                           mul_wide64(y0, (uint32_t)(w.x >> 32)) + mul_wide64(y1, (uint32_t)(w.y >> 32)) + (U >> 32);
-        const uint64_t low = (V << 32) | (uint32_t)U;
-        return mul_wide64((uint32_t)(V >> 32), c.pm_c) + (low >> c.pm_s);
+        uint64_t U = mul_wide64(x0, (uint32_t)v.x), V = mul_wide64(x0, (uint32_t)(v.x >> 32));
+        U = mad_wide64(x1, (uint32_t)v.y, U);
+        V = mad_wide64(x1, (uint32_t)(v.y >> 32), V);
+        U = mad_wide64(y0, (uint32_t)w.x, U);
+        V = mad_wide64(y0, (uint32_t)(w.x >> 32), V);
+        U = mad_wide64(y1, (uint32_t)w.y, U);
+        V = mad_wide64(y1, (uint32_t)(w.y >> 32), V);
+        return fold64(U, V, c);
     }
     return mul64<PM>(x, v, c) + mul64<PM>(y, w, c);
 }
@@ -116,7 +140,7 @@ __device__ __forceinline__ uint64_t reduce64(uint64_t x, const Ntt64Consts &c)
 {
     if (PM) {
         const uint32_t b = 64 - c.pm_s;
-        return (x & (~0ull >> c.pm_s)) + mul_wide64((uint32_t)(x >> b), c.pm_c);
+        return mad_wide64((uint32_t)(x >> b), c.pm_c, x & (~0ull >> c.pm_s));
     }
     return x - __umul64hi(x, c.mu64) * c.Q;
 }
@@ -213,18 +237,14 @@ __device__ __forceinline__ void digit_radix4(uint64_t &x0, uint64_t &x1, uint64_
                                              const ulonglong2 *__restrict__ tw, const Ntt64Consts &c)
 {
     if (PM) {
-        auto fold = [&](uint64_t U, uint64_t V) {
-            V += U >> 32;
-            return mul_wide64((uint32_t)(V >> 32), c.pm_c) + (((V << 32) | (uint32_t)U) >> c.pm_s);
-        };
         auto lo = [](uint64_t w) { return (uint32_t)w; };
         auto hi = [](uint64_t w) { return (uint32_t)(w >> 32); };
         const uint32_t d1 = (uint32_t)x1, d2 = (uint32_t)x2, d3 = (uint32_t)x3;
-        const uint64_t A = fold(mul_wide64(d2, lo(c.dw1)), mul_wide64(d2, hi(c.dw1)));
-        const uint64_t B = fold(mul_wide64(d1, lo(c.dw2)) + mul_wide64(d3, lo(c.dw21)),
-                                mul_wide64(d1, hi(c.dw2)) + mul_wide64(d3, hi(c.dw21)));
-        const uint64_t D = fold(mul_wide64(d1, lo(c.dw3)) + mul_wide64(d3, lo(c.dw31)),
-                                mul_wide64(d1, hi(c.dw3)) + mul_wide64(d3, hi(c.dw31)));
+        const uint64_t A = fold64(mul_wide64(d2, lo(c.dw1)), mul_wide64(d2, hi(c.dw1)), c);
+        const uint64_t B = fold64(mad_wide64(d1, lo(c.dw2), mul_wide64(d3, lo(c.dw21))),
+                                  mad_wide64(d1, hi(c.dw2), mul_wide64(d3, hi(c.dw21))), c);
+        const uint64_t D = fold64(mad_wide64(d1, lo(c.dw3), mul_wide64(d3, lo(c.dw31))),
+                                  mad_wide64(d1, hi(c.dw3), mul_wide64(d3, hi(c.dw31))), c);
         const uint64_t u = x0 + A, v = x0 + c.twoQ - A;
         x0 = u + B;
         x1 = u + c.twoQ - B;

@@ -410,7 +410,7 @@ int fheacc_server_create(fheacc_ctx *ctx, size_t max_batch, size_t pool_cipherte
     if (!ctx || !out || max_batch == 0 || max_batch > (1u << 24) || pool_ciphertexts > 0xFFFFFFF0u)
         return FHEACC_EINVAL;
     Context &c = *reinterpret_cast<Context *>(ctx);
-    if (c.wide ? (!c.d_btkey64 || !c.d_kskey64) : (!c.d_btkey || !c.d_kskey))
+    if (c.wide ? (!c.has_btkey() || !c.d_kskey64) : (!c.d_btkey || !c.d_kskey))
         return c.fail(FHEACC_ENOKEY, "server: keys must be uploaded first");
     DeviceGuard guard(c.device);
     Server *s = new Server();

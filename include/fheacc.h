@@ -244,6 +244,10 @@ int fheacc_lwe_modswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t cou
  *                             0 = the kernel's maximum, 24 for 32-bit words,
  *                             8 for 64-bit); the launch fits equal groups to
  *                             the batch under the cap
+ *  (64-bit words, Q = 2^b - c with 48 <= b <= 54 and c <= 2^(b-36): one kernel
+ *  on clusters of CTAs up to one ciphertext per SM, else one that takes items
+ *  of a few steps from a shared cursor; FHEACC_OPT_BR_PIPES other than 0 asks
+ *  for the second at any count, and GROUP, WINDOW and POOL do not apply)
  *  FHEACC_OPT_BR_WINDOW     : 64-bit words: steps per bucket of the step
  *                             window that keeps the CTAs of a launch within
  *                             two buckets of each other, so that the key tiles
@@ -286,10 +290,10 @@ int fheacc_lwe_modswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t cou
  *                             FHEACC_STATUS_WAIT_LIMIT is set and
  *                             fheacc_sync / fheacc_bootstrap return
  *                             FHEACC_EIO. Set it back to -1 afterwards.
- * Results never depend on the other options. The 64-bit blind rotation is a
- * cooperative launch whenever its CTAs wait on each other (the remainder
- * pool, the step window), so a grid that cannot be co-resident fails to
- * launch rather than waiting. */
+ * Results never depend on the other options. The 64-bit blind rotation of
+ * other moduli is a cooperative launch whenever its CTAs wait on each other
+ * (the remainder pool, the step window), so a grid that cannot be co-resident
+ * fails to launch rather than waiting. */
 #define FHEACC_OPT_BR_REGS_FOR_3  1
 #define FHEACC_OPT_BR_CTAS_PER_SM 2
 #define FHEACC_OPT_BR_GROUP       3

@@ -16,7 +16,7 @@ def host(t):
     return t.cpu().numpy().view(np.uint64)
 
 
-@pytest.mark.parametrize("nbit,bg", [(47, 9), (50, 9), (53, 27), (54, 9), (54, 27), (55, 9), (57, 9)])
+@pytest.mark.parametrize("nbit,bg", [(47, 9), (50, 9), (53, 27), (54, 7), (54, 9), (54, 27), (55, 9), (57, 9)])
 def test_moduli_vs_oracle(F, cuda_ok, nbit, bg):
     torch = cuda_ok
     from oracle_lib import Oracle
@@ -77,3 +77,41 @@ def test_moduli_vs_oracle(F, cuda_ok, nbit, bg):
             got = ctx.eval_bootstrap_batch(c1, c2, g[:count])
             want, failed = o.eval_bootstrap_batch(c1, c2, g[:count], bt, ks)
             assert failed == 0 and np.array_equal(got, want), count
+
+
+@pytest.fixture(scope="module")
+def small_wide(F, cuda_ok):
+    P = F.params_preset(1)
+    P.n = 5
+    F.derive(P)
+    lsk, rsk = F.LWE_secretkey(P, 1), F.RLWE_secretkey(P, 2)
+    with F.Context(P, 0) as ctx:
+        ctx.upload_bootstrap_key(F.bootstrap_key(P, 3, lsk, rsk))
+        ctx.upload_keyswitch_key(F.keyswitch_key(P, 4, rsk, lsk))
+        yield P, ctx, lsk
+
+
+@pytest.mark.parametrize("count", [1, 8, 17, 18, 19, 38, 39, 76, 77, 152, 153, 305])
+def test_forms_agree(F, cuda_ok, small_wide, count):
+    """The latency form's cluster sizes at the edges of their ranges against the
+    items form: accumulators and outputs, in the three issue orders."""
+    torch = cuda_ok
+    P, ctx, lsk = small_wide
+    rng = np.random.default_rng(count)
+    ct = F.LWE_encrypt(P, 40 + count, lsk, rng.integers(0, 2, 2 * count, dtype=np.uint8))
+    d1, d2 = dev(torch, ct[:count]), dev(torch, ct[count:])
+    dg = torch.from_numpy(rng.integers(0, 6, count).astype(np.int32)).cuda()
+    for flags in (0, F.FLAG_FPGA_COMPAT, F.FLAG_FPGA_X1):
+        got = []
+        for pipes in (0, 2):
+            ctx.set_option(F.OPT_BR_PIPES, pipes)
+            try:
+                acc = torch.zeros((count, 2 * P.N), dtype=torch.int64, device="cuda")
+                out = torch.zeros_like(d1)
+                ctx.blind_rotate_async(d1.data_ptr(), d2.data_ptr(), dg.data_ptr(), count, acc.data_ptr(), flags)
+                ctx.bootstrap_async(d1.data_ptr(), d2.data_ptr(), dg.data_ptr(), count, out.data_ptr(), flags)
+                ctx.sync()
+            finally:
+                ctx.set_option(F.OPT_BR_PIPES, 0)
+            got.append((acc, out))
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
