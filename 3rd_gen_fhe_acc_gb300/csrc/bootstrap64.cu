@@ -618,32 +618,57 @@ __global__ void __launch_bounds__(512) lwe_ks64_kernel(const __grid_constant__ K
     }
 }
 
-// Split form for a few ciphertexts (a lone gate's key switch would otherwise
-// run on one CTA): CTA (ci, slice) sums rows [slice * per, ...) of
-// ciphertext ci (per <= fold rows, so its 64-bit sums cannot overflow),
-// reduces them mod Q and adds them into part[ci][ks_row] (zeroed before;
-// slices * Q < 2^64); ks64_final_kernel reduces and writes the outputs.
+// Split form: CTA (slice, ci) sums rows [slice * per, ...) of ciphertext ci (per <=
+// fold <= 256 rows, so its 64-bit sums cannot overflow), reduces them mod Q and adds
+// them into part[ci][ks_row] (zeroed before; slices * Q < 2^64); ks64_final_kernel
+// reduces and writes the outputs. The slice is the slow index of the grid: the
+// ciphertexts' CTAs of one slice run together, and the slice's rows (33 MB of the
+// 3.1 GB key for 256 rows) come from L2 after the first read. The digits of the
+// CTA's rows are computed once into shared memory (magic: ks64_digit_magic, or 0:
+// divisions); computed by every thread for every row, with up to 11 divisions each,
+// they were the kernel's time (100 gates, n = 630: 13.0 ms, now 1.07).
+constexpr int kKs64MaxFold = 256;
+
 __global__ void __launch_bounds__(512) ks64_partial_kernel(const __grid_constant__ Ks64Args A,
-                                                           unsigned long long *part, int slices)
+                                                           unsigned long long *part, int slices, uint64_t magic)
 {
+    __shared__ uint8_t dig[kKs64MaxFold];
     const int N = A.N, D = A.digitKS, t = threadIdx.x;
     const uint64_t Q = A.Q;
     const size_t rs2 = A.ks_row / 2;
-    const ulonglong2 *key2 = reinterpret_cast<const ulonglong2 *>(A.kskey);
+    const ulonglong2 *key2 = reinterpret_cast<const ulonglong2 *>(A.kskey) + t;
     const int total = N * D, per = (total + slices - 1) / slices;
-    const size_t ci = blockIdx.x / slices;
-    const int r0 = (int)(blockIdx.x % slices) * per, r1 = min(total, r0 + per);
-    if (ci >= A.count) return;
+    const size_t ci = blockIdx.x % A.count;
+    const int r0 = (int)(blockIdx.x / A.count) * per, r1 = min(total, r0 + per);
     const uint64_t *ext = A.ext + ci * kExtract64;
-    uint64_t s0 = 0, s1 = 0;
-    for (int r = r0; r < r1; r++) {
-        const int i = r / D, j = r - i * D;
+    for (int i = r0 / D + t; i * D < r1; i += blockDim.x) {
         uint64_t a = ext[i];
-        for (int jj = 0; jj < j; jj++) a /= A.Bks;
-        const uint32_t d = (uint32_t)(a % A.Bks);
-        const ulonglong2 v = __ldg(key2 + ((size_t)(d * D + j) * N + i) * rs2 + t);
-        s0 += v.x;
-        s1 += v.y;
+        for (int j = 0; j < D; j++) {
+            const uint64_t qt = magic ? __umul64hi(a, magic) : a / A.Bks;
+            const int r = i * D + j;
+            if (r >= r0 && r < r1) dig[r - r0] = (uint8_t)(a - qt * A.Bks);
+            a = qt;
+        }
+    }
+    __syncthreads();
+    uint64_t s0 = 0, s1 = 0;
+    int i = r0 / D, j = r0 - i * D;
+    for (int r = r0; r < r1; r += kKs64Unroll) {
+        ulonglong2 v[kKs64Unroll];
+#pragma unroll
+        for (int u = 0; u < kKs64Unroll; u++) {
+            v[u] = make_ulonglong2(0, 0);
+            if (r + u < r1) v[u] = __ldg(key2 + ((size_t)(dig[r + u - r0] * D + j) * N + i) * rs2);
+            if (++j == D) {
+                j = 0;
+                ++i;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kKs64Unroll; u++) {
+            s0 += v[u].x;
+            s1 += v[u].y;
+        }
     }
     unsigned long long *p = part + ci * A.ks_row + 2 * (size_t)t;
     atomicAdd(p + 0, (unsigned long long)(s0 % Q));
@@ -920,26 +945,27 @@ int launch_lwe_keyswitch64(Context &c, const uint64_t *d_extract, size_t count, 
     A.n = c.p.n; A.N = c.p.N; A.digitKS = (int)c.p.digitKS; A.Bks = c.p.Bks; A.ks_row = c.dp.ks_row;
     A.q = c.p.q; A.modswitch = modswitch ? 1u : 0u; A.Q = c.p.Q;
     // key words are < Q: (fold + 1) Q must stay below 2^64
-    const uint64_t fold = std::min<uint64_t>(256, UINT64_MAX / c.p.Q - 1);
+    const uint64_t fold = std::min<uint64_t>(dev::kKs64MaxFold, UINT64_MAX / c.p.Q - 1);
     A.fold = (int)std::max<uint64_t>(8, fold & ~(uint64_t)7);
     const unsigned threads = c.dp.ks_row / 2;   // ks_row: a multiple of 32 words, > n
     const size_t sms = (size_t)sms_of(c);
-    // from two gates per SM: the tiled form (lwe_ks.cu), each row group read
-    // from L2 once per gate block
+    // large batches: the tiled form (lwe_ks.cu), each row group read from L2 once per
+    // gate block
     if (d_scratch && ks64_tiled_applies(c, count, (int)sms, scratch_bytes))
         return launch_ks64_tiled(c, d_extract, count, modswitch, d_out, d_out_idx, d_scratch, (int)sms, st);
-    // a few ciphertexts: each one's rows split over many CTAs, with at most
-    // `fold` rows per CTA and slices * Q < 2^64
+    // below that each ciphertext's rows are split over CTAs (ks_tiled = 0: only below two
+    // ciphertexts per SM), with at most `fold` rows per CTA and slices * Q < 2^64
     const int rows = c.p.N * (int)c.p.digitKS;
     const size_t max_slices = std::min<uint64_t>(UINT64_MAX / c.p.Q, 4096);
     const size_t slices = std::min<size_t>(max_slices, std::max<size_t>((size_t)(rows + A.fold - 1) / A.fold,
                                                                          sms * 8 / std::max<size_t>(count, 1)));
-    if (d_scratch && count < 2 * sms && count * c.dp.ks_row * sizeof(uint64_t) <= scratch_bytes &&
+    if (d_scratch && !(c.tune.ks_tiled == 0 && count >= 2 * sms) && count * c.dp.ks_row * sizeof(uint64_t) <= scratch_bytes &&
         (size_t)(rows + slices - 1) / slices <= (size_t)A.fold) {
         unsigned long long *part = reinterpret_cast<unsigned long long *>(d_scratch);
         cudaError_t e = cudaMemsetAsync(part, 0, count * c.dp.ks_row * sizeof(uint64_t), st);
         if (e != cudaSuccess) return c.cuda_fail(e, "key switch partials reset");
-        dev::ks64_partial_kernel<<<(unsigned)(count * slices), threads, 0, st>>>(A, part, (int)slices);
+        dev::ks64_partial_kernel<<<(unsigned)(count * slices), threads, 0, st>>>(A, part, (int)slices,
+                                                                                       ks64_digit_magic(c));
         c.launches++;
         e = cudaGetLastError();
         if (e != cudaSuccess) return c.cuda_fail(e, "key switch partial launch");

@@ -213,8 +213,12 @@ int launch_lwe_keyswitch32_indexed(Context &c, const uint32_t *d_extract, size_t
 int launch_lwe_keyswitch32(Context &c, const uint32_t *d_extract, size_t count, bool modswitch, uint64_t *d_out,
                            cudaStream_t st, void *d_scratch = nullptr, size_t scratch_bytes = 0,
                            const uint32_t *d_out_idx = nullptr);
-// Batches from this many gates take the tiled key switch.
-constexpr size_t kKsTiledMinGates = 1024;
+// Batches from this many gates per SM take the tiled key switch, smaller ones the
+// split form, whose time grows with the gates (one GB300: 1.1 us a gate for 32-bit
+// words, 7.8 us for 64-bit ones: the rows' bytes from L2 at 11 and 16 TB/s) where the
+// tiled form's grows slowly: 2000 gates 2.20 ms split, 2.59 tiled, 4096 gates 2.92 ms
+// tiled; 64-bit 1000 gates 7.8 split, 10.4 tiled, 2048 gates 14.5 ms tiled.
+constexpr size_t kKsTiledGatesPerSm = 16, kKs64TiledGatesPerSm = 11;
 int launch_extract_from_ntt32(Context &c, const uint64_t *d_rlwe, size_t count, uint32_t *d_extract,
                               cudaStream_t st);
 int launch_modswitch(Context &c, const uint64_t *d_in, size_t count, uint64_t *d_out, cudaStream_t st);
@@ -239,6 +243,8 @@ int launch_blind_rotate64_with(Context &c, const uint64_t *d_c1, const uint64_t 
 int launch_extract64(Context &c, const uint64_t *d_rlwe, size_t count, uint64_t *d_extract, cudaStream_t st);
 // Tiled 64-bit LWE key switch (lwe_ks.cu): whether it applies to `count` gates
 // with `scratch_bytes` of scratch for the digits, and the launch.
+// ceil(2^64 / Bks), the digits' quotient multiplier (0: not exact for every word below Q).
+uint64_t ks64_digit_magic(const Context &c);
 bool ks64_tiled_applies(const Context &c, size_t count, int sms, size_t scratch_bytes);
 int launch_ks64_tiled(Context &c, const uint64_t *d_extract, size_t count, bool modswitch, uint64_t *d_out,
                       const uint32_t *d_out_idx, void *scratch, int sms, cudaStream_t st);

@@ -11,8 +11,8 @@
 // b[0]). For every coefficient i < N and digit j < digitKS the LWE row
 // kskey[d][j][i], d = base-Bks digit j of a[i], is subtracted.
 //
-// Batches of 1024 gates and more take the tiled form (lwe_ks32_tiled_kernel;
-// 64-bit words from two gates per SM, lwe_ks64_tiled_kernel):
+// Large batches take the tiled form (kKsTiledGatesPerSm; lwe_ks32_tiled_kernel and
+// lwe_ks64_tiled_kernel):
 // ks_digits_kernel first writes every gate's digits gate-minor,
 // [(i * digitKS + j)][gate]; then a CTA takes a block of gates and a 512-byte
 // slice of the key rows and walks the N * digitKS row groups (the
@@ -23,10 +23,9 @@
 // 315 MB key 32 times instead of 4096), and because every CTA walks the groups
 // in the same order the key streams from HBM about once.
 //
-// Smaller batches: one CTA per ciphertext, the digits computed once into
-// shared memory, then the CTA walks the N * digitKS rows; a row is n+1
-// consecutive words, read by consecutive threads (coalesced). Below two gates
-// per SM each gate's rows are split over many CTAs (ks_partial_kernel).
+// Smaller batches split each gate's rows over several CTAs (ks_partial_kernel); a
+// row is n+1 consecutive words, read by consecutive threads (coalesced). Without
+// scratch: one CTA per ciphertext (lwe_ks32_kernel).
 // Sums are kept in 64-bit registers without reduction (N * digitKS * Q <
 // 2^64) and reduced once at the end; the modulus switch is fused into the
 // same epilogue.
@@ -123,32 +122,52 @@ __global__ void __launch_bounds__(kKsMaxThreads) lwe_ks32_kernel(const __grid_co
     }
 }
 
-// Split form for a few ciphertexts (the one-gate launches): CTA (ci, slice)
-// sums rows [slice * rows_per, ...) of ciphertext ci and adds its 64-bit
-// partial sums into part[ci][ks_row] (zeroed before; the sums stay below
-// N * digitKS * Q < 2^64); ks_final_kernel reduces them.
+// Split form: CTA (slice, ci) sums rows [slice * per, ...) of ciphertext ci and adds
+// its 64-bit partial sums into part[ci][ks_row] (zeroed before; the sums stay below
+// N * digitKS * Q < 2^64); ks_final_kernel reduces them. The slice is the slow index of
+// the grid (the ciphertexts' CTAs of one slice read its rows together, from L2), and
+// the CTA's digits are computed once into shared memory: computed by every thread for
+// every row, with up to digitKS - 1 divisions each, 96 gates took 0.42 ms.
 __global__ void __launch_bounds__(kKsMaxThreads) ks_partial_kernel(const __grid_constant__ KsArgs A,
                                                                    unsigned long long *part, int slices)
 {
+    extern __shared__ uint8_t dig[];   // [per]
     const int N = A.N, D = A.digitKS, t = threadIdx.x;
     const size_t rs4 = A.ks_row / 4;
-    const uint4 *key4 = reinterpret_cast<const uint4 *>(A.kskey);
+    const uint4 *key4 = reinterpret_cast<const uint4 *>(A.kskey) + t;
     const int total = N * D, per = (total + slices - 1) / slices;
-    const size_t ci = blockIdx.x / slices;
-    const int r0 = (int)(blockIdx.x % slices) * per, r1 = min(total, r0 + per);
-    if (ci >= A.count) return;
+    const size_t ci = blockIdx.x % A.count;
+    const int r0 = (int)(blockIdx.x / A.count) * per, r1 = min(total, r0 + per);
     const uint32_t *ext = A.ext + ci * kExtractStride;
-    uint64_t s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    for (int r = r0; r < r1; r++) {
-        const int i = r / D, j = r - i * D;
+    for (int i = r0 / D + t; i * D < r1; i += blockDim.x) {
         uint32_t a = ext[i];
-        for (int jj = 0; jj < j; jj++) a /= A.Bks;
-        const uint32_t d = a % A.Bks;
-        const uint4 v = __ldg(key4 + ((size_t)(d * D + j) * N + i) * rs4 + t);
-        s0 += v.x;
-        s1 += v.y;
-        s2 += v.z;
-        s3 += v.w;
+        for (int j = 0; j < D; j++) {
+            const int r = i * D + j;
+            if (r >= r0 && r < r1) dig[r - r0] = (uint8_t)(a % A.Bks);
+            a /= A.Bks;
+        }
+    }
+    __syncthreads();
+    uint64_t s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+    int i = r0 / D, j = r0 - i * D;
+    for (int r = r0; r < r1; r += kKsUnroll) {
+        uint4 v[kKsUnroll];
+#pragma unroll
+        for (int u = 0; u < kKsUnroll; u++) {
+            v[u] = make_uint4(0, 0, 0, 0);
+            if (r + u < r1) v[u] = __ldg(key4 + ((size_t)(dig[r + u - r0] * D + j) * N + i) * rs4);
+            if (++j == D) {
+                j = 0;
+                ++i;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kKsUnroll; u++) {
+            s0 += v[u].x;
+            s1 += v[u].y;
+            s2 += v[u].z;
+            s3 += v[u].w;
+        }
     }
     unsigned long long *p = part + ci * A.ks_row + 4 * (size_t)t;
     atomicAdd(p + 0, (unsigned long long)s0);
@@ -521,7 +540,7 @@ static bool ks_tiled_applies(const Context &c, size_t count, int sms, size_t scr
         return false;
     if (ks_tiled_digit_bytes(c, count, sms) > scratch_bytes) return false;
     if (c.tune.ks_tiled > 0) return true;
-    return count >= kKsTiledMinGates;
+    return count >= kKsTiledGatesPerSm * (size_t)sms;
 }
 
 static int launch_ks_tiled(Context &c, const dev::KsArgs &A, void *scratch, int sms, cudaStream_t st)
@@ -570,7 +589,7 @@ static int ks64_tiled_gw(size_t count, int sms, int slices)
 
 // ceil(2^64 / Bks), the digits kernel's quotient multiplier; 0 if its
 // quotients are not exact for every word below Q.
-static uint64_t ks64_digit_magic(const Context &c)
+uint64_t ks64_digit_magic(const Context &c)
 {
     const uint64_t B = c.p.Bks;
     if (B < 2) return 0;
@@ -591,7 +610,7 @@ bool ks64_tiled_applies(const Context &c, size_t count, int sms, size_t scratch_
     const size_t G = (size_t)dev::kKsTileWarps * ks64_tiled_gw(count, sms, slices);
     if ((count + G - 1) / G * G * (size_t)c.p.N * c.p.digitKS > scratch_bytes) return false;
     if (c.tune.ks_tiled > 0) return true;
-    return count >= 2 * (size_t)sms;
+    return count >= kKs64TiledGatesPerSm * (size_t)sms;
 }
 
 // Runs the tiled 64-bit key switch (ks64_tiled_applies must hold): the digits
@@ -655,16 +674,20 @@ int launch_lwe_keyswitch32(Context &c, const uint32_t *d_extract, size_t count, 
     A.n = c.p.n; A.N = c.p.N; A.digitKS = (int)c.p.digitKS; A.Bks = c.p.Bks; A.ks_row = c.dp.ks_row;
     A.q = c.p.q; A.modswitch = modswitch ? 1u : 0u; A.Q = c.p.Q;
     if (d_scratch && ks_tiled_applies(c, count, sms, scratch_bytes)) return launch_ks_tiled(c, A, d_scratch, sms, st);
-    // a few ciphertexts: split each one's rows over many CTAs
-    if (!d_scratch || count >= 2 * (size_t)sms || count * c.dp.ks_row * sizeof(uint64_t) > scratch_bytes)
+    // below that each ciphertext's rows are split over CTAs (ks_tiled = 0: only below two
+    // ciphertexts per SM)
+    if (!d_scratch || (c.tune.ks_tiled == 0 && count >= 2 * (size_t)sms) ||
+        count * c.dp.ks_row * sizeof(uint64_t) > scratch_bytes)
         return launch_lwe_keyswitch32_indexed(c, d_extract, count, modswitch, d_out, d_out_idx, st);
     uint64_t *d_partials = (uint64_t *)d_scratch;
     const int rows = c.p.N * (int)c.p.digitKS;
-    // about 8 CTAs per SM, at least 48 rows each
-    const int slices = (int)std::max<size_t>(1, std::min<size_t>((size_t)rows / 48, (size_t)sms * 8 / count));
+    // 32 CTAs (of 4 warps) per SM, at least 8 per ciphertext, at least 48 rows each
+    // (1000 gates: 1.14 ms; 8 per SM 1.73, 16 per SM 1.29, 64 per SM 1.13)
+    const int slices = (int)std::max<size_t>(
+        1, std::min<size_t>((size_t)rows / 48, std::max<size_t>(8, (size_t)sms * 32 / count)));
     cudaError_t e = cudaMemsetAsync(d_partials, 0, count * c.dp.ks_row * sizeof(uint64_t), st);
     if (e != cudaSuccess) return c.cuda_fail(e, "key switch partials reset");
-    dev::ks_partial_kernel<<<(unsigned)(count * slices), c.dp.ks_row / 4, 0, st>>>(
+    dev::ks_partial_kernel<<<(unsigned)(count * slices), c.dp.ks_row / 4, (size_t)(rows + slices - 1) / slices, st>>>(
         A, reinterpret_cast<unsigned long long *>(d_partials), slices);
     c.launches++;
     e = cudaGetLastError();

@@ -268,9 +268,10 @@ int fheacc_lwe_modswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t cou
  *  FHEACC_OPT_KS_TILED      : LWE key switch of a batched bootstrap:
  *                             1 = the tiled form (gate blocks sharing each
  *                             key row group through shared memory) for any
- *                             batch, 0 = one CTA per gate, -1 (default) =
- *                             tiled from 1024 gates (32-bit words) or from
- *                             two gates per SM (64-bit words)
+ *                             batch, 0 = one CTA per gate (several below two
+ *                             gates per SM), -1 (default) = tiled from 16
+ *                             (32-bit words) or 11 (64-bit) gates per SM,
+ *                             several CTAs per gate below
  *  FHEACC_OPT_BR_SOLO       : 32-bit words: the latency form of the blind
  *                             rotation (one CTA per ciphertext, accumulator in
  *                             shared memory, each step's key prefetched into
