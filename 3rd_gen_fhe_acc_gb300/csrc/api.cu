@@ -228,6 +228,13 @@ int build_tables(Context &c)
     if (e == cudaSuccess) e = cudaMalloc(&c.d_inv_tw, N * sizeof(uint2));
     if (e == cudaSuccess) e = cudaMemcpy(c.d_fwd_tw, fw.data(), N * sizeof(uint2), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(c.d_inv_tw, iw.data(), N * sizeof(uint2), cudaMemcpyHostToDevice);
+    std::vector<uint2> plain(2 * N);
+    for (int i = 0; i < N; i++) {
+        plain[i] = make_uint2((uint32_t)T.rou[i], shoup32_companion(T.rou[i], Q));
+        plain[N + i] = make_uint2((uint32_t)T.irou[i], shoup32_companion(T.irou[i], Q));
+    }
+    if (e == cudaSuccess) e = cudaMalloc(&c.d_plain_tw, 2 * N * sizeof(uint2));
+    if (e == cudaSuccess) e = cudaMemcpy(c.d_plain_tw, plain.data(), 2 * N * sizeof(uint2), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return c.cuda_fail(e, "twiddle upload");
     dev::Ntt32Consts &k = c.nc;
     std::memset(&k, 0, sizeof k);
@@ -393,6 +400,7 @@ int fheacc_destroy(fheacc_ctx *ctx)
     if (c->stream) cudaStreamSynchronize(c->stream);
     cudaFree(c->d_fwd_tw);
     cudaFree(c->d_inv_tw);
+    cudaFree(c->d_plain_tw);
     cudaFree(c->d_tw64);
     cudaFree(c->d_itw64);
     cudaFree(c->d_btkey64);

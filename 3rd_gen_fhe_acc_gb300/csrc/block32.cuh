@@ -1,0 +1,387 @@
+// block32.cuh -- latency form of the 32-bit blind rotation: one ciphertext per
+// cluster of C CTAs (included by blind_rotate32.cu, whose prologue, epilogue and
+// arithmetic it shares: outputs are identical word for word).
+//
+// With a gate or two per SM the pipelines have nothing to overlap: a lone
+// ciphertext's steps are a serial chain, and a transform on one warp takes longer
+// than all of a step's multiplications spread over the SM. X^1024 + 1 splits into
+// four factors X^256 - zeta: the 256-word blocks of the bit-reversed NTTs depend on
+// the polynomial only through its residue mod X^256 - zeta, so every transform is cut
+// into four 256-word transforms of one warp each (8 words a lane), and a CTA of the
+// cluster owns 4 / C blocks of the accumulator, the digit NTTs and the key rows:
+//   1. 2 * 4 / C warps: the inverse stages t = 1 .. 128 of a block of the accumulator
+//      (closed in the block), written to every CTA's shared memory; one cluster
+//      barrier per step;
+//   2. 512 threads: the stages t = 256, 512 of one tuple (x_j, x_{j+256}, ..) in
+//      registers, the canonical coefficients' digits and the first two forward stages
+//      of each digit, of which the CTA keeps its blocks' words;
+//   3. a warp per digit and block: forward stages t = 128 .. 1;
+//   4. multiply-accumulate of the CTA's words, keys from shared memory (copied
+//      a step ahead with cp.async, by the warps that have no part in 1).
+// One GB300, per step: 2.0 us on 4 CTAs, 2.5 on 2, 3.4 on one; a CTA of 8 warps with one
+// transform each took 3.8 (one gate) to 4.3 (152). On 4 CTAs a step is 4160 cycles: 830
+// for 1 (two warps, a chain of eight stages), 685 for the cluster barrier, 865 for 2
+// (every CTA does the last inverse stages of all words), 955 for 3 and 440 for 4.
+// Three CTA barriers and one cluster barrier per step; the transforms' own exchanges
+// stay inside a warp. Residues, accumulator, twiddles and keys live in shared memory
+// for the whole bootstrap.
+#pragma once
+
+namespace fheacc {
+namespace dev {
+
+constexpr int kB32 = 256, kB32E = 256 + 32;   // words of a block, with 4 words of padding after every 32
+
+// Padded position of word e of a block: the passes' accesses (32 consecutive words;
+// words grp * 32 + j + 4 k for j < 4; four consecutive words) fall on distinct banks.
+__device__ __forceinline__ constexpr int p4(int e) { return e + ((e >> 5) << 2); }
+
+template <int DG, int C>
+struct Block32Layout {
+    static constexpr int NB = 4 / C, ND = 2 * (DG - 1);
+    static constexpr int T = C == 1 ? 768 : 512;   // threads: 24 digit blocks (digitG = 4), or the 512 tuples
+    static constexpr size_t g_off = 0;                                             // [C > 1 ? 2 : 1][2][1024]
+    static constexpr size_t acc_off = (C > 1 ? 2 : 1) * 2 * kN32 * 4;              // [2 buffers][2][NB][kB32E]
+    static constexpr size_t d_off = acc_off + (size_t)2 * 2 * NB * kB32E * 4;      // [ND][NB][kB32E], or [2][NB][kB32E]
+    static constexpr size_t key_off = d_off + (size_t)ND * NB * kB32E * 4;         // [2][DG * 4][NB * 256]
+    static constexpr size_t key_words = (size_t)DG * 4 * NB * kB32;
+    static constexpr size_t tw_off = key_off + 2 * key_words * 4;                  // [fwd, inv][1024] (w, w')
+    static constexpr size_t res_off = tw_off + 2 * kN32 * sizeof(uint2);
+    static size_t bytes(size_t steps) { return res_off + (steps + 15) / 16 * 16; }
+};
+
+__device__ __forceinline__ void cp_async16_32(void *smem, const void *gmem)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
+}
+
+// E = 1, 2 or 4 consecutive words in one shared-memory access.
+template <int E>
+__device__ __forceinline__ void load_words(uint32_t (&v)[E], const uint32_t *p)
+{
+    if constexpr (E == 4) {
+        const uint4 x = *reinterpret_cast<const uint4 *>(p);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    } else if constexpr (E == 2) {
+        const uint2 x = *reinterpret_cast<const uint2 *>(p);
+        v[0] = x.x; v[1] = x.y;
+    } else {
+        v[0] = *p;
+    }
+}
+template <int E>
+__device__ __forceinline__ void store_words(uint32_t *p, const uint32_t (&v)[E])
+{
+    if constexpr (E == 4) *reinterpret_cast<uint4 *>(p) = make_uint4(v[0], v[1], v[2], v[3]);
+    else if constexpr (E == 2) *reinterpret_cast<uint2 *>(p) = make_uint2(v[0], v[1]);
+    else *p = v[0];
+}
+
+// Forward stages t = 128 .. 1 of block b (of four) at d by one warp.
+__device__ __forceinline__ void block32_fwd(uint32_t *d, int b, int lane, const Ntt32Consts &c, const uint2 *ftw)
+{
+    const uint32_t Q = c.Q, twoQ = c.twoQ;
+    {
+        uint32_t x[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) x[k] = d[lane + 36 * k];
+#pragma unroll
+        for (int st = 0; st < 3; st++)
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                if (!(k & (4 >> st))) {
+                    const int i = (4 << st) + (b << st) + (k >> (3 - st));
+                    ct_bfly(x[k], x[k + (4 >> st)], c.fw[i], c.fws[i], Q, twoQ);
+                }
+#pragma unroll
+        for (int k = 0; k < 8; k++) d[lane + 36 * k] = x[k];
+    }
+    __syncwarp();
+    {
+        const int grp = lane >> 2, G = 8 * b + grp;
+        uint32_t *const p = d + grp * 36 + (lane & 3);
+        uint32_t x[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) x[k] = p[4 * k];
+        const uint2 w0 = ftw[32 + G];
+        const uint4 w1 = *reinterpret_cast<const uint4 *>(ftw + 64 + 2 * G);
+        const uint4 w2 = *reinterpret_cast<const uint4 *>(ftw + 128 + 4 * G);
+        const uint4 w3 = *reinterpret_cast<const uint4 *>(ftw + 130 + 4 * G);
+#pragma unroll
+        for (int k = 0; k < 4; k++) ct_bfly(x[k], x[k + 4], w0.x, w0.y, Q, twoQ);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            ct_bfly(x[k], x[k + 2], w1.x, w1.y, Q, twoQ);
+            ct_bfly(x[k + 4], x[k + 6], w1.z, w1.w, Q, twoQ);
+        }
+        ct_bfly(x[0], x[1], w2.x, w2.y, Q, twoQ);
+        ct_bfly(x[2], x[3], w2.z, w2.w, Q, twoQ);
+        ct_bfly(x[4], x[5], w3.x, w3.y, Q, twoQ);
+        ct_bfly(x[6], x[7], w3.z, w3.w, Q, twoQ);
+#pragma unroll
+        for (int k = 0; k < 8; k++) p[4 * k] = x[k];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int q = lane + 32 * i, P = 64 * b + q;
+        uint4 *const p = reinterpret_cast<uint4 *>(d + p4(4 * q));
+        uint4 v = *p;
+        const uint2 w0 = ftw[256 + P];
+        const uint4 w1 = *reinterpret_cast<const uint4 *>(ftw + 512 + 2 * P);
+        ct_bfly(v.x, v.z, w0.x, w0.y, Q, twoQ);
+        ct_bfly(v.y, v.w, w0.x, w0.y, Q, twoQ);
+        ct_bfly(v.x, v.y, w1.x, w1.y, Q, twoQ);
+        ct_bfly(v.z, v.w, w1.z, w1.w, Q, twoQ);
+        *p = v;
+    }
+}
+
+// Inverse stages t = 1 .. 128 of block b at src (values < 2Q) by one warp; w: scratch
+// of kB32E words; out(k, x): word lane + 32 k of the block, < 2Q.
+template <class Out>
+__device__ __forceinline__ void block32_inv(const uint32_t *src, uint32_t *w, int b, int lane, const Ntt32Consts &c,
+                                            const uint2 *itw, Out out)
+{
+    const uint32_t Q = c.Q, twoQ = c.twoQ;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int q = lane + 32 * i, P = 64 * b + q;
+        uint4 v = *reinterpret_cast<const uint4 *>(src + p4(4 * q));
+        const uint4 w1 = *reinterpret_cast<const uint4 *>(itw + 512 + 2 * P);
+        const uint2 w0 = itw[256 + P];
+        gs_bfly(v.x, v.y, w1.x, w1.y, Q, twoQ);
+        gs_bfly(v.z, v.w, w1.z, w1.w, Q, twoQ);
+        gs_bfly(v.x, v.z, w0.x, w0.y, Q, twoQ);
+        gs_bfly(v.y, v.w, w0.x, w0.y, Q, twoQ);
+        *reinterpret_cast<uint4 *>(w + p4(4 * q)) = v;
+    }
+    __syncwarp();
+    {
+        const int grp = lane >> 2, G = 8 * b + grp;
+        uint32_t *const p = w + grp * 36 + (lane & 3);
+        uint32_t x[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) x[k] = p[4 * k];
+        const uint4 w2 = *reinterpret_cast<const uint4 *>(itw + 128 + 4 * G);
+        const uint4 w3 = *reinterpret_cast<const uint4 *>(itw + 130 + 4 * G);
+        const uint4 w1 = *reinterpret_cast<const uint4 *>(itw + 64 + 2 * G);
+        const uint2 w0 = itw[32 + G];
+        gs_bfly(x[0], x[1], w2.x, w2.y, Q, twoQ);
+        gs_bfly(x[2], x[3], w2.z, w2.w, Q, twoQ);
+        gs_bfly(x[4], x[5], w3.x, w3.y, Q, twoQ);
+        gs_bfly(x[6], x[7], w3.z, w3.w, Q, twoQ);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            gs_bfly(x[k], x[k + 2], w1.x, w1.y, Q, twoQ);
+            gs_bfly(x[k + 4], x[k + 6], w1.z, w1.w, Q, twoQ);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) gs_bfly(x[k], x[k + 4], w0.x, w0.y, Q, twoQ);
+#pragma unroll
+        for (int k = 0; k < 8; k++) p[4 * k] = x[k];
+    }
+    __syncwarp();
+    uint32_t x[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) x[k] = w[lane + 36 * k];
+#pragma unroll
+    for (int st = 0; st < 3; st++)
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (!(k & (1 << st))) {
+                const int i = (16 >> st) + (b << (2 - st)) + (k >> (st + 1));
+                gs_bfly(x[k], x[k + (1 << st)], c.iw[i], c.iws[i], Q, twoQ);
+            }
+#pragma unroll
+    for (int k = 0; k < 8; k++) out(k, x[k]);
+}
+
+template <int DG, int C>
+__global__ void __launch_bounds__(Block32Layout<DG, C>::T, 1)
+    br32_block_kernel(const __grid_constant__ PipeArgs A, const __grid_constant__ Ntt32Consts c,
+                      const uint2 *__restrict__ fwd_tw, const uint2 *__restrict__ inv_tw,
+                      const uint2 *__restrict__ plain_tw, uint32_t mu32)
+{
+    using L = Block32Layout<DG, C>;
+    constexpr int NB = L::NB, ND = L::ND, T = L::T, NW = T / 32;
+    constexpr int FW = ND * NB < NW ? ND * NB : 0;   // warps with a block in 3 (0: no other warp)
+    extern __shared__ __align__(16) unsigned char blk_smem[];
+    uint32_t *const g = reinterpret_cast<uint32_t *>(blk_smem + L::g_off);
+    uint32_t *const acc = reinterpret_cast<uint32_t *>(blk_smem + L::acc_off);
+    uint32_t *const dbuf = reinterpret_cast<uint32_t *>(blk_smem + L::d_off);
+    uint32_t *const keys = reinterpret_cast<uint32_t *>(blk_smem + L::key_off);
+    uint2 *const ftw = reinterpret_cast<uint2 *>(blk_smem + L::tw_off), *const itw = ftw + kN32;
+    uint8_t *const res = blk_smem + L::res_off;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = C > 1 ? (int)(blockIdx.x % C) : 0;
+    const int S = A.n * (int)A.digitR, mode = issue_mode(A.flags);
+    const uint32_t Q = c.Q, twoQ = c.twoQ, fourQ = 2 * twoQ, mask = (1u << A.bg_bits) - 1;
+    uint32_t *peer[C];
+    peer[0] = g;
+    if (C > 1) {
+        cg::cluster_group cl = cg::this_cluster();
+#pragma unroll
+        for (int r = 0; r < C; r++) peer[r] = cl.map_shared_rank(g, r);
+    }
+    for (int i = tid; i < 2 * kN32; i += T) ftw[i] = __ldg(plain_tw + i);
+    if (C > 1) cg::this_cluster().sync();
+
+    // the CTA's key words of step s into buffer b: of each row, in B-tile order, the
+    // chunks q * 32 + l (words 32 l + 4 q ..) of its blocks' rows l
+    auto fetch = [&](int s, int b, int t0, int nt) {
+        if (s < S && t0 >= 0) {
+            const uint4 *src = reinterpret_cast<const uint4 *>(A.btkey + ((size_t)s * A.Br + res[s]) * ((size_t)DG * 4 * kN32));
+            uint4 *dst = reinterpret_cast<uint4 *>(keys + b * L::key_words);
+            for (int x = t0; x < DG * 4 * NB * 64; x += nt) {
+                const int row = x / (NB * 64), y = x - row * (NB * 64), q = y / (8 * NB), l = y - q * (8 * NB);
+                cp_async16_32(dst + x, src + row * 256 + q * 32 + rank * NB * 8 + l);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    for (size_t gid = blockIdx.x / C; gid < A.count; gid += gridDim.x / C) {
+        // ---- LWE_evaluate, residues and the initial accumulator (global, B-tiled; the
+        // CTAs of a cluster write the same words)
+        if (warp == 0) pipe_init_item(A, c, fwd_tw, keys, res, gid, lane, mu32);
+        __syncthreads();
+        uint32_t *const ga = A.accs + gid * 2048;
+        for (int u = tid; u < 2 * NB * 64; u += T) {
+            const int p = u / (NB * 64), cc = u - p * (NB * 64);
+            *reinterpret_cast<uint4 *>(acc + (p * NB + (cc >> 6)) * kB32E + p4(4 * (cc & 63))) = __ldcg(
+                reinterpret_cast<const uint4 *>(ga) + p * 256 + (cc & 7) * 32 + rank * NB * 8 + (cc >> 3));
+        }
+        int s = solo_next_step(res, -1, S, mode), next = s < S ? solo_next_step(res, s, S, mode) : S;
+        fetch(s, 0, tid, T);
+        __syncthreads();
+        int ab = 0;   // accumulator buffer
+        for (int kb = 0, gb = 0; s < S; kb ^= 1, ab ^= 1, gb ^= C > 1) {
+            // ---- 1. inverse stages in the blocks
+            if (warp < 2 * NB) {
+                const int p = warp / NB, lb = warp - p * NB, b = rank * NB + lb;
+                const int o = gb * 2048 + p * kN32 + b * kB32 + lane;
+                block32_inv(acc + ab * (2 * NB * kB32E) + warp * kB32E, dbuf + warp * kB32E, b, lane, c, itw, [&](int k, uint32_t v) {
+#pragma unroll
+                    for (int r = 0; r < C; r++) peer[r][o + 32 * k] = v;
+                });
+            }
+            // warps without a block here (C = 1) or in 3 start the copy of the next step's
+            // keys into the buffer that the last products have freed (copies in flight would
+            // hold up the cluster barrier's release: C = 4, 2.01 -> 2.18 us per step)
+            if (C == 1) fetch(next, kb ^ 1, tid - 64 * NB, T - 64 * NB);
+            if (C > 1) cg::this_cluster().sync();
+            else __syncthreads();
+            // ---- 2. last inverse stages, digits, first two forward stages
+            if (tid < 512) {
+                const int p = tid >> 8, j = tid & 255;
+                const uint32_t *const x = g + gb * 2048 + p * kN32 + j;
+                uint32_t x0 = x[0], x1 = x[256], x2 = x[512], x3 = x[768];
+                gs_bfly(x0, x1, c.iw[2], c.iws[2], Q, twoQ);
+                gs_bfly(x2, x3, c.iw[3], c.iws[3], Q, twoQ);
+                auto last = [&](uint32_t &a, uint32_t &b) {   // as ntt_inv_1024_noscale
+                    uint32_t u = a + b;
+                    u = min(u, u - twoQ);
+                    const uint32_t v = shoup32(a - b + twoQ, c.iw[1], c.iws[1], Q);
+                    a = min(u, u - Q);
+                    b = min(v, v - Q);
+                };
+                last(x0, x2);
+                last(x1, x3);
+                uint32_t *o = dbuf + p * (DG - 1) * NB * kB32E + p4(j);
+#pragma unroll
+                for (int h = 0; h < DG - 1; h++, o += NB * kB32E) {
+                    const uint32_t sh = A.bg_bits * h;
+                    const uint32_t y0 = (x0 >> sh) & mask, y1 = (x1 >> sh) & mask, y2 = (x2 >> sh) & mask,
+                                   y3 = (x3 >> sh) & mask;
+                    // y0 +- w1 y2 +- (w2 y1 + w2 w1 y3), and with w3, -w3 w1 for the
+                    // lower half: each < 6Q + BG
+                    const uint32_t a = shoup32(y2, c.fw[1], c.fws[1], Q);
+                    if (C == 1 || rank < C / 2) {
+                        const uint32_t u = y0 + a;
+                        const uint32_t v = shoup32(y1, c.fw[2], c.fws[2], Q) + shoup32(y3, A.w21, A.w21s, Q);
+                        if (C < 4) {
+                            o[0] = u + v;
+                            o[kB32E] = u + fourQ - v;
+                        } else {
+                            o[0] = rank == 0 ? u + v : u + fourQ - v;
+                        }
+                    }
+                    if (C == 1 || rank >= C / 2) {
+                        const uint32_t u = y0 + twoQ - a;
+                        const uint32_t v = shoup32(y1, c.fw[3], c.fws[3], Q) + shoup32(y3, A.w31n, A.w31ns, Q);
+                        uint32_t *const q = C == 1 ? o + 2 * kB32E : o;
+                        if (C < 4) {
+                            q[0] = u + v;
+                            q[kB32E] = u + fourQ - v;
+                        } else {
+                            q[0] = rank == 2 ? u + v : u + fourQ - v;
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            // ---- 3. forward stages in the blocks
+            if (C > 1) fetch(next, kb ^ 1, tid - 32 * FW, T - 32 * FW);
+            for (int w = warp; w < ND * NB; w += NW)
+                block32_fwd(dbuf + w * kB32E, rank * NB + w % NB, lane, c, ftw);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+            // ---- 4. multiply-accumulate in the keys' B-tile order (conflict-free in the
+            // blocks too): C = 1, 256 threads with 4 words of both output polys each (a
+            // digit word is read once); else 512 threads with E words of one poly
+            constexpr int PP = C == 1 ? 2 : 1;   // output polys per thread
+            if (tid < 512 / PP) {
+                constexpr int E = NB;
+                const int P = tid >> 8, v = tid & 255, ch = v * E / 4, e0 = v * E % 4;
+                const int q = ch / (8 * NB), l = ch % (8 * NB), e = 36 * (l & 7) + 4 * q + e0, lb = l >> 3;
+                const uint32_t *const a0 = acc + ab * (2 * NB * kB32E) + lb * kB32E + e;
+                const uint32_t *const d0 = dbuf + lb * kB32E + e, *ka = keys + kb * L::key_words + P * (NB * kB32) + v * E;
+                uint64_t sum[PP][E];
+#pragma unroll
+                for (int o = 0; o < PP; o++)
+#pragma unroll
+                    for (int i = 0; i < E; i++) sum[o][i] = 0;
+#pragma unroll
+                for (int h = 0; h < DG; h++)
+#pragma unroll
+                    for (int p = 0; p < 2; p++, ka += 2 * NB * kB32) {
+                        uint32_t dv[E], kv[E];
+                        load_words<E>(dv, h < DG - 1 ? d0 + (p * (DG - 1) + h) * NB * kB32E : a0 + p * NB * kB32E);
+#pragma unroll
+                        for (int o = 0; o < PP; o++) {
+                            load_words<E>(kv, ka + o * NB * kB32);
+#pragma unroll
+                            for (int i = 0; i < E; i++) sum[o][i] += (uint64_t)dv[i] * kv[i];
+                        }
+                    }
+#pragma unroll
+                for (int o = 0; o < PP; o++) {
+                    uint32_t r[E];
+#pragma unroll
+                    for (int i = 0; i < E; i++) r[i] = mont_reduce_2q(sum[o][i], Q, A.qinv_neg);
+                    store_words<E>(acc + (ab ^ 1) * (2 * NB * kB32E) + ((P + o) * NB + lb) * kB32E + e, r);
+                }
+            }
+            __syncthreads();
+            s = next;
+            next = s < S ? solo_next_step(res, s, S, mode) : S;
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        // ---- accumulator back to global memory, then the outputs of the pipelines' epilogue
+        for (int u = tid; u < 2 * NB * 64; u += T) {
+            const int p = u / (NB * 64), cc = u - p * (NB * 64);
+            __stcg(reinterpret_cast<uint4 *>(ga) + p * 256 + (cc & 7) * 32 + rank * NB * 8 + (cc >> 3),
+                   *reinterpret_cast<const uint4 *>(acc + ab * (2 * NB * kB32E) + (p * NB + (cc >> 6)) * kB32E +
+                                                      p4(4 * (cc & 63))));
+        }
+        if (C > 1) cg::this_cluster().sync();
+        else __syncthreads();
+        if (rank == 0 && warp < 2) pipe_out_poly(A, c, inv_tw, keys + warp * kN32, gid, warp, lane);
+        if (C > 1) cg::this_cluster().sync();   // the next ciphertext's accumulator words, and this CTA's exit
+        else __syncthreads();
+    }
+}
+
+}  // namespace dev
+}  // namespace fheacc

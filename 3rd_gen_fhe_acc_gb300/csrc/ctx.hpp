@@ -119,6 +119,7 @@ struct Context {
 
     // twiddles: (w, w') pairs indexed like the reference tables
     uint2 *d_fwd_tw = nullptr, *d_inv_tw = nullptr;
+    uint2 *d_plain_tw = nullptr;   // [fwd, inv][N] in reference order (32-bit latency form)
     dev::Ntt32Consts nc{};
 
     // 64-bit path: twiddles as constant pairs (mul64 in ntt64.cuh) in reference order

@@ -273,11 +273,11 @@ int fheacc_lwe_modswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t cou
  *                             (32-bit words) or 11 (64-bit) gates per SM,
  *                             several CTAs per gate below
  *  FHEACC_OPT_BR_SOLO       : 32-bit words: the latency form of the blind
- *                             rotation (one CTA per ciphertext, accumulator in
- *                             shared memory, each step's key prefetched into
- *                             shared memory by bulk asynchronous copies) up
+ *                             rotation (a cluster of 4, 2 or 1 CTAs per
+ *                             ciphertext, as many as run at once, accumulator
+ *                             and the next step's keys in shared memory) up
  *                             to this many gates per SM; 0 = off, -1
- *                             (default) = 1. Not taken when
+ *                             (default) = 2. Not taken when
  *                             FHEACC_OPT_BR_PIPES or
  *                             FHEACC_OPT_DEBUG_WAIT_LIMIT is set.
  *  FHEACC_OPT_DEBUG_WAIT_LIMIT: for tests of the error path only. The
