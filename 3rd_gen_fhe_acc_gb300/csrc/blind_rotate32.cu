@@ -89,6 +89,7 @@ struct PipeArgs {
     uint64_t gate_constant[8];
     unsigned long long *claim_next;   // next unclaimed ciphertext (zeroed before the launch)
     unsigned *status;                 // set to kStatusWaitLimit if a pipeline gave up waiting
+    int items_ok;                     // the scratch holds the items form's done words and residues
     int idle_limit;                   // idle periods before such a wait gives up (kIdleLimit)
 };
 
@@ -552,10 +553,46 @@ static int launch_block32(Context &c, const dev::PipeArgs &A, int max_ctas, cuda
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "blind rotation (latency form) launch");
 }
 
+// Items form; scratch after the accumulators: claim words, done words, residues
+// (bootstrap_accs_bytes).
+template <int DG, int W>
+static int launch_items32(Context &c, dev::PipeArgs A, int max_ctas, cudaStream_t st)
+{
+    auto kern = dev::br32_items_kernel<DG, W>;
+    const size_t smem = dev::item32_bytes<DG, W>();
+    const uint32_t mu32 = (uint32_t)((1ULL << 32) / c.p.Q);
+    A.claim_next = reinterpret_cast<unsigned long long *>(A.accs + A.count * 2048);
+    int *done = reinterpret_cast<int *>(A.accs + A.count * 2048 + kClaimWords);
+    uint8_t *res = reinterpret_cast<uint8_t *>(done + A.count);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaMemsetAsync(A.claim_next, 0, kClaimWords * sizeof(uint32_t), st);
+    if (e != cudaSuccess) return c.cuda_fail(e, "blind rotation (items form) set-up");
+    dev::br32_begin_kernel<<<(unsigned)A.count, 32, 0, st>>>(A, c.nc, c.d_fwd_tw, res, done, mu32);
+    c.launches++;
+    size_t blocks = std::min<size_t>((size_t)sm_count(c), A.count);
+    if (max_ctas > 0) blocks = std::min<size_t>(blocks, (size_t)max_ctas);
+    kern<<<(unsigned)blocks, dev::kItem32Threads, smem, st>>>(A, c.nc, c.d_plain_tw, res, done,
+                                                                                    dev::kItem32WaitLimit);
+    c.launches++;
+    dev::br32_end_kernel<<<(unsigned)A.count, 64, 0, st>>>(A, c.nc, c.d_inv_tw);
+    c.launches++;
+    e = cudaGetLastError();
+    return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "blind rotation (items form) launch");
+}
+
 // Latency form up to this many gates per SM by default; FHEACC_OPT_BR_SOLO overrides, 0
-// turns it off. One GB300, n = 500: 152 gates 3.2 ms (pipelines 7.3), 304 gates in two
-// rounds 6.4 ms (7.4), three rounds 9.6 ms (333 gates 9.8).
-constexpr int kSoloGatesPerSm = 2;
+// turns it and the items form off.
+constexpr int kSoloGatesPerSm = 1;
+
+// Whether the items form is taken for `count` gates beyond the latency form's range.
+// Blind rotation per gate and SM (one GB300, n = 500, 152 SMs): items 2.42 ms (700 gates
+// 11.2 ms, 1000 gates 16.0, 2000 gates 31.8), pipelines 2.24 ms a round of one gate per SM
+// and 0.4 ms more (700 gates 11.8, 1000 gates 16.5, 2000 gates 31.4, 4096 gates 60.5): the
+// pipelines are faster per gate, but their last round is as long as a full one.
+static bool items32_pay(size_t count, size_t sms)
+{
+    return 2.42 * (double)count / (double)sms < 2.24 * (double)((count + sms - 1) / sms) + 0.4;
+}
 
 // Pipelines per CTA. By default from the gates per SM (one GB300, 4096-gate
 // key set): up to 2 a single pipeline per SM is fastest (its items do not
@@ -572,6 +609,10 @@ static int launch_pipe_shape(Context &c, const dev::PipeArgs &A, int max_ctas, c
         if (rc == 1) rc = launch_block32<DG, 1>(c, A, max_ctas, st);
         if (rc != 1) return rc;
     }
+    if (A.items_ok && c.tune.br_solo != 0 && c.tune.br_pipes == 0 && c.tune.debug_wait_limit < 0 &&
+        items32_pay(A.count, sms))
+        return 2 * A.count <= 5 * sms ? launch_items32<DG, 2>(c, A, max_ctas, st)
+                                      : launch_items32<DG, 3>(c, A, max_ctas, st);
     const int np = c.tune.br_pipes > 0 ? c.tune.br_pipes : A.count <= 2 * sms ? 1 : A.count <= 5 * sms ? 2 : 3;
     if (np == 3) return launch_pipe_dg<DG, 3, 1>(c, A, max_ctas, st);
     if (np == 2) return launch_pipe_dg<DG, 2, 1>(c, A, max_ctas, st);
@@ -628,6 +669,7 @@ int launch_blind_rotate32(Context &c, const uint64_t *d_c1, const uint64_t *d_c2
     dev::PipeArgs A{};
     A.c1 = d_c1; A.c2 = d_c2; A.gates = d_gates; A.count = count;
     A.accs = (uint32_t *)c.accs.ptr; A.acc_out = d_acc_out; A.extract = d_extract;
+    A.items_ok = 1;
     fill_pipe_params(c, A, flags);
     return launch_pipe(c, A, max_ctas, st);
 }
@@ -640,20 +682,22 @@ namespace fheacc {
 // by the caller (`accs`: bootstrap_accs_bytes, 16-byte aligned); allocates
 // nothing.
 int launch_blind_rotate32_with(Context &c, const uint64_t *d_c1, const uint64_t *d_c2, const int32_t *d_gates,
-                               size_t count, uint32_t flags, uint32_t *accs, uint32_t *d_extract, cudaStream_t st)
+                               size_t count, uint32_t flags, uint32_t *accs, uint32_t *d_extract, cudaStream_t st,
+                               bool full_scratch)
 {
-    return launch_blind_rotate32_indexed(c, d_c1, d_c2, nullptr, nullptr, d_gates, count, flags, accs, d_extract, st);
+    return launch_blind_rotate32_indexed(c, d_c1, d_c2, nullptr, nullptr, d_gates, count, flags, accs, d_extract, st,
+                                         full_scratch);
 }
 
 int launch_blind_rotate32_indexed(Context &c, const uint64_t *d_c1, const uint64_t *d_c2, const uint32_t *d_idx1,
                                   const uint32_t *d_idx2, const int32_t *d_gates, size_t count, uint32_t flags,
-                                  uint32_t *accs, uint32_t *d_extract, cudaStream_t st)
+                                  uint32_t *accs, uint32_t *d_extract, cudaStream_t st, bool full_scratch)
 {
     if (!count) return FHEACC_OK;
     if (!c.d_btkey) return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
     dev::PipeArgs A{};
     A.c1 = d_c1; A.c2 = d_c2; A.idx1 = d_idx1; A.idx2 = d_idx2; A.gates = d_gates; A.count = count;
-    A.accs = accs; A.acc_out = nullptr; A.extract = d_extract;
+    A.accs = accs; A.acc_out = nullptr; A.extract = d_extract; A.items_ok = full_scratch;
     fill_pipe_params(c, A, flags);
     return launch_pipe(c, A, 0, st);
 }

@@ -197,6 +197,138 @@ __device__ __forceinline__ void block32_inv(const uint32_t *src, uint32_t *w, in
     for (int k = 0; k < 8; k++) out(k, x[k]);
 }
 
+// What a step works on: shared memory of the CTA (or worker), the cluster's g buffers
+// of this step, the accumulator read and the one written.
+template <int C>
+struct Block32Cta {
+    uint32_t *g, *acc, *acc_out, *dbuf;
+    uint32_t *peer[C];
+    const uint2 *ftw, *itw;
+    int rank;
+};
+
+// One step of the CTA's blocks by T threads (tid < T) that share named barrier `bar` (0:
+// the CTA). key: the RGSW's rows of the CTA's blocks, in B-tile order (KG: global
+// memory). mid(0), mid(1), mid(2): run before the barrier of 1, at the start of 3 and
+// before the products.
+template <int DG, int C, int T, bool KG, class Mid>
+__device__ __forceinline__ void block32_step(const Block32Cta<C> &s, const PipeArgs &A, const Ntt32Consts &c,
+                                             const uint32_t *key, int tid, int bar, Mid mid)
+{
+    constexpr int NB = 4 / C, ND = 2 * (DG - 1), NW = T / 32;
+    const int warp = tid >> 5, lane = tid & 31;
+    const uint32_t Q = c.Q, twoQ = c.twoQ, fourQ = 2 * twoQ, mask = (1u << A.bg_bits) - 1;
+    // ---- 1. inverse stages in the blocks
+    for (int w = warp; w < 2 * NB; w += NW) {
+        const int p = w / NB, lb = w - p * NB, b = s.rank * NB + lb;
+        const int o = p * kN32 + b * kB32 + lane;
+        block32_inv(s.acc + w * kB32E, s.dbuf + w * kB32E, b, lane, c, s.itw, [&](int k, uint32_t v) {
+#pragma unroll
+            for (int r = 0; r < C; r++) s.peer[r][o + 32 * k] = v;
+        });
+    }
+    mid(0);
+    if (C > 1) cg::this_cluster().sync();
+    else pipe_barrier(bar, T);
+    // ---- 2. last inverse stages, digits, first two forward stages
+    for (int u = tid; u < 512; u += T) {
+        const int p = u >> 8, j = u & 255;
+        const uint32_t *const x = s.g + p * kN32 + j;
+        uint32_t x0 = x[0], x1 = x[256], x2 = x[512], x3 = x[768];
+        gs_bfly(x0, x1, c.iw[2], c.iws[2], Q, twoQ);
+        gs_bfly(x2, x3, c.iw[3], c.iws[3], Q, twoQ);
+        auto last = [&](uint32_t &a, uint32_t &b) {   // as ntt_inv_1024_noscale
+            uint32_t u = a + b;
+            u = min(u, u - twoQ);
+            const uint32_t v = shoup32(a - b + twoQ, c.iw[1], c.iws[1], Q);
+            a = min(u, u - Q);
+            b = min(v, v - Q);
+        };
+        last(x0, x2);
+        last(x1, x3);
+        uint32_t *o = s.dbuf + p * (DG - 1) * NB * kB32E + p4(j);
+#pragma unroll
+        for (int h = 0; h < DG - 1; h++, o += NB * kB32E) {
+            const uint32_t sh = A.bg_bits * h;
+            const uint32_t y0 = (x0 >> sh) & mask, y1 = (x1 >> sh) & mask, y2 = (x2 >> sh) & mask,
+                           y3 = (x3 >> sh) & mask;
+            // y0 +- w1 y2 +- (w2 y1 + w2 w1 y3), and with w3, -w3 w1 for the
+            // lower half: each < 6Q + BG
+            const uint32_t a = shoup32(y2, c.fw[1], c.fws[1], Q);
+            if (C == 1 || s.rank < C / 2) {
+                const uint32_t z = y0 + a;
+                const uint32_t v = shoup32(y1, c.fw[2], c.fws[2], Q) + shoup32(y3, A.w21, A.w21s, Q);
+                if (C < 4) {
+                    o[0] = z + v;
+                    o[kB32E] = z + fourQ - v;
+                } else {
+                    o[0] = s.rank == 0 ? z + v : z + fourQ - v;
+                }
+            }
+            if (C == 1 || s.rank >= C / 2) {
+                const uint32_t z = y0 + twoQ - a;
+                const uint32_t v = shoup32(y1, c.fw[3], c.fws[3], Q) + shoup32(y3, A.w31n, A.w31ns, Q);
+                uint32_t *const q = C == 1 ? o + 2 * kB32E : o;
+                if (C < 4) {
+                    q[0] = z + v;
+                    q[kB32E] = z + fourQ - v;
+                } else {
+                    q[0] = s.rank == 2 ? z + v : z + fourQ - v;
+                }
+            }
+        }
+    }
+    pipe_barrier(bar, T);
+    // ---- 3. forward stages in the blocks
+    mid(1);
+    for (int w = warp; w < ND * NB; w += NW)
+        block32_fwd(s.dbuf + w * kB32E, s.rank * NB + w % NB, lane, c, s.ftw);
+    mid(2);
+    pipe_barrier(bar, T);
+    // ---- 4. multiply-accumulate in the keys' B-tile order (conflict-free in the
+    // blocks too): C = 1, 256 threads with 4 words of both output polys each (a
+    // digit word is read once); else 512 threads with E words of one poly
+    constexpr int PP = C == 1 ? 2 : 1;   // output polys per thread
+    if (tid < 512 / PP) {
+        constexpr int E = NB;
+        const int P = tid >> 8, v = tid & 255, ch = v * E / 4, e0 = v * E % 4;
+        const int q = ch / (8 * NB), l = ch % (8 * NB), e = 36 * (l & 7) + 4 * q + e0, lb = l >> 3;
+        const uint32_t *const a0 = s.acc + lb * kB32E + e;
+        const uint32_t *const d0 = s.dbuf + lb * kB32E + e, *ka = key + P * (NB * kB32) + v * E;
+        uint64_t sum[PP][E];
+#pragma unroll
+        for (int o = 0; o < PP; o++)
+#pragma unroll
+            for (int i = 0; i < E; i++) sum[o][i] = 0;
+#pragma unroll
+        for (int h = 0; h < DG; h++)
+#pragma unroll
+            for (int p = 0; p < 2; p++, ka += 2 * NB * kB32) {
+                uint32_t dv[E], kv[E];
+                load_words<E>(dv, h < DG - 1 ? d0 + (p * (DG - 1) + h) * NB * kB32E : a0 + p * NB * kB32E);
+#pragma unroll
+                for (int o = 0; o < PP; o++) {
+                    if constexpr (KG) {
+                        const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(ka + o * NB * kB32));
+                        kv[0] = x.x; kv[1] = x.y; kv[2] = x.z; kv[3] = x.w;
+                    } else {
+                        load_words<E>(kv, ka + o * NB * kB32);
+                    }
+#pragma unroll
+                    for (int i = 0; i < E; i++) sum[o][i] += (uint64_t)dv[i] * kv[i];
+                }
+            }
+#pragma unroll
+        for (int o = 0; o < PP; o++) {
+            uint32_t r[E];
+#pragma unroll
+            for (int i = 0; i < E; i++) r[i] = mont_reduce_2q(sum[o][i], Q, A.qinv_neg);
+            store_words<E>(s.acc_out + ((P + o) * NB + lb) * kB32E + e, r);
+        }
+    }
+    pipe_barrier(bar, T);
+}
+
 template <int DG, int C>
 __global__ void __launch_bounds__(Block32Layout<DG, C>::T, 1)
     br32_block_kernel(const __grid_constant__ PipeArgs A, const __grid_constant__ Ntt32Consts c,
@@ -216,7 +348,6 @@ __global__ void __launch_bounds__(Block32Layout<DG, C>::T, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = C > 1 ? (int)(blockIdx.x % C) : 0;
     const int S = A.n * (int)A.digitR, mode = issue_mode(A.flags);
-    const uint32_t Q = c.Q, twoQ = c.twoQ, fourQ = 2 * twoQ, mask = (1u << A.bg_bits) - 1;
     uint32_t *peer[C];
     peer[0] = g;
     if (C > 1) {
@@ -257,113 +388,22 @@ __global__ void __launch_bounds__(Block32Layout<DG, C>::T, 1)
         __syncthreads();
         int ab = 0;   // accumulator buffer
         for (int kb = 0, gb = 0; s < S; kb ^= 1, ab ^= 1, gb ^= C > 1) {
-            // ---- 1. inverse stages in the blocks
-            if (warp < 2 * NB) {
-                const int p = warp / NB, lb = warp - p * NB, b = rank * NB + lb;
-                const int o = gb * 2048 + p * kN32 + b * kB32 + lane;
-                block32_inv(acc + ab * (2 * NB * kB32E) + warp * kB32E, dbuf + warp * kB32E, b, lane, c, itw, [&](int k, uint32_t v) {
+            const Block32Cta<C> cta = [&]() {
+                Block32Cta<C> v{g + gb * 2048, acc + ab * (2 * NB * kB32E), acc + (ab ^ 1) * (2 * NB * kB32E), dbuf, {},
+                                ftw, itw, rank};
 #pragma unroll
-                    for (int r = 0; r < C; r++) peer[r][o + 32 * k] = v;
-                });
-            }
-            // warps without a block here (C = 1) or in 3 start the copy of the next step's
-            // keys into the buffer that the last products have freed (copies in flight would
-            // hold up the cluster barrier's release: C = 4, 2.01 -> 2.18 us per step)
-            if (C == 1) fetch(next, kb ^ 1, tid - 64 * NB, T - 64 * NB);
-            if (C > 1) cg::this_cluster().sync();
-            else __syncthreads();
-            // ---- 2. last inverse stages, digits, first two forward stages
-            if (tid < 512) {
-                const int p = tid >> 8, j = tid & 255;
-                const uint32_t *const x = g + gb * 2048 + p * kN32 + j;
-                uint32_t x0 = x[0], x1 = x[256], x2 = x[512], x3 = x[768];
-                gs_bfly(x0, x1, c.iw[2], c.iws[2], Q, twoQ);
-                gs_bfly(x2, x3, c.iw[3], c.iws[3], Q, twoQ);
-                auto last = [&](uint32_t &a, uint32_t &b) {   // as ntt_inv_1024_noscale
-                    uint32_t u = a + b;
-                    u = min(u, u - twoQ);
-                    const uint32_t v = shoup32(a - b + twoQ, c.iw[1], c.iws[1], Q);
-                    a = min(u, u - Q);
-                    b = min(v, v - Q);
-                };
-                last(x0, x2);
-                last(x1, x3);
-                uint32_t *o = dbuf + p * (DG - 1) * NB * kB32E + p4(j);
-#pragma unroll
-                for (int h = 0; h < DG - 1; h++, o += NB * kB32E) {
-                    const uint32_t sh = A.bg_bits * h;
-                    const uint32_t y0 = (x0 >> sh) & mask, y1 = (x1 >> sh) & mask, y2 = (x2 >> sh) & mask,
-                                   y3 = (x3 >> sh) & mask;
-                    // y0 +- w1 y2 +- (w2 y1 + w2 w1 y3), and with w3, -w3 w1 for the
-                    // lower half: each < 6Q + BG
-                    const uint32_t a = shoup32(y2, c.fw[1], c.fws[1], Q);
-                    if (C == 1 || rank < C / 2) {
-                        const uint32_t u = y0 + a;
-                        const uint32_t v = shoup32(y1, c.fw[2], c.fws[2], Q) + shoup32(y3, A.w21, A.w21s, Q);
-                        if (C < 4) {
-                            o[0] = u + v;
-                            o[kB32E] = u + fourQ - v;
-                        } else {
-                            o[0] = rank == 0 ? u + v : u + fourQ - v;
-                        }
-                    }
-                    if (C == 1 || rank >= C / 2) {
-                        const uint32_t u = y0 + twoQ - a;
-                        const uint32_t v = shoup32(y1, c.fw[3], c.fws[3], Q) + shoup32(y3, A.w31n, A.w31ns, Q);
-                        uint32_t *const q = C == 1 ? o + 2 * kB32E : o;
-                        if (C < 4) {
-                            q[0] = u + v;
-                            q[kB32E] = u + fourQ - v;
-                        } else {
-                            q[0] = rank == 2 ? u + v : u + fourQ - v;
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-            // ---- 3. forward stages in the blocks
-            if (C > 1) fetch(next, kb ^ 1, tid - 32 * FW, T - 32 * FW);
-            for (int w = warp; w < ND * NB; w += NW)
-                block32_fwd(dbuf + w * kB32E, rank * NB + w % NB, lane, c, ftw);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-            __syncthreads();
-            // ---- 4. multiply-accumulate in the keys' B-tile order (conflict-free in the
-            // blocks too): C = 1, 256 threads with 4 words of both output polys each (a
-            // digit word is read once); else 512 threads with E words of one poly
-            constexpr int PP = C == 1 ? 2 : 1;   // output polys per thread
-            if (tid < 512 / PP) {
-                constexpr int E = NB;
-                const int P = tid >> 8, v = tid & 255, ch = v * E / 4, e0 = v * E % 4;
-                const int q = ch / (8 * NB), l = ch % (8 * NB), e = 36 * (l & 7) + 4 * q + e0, lb = l >> 3;
-                const uint32_t *const a0 = acc + ab * (2 * NB * kB32E) + lb * kB32E + e;
-                const uint32_t *const d0 = dbuf + lb * kB32E + e, *ka = keys + kb * L::key_words + P * (NB * kB32) + v * E;
-                uint64_t sum[PP][E];
-#pragma unroll
-                for (int o = 0; o < PP; o++)
-#pragma unroll
-                    for (int i = 0; i < E; i++) sum[o][i] = 0;
-#pragma unroll
-                for (int h = 0; h < DG; h++)
-#pragma unroll
-                    for (int p = 0; p < 2; p++, ka += 2 * NB * kB32) {
-                        uint32_t dv[E], kv[E];
-                        load_words<E>(dv, h < DG - 1 ? d0 + (p * (DG - 1) + h) * NB * kB32E : a0 + p * NB * kB32E);
-#pragma unroll
-                        for (int o = 0; o < PP; o++) {
-                            load_words<E>(kv, ka + o * NB * kB32);
-#pragma unroll
-                            for (int i = 0; i < E; i++) sum[o][i] += (uint64_t)dv[i] * kv[i];
-                        }
-                    }
-#pragma unroll
-                for (int o = 0; o < PP; o++) {
-                    uint32_t r[E];
-#pragma unroll
-                    for (int i = 0; i < E; i++) r[i] = mont_reduce_2q(sum[o][i], Q, A.qinv_neg);
-                    store_words<E>(acc + (ab ^ 1) * (2 * NB * kB32E) + ((P + o) * NB + lb) * kB32E + e, r);
-                }
-            }
-            __syncthreads();
+                for (int r = 0; r < C; r++) v.peer[r] = peer[r] + gb * 2048;
+                return v;
+            }();
+            block32_step<DG, C, T, false>(cta, A, c, keys + kb * L::key_words, tid, 0, [&](int at) {
+                // warps without a block in 1 (C = 1) or in 3 start the copy of the next
+                // step's keys into the buffer that the last products have freed (copies in
+                // flight would hold up the cluster barrier's release: C = 4, 2.01 -> 2.18
+                // us per step)
+                if (at == 0 && C == 1) fetch(next, kb ^ 1, tid - 64 * NB, T - 64 * NB);
+                if (at == 1 && C > 1) fetch(next, kb ^ 1, tid - 32 * FW, T - 32 * FW);
+                if (at == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            });
             s = next;
             next = s < S ? solo_next_step(res, s, S, mode) : S;
         }
@@ -380,6 +420,122 @@ __global__ void __launch_bounds__(Block32Layout<DG, C>::T, 1)
         if (rank == 0 && warp < 2) pipe_out_poly(A, c, inv_tw, keys + warp * kN32, gid, warp, lane);
         if (C > 1) cg::this_cluster().sync();   // the next ciphertext's accumulator words, and this CTA's exit
         else __syncthreads();
+    }
+}
+
+// ---- Items form (a few gates per SM): W workers of 768 / W threads per CTA, whose
+// barriers and loads overlap, take items, consecutive steps of one ciphertext, from a
+// cursor that walks them step-major; the accumulator goes through L2 between items. So
+// the work spreads evenly over the SMs whatever the batch, where the pipelines give whole
+// ciphertexts to CTAs (333 gates: 3 each to 111 of the 152). An item waits for the item
+// before it of its ciphertext (done[]), taken earlier by a worker that is running. Three
+// workers of 8 warps divide every phase evenly over the four schedulers and reach 2.5 us
+// per step and SM; with two of 12 the few ciphertexts of a small batch advance faster
+// (blind rotation, two / three workers: 304 gates 5.6 / 6.1 ms, 512 gates 9.1 / 8.2 ms).
+// Bound by the multiply pipe (61 % busy; a loop of butterflies alone reaches 82 %).
+// Digit tables instead of multiplications did not pay here: 1000 gates 16.0 -> 16.1 ms.
+constexpr int kItem32Threads = 768;   // of a CTA
+__host__ __device__ constexpr int item32_steps(int W) { return W == 2 ? 8 : 16; }
+
+// Polls of such a wait (about 60 ns each) before it gives up and flags the launch.
+constexpr unsigned kItem32WaitLimit = 1u << 26;
+
+// Dynamic shared memory: twiddles, then per worker [g | acc x 2 | dbuf].
+template <int DG>
+__host__ __device__ constexpr size_t item32_worker_bytes()
+{
+    return 4 * (2 * kN32 + (size_t)2 * 2 * 4 * kB32E + (size_t)2 * (DG - 1) * 4 * kB32E);
+}
+template <int DG, int W>
+constexpr size_t item32_bytes()
+{
+    return 2 * kN32 * sizeof(uint2) + W * item32_worker_bytes<DG>();
+}
+
+// Residues and initial accumulators, one warp per ciphertext.
+__global__ void __launch_bounds__(32) br32_begin_kernel(const __grid_constant__ PipeArgs A,
+                                                        const __grid_constant__ Ntt32Consts c,
+                                                        const uint2 *__restrict__ fwd_tw, uint8_t *res, int *done,
+                                                        uint32_t mu32)
+{
+    __shared__ __align__(16) uint32_t buf[kN32];
+    const size_t gid = blockIdx.x;
+    if (threadIdx.x == 0) done[gid] = -1;
+    pipe_init_item(A, c, fwd_tw, buf, res + gid * (size_t)(A.n * (int)A.digitR), gid, threadIdx.x, mu32);
+}
+
+__global__ void __launch_bounds__(64) br32_end_kernel(const __grid_constant__ PipeArgs A,
+                                                      const __grid_constant__ Ntt32Consts c,
+                                                      const uint2 *__restrict__ inv_tw)
+{
+    __shared__ __align__(16) uint32_t buf[2][kN32];
+    pipe_out_poly(A, c, inv_tw, buf[threadIdx.x >> 5], blockIdx.x, threadIdx.x >> 5, threadIdx.x & 31);
+}
+
+template <int DG, int W>
+__global__ void __launch_bounds__(kItem32Threads, 1)
+    br32_items_kernel(const __grid_constant__ PipeArgs A, const __grid_constant__ Ntt32Consts c,
+                      const uint2 *__restrict__ plain_tw, const uint8_t *__restrict__ all_res, int *done,
+                      unsigned wait_limit)
+{
+    constexpr int T = kItem32Threads / W, K = item32_steps(W);
+    extern __shared__ __align__(16) unsigned char blk_smem[];
+    __shared__ int plans[W][2];   // item of the ciphertext (-1: none left), ciphertext
+    uint2 *const ftw = reinterpret_cast<uint2 *>(blk_smem), *const itw = ftw + kN32;
+    const int wk = threadIdx.x / T, tid = threadIdx.x - wk * T, bar = 1 + wk;
+    uint32_t *const g = reinterpret_cast<uint32_t *>(blk_smem + 2 * kN32 * sizeof(uint2) + wk * item32_worker_bytes<DG>());
+    uint32_t *const acc = g + 2 * kN32, *const dbuf = acc + 2 * 2 * 4 * kB32E;
+    const int S = A.n * (int)A.digitR, mode = issue_mode(A.flags);
+    for (int i = threadIdx.x; i < 2 * kN32; i += kItem32Threads) ftw[i] = __ldg(plain_tw + i);
+    __syncthreads();
+    const unsigned long long items = (unsigned long long)((S + K - 1) / K) * A.count;
+    int *const plan = plans[wk];
+    for (;;) {
+        if (tid == 0) {
+            const unsigned long long v = atomicAdd(A.claim_next, 1ull);
+            const int it = v < items ? (int)(v / A.count) : -1;
+            const size_t k = it < 0 ? 0 : (size_t)(v - (unsigned long long)it * A.count);
+            plan[0] = it;
+            plan[1] = (int)k;
+            if (it >= 0) {
+                const volatile int *d = done + k;
+                unsigned polls = 0;
+                while (*d != it - 1) {
+                    if (++polls > wait_limit) {
+                        atomicOr(A.status, kStatusWaitLimit);
+                        plan[0] = -1;
+                        break;
+                    }
+                    __nanosleep(32);
+                }
+                __threadfence();
+            }
+        }
+        pipe_barrier(bar, T);
+        const int it = plan[0], k = plan[1];
+        if (it < 0) break;
+        const uint8_t *const res = all_res + (size_t)k * S;
+        uint4 *const ga = reinterpret_cast<uint4 *>(A.accs + (size_t)k * 2048);
+        const uint64_t pol = l2_keep_policy();
+        // B-tile chunk q * 32 + l holds words 32 l + 4 q ..
+        for (int u = tid; u < 512; u += T)
+            *reinterpret_cast<uint4 *>(acc + (u >> 8) * 4 * kB32E + 36 * (u & 31) + 4 * ((u >> 5) & 7)) = ld_keep(ga + u, pol);
+        pipe_barrier(bar, T);
+        int ab = 0;
+        const int end = min(S, (it + 1) * K);
+        for (int st = it * K; st < end; st++) {
+            if (!step_issued(res, st, mode)) continue;
+            const Block32Cta<1> cta{g, acc + ab * (8 * kB32E), acc + (ab ^ 1) * (8 * kB32E), dbuf, {g}, ftw, itw, 0};
+            block32_step<DG, 1, T, true>(cta, A, c, A.btkey + ((size_t)st * A.Br + res[st]) * ((size_t)DG * 4 * kN32),
+                                         tid, bar, [](int) {});
+            ab ^= 1;
+        }
+        for (int u = tid; u < 512; u += T)
+            st_keep(ga + u, *reinterpret_cast<const uint4 *>(acc + ab * (8 * kB32E) + (u >> 8) * 4 * kB32E + 36 * (u & 31) +
+                                                             4 * ((u >> 5) & 7)), pol);
+        __threadfence();
+        pipe_barrier(bar, T);
+        if (tid == 0) atomicExch(done + k, it);
     }
 }
 

@@ -194,14 +194,17 @@ int launch_blind_rotate32(Context &c, const uint64_t *d_c1, const uint64_t *d_c2
                           size_t count, uint32_t flags, uint64_t *d_acc_out, uint32_t *d_extract,
                           int max_ctas, cudaStream_t st);
 // The same blind rotation writing extracted RLWEs, with caller-supplied
-// accumulator scratch (bootstrap_accs_bytes); performs no allocation.
+// accumulator scratch (bootstrap_accs_bytes; full_scratch = false: only the
+// accumulators and the claim words); performs no allocation.
 int launch_blind_rotate32_with(Context &c, const uint64_t *d_c1, const uint64_t *d_c2, const int32_t *d_gates,
-                               size_t count, uint32_t flags, uint32_t *accs, uint32_t *d_extract, cudaStream_t st);
+                               size_t count, uint32_t flags, uint32_t *accs, uint32_t *d_extract, cudaStream_t st,
+                               bool full_scratch = true);
 // Blind rotation whose gate g reads c1 + idx1[g] * (n+1) and c2 + idx2[g] *
 // (n+1) (index arrays optional), caller-supplied accumulator scratch.
 int launch_blind_rotate32_indexed(Context &c, const uint64_t *d_c1, const uint64_t *d_c2, const uint32_t *d_idx1,
                                   const uint32_t *d_idx2, const int32_t *d_gates, size_t count, uint32_t flags,
-                                  uint32_t *accs, uint32_t *d_extract, cudaStream_t st);
+                                  uint32_t *accs, uint32_t *d_extract, cudaStream_t st,
+                                  bool full_scratch = true);
 // Key switch writing ciphertext ci to d_out + out_idx[ci] * (n+1) (optional).
 int launch_lwe_keyswitch32_indexed(Context &c, const uint32_t *d_extract, size_t count, bool modswitch,
                                    uint64_t *d_out, const uint32_t *d_out_idx, cudaStream_t st);
@@ -284,7 +287,7 @@ inline size_t bootstrap_accs_bytes(const Context &c, size_t count)
     const size_t S = (size_t)c.p.n * c.p.digitR;   // residues: of every gate (block form) or of the pool's
     return c.wide ? count * 4096 * sizeof(uint64_t) + kClaimWords * sizeof(uint32_t) +
                         std::max(count * (sizeof(int) + S), kPool64 * (2 * sizeof(int) + S))
-                  : (count * 2048 + kClaimWords) * sizeof(uint32_t);
+                  : (count * 2048 + kClaimWords) * sizeof(uint32_t) + count * (sizeof(int) + S);
 }
 inline size_t bootstrap_extract_bytes(const Context &c, size_t count)
 {

@@ -92,7 +92,7 @@ extern "C" int fheacc_bootstrap_noalloc(fheacc_ctx *ctx, const uint64_t *d_c1, c
         const bool prof = (flags & FHEACC_FLAG_PROFILE) != 0;
         flags &= ~(uint32_t)FHEACC_FLAG_PROFILE;
         if (prof) cudaEventRecord(c.prof[0], st);
-        rc = launch_blind_rotate32_with(c, d_c1, d_c2, d_gates, count, flags, accs, ext, st);
+        rc = launch_blind_rotate32_with(c, d_c1, d_c2, d_gates, count, flags, accs, ext, st, false);
         if (rc == FHEACC_OK && prof) cudaEventRecord(c.prof[1], st);
         if (rc == FHEACC_OK)
             rc = launch_lwe_keyswitch32(c, ext, count, true, d_out, st, accs,

@@ -276,8 +276,10 @@ int fheacc_lwe_modswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t cou
  *                             rotation (a cluster of 4, 2 or 1 CTAs per
  *                             ciphertext, as many as run at once, accumulator
  *                             and the next step's keys in shared memory) up
- *                             to this many gates per SM; 0 = off, -1
- *                             (default) = 2. Not taken when
+ *                             to this many gates per SM; -1 (default) = 1,
+ *                             0 = off, and so is the form for a few gates
+ *                             per SM (workers that take items of a few
+ *                             steps from a shared cursor). Not taken when
  *                             FHEACC_OPT_BR_PIPES or
  *                             FHEACC_OPT_DEBUG_WAIT_LIMIT is set.
  *  FHEACC_OPT_DEBUG_WAIT_LIMIT: for tests of the error path only. The

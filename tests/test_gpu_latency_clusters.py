@@ -1,6 +1,6 @@
 """The 32-bit latency form at the edges of its cluster sizes' ranges (4, 2 and 1 CTAs
-per ciphertext, more than one round), for every digitG the path takes, against the
-pipelines and the oracle."""
+per ciphertext) and the items form with two and three workers, for every digitG the
+path takes, against the pipelines and the oracle."""
 import numpy as np
 import pytest
 
@@ -25,7 +25,7 @@ def small(F, cuda_ok, request):
         yield P, ctx, lsk, bt, ks, Oracle.from_params(P)
 
 
-@pytest.mark.parametrize("count", [1, 2, 35, 38, 39, 76, 77, 152, 153, 304, 305])
+@pytest.mark.parametrize("count", [1, 2, 35, 38, 39, 76, 77, 152, 153, 304, 380, 381, 1000])
 def test_clusters(F, cuda_ok, small, count):
     torch = cuda_ok
     P, ctx, lsk, bt, ks, o = small
