@@ -34,18 +34,11 @@
 // bound by the multiply pipe: 48 k of its instructions a step, of which 29 k are
 // 32 x 32 -> 64 multiplies; a loop of butterflies on registers alone keeps the pipe 74 %
 // busy, the items form 62 %.
-#include "br64.cuh"
+#include "block64.cuh"
 #include <algorithm>
-#include <cooperative_groups.h>
-
-namespace cg = cooperative_groups;
 
 namespace fheacc {
 namespace dev {
-
-// Threads of a CTA: the 10 digits' 512-word blocks are 640 octets (digitG = 6), all
-// at once in the latency form, half of them in the throughput form (two CTAs per SM).
-constexpr int kTB = 640, kTP = 320;
 
 // Polls of an mbarrier before a key wait gives up and flags the launch.
 constexpr unsigned kKeyWaitLimit = 1u << 22;
@@ -62,327 +55,11 @@ struct BlockArgs {
     unsigned wait_limit;
 };
 
-// x w of the MAC: sums[0] + 2^27 sums[1] + 2^54 sums[2] (x < 2^59, limbs < 2^27,
-// at most 16 products: sums[1] < 16 (2^59 + 2^54) < 2^64).
-__device__ __forceinline__ void mac27(uint64_t (&s)[3], uint32_t x0, uint32_t x1, uint2 w)
-{
-    s[0] += mul_wide64(x0, w.x);
-    s[1] += mul_wide64(x0, w.y);
-    s[1] += mul_wide64(x1, w.x);
-    s[2] += mul_wide64(x1, w.y);
-}
-
-// The value of the sums mod Q, below 2Q: c54 (2^54 mod Q, below 2^19) folds the part
-// Y above 2^54 (Y < 2^64) twice.
-__device__ __forceinline__ uint64_t mac27_reduce(const uint64_t (&s)[3], uint32_t c54, const Ntt64Consts &c)
-{
-    constexpr uint64_t m27 = (1u << 27) - 1;
-    const uint64_t T = s[1] + (s[0] >> 27);
-    const uint64_t low = (s[0] & m27) | ((T & m27) << 27);
-    const uint64_t Y = s[2] + (T >> 27);
-    const uint64_t zl = mul_wide64((uint32_t)Y, c54);
-    const uint64_t zm = mad_wide64((uint32_t)(Y >> 32), c54, zl >> 32);   // Z = zm 2^32 + low word of zl
-    const uint64_t z0 = ((zm << 32) | (uint32_t)zl) & (((uint64_t)1 << 54) - 1);
-    return reduce64<true>(mad_wide64((uint32_t)(zm >> 22), c54, low + z0), c);
-}
-
-template <int B, int C>
-struct BlockLayout {
-    static constexpr int M = 2048 / B, NB = B / C, ME = M + M / 16;   // words of a block, blocks of a CTA
-    static constexpr int GBUF = C > 1 ? 2 : 1;
-    static constexpr size_t g_off = 0;                                  // [GBUF][2][2048]
-    static constexpr size_t acc_off = (size_t)GBUF * 2 * 2048 * 8;      // [2][NB * ME], layout px
-    static size_t __host__ __device__ work_off(int) { return acc_off + (size_t)2 * NB * ME * 8; }
-    // digit NTTs [2 (DG - 1)][ME]; the inverse NTT's [2][NB * ME] before them
-    static size_t __host__ __device__ work_words(int DG)
-    {
-        const int d = 2 * (DG - 1), i = 2 * NB;
-        return (size_t)(d > i ? d : i) * ME;
-    }
-    // the latency form's key buffer: the rows of one block
-    static size_t __host__ __device__ key_off(int DG) { return work_off(DG) + work_words(DG) * 8; }
-    static size_t __host__ __device__ key_bytes(int DG) { return (size_t)DG * 4 * M * 8; }
-};
-
-// Threads that share a 512- or 256-word transform: GS = 32 or 64 consecutive ones,
-// group gi of the CTA. A transform's passes then need no CTA barrier between them.
-template <int GS>
-__device__ __forceinline__ void group_sync64(int gi)
-{
-    if (GS == 32) __syncwarp();
-    else group_sync(1 + gi, GS);
-}
-
-// One radix-2^R forward pass of a digit's block d (M words, layout px) by a group:
-// stages t, t/2, ..; blk: the block, gt: the thread in the group.
-template <int M, int R, int GS>
-__device__ __forceinline__ void blk_fwd_pass(uint64_t *d, int blk, int t, int gt, const ulonglong2 *__restrict__ tw,
-                                             const Ntt64Consts &c)
-{
-    constexpr int K = 1 << R, per = M / K;
-    const int h = t >> (R - 1), m = 1024 / t;
-    for (int q = gt; q < per; q += GS) {
-        const int gl = q / h, j = q - gl * h;
-        const int grp = blk * (M / (2 * t)) + gl;
-        uint64_t *const b = d + px(gl * 2 * t + j);
-        uint64_t x[K];
-#pragma unroll
-        for (int k = 0; k < K; k++) x[k] = b[px(k * h)];
-#pragma unroll
-        for (int st = 0; st < R; st++) {
-            const int dl = K >> (st + 1);
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                if (k & dl) continue;
-                ct64<true>(x[k], x[k + dl], __ldg(tw + ((m + grp) << st) + (k >> (R - st))), c);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < K; k++) b[px(k * h)] = x[k];
-    }
-}
-
-// The first pass (M = 512: t = 256 .. 64; 256: t = 128, 64) with the digit's residue
-// mod X^M - zeta computed as it loads: word j is the digit of x[j] plus
-// z[i - 1] times the digit of x[j + i M].
-template <int B, int GS>
-__device__ __forceinline__ void blk_fwd_first(uint64_t *d, const uint64_t *x, const uint64_t (&z)[B - 1], uint32_t sh,
-                                              uint32_t mask, int blk, int gt, const ulonglong2 *__restrict__ tw,
-                                              const Ntt64Consts &c)
-{
-    constexpr int M = 2048 / B, R = M == 512 ? 3 : 2, K = 1 << R;
-    for (int j = gt; j < 64; j += GS) {
-        uint64_t v[K];
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const uint64_t *b = x + j + 64 * k;
-            uint64_t U = 0, V = 0;
-#pragma unroll
-            for (int i = 1; i < B; i++) {
-                const uint32_t y = (uint32_t)(b[i * M] >> sh) & mask;
-                U = mad_wide64(y, (uint32_t)z[i - 1], U);
-                V = mad_wide64(y, (uint32_t)(z[i - 1] >> 32), V);
-            }
-            v[k] = fold64(U, V, c) + ((uint32_t)(b[0] >> sh) & mask);
-        }
-#pragma unroll
-        for (int st = 0; st < R; st++) {
-            const int dl = K >> (st + 1);
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                if (k & dl) continue;
-                ct64<true>(v[k], v[k + dl], __ldg(tw + ((B + blk) << st) + (k >> (R - st))), c);
-            }
-        }
-        uint64_t *const o = d + px(j);
-#pragma unroll
-        for (int k = 0; k < K; k++) o[px(64 * k)] = v[k];
-    }
-}
-
-// One radix-8 inverse pass of a block (M words, layout px) by a group, src to
-// out(word, x); stages t, 2t, 4t. Inputs below 2^K0 Q, outputs below 2^(K0+3) Q, or
-// below 2Q with FOLD.
-template <int M, int K0, bool FOLD, int GS, class Out>
-__device__ __forceinline__ void blk_inv_pass8(const uint64_t *src, int blk, int t, int gt,
-                                              const ulonglong2 *__restrict__ itw, const Ntt64Consts &c, Out out)
-{
-    constexpr int per = M / 8;
-    const int m = 1024 / t;
-    for (int q = gt; q < per; q += GS) {
-        int gl = q / t;
-        const int j = q - gl * t;
-        if (t == 8) gl = (gl & ~3) | ((gl & 1) << 1) | ((gl >> 1) & 1);   // as inv_pass8
-        const int grp = blk * (M / (8 * t)) + gl, e0 = gl * 8 * t + j;
-        const uint64_t *b = src + px(e0);
-        uint64_t x[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) x[k] = b[px(k * t)];
-#pragma unroll
-        for (int k = 0; k < 4; k++) gs64<true, K0>(x[2 * k], x[2 * k + 1], __ldg(itw + m + 4 * grp + k), c);
-        const ulonglong2 w2a = __ldg(itw + (m >> 1) + 2 * grp), w2b = __ldg(itw + (m >> 1) + 2 * grp + 1);
-        gs64<true, K0 + 1>(x[0], x[2], w2a, c);
-        gs64<true, K0 + 1>(x[1], x[3], w2a, c);
-        gs64<true, K0 + 1>(x[4], x[6], w2b, c);
-        gs64<true, K0 + 1>(x[5], x[7], w2b, c);
-        const ulonglong2 w4 = __ldg(itw + (m >> 2) + grp);
-#pragma unroll
-        for (int k = 0; k < 4; k++) gs64<true, K0 + 2>(x[k], x[k + 4], w4, c);
-        if (FOLD) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) x[k] = reduce64<true>(x[k], c);
-        }
-        out(e0, x);
-    }
-}
-
-// The last inverse stages (t = M .. 1024, N^-1 folded in) of the tuple x_i = word
-// j + i M, canonical; inputs below 2^K Q (K <= 4).
-template <int B>
-__device__ __forceinline__ void blk_inv_last(uint64_t (&x)[B], const ulonglong2 *__restrict__ itw, const Ntt64Consts &c)
-{
-    if (B == 8) {
-#pragma unroll
-        for (int i = 0; i < B / 2; i++) gs64<true, 3>(x[2 * i], x[2 * i + 1], __ldg(itw + 4 + i), c);
-#pragma unroll
-        for (int i = 0; i < B / 4; i++) {
-            const ulonglong2 w = __ldg(itw + 2 + i);
-            gs64<true, 4>(x[4 * i], x[4 * i + 2], w, c);
-            gs64<true, 4>(x[4 * i + 1], x[4 * i + 3], w, c);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < B / 2; i++) gs64<true, 4>(x[2 * i], x[2 * i + 1], __ldg(itw + 2 + i), c);
-    }
-    const ulonglong2 wu = make_ulonglong2(c.iN, c.iNs), wv = make_ulonglong2(c.iw1N, c.iw1Ns);
-#pragma unroll
-    for (int i = 0; i < B / 2; i++) {
-        const uint64_t a = x[i], b = x[i + B / 2];
-        const uint64_t u = mul64<true>(a + b, wu, c), v = mul64<true>(a - b + (c.Q << 5), wv, c);
-        x[i] = u >= c.Q ? u - c.Q : u;
-        x[i + B / 2] = v >= c.Q ? v - c.Q : v;
-    }
-}
-
 __device__ __forceinline__ int next_issued(const uint8_t *res, int s, int S, int mode)
 {
     for (s++; s < S; s++)
         if (step_issued(res, s, mode)) return s;
     return S;
-}
-
-// What a CTA of a cluster of C brings to a step.
-template <int B, int C>
-struct BlockCta {
-    uint64_t *g, *acc, *work;      // shared memory (BlockLayout); g: the buffer of this step
-    uint64_t *peer[C];             // the cluster's g buffers of this step
-    const uint64_t (*zeta)[B - 1]; // powers of the blocks' zeta, times 2^pm_s
-    int rank;
-};
-
-// One step of the CTA's blocks by T threads (tid < T) that share the named barrier
-// `bar` (0: the whole CTA). keys(lb): waits for and returns
-// the key rows of block lb, [DG][2][2] rows of M words `row` words apart (KG: in global
-// memory, read past L1, which then keeps the twiddles of the block);
-// done(lb) runs after the block's products.
-template <int B, int C, int T, bool KG, class Keys, class Done>
-__device__ __forceinline__ void block_step(const BlockCta<B, C> &s, const BlockArgs &A,
-                                           const ulonglong2 *__restrict__ tw, const ulonglong2 *__restrict__ itw,
-                                           const Ntt64Consts &c, size_t row, int tid, int bar, Keys keys,
-                                           Done done)
-{
-    using L = BlockLayout<B, C>;
-    constexpr int M = L::M, NB = L::NB, ME = L::ME, NW = NB * M;
-    const int DG = A.DG, nd = 2 * (DG - 1);
-    const uint32_t mask = (1u << A.bg_bits) - 1;
-    uint64_t *const work = s.work, *const acc = s.acc;
-    constexpr int GS = M == 512 && T == kTB ? 64 : 32, NG = T / GS;
-    const int gi = tid / GS, gt = tid - gi * GS;
-    // ---- 1. inverse stages inside the blocks, a group per block
-    for (int u = gi; u < 2 * NB; u += NG) {
-        const int p = u / NB, lb = u - p * NB, blk = s.rank * NB + lb, base = p * 2048 + blk * M;
-        uint64_t *const w = work + u * ME;
-        blk_inv_pass8<M, 1, false, GS>(acc + p * px(NW) + lb * ME, blk, 1, gt, itw, c, [&](int e0, uint64_t (&x)[8]) {
-#pragma unroll
-            for (int k = 0; k < 8; k++) w[px(e0) + k] = x[k];   // 2Q -> 16Q
-        });
-        group_sync64<GS>(gi);
-        blk_inv_pass8<M, 4, true, GS>(w, blk, 8, gt, itw, c, [&](int e0, uint64_t (&x)[8]) {   // -> 2Q
-#pragma unroll
-            for (int k = 0; k < 8; k++) w[px(e0) + px(8 * k)] = x[k];
-        });
-        group_sync64<GS>(gi);
-        if (B == 8) {   // t = 64, 128: 2Q -> 8Q
-            for (int j = gt; j < 64; j += GS) {
-                uint64_t x[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) x[k] = w[px(j) + px(64 * k)];
-                gs64<true, 1>(x[0], x[1], __ldg(itw + 16 + 2 * blk), c);
-                gs64<true, 1>(x[2], x[3], __ldg(itw + 16 + 2 * blk + 1), c);
-                const ulonglong2 w2 = __ldg(itw + 8 + blk);
-                gs64<true, 2>(x[0], x[2], w2, c);
-                gs64<true, 2>(x[1], x[3], w2, c);
-#pragma unroll
-                for (int r = 0; r < C; r++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++) s.peer[r][base + j + 64 * k] = x[k];
-            }
-        } else {        // t = 64, 128, 256: 2Q -> 16Q
-            blk_inv_pass8<M, 1, false, GS>(w, blk, 64, gt, itw, c, [&](int e0, uint64_t (&x)[8]) {
-#pragma unroll
-                for (int r = 0; r < C; r++)
-#pragma unroll
-                    for (int k = 0; k < 8; k++) s.peer[r][base + e0 + 64 * k] = x[k];
-            });
-        }
-    }
-    if (C > 1) cg::this_cluster().sync();
-    else group_sync(bar, T);
-    // ---- 2. last inverse stages of all words
-    for (int u = tid; u < 2 * M; u += T) {
-        uint64_t *const b = s.g + (u / M) * 2048 + u % M;
-        uint64_t x[B];
-#pragma unroll
-        for (int i = 0; i < B; i++) x[i] = b[i * M];
-        blk_inv_last<B>(x, itw, c);
-#pragma unroll
-        for (int i = 0; i < B; i++) b[i * M] = x[i];
-    }
-    group_sync(bar, T);
-    for (int lb = 0; lb < NB; lb++) {
-        const int blk = s.rank * NB + lb;
-        // ---- 3. the digits' NTTs in the block, a group per digit
-        for (int dd = gi; dd < nd; dd += NG) {
-            const int p = dd / (DG - 1), h = dd - p * (DG - 1);
-            uint64_t z[B - 1];
-#pragma unroll
-            for (int i = 0; i < B - 1; i++) z[i] = s.zeta[lb][i];
-            uint64_t *const d = work + dd * ME;
-            blk_fwd_first<B, GS>(d, s.g + p * 2048, z, A.bg_bits * (uint32_t)h, mask, blk, gt, tw, c);
-            group_sync64<GS>(gi);
-            blk_fwd_pass<M, 3, GS>(d, blk, 32, gt, tw, c);   // t = 32 .. 8
-            group_sync64<GS>(gi);
-            blk_fwd_pass<M, 3, GS>(d, blk, 4, gt, tw, c);    // t = 4, 2, 1
-        }
-        const uint2 *const kb = keys(lb);
-        group_sync(bar, T);
-        // ---- multiply-accumulate
-        for (int k = tid; k < M; k += T) {
-            uint64_t sa[3] = {0, 0, 0}, sb[3] = {0, 0, 0};
-            const uint2 *kk = kb + k;
-            uint64_t *const a0 = acc + lb * ME + px(k);
-#pragma unroll 6
-            for (int h = 0; h < DG; h++, kk += 4 * row) {
-#pragma unroll
-                for (int p = 0; p < 2; p++) {
-                    const uint64_t v = h < DG - 1 ? work[(p * (DG - 1) + h) * ME + px(k)] : a0[p * px(NW)];
-                    const uint32_t x0 = (uint32_t)v & ((1u << 27) - 1), x1 = (uint32_t)(v >> 27);
-                    mac27(sa, x0, x1, KG ? __ldcg(kk + (p * 2 + 0) * row) : kk[(p * 2 + 0) * row]);
-                    mac27(sb, x0, x1, KG ? __ldcg(kk + (p * 2 + 1) * row) : kk[(p * 2 + 1) * row]);
-                }
-            }
-            a0[0] = mac27_reduce(sa, A.c54, c);
-            a0[px(NW)] = mac27_reduce(sb, A.c54, c);
-        }
-        group_sync(bar, T);
-        done(lb);
-    }
-}
-
-// Powers 1 .. B - 1 of the zeta of blocks first .. first + NB - 1.
-template <int B, int NB>
-__device__ __forceinline__ void block_zeta(uint64_t (*zeta)[B - 1], int first, const ulonglong2 *tw, const Ntt64Consts &c)
-{
-    const int tid = threadIdx.x;
-    if (tid < NB) {
-        const int d = first + tid;
-        const uint64_t w = tw[B / 2 + d / 2].x >> c.pm_s, z = (d & 1) ? c.Q - w : w;
-        uint64_t v = z;
-        for (int i = 0; i < B - 1; i++) {
-            zeta[tid][i] = v << c.pm_s;
-            v = (uint64_t)((unsigned __int128)v * z % c.Q);
-        }
-    }
 }
 
 // Latency form: one ciphertext per cluster of C CTAs at a time, its accumulator in
@@ -607,7 +284,42 @@ __global__ void limb_words64_kernel(const uint64_t *__restrict__ in, uint2 *__re
     }
 }
 
+// The same with the last-digit identity (derive_keys64_kernel) applied on the way, to
+// `count` RGSWs [DG][4][2048].
+__global__ void derive_limbs64_kernel(const uint64_t *__restrict__ in, uint2 *__restrict__ out, size_t count, int DG,
+                                      const ulonglong2 *__restrict__ cf, const __grid_constant__ Ntt64Consts c)
+{
+    constexpr size_t plane = 4 * 2048;
+    constexpr uint32_t m27 = (1u << 27) - 1;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count * plane;
+         i += (size_t)gridDim.x * blockDim.x) {
+        const size_t at = i / plane * (size_t)DG * plane + i % plane;
+        const uint64_t last = in[at + (size_t)(DG - 1) * plane] % c.Q;
+        for (int h = 0; h < DG; h++) {
+            uint64_t m = mul64<true>(last, cf[h], c), w;
+            m = m >= c.Q ? m - c.Q : m;
+            if (h + 1 < DG) {
+                const uint64_t k = in[at + (size_t)h * plane] % c.Q;
+                w = k >= m ? k - m : k + c.Q - m;
+            } else {
+                w = m;
+            }
+            out[at + (size_t)h * plane] = make_uint2((uint32_t)w & m27, (uint32_t)(w >> 27));
+        }
+    }
+}
+
 }  // namespace dev
+
+int launch_derive_limbs64(Context &c, const uint64_t *d_in, uint2 *d_out, size_t count, cudaStream_t st)
+{
+    if (!count) return FHEACC_OK;
+    dev::derive_limbs64_kernel<<<(unsigned)std::min<size_t>(count * 32, 4096), 256, 0, st>>>(
+        d_in, d_out, count, (int)c.p.digitG, c.d_cf64, c.nc64);
+    c.launches++;
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "derived limb words launch");
+}
 
 int launch_limb_words64(Context &c, const uint64_t *d_in, uint2 *d_out, size_t n, cudaStream_t st)
 {
@@ -690,7 +402,7 @@ int launch_blind_rotate64_blocks(Context &c, const dev::Br64Args &R, int max_cta
     A.btkey = c.d_btkey64_limbs; A.accs = R.accs; A.count = R.count;
     A.S = c.p.n * (int)c.p.digitR; A.DG = (int)c.p.digitG;
     A.bg_bits = c.p.BG_bits; A.Br = c.p.Br; A.flags = R.flags;
-    A.c54 = c.nc64.pm_c << (c.nc64.pm_s - 10);   // 2^54 = 2^(54-b) 2^b
+    A.c54 = limb_c54(c);
     A.status = c.d_status;
     A.wait_limit = c.tune.debug_wait_limit >= 0 ? (unsigned)c.tune.debug_wait_limit : dev::kKeyWaitLimit;
     // after the accumulators: claim words, done words, residues

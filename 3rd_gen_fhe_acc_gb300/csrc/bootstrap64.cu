@@ -740,6 +740,16 @@ int launch_rlwe_mult_rgsw64(Context &c, const uint64_t *d_acc, const uint64_t *d
     const size_t rw = (size_t)c.p.digitG * 4 * 2048;
     if (stride != 0 && stride != rw) return c.fail(FHEACC_EINVAL, "RGSW stride: 0 or one RGSW");
     const size_t words = (stride ? count : 1) * rw;
+    if (products64_apply(c)) {
+        int rc = ensure_scratch(c, c.io, words * sizeof(uint2));
+        if (!rc) rc = launch_derive_limbs64(c, d_rgsw, (uint2 *)c.io.ptr, words / rw, st);
+        if (rc) return rc;
+        Products64 A{};
+        A.in1 = d_acc; A.in_stride = 4096;
+        A.keys = (const uint2 *)c.io.ptr; A.key_stride = stride;
+        A.out = d_out; A.out_per = 1; A.out_s1 = 4096; A.count = count;
+        return launch_products64(c, A, st);
+    }
     // constant pairs of the RGSWs, after the last-digit identity when it applies
     // (2 of the 2 digitG digit NTTs of a product saved); a call of a few
     // products keeps the plain RGSWs, whose derivation would cost it more

@@ -135,6 +135,32 @@ __device__ __noinline__ void br64_output(const Br64Args &A, const Ntt64Consts &c
 // Blind rotation in block form (blind_rotate64.cu); R: inputs, outputs, flags and
 // the accumulator scratch, followed by the claim words and [count][n * digitR] bytes.
 int launch_blind_rotate64_blocks(Context &c, const dev::Br64Args &R, int max_ctas, cudaStream_t st);
+int launch_derive_limbs64(Context &c, const uint64_t *d_in, uint2 *d_out, size_t count, cudaStream_t st);
 int launch_limb_words64(Context &c, const uint64_t *d_in, uint2 *d_out, size_t n, cudaStream_t st);
+
+// RLWE x RGSW products in block form (products64.cu; moduli Q = 2^b - c). Product i: of
+// in1[i] (in0 null), in1[i] - in0[i], or in0[i] times rot minus in0[i] (rot: constant
+// pairs), i-th RLWEs in_stride words apart, with RGSW i (limb words with the last-digit
+// identity, launch_derive_limbs64; one RGSW for all: key_stride 0); plus in0[i] with
+// add0; to out + i / out_per * out_s1 + i % out_per * out_s2 words, and with copy_in the
+// input after it. All RLWEs canonical NTT, [2][2048]; out may be in0 or in1 of equal
+// strides.
+struct Products64 {
+    const uint64_t *in0, *in1;
+    size_t in_stride;
+    const ulonglong2 *rot;
+    const uint2 *keys;
+    size_t key_stride;
+    uint64_t *out;
+    size_t out_per, out_s1, out_s2;
+    int add0, copy_in;
+    size_t count;
+    int DG;
+    uint32_t bg_bits, c54;
+};
+int launch_products64(Context &c, Products64 A, cudaStream_t st);
+// Whether the block form's products and key words apply to the context.
+inline bool products64_apply(const Context &c) { return c.wide && c.nc64.pm_c && c.dp.last_digit_from_acc; }
+inline uint32_t limb_c54(const Context &c) { return c.nc64.pm_c << (c.nc64.pm_s - 10); }   // 2^54 = 2^(54-b) 2^b
 
 }  // namespace fheacc

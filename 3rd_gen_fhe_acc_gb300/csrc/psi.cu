@@ -13,6 +13,7 @@
 // addition, and the NTT-domain rotation RLWE_rotate_freq, RLWE.cpp:411-430).
 // Ciphertexts are canonical NTT-domain RLWEs, [count][2N] u64, as in the
 // reference; results are bit-identical to it.
+#include "br64.cuh"
 #include "ctx.hpp"
 #include <algorithm>
 
@@ -102,6 +103,18 @@ static int cmux_device(Context &c, const uint64_t *c0, const uint64_t *c1, size_
                        size_t sel_stride, uint64_t *out, size_t count, uint64_t *scratch, cudaStream_t st)
 {
     const size_t rw = 2 * (size_t)c.p.N;
+    if (products64_apply(c)) {
+        const size_t gw = (size_t)c.p.digitG * 4 * c.p.N, keys = sel_stride ? count : 1;
+        int rc = ensure_scratch(c, c.io, keys * gw * sizeof(uint2));
+        if (!rc) rc = launch_derive_limbs64(c, sel, (uint2 *)c.io.ptr, keys, st);
+        if (rc) return rc;
+        Products64 A{};
+        A.in0 = c0; A.in1 = c1; A.in_stride = in_stride;
+        A.keys = (const uint2 *)c.io.ptr; A.key_stride = sel_stride;
+        A.out = out; A.out_per = 1; A.out_s1 = rw;
+        A.add0 = 1; A.count = count;
+        return launch_products64(c, A, st);
+    }
     uint64_t *diff = scratch, *mult = scratch + count * rw;
     int rc = launch_elementwise(c, dev::kEwSub, c1, in_stride, c0, in_stride, nullptr, diff, count, st);
     if (!rc) rc = mult_rgsw(c, diff, sel, sel_stride, mult, count, st);
@@ -127,7 +140,7 @@ int fheacc_cmux_async(fheacc_ctx *ctx, const uint64_t *d_c0, const uint64_t *d_c
     if (!count) return FHEACC_OK;
     DeviceGuard g(c.device);
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = ensure_scratch(c, c.psi, 2 * count * rw * sizeof(uint64_t));
+    int rc = products64_apply(c) ? FHEACC_OK : ensure_scratch(c, c.psi, 2 * count * rw * sizeof(uint64_t));
     if (rc) return rc;
     const size_t gw = (size_t)c.p.digitG * 4 * c.p.N;
     return cmux_device(c, d_c0, d_c1, in_stride, d_sel, sel_shared ? 0 : gw, d_out, count, (uint64_t *)c.psi.ptr,
@@ -144,6 +157,22 @@ int fheacc_rlwe_blind_rotate_async(fheacc_ctx *ctx, const uint64_t *d_in, const 
     DeviceGuard g(c.device);
     cudaStream_t st = (cudaStream_t)stream;
     const int N = c.p.N, logN = c.wide ? 11 : 10;
+    if (products64_apply(c)) {
+        // the RGSWs' key words once, then one launch per CMUX: acc = CMUX(acc, acc rotated, C[i])
+        const size_t words = (size_t)c.p.digitG * 4 * N, rlwe = 2 * (size_t)N;
+        int rc = ensure_scratch(c, c.io, (size_t)logN * words * sizeof(uint2));
+        if (!rc) rc = launch_derive_limbs64(c, d_rgsws, (uint2 *)c.io.ptr, (size_t)logN, st);
+        for (int i = 0; i < logN && !rc; i++) {
+            Products64 A{};
+            A.in0 = i ? d_out : d_in; A.in_stride = rlwe;
+            A.rot = (forward ? c.d_rot_fwd64 : c.d_rot64) + (size_t)i * N;
+            A.keys = (const uint2 *)c.io.ptr + (size_t)i * words;
+            A.out = d_out; A.out_per = 1; A.out_s1 = rlwe;
+            A.add0 = 1; A.count = count;
+            rc = launch_products64(c, A, st);
+        }
+        return rc;
+    }
     const size_t rw = 2 * (size_t)N, gw = (size_t)c.p.digitG * 4 * N;
     // tmp (rotated acc) + the CMUX scratch
     int rc = ensure_scratch(c, c.psi, 3 * count * rw * sizeof(uint64_t));
@@ -172,6 +201,21 @@ int fheacc_homo_expand(fheacc_ctx *ctx, const uint64_t *d_packed, const uint64_t
     const size_t N = (size_t)c.p.N, rw = 2 * N, dG = c.p.digitG, gw = dG * 4 * N;
     // all digits at once: the dG x N expanded RLWEs (the dG expansions level by
     // level, one launch per level) and their products with enc_sec (one launch)
+    if (products64_apply(c)) {
+        int rc = ensure_scratch(c, c.psi, dG * N * rw * sizeof(uint64_t));
+        if (!rc) rc = ensure_scratch(c, c.io, gw * sizeof(uint2));
+        uint64_t *u = (uint64_t *)c.psi.ptr;
+        if (!rc) rc = expand_device(c, d_packed, u, st, dG);
+        if (!rc) rc = launch_derive_limbs64(c, d_enc_sec, (uint2 *)c.io.ptr, 1, st);
+        if (rc) return rc;
+        Products64 A{};
+        A.in1 = u; A.in_stride = rw;
+        A.keys = (const uint2 *)c.io.ptr;
+        // product j N + i to row j of RGSW i: c_text[j][0], with u[j][i] as c_text[j][1]
+        A.out = d_out; A.out_per = N; A.out_s1 = 2 * rw; A.out_s2 = gw;
+        A.copy_in = 1; A.count = dG * N;
+        return launch_products64(c, A, st);
+    }
     int rc = ensure_scratch(c, c.psi, 2 * dG * N * rw * sizeof(uint64_t));
     if (rc) return rc;
     uint64_t *u = (uint64_t *)c.psi.ptr, *m = u + dG * N * rw;
