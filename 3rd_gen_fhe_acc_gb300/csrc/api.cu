@@ -657,33 +657,37 @@ static int subs_key_pass(Context &c, const uint64_t *subs_key, size_t words, boo
     if (verify && !(c.wide ? (void *)c.d_subs64 : (void *)c.d_subs))
         return c.fail(FHEACC_ENOKEY, "substitute key not uploaded");
     if (c.wide) {
+        const bool limbs = products64_apply(c);
+        const size_t wb = limbs ? sizeof(uint2) : sizeof(ulonglong2);   // bytes of a device word
         if (!verify && !c.d_subs64) {
-            cudaError_t e = cudaMalloc(&c.d_subs64, words * sizeof(ulonglong2));
+            cudaError_t e = cudaMalloc(&c.d_subs64, words * wb);
             if (e != cudaSuccess) {
                 cudaGetLastError();
                 c.d_subs64 = nullptr;
                 return c.fail(FHEACC_ENOMEM, "device memory for the substitute key");
             }
-            c.subs_bytes = words * sizeof(ulonglong2);
+            c.subs_bytes = words * wb;
         }
         uint64_t *d_stage = nullptr;
-        ulonglong2 *d_check = nullptr;   // verify: the pairs as the upload makes them
+        void *d_check = nullptr;   // verify: the words as the upload makes them
         cudaError_t e = cudaMalloc(&d_stage, words * sizeof(uint64_t));
-        if (e == cudaSuccess && verify) e = cudaMalloc(&d_check, words * sizeof(ulonglong2));
+        if (e == cudaSuccess && verify) e = cudaMalloc(&d_check, words * wb);
         if (e == cudaSuccess) e = cudaMemcpy(d_stage, subs_key, words * sizeof(uint64_t), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
             cudaFree(d_stage);
             cudaFree(d_check);
             return c.cuda_fail(e, "substitute key upload");
         }
-        int rc = launch_const_pairs64(c, d_stage, verify ? d_check : c.d_subs64, words, c.stream);
-        if (!rc && cudaStreamSynchronize(c.stream) != cudaSuccess) rc = c.cuda_fail(cudaGetLastError(), "key pairs");
+        void *const to = verify ? d_check : c.d_subs64;
+        int rc = limbs ? launch_limb_words64(c, d_stage, (uint2 *)to, words, c.stream)
+                       : launch_const_pairs64(c, d_stage, (ulonglong2 *)to, words, c.stream);
+        if (!rc && cudaStreamSynchronize(c.stream) != cudaSuccess) rc = c.cuda_fail(cudaGetLastError(), "key words");
         if (!rc && verify) {
-            std::vector<ulonglong2> made(words), held(words);
-            e = cudaMemcpy(made.data(), d_check, words * sizeof(ulonglong2), cudaMemcpyDeviceToHost);
-            if (e == cudaSuccess) e = cudaMemcpy(held.data(), c.d_subs64, words * sizeof(ulonglong2), cudaMemcpyDeviceToHost);
+            std::vector<char> made(words * wb), held(words * wb);
+            e = cudaMemcpy(made.data(), d_check, words * wb, cudaMemcpyDeviceToHost);
+            if (e == cudaSuccess) e = cudaMemcpy(held.data(), c.d_subs64, words * wb, cudaMemcpyDeviceToHost);
             if (e != cudaSuccess) rc = c.cuda_fail(e, "key read-back");
-            else if (std::memcmp(made.data(), held.data(), words * sizeof(ulonglong2)) != 0)
+            else if (std::memcmp(made.data(), held.data(), words * wb) != 0)
                 rc = c.fail(FHEACC_EMISMATCH, "device substitute key differs from the given key");
         }
         cudaFree(d_stage);
@@ -947,7 +951,8 @@ int fheacc_measure_components(fheacc_ctx *ctx, double ns[4])
 static const void *subs_key_level(Context &c, int f)
 {
     const size_t per = (size_t)c.p.digitKS_R * 2 * c.p.N;
-    if (c.wide) return c.d_subs64 ? (const void *)(c.d_subs64 + (size_t)f * per) : nullptr;
+    const size_t wb = products64_apply(c) ? sizeof(uint2) : sizeof(ulonglong2);   // as uploaded
+    if (c.wide) return c.d_subs64 ? (const void *)((const char *)c.d_subs64 + (size_t)f * per * wb) : nullptr;
     return c.d_subs ? (const void *)(c.d_subs + (size_t)f * per) : nullptr;
 }
 
@@ -972,8 +977,9 @@ int fheacc_rlwe_keyswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t co
     const size_t words = (size_t)c.p.digitKS_R * 2 * c.p.N;
     int rc = ensure_scratch(c, c.io, words * (c.wide ? sizeof(ulonglong2) : sizeof(uint32_t)));
     if (rc) return rc;
-    rc = c.wide ? launch_const_pairs64(c, d_ksk, (ulonglong2 *)c.io.ptr, words, st)
-                : launch_to_u32(c, d_ksk, (uint32_t *)c.io.ptr, words, st);
+    rc = products64_apply(c) ? launch_limb_words64(c, d_ksk, (uint2 *)c.io.ptr, words, st)
+         : c.wide            ? launch_const_pairs64(c, d_ksk, (ulonglong2 *)c.io.ptr, words, st)
+                             : launch_to_u32(c, d_ksk, (uint32_t *)c.io.ptr, words, st);
     if (rc) return rc;
     return mark_done(c, st, launch_expand(c, 1, d_in, d_out, count, 0, c.io.ptr, st));
 }

@@ -95,29 +95,31 @@ __device__ __forceinline__ void blk_fwd_pass(uint64_t *d, int blk, int t, int gt
     }
 }
 
-// The first pass (M = 512: t = 256 .. 64; 256: t = 128, 64) with the digit's residue
-// mod X^M - zeta computed as it loads: word j is the digit of x[j] plus
-// z[i - 1] times the digit of x[j + i M].
-template <int B, int GS>
-__device__ __forceinline__ void blk_fwd_first(uint64_t *d, const uint64_t *x, const uint64_t (&z)[B - 1], uint32_t sh,
-                                              uint32_t mask, int blk, int gt, const ulonglong2 *__restrict__ tw,
-                                              const Ntt64Consts &c)
+// A word of a digit's residue: y(0) plus z[i - 1] (zeta^i times 2^pm_s) times y(i), y < 2^30.
+template <int B, class Y>
+__device__ __forceinline__ uint64_t digit_residue(const uint64_t (&z)[B - 1], const Ntt64Consts &c, Y y)
+{
+    uint64_t U = 0, V = 0;
+#pragma unroll
+    for (int i = 1; i < B; i++) {
+        const uint32_t v = y(i);
+        U = mad_wide64(v, (uint32_t)z[i - 1], U);
+        V = mad_wide64(v, (uint32_t)(z[i - 1] >> 32), V);
+    }
+    return fold64(U, V, c) + y(0);
+}
+
+// The first pass (M = 512: t = 256 .. 64; 256: t = 128, 64) of a polynomial's residue mod
+// X^M - zeta, computed as it loads: word(j, k) is word j + 64 k of the residue.
+template <int B, int GS, class Word>
+__device__ __forceinline__ void blk_fwd_first(uint64_t *d, Word word, int blk, int gt,
+                                              const ulonglong2 *__restrict__ tw, const Ntt64Consts &c)
 {
     constexpr int M = 2048 / B, R = M == 512 ? 3 : 2, K = 1 << R;
     for (int j = gt; j < 64; j += GS) {
         uint64_t v[K];
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-            const uint64_t *b = x + j + 64 * k;
-            uint64_t U = 0, V = 0;
-#pragma unroll
-            for (int i = 1; i < B; i++) {
-                const uint32_t y = (uint32_t)(b[i * M] >> sh) & mask;
-                U = mad_wide64(y, (uint32_t)z[i - 1], U);
-                V = mad_wide64(y, (uint32_t)(z[i - 1] >> 32), V);
-            }
-            v[k] = fold64(U, V, c) + ((uint32_t)(b[0] >> sh) & mask);
-        }
+        for (int k = 0; k < K; k++) v[k] = word(j, k);
 #pragma unroll
         for (int st = 0; st < R; st++) {
             const int dl = K >> (st + 1);
@@ -207,8 +209,8 @@ struct BlockCta {
 };
 
 // The accumulator's inverse NTT by T threads (tid < T) that share the named barrier `bar`
-// (0: the whole CTA): canonical coefficients of both polys in s.g.
-template <int B, int C, int T>
+// (0: the whole CTA): canonical coefficients of its NP polys in s.g.
+template <int B, int C, int T, int NP = 2>
 __device__ __forceinline__ void block_to_time(const BlockCta<B, C> &s, const ulonglong2 *__restrict__ itw,
                                               const Ntt64Consts &c, int tid, int bar)
 {
@@ -218,7 +220,7 @@ __device__ __forceinline__ void block_to_time(const BlockCta<B, C> &s, const ulo
     constexpr int GS = M == 512 && T == kTB ? 64 : 32, NG = T / GS;
     const int gi = tid / GS, gt = tid - gi * GS;
     // ---- 1. inverse stages inside the blocks, a group per block
-    for (int u = gi; u < 2 * NB; u += NG) {
+    for (int u = gi; u < NP * NB; u += NG) {
         const int p = u / NB, lb = u - p * NB, blk = s.rank * NB + lb, base = p * 2048 + blk * M;
         uint64_t *const w = work + u * ME;
         blk_inv_pass8<M, 1, false, GS>(acc + p * px(NW) + lb * ME, blk, 1, gt, itw, c, [&](int e0, uint64_t (&x)[8]) {
@@ -258,7 +260,7 @@ __device__ __forceinline__ void block_to_time(const BlockCta<B, C> &s, const ulo
     if (C > 1) cg::this_cluster().sync();
     else group_sync(bar, T);
     // ---- 2. last inverse stages of all words
-    for (int u = tid; u < 2 * M; u += T) {
+    for (int u = tid; u < NP * M; u += T) {
         uint64_t *const b = s.g + (u / M) * 2048 + u % M;
         uint64_t x[B];
 #pragma unroll
@@ -298,7 +300,12 @@ __device__ __forceinline__ void block_step(const BlockCta<B, C> &s, const Args &
 #pragma unroll
             for (int i = 0; i < B - 1; i++) z[i] = s.zeta[lb][i];
             uint64_t *const d = work + dd * ME;
-            blk_fwd_first<B, GS>(d, s.g + p * 2048, z, A.bg_bits * (uint32_t)h, mask, blk, gt, tw, c);
+            const uint64_t *const x = s.g + p * 2048;
+            const uint32_t sh = A.bg_bits * (uint32_t)h;
+            blk_fwd_first<B, GS>(d, [&](int j, int k) {
+                const uint64_t *b = x + j + 64 * k;
+                return digit_residue<B>(z, c, [&](int i) { return (uint32_t)(b[i * M] >> sh) & mask; });
+            }, blk, gt, tw, c);
             group_sync64<GS>(gi);
             blk_fwd_pass<M, 3, GS>(d, blk, 32, gt, tw, c);   // t = 32 .. 8
             group_sync64<GS>(gi);

@@ -130,7 +130,7 @@ struct Context {
     uint2 *d_btkey64_limbs = nullptr;
     ulonglong2 *d_btkey64 = nullptr;   // constant pairs, [(i*digitR + j)*Br + r][digitG][2][2][N]
     ulonglong2 *d_cf64 = nullptr;      // factors of the last-digit identity, digitG constant pairs
-    ulonglong2 *d_subs64 = nullptr;    // constant pairs, [logN][digitKS_R][2][N]
+    void *d_subs64 = nullptr;    // limb words or constant pairs, [logN][digitKS_R][2][N]
     // rotations, [logN][N]: NTT(-X^(N - 2^j)), rotate_vector_gen(false), and
     // NTT(X^(2^j)), rotate_vector_gen(true); wide: constant pairs
     uint64_t *d_rot = nullptr, *d_rot_fwd = nullptr;

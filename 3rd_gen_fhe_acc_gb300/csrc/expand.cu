@@ -19,6 +19,7 @@
 //   SUBS_KS   out = RLWE_keyswitch(RLWE_substitute(c, f), ksk)
 //   EXPAND    r[j] <- r[j] + s, r[j + 2^f] <- (r[j] - s) * NTT(-X^(N - 2^f)),
 //             s = SUBS_KS(r[j], f, subs_key[f]), for every j < 2^f (one level)
+#include "block64.cuh"
 #include "ctx.hpp"
 #include "step32.cuh"
 #include <algorithm>
@@ -39,6 +40,8 @@ struct ExpArgs {
     uint32_t ipow;           // (N / 2^f + 1)^-1 mod 2N
     const uint32_t *ksk32;   // [L][2][N] u32 (narrow)
     const ulonglong2 *ksk64; // [L][2][N] constant pairs (wide)
+    const uint2 *ksk_limbs;  // the same as limb words (wide, block form)
+    uint32_t c54, power;     // block form: 2^54 mod Q, N / 2^f + 1 (KS: 1)
     const uint64_t *rot;     // [N] NTT(-X^(N - 2^f)) (EXPAND, narrow)
     const ulonglong2 *rot64; // the same as constant pairs (wide)
     uint64_t Q, mu64;
@@ -160,7 +163,6 @@ struct LoadSubs64 {
 };
 
 // 256 threads in two 128-thread groups; group g transforms poly g.
-template <bool PM>
 __global__ void __launch_bounds__(256, 2) expand64_kernel(const __grid_constant__ ExpArgs A,
                                                       const ulonglong2 *__restrict__ tw,
                                                       const ulonglong2 *__restrict__ itw,
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(256, 2) expand64_kernel(const __grid_constant_
         const uint64_t *in = A.in + bo + jt * 4096;
         for (int e = gtid; e < 2048; e += 128) t[grp][px(e)] = in[grp * 2048 + e];
         group_sync(1 + grp, 128);
-        ntt64_inv_2048<PM, 128, true>(t[grp], itw, c, gtid, 1 + grp);
+        ntt64_inv_2048<false, 128, true>(t[grp], itw, c, gtid, 1 + grp);
         __syncthreads();
         // transforms: L digits of sigma(a) and sigma(b) (SUBS: sigma(a), sigma(b)),
         // two at a time; MAC after each pair
@@ -193,11 +195,11 @@ __global__ void __launch_bounds__(256, 2) expand64_kernel(const __grid_constant_
                 const int poly = A.mode == kSubs ? tr : (tr == L ? 1 : 0);
                 // A.ipow = 1 is the identity (kKs)
                 if (A.mode != kSubs && tr < L) {
-                    ntt64_fwd_2048_load<PM, 128, true, true>(
+                    ntt64_fwd_2048_load<false, 128, true, true>(
                         buf[grp], LoadSubs64{t[poly], Q, A.ipow, A.bits * (uint32_t)tr, (1u << A.bits) - 1}, tw, c, gtid,
                         1 + grp);
                 } else {
-                    ntt64_fwd_2048_load<PM, 128, true, false>(buf[grp], LoadSubs64{t[poly], Q, A.ipow, 0, 0}, tw, c,
+                    ntt64_fwd_2048_load<false, 128, true, false>(buf[grp], LoadSubs64{t[poly], Q, A.ipow, 0, 0}, tw, c,
                                                                gtid, 1 + grp);
                 }
             }
@@ -211,14 +213,14 @@ __global__ void __launch_bounds__(256, 2) expand64_kernel(const __grid_constant_
                     if (tr >= nt) continue;
                     const uint64_t dv = buf[g2][px(k)];
                     if (A.mode == kSubs || tr == L) {
-                        const uint64_t v = reduce64<PM>(dv, c);
+                        const uint64_t v = reduce64<false>(dv, c);
                         if (A.mode == kSubs && tr == 0) sa[i] = v;
                         else fb[i] = v;
                     } else {
                         const ulonglong2 ka = __ldg(A.ksk64 + (size_t)(tr * 2 + 0) * 2048 + k);
                         const ulonglong2 kb = __ldg(A.ksk64 + (size_t)(tr * 2 + 1) * 2048 + k);
-                        sa[i] += mul64<PM>(dv, ka, c);
-                        sb[i] += mul64<PM>(dv, kb, c);
+                        sa[i] += mul64<false>(dv, ka, c);
+                        sb[i] += mul64<false>(dv, kb, c);
                     }
                 }
             }
@@ -233,7 +235,7 @@ __global__ void __launch_bounds__(256, 2) expand64_kernel(const __grid_constant_
                 oa = sa[i] >= Q ? sa[i] - Q : sa[i];
                 ob = fb[i] >= Q ? fb[i] - Q : fb[i];
             } else {
-                uint64_t ra = reduce64<PM>(sa[i], c), rb = reduce64<PM>(sb[i], c);
+                uint64_t ra = reduce64<false>(sa[i], c), rb = reduce64<false>(sb[i], c);
                 ra = ra >= Q ? ra - Q : ra;
                 rb = rb >= Q ? rb - Q : rb;
                 const uint64_t nb = fb[i] >= Q ? fb[i] - Q : fb[i];
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(256, 2) expand64_kernel(const __grid_constant_
                 out[k] = s1 >= Q ? s1 - Q : s1;
                 out[2048 + k] = s2 >= Q ? s2 - Q : s2;
                 const uint64_t d1 = ta >= oa ? ta - oa : ta + Q - oa, d2 = tb >= ob ? tb - ob : tb + Q - ob;
-                const uint64_t h1 = mul64<PM>(d1, rot, c), h2 = mul64<PM>(d2, rot, c);
+                const uint64_t h1 = mul64<false>(d1, rot, c), h2 = mul64<false>(d2, rot, c);
                 hi[k] = h1 >= Q ? h1 - Q : h1;
                 hi[2048 + k] = h2 >= Q ? h2 - Q : h2;
             } else {
@@ -267,7 +269,6 @@ __global__ void __launch_bounds__(256, 2) expand64_kernel(const __grid_constant_
 // part[item][p] as [sa | sb | fb][2048], each word < 4Q. expand64_combine_kernel
 // adds the shares and applies the level's epilogue. One RLWE's transforms then
 // take two rounds instead of 1 + ceil((L + 1) / 2).
-template <bool PM>
 __global__ void __launch_bounds__(256) expand64_split_kernel(const __grid_constant__ ExpArgs A,
                                                             uint64_t *__restrict__ part, int P,
                                                             const ulonglong2 *__restrict__ tw,
@@ -287,15 +288,15 @@ __global__ void __launch_bounds__(256) expand64_split_kernel(const __grid_consta
     const uint64_t *in = A.in + bo + jt * 4096;
     for (int e = gtid; e < 2048; e += 128) t[grp][px(e)] = in[grp * 2048 + e];
     group_sync(1 + grp, 128);
-    ntt64_inv_2048<PM, 128, true>(t[grp], itw, c, gtid, 1 + grp);
+    ntt64_inv_2048<false, 128, true>(t[grp], itw, c, gtid, 1 + grp);
     __syncthreads();
     const int tr = 2 * p + grp;
     if (tr < nt) {
         if (tr < L)
-            ntt64_fwd_2048_load<PM, 128, true, true>(
+            ntt64_fwd_2048_load<false, 128, true, true>(
                 buf[grp], LoadSubs64{t[0], Q, A.ipow, A.bits * (uint32_t)tr, (1u << A.bits) - 1}, tw, c, gtid, 1 + grp);
         else
-            ntt64_fwd_2048_load<PM, 128, true, false>(buf[grp], LoadSubs64{t[1], Q, A.ipow, 0, 0}, tw, c, gtid,
+            ntt64_fwd_2048_load<false, 128, true, false>(buf[grp], LoadSubs64{t[1], Q, A.ipow, 0, 0}, tw, c, gtid,
                                                        1 + grp);
     }
     __syncthreads();
@@ -310,12 +311,12 @@ __global__ void __launch_bounds__(256) expand64_split_kernel(const __grid_consta
             if (tq >= nt) continue;
             const uint64_t dv = buf[g2][px(k)];
             if (tq == L) {
-                fb = reduce64<PM>(dv, c);
+                fb = reduce64<false>(dv, c);
             } else {
                 const ulonglong2 ka = __ldg(A.ksk64 + (size_t)(tq * 2 + 0) * 2048 + k);
                 const ulonglong2 kb = __ldg(A.ksk64 + (size_t)(tq * 2 + 1) * 2048 + k);
-                sa += mul64<PM>(dv, ka, c);
-                sb += mul64<PM>(dv, kb, c);
+                sa += mul64<false>(dv, ka, c);
+                sb += mul64<false>(dv, kb, c);
             }
         }
         o[k] = sa;
@@ -327,7 +328,6 @@ __global__ void __launch_bounds__(256) expand64_split_kernel(const __grid_consta
 // The shares of expand64_split_kernel added (P of them, < 4PQ < 2^64, checked
 // by the launcher) and the expand level's epilogue, one thread per item word:
 // s = (-sa, sigma(b) - sb), r[j] <- r[j] + s, r[j + 2^f] <- (r[j] - s) * rot.
-template <bool PM>
 __global__ void expand64_combine_kernel(const __grid_constant__ ExpArgs A, const uint64_t *__restrict__ part, int P,
                                         size_t items, const __grid_constant__ Ntt64Consts c)
 {
@@ -345,7 +345,7 @@ __global__ void expand64_combine_kernel(const __grid_constant__ ExpArgs A, const
             sb += pp[(size_t)(p * 3 + 1) * 2048];
             fb += pp[(size_t)(p * 3 + 2) * 2048];
         }
-        uint64_t ra = reduce64<PM>(sa, c), rb = reduce64<PM>(sb, c);
+        uint64_t ra = reduce64<false>(sa, c), rb = reduce64<false>(sb, c);
         ra = ra >= Q ? ra - Q : ra;
         rb = rb >= Q ? rb - Q : rb;
         const uint64_t nb = fb >= Q ? fb - Q : fb;
@@ -360,10 +360,183 @@ __global__ void expand64_combine_kernel(const __grid_constant__ ExpArgs A, const
         out[k] = s1 >= Q ? s1 - Q : s1;
         out[2048 + k] = s2 >= Q ? s2 - Q : s2;
         const uint64_t d1 = ta >= oa ? ta - oa : ta + Q - oa, d2 = tb >= ob ? tb - ob : tb + Q - ob;
-        const uint64_t h1 = mul64<PM>(d1, rot, c), h2 = mul64<PM>(d2, rot, c);
+        const uint64_t h1 = mul64<false>(d1, rot, c), h2 = mul64<false>(d2, rot, c);
         hi[k] = h1 >= Q ? h1 - Q : h1;
         hi[2048 + k] = h2 >= Q ? h2 - Q : h2;
     }
+}
+
+// ---- Block form (moduli Q = 2^b - c; block64.cuh), every mode. The automorphism permutes
+// the words of an NTT: word j is the value at psi^(2 rev(j) + 1), and p(X^power) there is
+// p at psi^(power (2 rev(j) + 1)). So sigma(b), of which only the NTT is needed, takes no
+// transform (nor does SUBS), and a step is one inverse NTT and the L digits' instead of
+// two and L + 1. A cluster of C CTAs per RLWE up to one RLWE per SM (a level of few RLWEs
+// is a chain of transforms: 16 us, 36 split over transform pairs with a second launch for
+// their sum), else three workers of 192 threads per CTA, a warp per digit. The large
+// levels are bound by the multiply pipe.
+
+// Where word e of the NTT of the substituted polynomial comes from.
+__device__ __forceinline__ uint32_t subs_ntt_src(uint32_t e, uint32_t power)
+{
+    const uint32_t x = ((2 * (__brev(e) >> 21) + 1) * power) & 4095;
+    return __brev(x >> 1) >> 21;
+}
+
+// Shared memory: as BlockLayout with one poly to transform; g: [GBUF][2][2048] (a's
+// coefficients; b as it came in), acc: sigma(a) afterwards (C = 1).
+template <int B, int C>
+struct ExpandLayout {
+    using L = BlockLayout<B, C>;
+    static constexpr size_t work_off = L::acc_off + (size_t)(C == 1 ? px(2048) : L::NB * L::ME) * 8;
+    static size_t __host__ __device__ bytes(int nd) { return work_off + (size_t)(nd > L::NB ? nd : L::NB) * L::ME * 8; }
+};
+
+// RLWE `it` on the CTA's blocks by T threads.
+template <int B, int C, int T>
+__device__ __forceinline__ void expand_item(const BlockCta<B, C> &s, const ExpArgs &A, size_t it,
+                                            const ulonglong2 *__restrict__ tw, const ulonglong2 *__restrict__ itw,
+                                            const Ntt64Consts &c, int tid, int bar)
+{
+    using L = BlockLayout<B, C>;
+    constexpr int M = L::M, NB = L::NB, ME = L::ME, NW = NB * M;
+    constexpr int GS = M == 512 && T == kTB ? 64 : 32, NG = T / GS;
+    const int gi = tid / GS, gt = tid - gi * GS, first = s.rank * NW;
+    const size_t per = A.mode == kExpand ? ((size_t)1 << A.f) : A.count;
+    const size_t bo = it / per * A.bstride, jt = it % per;   // batch offset, item within the batch
+    const uint64_t *in = A.in + bo + jt * 4096;
+    uint64_t *out = A.out + bo + jt * 4096;
+    const uint64_t Q = c.Q;
+    uint64_t *const gb = s.g + 2048;   // b
+    for (int e = tid; e < 2048; e += T) gb[e] = in[2048 + e];
+    if (A.mode == kSubs) {
+        for (int e = tid; e < 2048; e += T) s.g[e] = in[e];
+        if (C > 1) cg::this_cluster().sync();   // out may be in
+        else group_sync(bar, T);
+        for (int u = tid; u < 2 * NW; u += T) {
+            const int p = u / NW, e = first + u - p * NW;
+            out[p * 2048 + e] = s.g[p * 2048 + subs_ntt_src((uint32_t)e, A.power)];
+        }
+        group_sync(bar, T);
+        return;
+    }
+    for (int e = tid; e < NW; e += T) s.acc[px(e)] = in[first + e];
+    group_sync(bar, T);
+    block_to_time<B, C, T, 1>(s, itw, c, tid, bar);
+    // sigma(a) once for all digits, into the accumulator's words (C = 1, free by now) or
+    // the other g buffer (one RLWE per cluster: free)
+    uint64_t *const sg = C == 1 ? s.acc : s.g + 4096;
+    for (int e = tid; e < 2048; e += T) {
+        bool neg;
+        const uint64_t v = s.g[subs_src((uint32_t)e, A.ipow, 2048, neg)];
+        sg[e] = neg && v ? Q - v : v;
+    }
+    group_sync(bar, T);
+    const int nd = A.L;
+    const uint32_t mask = (1u << A.bits) - 1;
+    for (int lb = 0; lb < NB; lb++) {
+        const int blk = s.rank * NB + lb;
+        for (int dd = gi; dd < nd; dd += NG) {
+            uint64_t *const d = s.work + dd * ME;
+            const uint32_t sh = A.bits * (uint32_t)dd;
+            uint64_t z[B - 1];
+#pragma unroll
+            for (int i = 0; i < B - 1; i++) z[i] = s.zeta[lb][i];
+            blk_fwd_first<B, GS>(d, [&](int j, int k) {
+                const uint64_t *b = sg + j + 64 * k;
+                return digit_residue<B>(z, c, [&](int i) { return (uint32_t)(b[i * M] >> sh) & mask; });
+            }, blk, gt, tw, c);
+            group_sync64<GS>(gi);
+            blk_fwd_pass<M, 3, GS>(d, blk, 32, gt, tw, c);
+            group_sync64<GS>(gi);
+            blk_fwd_pass<M, 3, GS>(d, blk, 4, gt, tw, c);
+        }
+        group_sync(bar, T);
+        for (int k = tid; k < M; k += T) {
+            const int e = blk * M + k;
+            uint64_t sa[3] = {0, 0, 0}, sb[3] = {0, 0, 0};
+            const uint2 *kk = A.ksk_limbs + e;
+#pragma unroll 3
+            for (int h = 0; h < nd; h++, kk += 4096) {
+                const uint64_t v = s.work[h * ME + px(k)];
+                const uint32_t x0 = (uint32_t)v & ((1u << 27) - 1), x1 = (uint32_t)(v >> 27);
+                mac27(sa, x0, x1, __ldcg(kk));
+                mac27(sb, x0, x1, __ldcg(kk + 2048));
+            }
+            uint64_t ra = mac27_reduce(sa, A.c54, c), rb = mac27_reduce(sb, A.c54, c);
+            ra = ra >= Q ? ra - Q : ra;
+            rb = rb >= Q ? rb - Q : rb;
+            const uint64_t nb = gb[subs_ntt_src((uint32_t)e, A.power)];
+            const uint64_t oa = ra ? Q - ra : 0;
+            const uint64_t ob = nb >= rb ? nb - rb : nb + Q - rb;
+            if (A.mode == kExpand) {
+                const uint64_t ta = in[e], tb = gb[e];
+                const ulonglong2 rot = __ldg(A.rot64 + e);
+                uint64_t *hi = A.out + bo + (jt + per) * 4096;
+                const uint64_t s1 = ta + oa, s2 = tb + ob;
+                out[e] = s1 >= Q ? s1 - Q : s1;
+                out[2048 + e] = s2 >= Q ? s2 - Q : s2;
+                const uint64_t d1 = ta >= oa ? ta - oa : ta + Q - oa, d2 = tb >= ob ? tb - ob : tb + Q - ob;
+                const uint64_t h1 = mul64<true>(d1, rot, c), h2 = mul64<true>(d2, rot, c);
+                hi[e] = h1 >= Q ? h1 - Q : h1;
+                hi[2048 + e] = h2 >= Q ? h2 - Q : h2;
+            } else {
+                out[e] = oa;
+                out[2048 + e] = ob;
+            }
+        }
+        group_sync(bar, T);
+    }
+}
+
+template <int B, int C>
+__global__ void __launch_bounds__(kTB, 1) expand64_cluster_kernel(const __grid_constant__ ExpArgs A, size_t items,
+                                                                 const ulonglong2 *__restrict__ tw,
+                                                                 const ulonglong2 *__restrict__ itw,
+                                                                 const __grid_constant__ Ntt64Consts c)
+{
+    using L = BlockLayout<B, C>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ uint64_t zeta[L::NB][B - 1];
+    uint64_t *const g = reinterpret_cast<uint64_t *>(smem_raw + L::g_off);
+    const int rank = C > 1 ? (int)(blockIdx.x % C) : 0;
+    BlockCta<B, C> cta{g, reinterpret_cast<uint64_t *>(smem_raw + L::acc_off),
+                       reinterpret_cast<uint64_t *>(smem_raw + ExpandLayout<B, C>::work_off), {}, zeta, rank};
+    cta.peer[0] = g;
+    if (C > 1) {
+        cg::cluster_group cl = cg::this_cluster();
+#pragma unroll
+        for (int r = 0; r < C; r++) cta.peer[r] = cl.map_shared_rank(g, r);
+    }
+    block_zeta<B, L::NB>(zeta, rank * L::NB, tw, c);
+    if (C > 1) cg::this_cluster().sync();
+    else __syncthreads();
+    // one RLWE per cluster (the launcher's rule)
+    if (blockIdx.x / C < items)
+        expand_item<B, C, kTB>(cta, A, blockIdx.x / C, tw, itw, c, threadIdx.x, 0);
+    if (C > 1) cg::this_cluster().sync();
+}
+
+constexpr int kTE = 192;   // threads of an expand worker
+
+template <int B, int W>
+__global__ void __launch_bounds__(W * kTE, 1) expand64_workers_kernel(const __grid_constant__ ExpArgs A, size_t items,
+                                                                     int worker_bytes,
+                                                                     const ulonglong2 *__restrict__ tw,
+                                                                     const ulonglong2 *__restrict__ itw,
+                                                                     const __grid_constant__ Ntt64Consts c)
+{
+    using L = BlockLayout<B, 1>;
+    extern __shared__ __align__(128) unsigned char smem_all[];
+    __shared__ uint64_t zeta[B][B - 1];
+    const int wk = threadIdx.x / kTE, tid = threadIdx.x - wk * kTE;
+    unsigned char *const smem_raw = smem_all + wk * worker_bytes;
+    uint64_t *const g = reinterpret_cast<uint64_t *>(smem_raw + L::g_off);
+    block_zeta<B, B>(zeta, 0, tw, c);
+    __syncthreads();
+    const BlockCta<B, 1> cta{g, reinterpret_cast<uint64_t *>(smem_raw + L::acc_off),
+                             reinterpret_cast<uint64_t *>(smem_raw + ExpandLayout<B, 1>::work_off), {g}, zeta, 0};
+    for (size_t it = (size_t)wk * gridDim.x + blockIdx.x; it < items; it += (size_t)gridDim.x * W)
+        expand_item<B, 1, kTE>(cta, A, it, tw, itw, c, tid, 1 + wk);
 }
 
 __global__ void to_u32_kernel(const uint64_t *__restrict__ in, uint32_t *__restrict__ out, size_t n, uint64_t Q)
@@ -389,7 +562,73 @@ static uint32_t inv_power(int N, int f)
     return 1;
 }
 
-// ksk: narrow, u32 [L][2][N] device words; wide, constant pairs (mul64).
+template <int B, int C>
+static int launch_expand_cluster(Context &c, const dev::ExpArgs &A, size_t items, cudaStream_t st, bool *fits)
+{
+    auto kern = dev::expand64_cluster_kernel<B, C>;
+    const size_t smem = dev::ExpandLayout<B, C>::bytes(A.L);
+    *fits = false;
+    if (smem > 227 * 1024 || items * C > (size_t)sms(c)) return FHEACC_OK;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return c.cuda_fail(e, "expand smem attribute");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(items * C));
+    cfg.blockDim = dim3(dev::kTB);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    if (C > 1) {
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return FHEACC_OK;
+        }
+        if (items > (size_t)n) return FHEACC_OK;   // more than one round: fewer CTAs per RLWE
+    }
+    *fits = true;
+    e = cudaLaunchKernelEx(&cfg, kern, A, items, (const ulonglong2 *)c.d_tw64, (const ulonglong2 *)c.d_itw64, c.nc64);
+    c.launches++;
+    if (e == cudaSuccess) e = cudaGetLastError();
+    return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "expand launch");
+}
+
+template <int W>
+static int launch_expand_workers(Context &c, const dev::ExpArgs &A, size_t items, cudaStream_t st)
+{
+    auto kern = dev::expand64_workers_kernel<4, W>;
+    const int bytes = (int)dev::ExpandLayout<4, 1>::bytes(A.L);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, W * bytes);
+    if (e != cudaSuccess) return c.cuda_fail(e, "expand smem attribute");
+    kern<<<(unsigned)std::min<size_t>(items, (size_t)sms(c)), W * dev::kTE, W * bytes, st>>>(
+        A, items, bytes, c.d_tw64, c.d_itw64, c.nc64);
+    c.launches++;
+    e = cudaGetLastError();
+    return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "expand launch");
+}
+
+// The block form of a launch of `items` RLWEs.
+static int launch_expand_blocks(Context &c, const dev::ExpArgs &A, size_t items, cudaStream_t st)
+{
+    bool fits = false;
+    int rc = FHEACC_OK;
+    if (A.bits <= 29) rc = launch_expand_cluster<8, 8>(c, A, items, st, &fits);
+    if (!rc && !fits) rc = launch_expand_cluster<4, 4>(c, A, items, st, &fits);
+    if (!rc && !fits) rc = launch_expand_cluster<4, 2>(c, A, items, st, &fits);
+    if (!rc && !fits) rc = launch_expand_cluster<4, 1>(c, A, items, st, &fits);
+    if (rc || fits) return rc;
+    const size_t one = dev::ExpandLayout<4, 1>::bytes(A.L), most = 227 * 1024 - 512;   // 512: the kernel's static part
+    return 3 * one <= most   ? launch_expand_workers<3>(c, A, items, st)
+           : 2 * one <= most ? launch_expand_workers<2>(c, A, items, st)
+                             : launch_expand_workers<1>(c, A, items, st);
+}
+
+// ksk: narrow, u32 [L][2][N] device words; wide, limb words (block form,
+// products64_apply) or constant pairs (mul64).
 int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, size_t count, int f,
                   const void *ksk, cudaStream_t st, size_t batches, size_t bstride)
 {
@@ -412,6 +651,12 @@ int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, s
     cudaError_t e;
     if (c.wide) {
         if (A.L > 8) return c.fail(FHEACC_EINVAL, "digitKS_R too large");
+        if (products64_apply(c)) {
+            A.ksk_limbs = (const uint2 *)ksk;
+            A.c54 = limb_c54(c);
+            A.power = mode == dev::kKs ? 1u : (uint32_t)(c.p.N >> f) + 1u;
+            return launch_expand_blocks(c, A, items, st);
+        }
         A.ksk64 = (const ulonglong2 *)ksk;
         const size_t smem = 4 * dev::kPoly64 * sizeof(uint64_t);
         // an expand level of at most two CTAs per SM of (item, transform pair)
@@ -422,20 +667,20 @@ int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, s
             int rc = ensure_scratch(c, c.expand, words * sizeof(uint64_t));
             if (rc) return rc;
             uint64_t *part = (uint64_t *)c.expand.ptr;
-            auto split = c.nc64.pm_c ? dev::expand64_split_kernel<true> : dev::expand64_split_kernel<false>;
+            auto split = dev::expand64_split_kernel;
             cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             split<<<(unsigned)(items * P), 256, smem, st>>>(A, part, P, c.d_tw64, c.d_itw64, c.nc64);
             c.launches++;
             e = cudaGetLastError();
             if (e != cudaSuccess) return c.cuda_fail(e, "expand split launch");
             const unsigned cb = (unsigned)std::min<size_t>((items * 2048 + 255) / 256, (size_t)sms(c) * 4);
-            auto combine = c.nc64.pm_c ? dev::expand64_combine_kernel<true> : dev::expand64_combine_kernel<false>;
+            auto combine = dev::expand64_combine_kernel;
             combine<<<cb, 256, 0, st>>>(A, part, P, items, c.nc64);
             c.launches++;
             e = cudaGetLastError();
             return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "expand combine launch");
         }
-        auto kern = c.nc64.pm_c ? dev::expand64_kernel<true> : dev::expand64_kernel<false>;
+        auto kern = dev::expand64_kernel;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         kern<<<(unsigned)blocks, 256, smem, st>>>(A, c.d_tw64, c.d_itw64, c.nc64);
         c.launches++;
