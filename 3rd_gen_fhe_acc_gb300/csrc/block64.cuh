@@ -15,22 +15,22 @@ namespace cg = cooperative_groups;
 // at once in the latency form, half of them in the throughput form (two CTAs per SM).
 constexpr int kTB = 640, kTP = 320;
 
-// x w of the MAC: sums[0] + 2^27 sums[1] + 2^54 sums[2] (x < 2^59, limbs < 2^27,
-// at most 16 products: sums[1] < 16 (2^59 + 2^54) < 2^64).
+// x w of the MAC, x = x1 2^27 + x0 < 2^59 and limbs w < 2^27: the sums of x0 w0, of
+// (x0 + x1) (w0 + w1) and of x1 w1, three multiplies (Karatsuba; four without: 2048 gates
+// 1 % slower). At most 16 products: the middle sum < 16 2^31.6 2^28 < 2^64.
 __device__ __forceinline__ void mac27(uint64_t (&s)[3], uint32_t x0, uint32_t x1, uint2 w)
 {
     s[0] += mul_wide64(x0, w.x);
-    s[1] += mul_wide64(x0, w.y);
-    s[1] += mul_wide64(x1, w.x);
+    s[1] += mul_wide64(x0 + x1, w.x + w.y);
     s[2] += mul_wide64(x1, w.y);
 }
 
-// The value of the sums mod Q, below 2Q: c54 (2^54 mod Q, below 2^19) folds the part
+// The value sums[0] + 2^27 (sums[1] - sums[0] - sums[2]) + 2^54 sums[2] mod Q, below 2Q: c54 (2^54 mod Q, below 2^19) folds the part
 // Y above 2^54 (Y < 2^64) twice.
 __device__ __forceinline__ uint64_t mac27_reduce(const uint64_t (&s)[3], uint32_t c54, const Ntt64Consts &c)
 {
     constexpr uint64_t m27 = (1u << 27) - 1;
-    const uint64_t T = s[1] + (s[0] >> 27);
+    const uint64_t T = s[1] - s[0] - s[2] + (s[0] >> 27);
     const uint64_t low = (s[0] & m27) | ((T & m27) << 27);
     const uint64_t Y = s[2] + (T >> 27);
     const uint64_t zl = mul_wide64((uint32_t)Y, c54);
