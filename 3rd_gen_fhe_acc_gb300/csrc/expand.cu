@@ -41,7 +41,7 @@ struct ExpArgs {
     const uint32_t *ksk32;   // [L][2][N] u32 (narrow)
     const ulonglong2 *ksk64; // [L][2][N] constant pairs (wide)
     const uint2 *ksk_limbs;  // the same as limb words (wide, block form)
-    uint32_t c54, power;     // block form: 2^54 mod Q, N / 2^f + 1 (KS: 1)
+    uint32_t c54, power;     // 2^54 mod Q (block form); N / 2^f + 1 (KS: 1)
     const uint64_t *rot;     // [N] NTT(-X^(N - 2^f)) (EXPAND, narrow)
     const ulonglong2 *rot64; // the same as constant pairs (wide)
     uint64_t Q, mu64;
@@ -54,9 +54,18 @@ __device__ __forceinline__ uint32_t subs_src(uint32_t e, uint32_t ipow, uint32_t
     return neg ? ip - N : ip;
 }
 
+// Where word e of the NTT of the substituted polynomial comes from: word j of an NTT is
+// the value at psi^(2 rev(j) + 1), and p(X^power) there is p at psi^(power (2 rev(j) + 1)).
+__device__ __forceinline__ uint32_t subs_ntt_src(uint32_t e, uint32_t power, int logN)
+{
+    const uint32_t x = ((2 * (__brev(e) >> (32 - logN)) + 1) * power) & ((2u << logN) - 1);
+    return __brev(x >> 1) >> (32 - logN);
+}
+
 // ---------------------------------------------------------------- narrow
-// 8 warps: warps 0/1 inverse NTTs, then warps 0..L-1 the digits of sigma(a)
-// and warp L sigma(b), then all threads the MAC and the epilogue.
+// 8 warps: warp 0 the inverse NTT of a, then warps 0..L-1 the digits of sigma(a),
+// then all threads the MAC and the epilogue. Only NTT(sigma(b)) is needed, whose words
+// the automorphism permutes (subs_ntt_src), so b takes no transform, nor does SUBS.
 __global__ void __launch_bounds__(256) expand32_kernel(const __grid_constant__ ExpArgs A,
                                                       const __grid_constant__ Ntt32Consts c,
                                                       const uint2 *__restrict__ fwd_tw,
@@ -67,42 +76,39 @@ __global__ void __launch_bounds__(256) expand32_kernel(const __grid_constant__ E
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t Q = c.Q;
     const int L = A.L;
-    const bool subs = A.mode != kKs;
     const size_t per = A.mode == kExpand ? ((size_t)1 << A.f) : A.count;
     const size_t items = per * A.batches;
     for (size_t it = blockIdx.x; it < items; it += gridDim.x) {
         const size_t bo = it / per * A.bstride, jt = it % per;   // batch offset, item within the batch
         const uint64_t *in = A.in + bo + jt * 2048;
-        if (warp < 2) {
+        // a to the time domain (warp 0); b, and a of SUBS, as NTTs (subs_ntt_src)
+        if (warp == 0 && A.mode != kSubs) {
             uint32_t x[32];
 #pragma unroll
-            for (int r = 0; r < 32; r++) x[r] = (uint32_t)in[warp * 1024 + 32 * lane + r];
+            for (int r = 0; r < 32; r++) x[r] = (uint32_t)in[32 * lane + r];
             ntt_inv_1024(x, c, inv_tw, d[warp], lane);
 #pragma unroll
-            for (int r = 0; r < 32; r++) t[warp][pad32(lane + 32 * r)] = x[r];
+            for (int r = 0; r < 32; r++) t[0][pad32(lane + 32 * r)] = x[r];
+        } else if (warp >= 1) {
+            for (int e = threadIdx.x - 32; e < 1024; e += blockDim.x - 32) {
+                const uint32_t v = (uint32_t)in[1024 + e];
+                t[1][pad32(e)] = min(v, v - Q);
+                if (A.mode == kSubs) {
+                    const uint32_t u = (uint32_t)in[e];
+                    t[0][pad32(e)] = min(u, u - Q);
+                }
+            }
         }
         __syncthreads();
-        const int nt = A.mode == kSubs ? 2 : L + 1;   // transforms of phase 2
-        if (warp < nt) {
-            // kSubs: warps 0, 1 transform sigma(a), sigma(b); else warps < L
-            // the digits of sigma(a) and warp L sigma(b)
-            const int poly = A.mode == kSubs ? warp : (warp == L ? 1 : 0);
-            const bool digit = A.mode != kSubs && warp < L;
+        if (A.mode != kSubs && warp < L) {   // the digits of sigma(a)
             const uint32_t sh = A.bits * (uint32_t)warp, mask = (1u << A.bits) - 1;
             uint32_t x[32];
 #pragma unroll
             for (int r = 0; r < 32; r++) {
-                const uint32_t e = lane + 32 * r;
-                uint32_t v;
-                if (subs) {
-                    bool neg;
-                    const uint32_t s = subs_src(e, A.ipow, 1024, neg);
-                    v = t[poly][pad32(s)];
-                    if (neg && v) v = Q - v;
-                } else {
-                    v = t[poly][pad32(e)];
-                }
-                x[r] = digit ? (v >> sh) & mask : v;
+                bool neg;
+                uint32_t v = t[0][pad32(subs_src(lane + 32 * r, A.ipow, 1024, neg))];   // ipow = 1 for KS
+                if (neg && v) v = Q - v;
+                x[r] = (v >> sh) & mask;
             }
             ntt_fwd_1024(x, c, fwd_tw, d[warp], lane);
 #pragma unroll
@@ -113,8 +119,9 @@ __global__ void __launch_bounds__(256) expand32_kernel(const __grid_constant__ E
         for (int k = threadIdx.x; k < 1024; k += blockDim.x) {
             uint64_t oa, ob;
             if (A.mode == kSubs) {
-                oa = d[0][pad32(k)];
-                ob = d[1][pad32(k)];
+                const uint32_t j = subs_ntt_src((uint32_t)k, A.power, 10);
+                oa = t[0][pad32(j)];
+                ob = t[1][pad32(j)];
             } else {
                 uint64_t sa = 0, sb = 0;
                 for (int h = 0; h < L; h++) {
@@ -125,7 +132,7 @@ __global__ void __launch_bounds__(256) expand32_kernel(const __grid_constant__ E
                 const uint32_t ra = barrett64_lazy(sa, A.mu64, Q), rb = barrett64_lazy(sb, A.mu64, Q);
                 const uint32_t ca = min(ra, ra - Q), cb = min(rb, rb - Q);
                 oa = ca ? Q - ca : 0;
-                const uint32_t nb = d[L][pad32(k)];
+                const uint32_t nb = t[1][pad32(subs_ntt_src((uint32_t)k, A.power, 10))];
                 ob = nb >= cb ? nb - cb : nb + Q - cb;
             }
             if (A.mode == kExpand) {
@@ -367,20 +374,12 @@ __global__ void expand64_combine_kernel(const __grid_constant__ ExpArgs A, const
 }
 
 // ---- Block form (moduli Q = 2^b - c; block64.cuh), every mode. The automorphism permutes
-// the words of an NTT: word j is the value at psi^(2 rev(j) + 1), and p(X^power) there is
-// p at psi^(power (2 rev(j) + 1)). So sigma(b), of which only the NTT is needed, takes no
+// the words of an NTT (subs_ntt_src), so sigma(b), of which only the NTT is needed, takes no
 // transform (nor does SUBS), and a step is one inverse NTT and the L digits' instead of
 // two and L + 1. A cluster of C CTAs per RLWE up to one RLWE per SM (a level of few RLWEs
 // is a chain of transforms: 16 us, 36 split over transform pairs with a second launch for
 // their sum), else three workers of 192 threads per CTA, a warp per digit. The large
 // levels are bound by the multiply pipe.
-
-// Where word e of the NTT of the substituted polynomial comes from.
-__device__ __forceinline__ uint32_t subs_ntt_src(uint32_t e, uint32_t power)
-{
-    const uint32_t x = ((2 * (__brev(e) >> 21) + 1) * power) & 4095;
-    return __brev(x >> 1) >> 21;
-}
 
 // Shared memory: as BlockLayout with one poly to transform; g: [GBUF][2][2048] (a's
 // coefficients; b as it came in), acc: sigma(a) afterwards (C = 1).
@@ -407,14 +406,14 @@ __device__ __forceinline__ void expand_item(const BlockCta<B, C> &s, const ExpAr
     uint64_t *out = A.out + bo + jt * 4096;
     const uint64_t Q = c.Q;
     uint64_t *const gb = s.g + 2048;   // b
-    for (int e = tid; e < 2048; e += T) gb[e] = in[2048 + e];
+    for (int e = tid; e < 2048; e += T) gb[e] = canonical64<true>(in[2048 + e], c);
     if (A.mode == kSubs) {
-        for (int e = tid; e < 2048; e += T) s.g[e] = in[e];
+        for (int e = tid; e < 2048; e += T) s.g[e] = canonical64<true>(in[e], c);
         if (C > 1) cg::this_cluster().sync();   // out may be in
         else group_sync(bar, T);
         for (int u = tid; u < 2 * NW; u += T) {
             const int p = u / NW, e = first + u - p * NW;
-            out[p * 2048 + e] = s.g[p * 2048 + subs_ntt_src((uint32_t)e, A.power)];
+            out[p * 2048 + e] = s.g[p * 2048 + subs_ntt_src((uint32_t)e, A.power, 11)];
         }
         group_sync(bar, T);
         return;
@@ -465,7 +464,7 @@ __device__ __forceinline__ void expand_item(const BlockCta<B, C> &s, const ExpAr
             uint64_t ra = mac27_reduce(sa, A.c54, c), rb = mac27_reduce(sb, A.c54, c);
             ra = ra >= Q ? ra - Q : ra;
             rb = rb >= Q ? rb - Q : rb;
-            const uint64_t nb = gb[subs_ntt_src((uint32_t)e, A.power)];
+            const uint64_t nb = gb[subs_ntt_src((uint32_t)e, A.power, 11)];
             const uint64_t oa = ra ? Q - ra : 0;
             const uint64_t ob = nb >= rb ? nb - rb : nb + Q - rb;
             if (A.mode == kExpand) {
@@ -641,6 +640,7 @@ int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, s
     A.L = (int)c.p.digitKS_R; A.bits = c.p.Bks_R_bits; A.ipow = inv_power(c.p.N, mode == dev::kKs ? 0 : f);
     A.Q = c.p.Q; A.mu64 = c.dp.mu64;
     if (mode == dev::kKs) A.ipow = 1;
+    A.power = mode == dev::kKs ? 1u : (uint32_t)(c.p.N >> f) + 1u;
     if (mode == dev::kExpand) {
         if (c.wide) A.rot64 = c.d_rot64 + (size_t)f * c.p.N;
         else A.rot = c.d_rot + (size_t)f * c.p.N;
@@ -654,7 +654,6 @@ int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, s
         if (products64_apply(c)) {
             A.ksk_limbs = (const uint2 *)ksk;
             A.c54 = limb_c54(c);
-            A.power = mode == dev::kKs ? 1u : (uint32_t)(c.p.N >> f) + 1u;
             return launch_expand_blocks(c, A, items, st);
         }
         A.ksk64 = (const ulonglong2 *)ksk;
