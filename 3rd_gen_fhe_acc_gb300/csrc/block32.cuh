@@ -208,12 +208,13 @@ struct Block32Cta {
 };
 
 // One step of the CTA's blocks by T threads (tid < T) that share named barrier `bar` (0:
-// the CTA). key: the RGSW's rows of the CTA's blocks, in B-tile order (KG: global
-// memory). mid(0), mid(1), mid(2): run before the barrier of 1, at the start of 3 and
+// the CTA). key: the RGSW's rows of the CTA's blocks, in B-tile order, in shared memory,
+// or (KG: C = 1, global memory) in global memory but for its first KP, which are at
+// head. mid(0), mid(1), mid(2): run before the barrier of 1, at the start of 3 and
 // before the products.
-template <int DG, int C, int T, bool KG, class Mid>
+template <int DG, int C, int T, bool KG, int KP, class Mid>
 __device__ __forceinline__ void block32_step(const Block32Cta<C> &s, const PipeArgs &A, const Ntt32Consts &c,
-                                             const uint32_t *key, int tid, int bar, Mid mid)
+                                             const uint32_t *key, const uint32_t *head, int tid, int bar, Mid mid)
 {
     constexpr int NB = 4 / C, ND = 2 * (DG - 1), NW = T / 32;
     const int warp = tid >> 5, lane = tid & 31;
@@ -309,7 +310,9 @@ __device__ __forceinline__ void block32_step(const Block32Cta<C> &s, const PipeA
 #pragma unroll
                 for (int o = 0; o < PP; o++) {
                     if constexpr (KG) {
-                        const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(ka + o * NB * kB32));
+                        const int row = (h * 2 + p) * 2 + o;   // compile-time: the loops are unrolled
+                        const uint4 x = row < KP ? *reinterpret_cast<const uint4 *>(head + row * kN32 + 4 * v)
+                                                 : __ldcg(reinterpret_cast<const uint4 *>(ka + o * NB * kB32));
                         kv[0] = x.x; kv[1] = x.y; kv[2] = x.z; kv[3] = x.w;
                     } else {
                         load_words<E>(kv, ka + o * NB * kB32);
@@ -395,7 +398,7 @@ __global__ void __launch_bounds__(Block32Layout<DG, C>::T, 1)
                 for (int r = 0; r < C; r++) v.peer[r] = peer[r] + gb * 2048;
                 return v;
             }();
-            block32_step<DG, C, T, false>(cta, A, c, keys + kb * L::key_words, tid, 0, [&](int at) {
+            block32_step<DG, C, T, false, 0>(cta, A, c, keys + kb * L::key_words, nullptr, tid, 0, [&](int at) {
                 // warps without a block in 1 (C = 1) or in 3 start the copy of the next
                 // step's keys into the buffer that the last products have freed (copies in
                 // flight would hold up the cluster barrier's release: C = 4, 2.01 -> 2.18
@@ -434,22 +437,28 @@ __global__ void __launch_bounds__(Block32Layout<DG, C>::T, 1)
 // (blind rotation, two / three workers: 304 gates 5.6 / 6.1 ms, 512 gates 9.1 / 8.2 ms).
 // Bound by the multiply pipe (61 % busy; a loop of butterflies alone reaches 82 %).
 // Digit tables instead of multiplications did not pay here: 1000 gates 16.0 -> 16.1 ms.
+// With three workers the shared memory left holds the first 4 of a step's 16 key rows,
+// by one bulk copy that the transforms hide; the others come from L2 as they are
+// multiplied (1000 gates 15.95 -> 15.70 ms). With two workers 4 to 12 rows gained nothing.
 constexpr int kItem32Threads = 768;   // of a CTA
+__host__ __device__ constexpr int item32_key_rows(int W) { return W == 2 ? 0 : 4; }
+constexpr int kItem32KeyWaitLimit = 1 << 22;   // polls before a key wait gives up
 __host__ __device__ constexpr int item32_steps(int W) { return W == 2 ? 8 : 16; }
 
 // Polls of such a wait (about 60 ns each) before it gives up and flags the launch.
 constexpr unsigned kItem32WaitLimit = 1u << 26;
 
-// Dynamic shared memory: twiddles, then per worker [g | acc x 2 | dbuf].
-template <int DG>
+// Dynamic shared memory: twiddles, then per worker [g | acc x 2 | dbuf | key rows].
+template <int DG, int W>
 __host__ __device__ constexpr size_t item32_worker_bytes()
 {
-    return 4 * (2 * kN32 + (size_t)2 * 2 * 4 * kB32E + (size_t)2 * (DG - 1) * 4 * kB32E);
+    return 4 * (2 * kN32 + (size_t)2 * 2 * 4 * kB32E + (size_t)2 * (DG - 1) * 4 * kB32E +
+                (size_t)item32_key_rows(W) * kN32);
 }
 template <int DG, int W>
 constexpr size_t item32_bytes()
 {
-    return 2 * kN32 * sizeof(uint2) + W * item32_worker_bytes<DG>();
+    return 2 * kN32 * sizeof(uint2) + W * item32_worker_bytes<DG, W>();
 }
 
 // Residues and initial accumulators, one warp per ciphertext.
@@ -483,8 +492,16 @@ __global__ void __launch_bounds__(kItem32Threads, 1)
     __shared__ int plans[W][2];   // item of the ciphertext (-1: none left), ciphertext
     uint2 *const ftw = reinterpret_cast<uint2 *>(blk_smem), *const itw = ftw + kN32;
     const int wk = threadIdx.x / T, tid = threadIdx.x - wk * T, bar = 1 + wk;
-    uint32_t *const g = reinterpret_cast<uint32_t *>(blk_smem + 2 * kN32 * sizeof(uint2) + wk * item32_worker_bytes<DG>());
-    uint32_t *const acc = g + 2 * kN32, *const dbuf = acc + 2 * 2 * 4 * kB32E;
+    uint32_t *const g = reinterpret_cast<uint32_t *>(blk_smem + 2 * kN32 * sizeof(uint2) + wk * item32_worker_bytes<DG, W>());
+    uint32_t *const acc = g + 2 * kN32, *const dbuf = acc + 2 * 2 * 4 * kB32E, *const head = dbuf + 2 * (DG - 1) * 4 * kB32E;
+    constexpr int KP = item32_key_rows(W);
+    __shared__ __align__(8) uint64_t bars[W];
+    unsigned parity = 0;
+    bool failed = false;
+    if (tid == 0) {
+        mbar_init(&bars[wk], 1);
+        mbar_fence_init();
+    }
     const int S = A.n * (int)A.digitR, mode = issue_mode(A.flags);
     for (int i = threadIdx.x; i < 2 * kN32; i += kItem32Threads) ftw[i] = __ldg(plain_tw + i);
     __syncthreads();
@@ -526,8 +543,20 @@ __global__ void __launch_bounds__(kItem32Threads, 1)
         for (int st = it * K; st < end; st++) {
             if (!step_issued(res, st, mode)) continue;
             const Block32Cta<1> cta{g, acc + ab * (8 * kB32E), acc + (ab ^ 1) * (8 * kB32E), dbuf, {g}, ftw, itw, 0};
-            block32_step<DG, 1, T, true>(cta, A, c, A.btkey + ((size_t)st * A.Br + res[st]) * ((size_t)DG * 4 * kN32),
-                                         tid, bar, [](int) {});
+            const uint32_t *const key = A.btkey + ((size_t)st * A.Br + res[st]) * ((size_t)DG * 4 * kN32);
+            if (KP && tid == 0 && !failed) {
+                mbar_expect_tx(&bars[wk], KP * kN32 * 4);
+                bulk_copy_g2s(head, key, KP * kN32 * 4, &bars[wk]);
+            }
+            block32_step<DG, 1, T, true, KP>(cta, A, c, key, head, tid, bar, [&](int at) {
+                if (!KP || at != 2 || failed) return;
+                if (mbar_wait_bounded(&bars[wk], parity, kItem32KeyWaitLimit)) {
+                    parity ^= 1u;
+                } else {   // flag the launch and go on without
+                    failed = true;
+                    atomicOr(A.status, kStatusWaitLimit);
+                }
+            });
             ab ^= 1;
         }
         for (int u = tid; u < 512; u += T)
@@ -537,6 +566,8 @@ __global__ void __launch_bounds__(kItem32Threads, 1)
         pipe_barrier(bar, T);
         if (tid == 0) atomicExch(done + k, it);
     }
+    // a copy that was given up must land before the CTA's shared memory goes
+    if (failed && tid == 0) mbar_wait_bounded(&bars[wk], parity, kItem32KeyWaitLimit);
 }
 
 }  // namespace dev
