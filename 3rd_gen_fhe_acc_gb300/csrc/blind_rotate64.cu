@@ -23,17 +23,16 @@
 //      digit times a constant: two 32 x 32 -> 64 multiplies), three passes of
 //      butterflies, and the multiply-accumulate of all digits with the block's
 //      key rows, whose sums stay in registers: each key word is two limbs of 27
-//      bits (8 bytes, half of a constant pair's), each product four multiplies into
+//      bits (8 bytes, half of a Shoup pair's), each product three multiplies into
 //      three 64-bit sums, reduced once per output.
 // The last digit's NTT is the accumulator itself (DevParams::last_digit_from_acc).
 //
 // Two kernels. br64_cluster_kernel (up to one ciphertext per SM) is for latency: per
 // step 8.5 us on 8 CTAs, 10.5 on 4, 17.6 on 2, 31.4 on one, where a 256-thread worker
-// took 75 us (40 with its register spills gone). br64_items_kernel is for batches: 27.8
-// us per step and SM (2048 gates: 451 ms; 582 before the moduli's fold form). Both are
-// bound by the multiply pipe: 48 k of its instructions a step, of which 29 k are
-// 32 x 32 -> 64 multiplies; a loop of butterflies on registers alone keeps the pipe 74 %
-// busy, the items form 62 %.
+// took 75 us (40 with its register spills gone). br64_items_kernel is for batches: 27.5
+// us per step and SM (2048 gates: 446 ms; 582 before the moduli's fold form). Both are
+// bound by the multiply pipe: a loop of butterflies on registers alone keeps it 74 %
+// busy, the items form 67 %, the latency form on one CTA 62 %.
 #include "block64.cuh"
 #include <algorithm>
 
@@ -170,7 +169,7 @@ constexpr unsigned kItemWaitLimit = 1u << 26;
 // 27.8 with 4 and with 6, 28.2 with 8.
 constexpr int kItemSteps = 4;
 
-// Throughput form: W workers of kTP threads per CTA (two, so that one's barriers and
+// Throughput form: W workers per CTA (two of kTP threads, so that one's barriers and
 // loads overlap the other's arithmetic; in one CTA, because their 20 warps then spread
 // evenly over the SM's four schedulers: as two CTAs of 10 warps, two schedulers get 6
 // and two get 4, 30.0 against 29.4 us per step and SM). Each worker takes items,
@@ -181,16 +180,16 @@ constexpr int kItemSteps = 4;
 // before it has finished (done[]); that one was taken earlier, by a worker that is
 // running, so the wait ends whether or not the whole grid is resident.
 template <int B, int W>
-__global__ void __launch_bounds__(W * kTP, 1) br64_items_kernel(const __grid_constant__ BlockArgs A,
+__global__ void __launch_bounds__(W * worker_threads64(W), 1) br64_items_kernel(const __grid_constant__ BlockArgs A,
                                                            unsigned long long *cursor, int *done,
                                                            const ulonglong2 *__restrict__ tw,
                                                            const ulonglong2 *__restrict__ itw,
                                                            const __grid_constant__ Ntt64Consts c)
 {
     using L = BlockLayout<B, 1>;
-    constexpr int T = kTP;
+    constexpr int T = worker_threads64(W);
     extern __shared__ __align__(128) unsigned char smem_all[];
-    const int wk = threadIdx.x / T, tid = threadIdx.x - wk * T, bar = 1 + wk;
+    const int wk = threadIdx.x / T, tid = threadIdx.x - wk * T, bar = W == 1 ? 0 : 1 + wk;
     unsigned char *const smem_raw = smem_all + wk * L::key_off(A.DG);
     uint64_t *const g = reinterpret_cast<uint64_t *>(smem_raw + L::g_off);
     uint64_t *const acc = reinterpret_cast<uint64_t *>(smem_raw + L::acc_off);
@@ -390,7 +389,7 @@ static int launch_items(Context &c, dev::BlockArgs A, unsigned long long *cursor
     e = cudaMemsetAsync(cursor, 0, sizeof(*cursor), st);
     if (e != cudaSuccess) return c.cuda_fail(e, "blind rotation cursor reset");
     A.wait_limit = c.tune.debug_wait_limit >= 0 ? (unsigned)c.tune.debug_wait_limit : dev::kItemWaitLimit;
-    kern<<<(unsigned)blocks, W * dev::kTP, smem, st>>>(A, cursor, done, c.d_tw64, c.d_itw64, c.nc64);
+    kern<<<(unsigned)blocks, W * dev::worker_threads64(W), smem, st>>>(A, cursor, done, c.d_tw64, c.d_itw64, c.nc64);
     c.launches++;
     e = cudaGetLastError();
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "blind rotation launch");

@@ -14,6 +14,10 @@ namespace cg = cooperative_groups;
 // Threads of a CTA: the 10 digits' 512-word blocks are 640 octets (digitG = 6), all
 // at once in the latency form, half of them in the throughput form (two CTAs per SM).
 constexpr int kTB = 640, kTP = 320;
+// A worker alone on its SM (digitG = 7 and 8, whose work areas fill more than half of the
+// shared memory) has kTB threads: 1000 products at digitG = 8 451 us with kTP, 344 so;
+// 912 gates of n = 32 19.8 ms, 16.2 so.
+__host__ __device__ constexpr int worker_threads64(int W) { return W == 1 ? kTB : kTP; }
 
 // x w of the MAC, x = x1 2^27 + x0 < 2^59 and limbs w < 2^27: the sums of x0 w0, of
 // (x0 + x1) (w0 + w1) and of x1 w1, three multiplies (Karatsuba; four without: 2048 gates

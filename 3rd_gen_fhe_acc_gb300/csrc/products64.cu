@@ -97,14 +97,15 @@ __global__ void __launch_bounds__(kTB, 1) products64_cluster_kernel(const __grid
 }
 
 template <int B, int W>
-__global__ void __launch_bounds__(W * kTP, 1) products64_workers_kernel(const __grid_constant__ Products64 A,
+__global__ void __launch_bounds__(W * worker_threads64(W), 1) products64_workers_kernel(const __grid_constant__ Products64 A,
                                                                        const ulonglong2 *__restrict__ tw,
                                                                        const ulonglong2 *__restrict__ itw,
                                                                        const __grid_constant__ Ntt64Consts c)
 {
     using L = BlockLayout<B, 1>;
     extern __shared__ __align__(128) unsigned char smem_all[];
-    const int wk = threadIdx.x / kTP, tid = threadIdx.x - wk * kTP;
+    constexpr int T = worker_threads64(W);
+    const int wk = threadIdx.x / T, tid = threadIdx.x - wk * T;
     unsigned char *const smem_raw = smem_all + wk * L::key_off(A.DG);
     uint64_t *const g = reinterpret_cast<uint64_t *>(smem_raw + L::g_off);
     __shared__ uint64_t zeta[B][B - 1];
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(W * kTP, 1) products64_workers_kernel(const __
     const BlockCta<B, 1> cta{g, reinterpret_cast<uint64_t *>(smem_raw + L::acc_off),
                              reinterpret_cast<uint64_t *>(smem_raw + L::work_off(A.DG)), {g}, zeta, 0};
     for (size_t i = (size_t)wk * gridDim.x + blockIdx.x; i < A.count; i += (size_t)gridDim.x * W)
-        product_item<B, 1, kTP>(cta, A, i, tw, itw, c, tid, 1 + wk);
+        product_item<B, 1, T>(cta, A, i, tw, itw, c, tid, W == 1 ? 0 : 1 + wk);
 }
 
 }  // namespace dev
@@ -168,7 +169,7 @@ static int launch_products_workers(Context &c, const Products64 &A, cudaStream_t
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return c.cuda_fail(e, "products smem attribute");
     const size_t blocks = std::min<size_t>((size_t)sms_products(c), A.count);
-    kern<<<(unsigned)blocks, W * dev::kTP, smem, st>>>(A, c.d_tw64, c.d_itw64, c.nc64);
+    kern<<<(unsigned)blocks, W * dev::worker_threads64(W), smem, st>>>(A, c.d_tw64, c.d_itw64, c.nc64);
     c.launches++;
     e = cudaGetLastError();
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "products launch");
