@@ -171,12 +171,6 @@ int build_tables64(Context &c)
     };
     put(c.p.iN, k.iN, k.iNs);
     put(host::mulmod(T.irou[1], c.p.iN, Q), k.iw1N, k.iw1Ns);
-    put(((uint64_t)1 << 30) % Q, k.p30, k.p30s);
-    k.dw1 = T.rou[1] << k.pm_s;
-    k.dw2 = T.rou[2] << k.pm_s;
-    k.dw3 = T.rou[3] << k.pm_s;
-    k.dw21 = host::mulmod(T.rou[2], T.rou[1], Q) << k.pm_s;
-    k.dw31 = (Q - host::mulmod(T.rou[3], T.rou[1], Q)) << k.pm_s;
     std::vector<ulonglong2> fw(N), iw(N);
     for (int i = 0; i < N; i++) {
         fw[i] = const_pair64(c, T.rou[i]);
@@ -459,7 +453,7 @@ static int bootstrap_key_pass(Context &c, const uint64_t *btkey, size_t words, b
         return c.fail(FHEACC_ENOKEY, "bootstrap key not uploaded");
     if (c.wide) {
         // device order, one step (all residues) per chunk, device words made on the GPU
-        const bool limbs = c.nc64.pm_c && c.dp.last_digit_from_acc;
+        const bool limbs = products64_apply(c);
         const size_t wb = limbs ? sizeof(uint2) : sizeof(ulonglong2);   // bytes of a device word
         if (!verify && !c.has_btkey()) {
             void *ptr = nullptr;
@@ -501,7 +495,7 @@ static int bootstrap_key_pass(Context &c, const uint64_t *btkey, size_t words, b
                 char *to = verify ? d_check : chunk;
                 if (!rc)
                     rc = limbs ? launch_limb_words64(c, d_stage, (uint2 *)to, Br * rw, c.stream)
-                               : launch_const_pairs64(c, d_stage, (ulonglong2 *)to, Br * rw, c.stream);
+                               : launch_shoup_pairs64(c, d_stage, (ulonglong2 *)to, Br * rw, c.stream);
                 if (!rc && cudaStreamSynchronize(c.stream) != cudaSuccess) rc = c.cuda_fail(cudaGetLastError(), "key words");
                 if (!rc && verify) {
                     e = cudaMemcpy(made.data(), d_check, cb, cudaMemcpyDeviceToHost);
@@ -680,7 +674,7 @@ static int subs_key_pass(Context &c, const uint64_t *subs_key, size_t words, boo
         }
         void *const to = verify ? d_check : c.d_subs64;
         int rc = limbs ? launch_limb_words64(c, d_stage, (uint2 *)to, words, c.stream)
-                       : launch_const_pairs64(c, d_stage, (ulonglong2 *)to, words, c.stream);
+                       : launch_shoup_pairs64(c, d_stage, (ulonglong2 *)to, words, c.stream);
         if (!rc && cudaStreamSynchronize(c.stream) != cudaSuccess) rc = c.cuda_fail(cudaGetLastError(), "key words");
         if (!rc && verify) {
             std::vector<char> made(words * wb), held(words * wb);
@@ -978,7 +972,7 @@ int fheacc_rlwe_keyswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t co
     int rc = ensure_scratch(c, c.io, words * (c.wide ? sizeof(ulonglong2) : sizeof(uint32_t)));
     if (rc) return rc;
     rc = products64_apply(c) ? launch_limb_words64(c, d_ksk, (uint2 *)c.io.ptr, words, st)
-         : c.wide            ? launch_const_pairs64(c, d_ksk, (ulonglong2 *)c.io.ptr, words, st)
+         : c.wide            ? launch_shoup_pairs64(c, d_ksk, (ulonglong2 *)c.io.ptr, words, st)
                              : launch_to_u32(c, d_ksk, (uint32_t *)c.io.ptr, words, st);
     if (rc) return rc;
     return mark_done(c, st, launch_expand(c, 1, d_in, d_out, count, 0, c.io.ptr, st));

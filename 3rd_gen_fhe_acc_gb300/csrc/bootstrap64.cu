@@ -7,16 +7,15 @@
 // digit_decompose (RLWE.cpp:623-640), acc_initialization (RLWE.cpp:706-724),
 // LWE_keyswitch / LWE_modswitch (LWE.cpp:233-269).
 //
-// One RLWE x RGSW step runs on a CTA of 256 threads in two 128-thread groups,
-// group p owning poly p of the accumulator: inverse NTT in shared memory, then
-// for each digit h both groups transform digit h of their poly and all 256
-// threads multiply-accumulate it with the key rows. Keys are stored as constant
-// pairs (mul64 in ntt64.cuh: 16 bytes a word); the two products of a digit and
-// an output are folded together (mul64_2), and the digitG sums are reduced
-// once. As in the 32-bit kernel, steps are the outer loop over a
-// group of ciphertexts per CTA, so the CTAs stream each step's 23 RGSW keys
-// (18 MB) through L2 together; accumulators live in global
-// memory (32 KB per gate).
+// The blind rotation and the products here are for the moduli without the fold form
+// (pm64_shift in ntt64.cuh; Shoup multiplications); the others' are in block form
+// (blind_rotate64.cu, products64.cu). One RLWE x RGSW step runs on a worker of 256
+// threads in two 128-thread groups, group p owning poly p of the accumulator: inverse
+// NTT in shared memory, then for each digit h both groups transform digit h of their
+// poly and all 256 threads multiply-accumulate it with the key rows, kept as Shoup
+// pairs (16 bytes a word). Steps are the outer loop over a group of ciphertexts per
+// CTA, so the CTAs stream each step's RGSW keys through L2 together; accumulators
+// live in global memory (32 KB per gate).
 #include "ctx.hpp"
 #include "br64.cuh"
 #include "l2hint.cuh"
@@ -28,22 +27,14 @@ namespace dev {
 
 constexpr int kMaxGroup64 = 8;   // ciphertexts per worker and claim
 
-// One worker's polys in shared memory, layout pi<P> (ntt64.cuh).
-//
-// What the step costs (2048 gates, blind rotation of the n = 630 set): the L1 /
-// shared-memory data pipe was the busiest unit (72 %, 27 % of all cycles in bank
-// conflicts: the digit tables' gathers and a padding of one word in 8), the
-// multiply pipe 60 %. Folded multiplications alone: 582 -> 523 ms; digits
-// extracted inside the first pass, its first two stages from small products
-// instead of tables, one padding word in 16: 464 ms.
-template <bool P>
-struct Step64SmemT {
-    uint64_t acc[2][poly_words64<P>()];   // accumulator; time domain inside a step
-    uint64_t buf[2][poly_words64<P>()];   // digit NTTs
+// One worker's polys in shared memory, layout px (ntt64.cuh).
+struct Step64Smem {
+    uint64_t acc[2][kPoly64];   // accumulator; time domain inside a step
+    uint64_t buf[2][kPoly64];   // digit NTTs
 };
 
 // One RLWE x RGSW step on s.acc (NTT domain, values < 2Q) with the key
-// `key` (constant pairs, [digitG][2][2][2048]), run by the 256 threads tid of a
+// `key` (Shoup pairs, [digitG][2][2][2048]), run by the 256 threads tid of a
 // worker that synchronises on named barrier `bar` (its two 128-thread groups
 // on bar + 1 and bar + 2).
 // With acc_nd (the step's NTT-domain accumulator in global memory, read before
@@ -51,13 +42,13 @@ struct Step64SmemT {
 // keys were uploaded with K'_h = K_h - BG^(h-DG+1) K_last, K'_last =
 // BG^-(DG-1) K_last (Q < BG^DG, so sum_h BG^h NTT(digit_h) = acc).
 // KEEP: acc_nd is read with the L2 evict-last policy (l2hint.cuh).
-template <bool PM, bool P, bool KEEP = false>
-__device__ __forceinline__ void step64(Step64SmemT<P> &s, const ulonglong2 *__restrict__ key, int DG, uint32_t bg_bits,
+template <bool KEEP = false>
+__device__ __forceinline__ void step64(Step64Smem &s, const ulonglong2 *__restrict__ key, int DG, uint32_t bg_bits,
                                        const ulonglong2 *__restrict__ tw, const ulonglong2 *__restrict__ itw,
                                        const Ntt64Consts &c, const uint64_t *acc_nd, int tid, int bar)
 {
     const int grp = tid >> 7, gtid = tid & 127;
-    ntt64_inv_2048<PM, 128, P>(s.acc[grp], itw, c, gtid, bar + 1 + grp);
+    ntt64_inv_2048<false, 128, true>(s.acc[grp], itw, c, gtid, bar + 1 + grp);
     group_sync(bar, kT64);
     uint64_t sa[8], sb[8];
 #pragma unroll
@@ -65,7 +56,7 @@ __device__ __forceinline__ void step64(Step64SmemT<P> &s, const ulonglong2 *__re
     const uint32_t mask = (1u << bg_bits) - 1;
     const int DH = acc_nd ? DG - 1 : DG;   // digits transformed
     for (int h = 0; h < DH; h++) {
-        ntt64_fwd_2048_load<PM, 128, P, true>(s.buf[grp], LoadDigit64<P>{s.acc[grp], bg_bits * h, mask}, tw, c, gtid,
+        ntt64_fwd_2048_load<false, 128, true>(s.buf[grp], LoadDigit64<true>{s.acc[grp], bg_bits * h, mask}, tw, c, gtid,
                                               bar + 1 + grp);
         group_sync(bar, kT64);
         const ulonglong2 *k0 = key + (size_t)(h * 2 + 0) * 2 * 2048;   // row c_text[h][0]: times digit of a
@@ -73,11 +64,11 @@ __device__ __forceinline__ void step64(Step64SmemT<P> &s, const ulonglong2 *__re
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const int k = tid + 256 * i;
-            const uint64_t da = s.buf[0][pi<P>(k)], db = s.buf[1][pi<P>(k)];
+            const uint64_t da = s.buf[0][px(k)], db = s.buf[1][px(k)];
             const ulonglong2 a0 = __ldg(k0 + k), b0 = __ldg(k0 + 2048 + k);
             const ulonglong2 a1 = __ldg(k1 + k), b1 = __ldg(k1 + 2048 + k);
-            sa[i] += mul64_2<PM>(da, a0, db, a1, c);
-            sb[i] += mul64_2<PM>(da, b0, db, b1, c);
+            sa[i] += mul64<false>(da, a0, c) + mul64<false>(db, a1, c);
+            sb[i] += mul64<false>(da, b0, c) + mul64<false>(db, b1, c);
         }
         group_sync(bar, kT64);
     }
@@ -98,15 +89,15 @@ __device__ __forceinline__ void step64(Step64SmemT<P> &s, const ulonglong2 *__re
             }
             const ulonglong2 a0 = __ldg(k0 + k), b0 = __ldg(k0 + 2048 + k);
             const ulonglong2 a1 = __ldg(k1 + k), b1 = __ldg(k1 + 2048 + k);
-            sa[i] += mul64_2<PM>(da, a0, db, a1, c);
-            sb[i] += mul64_2<PM>(da, b0, db, b1, c);
+            sa[i] += mul64<false>(da, a0, c) + mul64<false>(db, a1, c);
+            sb[i] += mul64<false>(da, b0, c) + mul64<false>(db, b1, c);
         }
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int k = tid + 256 * i;
-        s.acc[0][pi<P>(k)] = reduce64<PM>(sa[i], c);
-        s.acc[1][pi<P>(k)] = reduce64<PM>(sb[i], c);
+        s.acc[0][px(k)] = reduce64<false>(sa[i], c);
+        s.acc[1][px(k)] = reduce64<false>(sb[i], c);
     }
     group_sync(bar, kT64);
 }
@@ -165,27 +156,18 @@ __global__ void derive_keys64_kernel(uint64_t *__restrict__ keys, size_t count, 
     }
 }
 
-// Constant pairs (mul64) of key words (reduced mod Q first).
-template <bool PM>
-__global__ void const_pairs64_kernel(const uint64_t *__restrict__ in, ulonglong2 *__restrict__ out, size_t n,
-                                     const __grid_constant__ Ntt64Consts c)
+// Shoup pairs of key words (reduced mod Q first).
+__global__ void shoup_pairs64_kernel(const uint64_t *__restrict__ in, ulonglong2 *__restrict__ out, size_t n, uint64_t Q)
 {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const uint64_t w = in[i] % c.Q;
-        if (PM) {
-            uint64_t v = mul64<PM>(w, make_ulonglong2(c.p30, c.p30s), c);
-            v = v >= c.Q ? v - c.Q : v;
-            out[i] = make_ulonglong2(w << c.pm_s, v << c.pm_s);
-        } else {
-            out[i] = make_ulonglong2(w, (uint64_t)(((unsigned __int128)w << 64) / c.Q));
-        }
+        const uint64_t w = in[i] % Q;
+        out[i] = make_ulonglong2(w, (uint64_t)(((unsigned __int128)w << 64) / Q));
     }
 }
 
 // RLWE_mult_RGSW of count (acc, RGSW-pairs) in reference order; acc canonical.
 // derive: the RGSWs carry the last-digit identity (derive_keys64_kernel) and the
 // last digit's NTT is the input accumulator itself.
-template <bool PM>
 __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_kernel(const uint64_t *__restrict__ acc_in,
                                                                const ulonglong2 *__restrict__ rgsw, uint64_t *acc_out,
                                                                size_t count, size_t rgsw_stride, int DG, uint32_t bg_bits,
@@ -194,11 +176,11 @@ __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_kernel(const uint64_t *
                                                                const __grid_constant__ Ntt64Consts c, int derive)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Step64SmemT<true> &s = *reinterpret_cast<Step64SmemT<true> *>(smem_raw);
+    Step64Smem &s = *reinterpret_cast<Step64Smem *>(smem_raw);
     for (size_t ci = blockIdx.x; ci < count; ci += gridDim.x) {
         for (int e = threadIdx.x; e < 4096; e += kT64) s.acc[e >> 11][px(e & 2047)] = acc_in[ci * 4096 + e];
         __syncthreads();
-        step64<PM>(s, rgsw + ci * rgsw_stride, DG, bg_bits, tw, itw, c, derive ? acc_in + ci * 4096 : nullptr,
+        step64(s, rgsw + ci * rgsw_stride, DG, bg_bits, tw, itw, c, derive ? acc_in + ci * 4096 : nullptr,
                threadIdx.x, 1);
         for (int e = threadIdx.x; e < 4096; e += kT64) {
             const uint64_t v = s.acc[e >> 11][px(e & 2047)];
@@ -214,7 +196,6 @@ __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_kernel(const uint64_t *
 // the multiply-accumulate to partial[ci][h] (two Shoup products per word, < 4Q);
 // rlwe_split_sum64_kernel adds the digitG shares. A lone product's inverse and
 // digit NTTs then take two rounds instead of 1 + digitG.
-template <bool PM>
 __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_split_kernel(const uint64_t *__restrict__ acc_in,
                                                                      const ulonglong2 *__restrict__ rgsw,
                                                                      uint64_t *__restrict__ partial, size_t rgsw_stride,
@@ -224,14 +205,14 @@ __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_split_kernel(const uint
                                                                      const __grid_constant__ Ntt64Consts c)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Step64SmemT<true> &s = *reinterpret_cast<Step64SmemT<true> *>(smem_raw);
+    Step64Smem &s = *reinterpret_cast<Step64Smem *>(smem_raw);
     const size_t ci = blockIdx.x / (unsigned)DG;
     const int h = (int)(blockIdx.x - ci * (unsigned)DG);
     const int tid = threadIdx.x, grp = tid >> 7, gtid = tid & 127;
     for (int e = tid; e < 4096; e += kT64) s.acc[e >> 11][px(e & 2047)] = acc_in[ci * 4096 + e];
     __syncthreads();
-    ntt64_inv_2048<PM, 128, true>(s.acc[grp], itw, c, gtid, 2 + grp);   // ends with the group's barrier
-    ntt64_fwd_2048_load<PM, 128, true, true>(
+    ntt64_inv_2048<false, 128, true>(s.acc[grp], itw, c, gtid, 2 + grp);   // ends with the group's barrier
+    ntt64_fwd_2048_load<false, 128, true>(
         s.buf[grp], LoadDigit64<true>{s.acc[grp], bg_bits * (uint32_t)h, (1u << bg_bits) - 1}, tw, c, gtid, 2 + grp);
     __syncthreads();
     const ulonglong2 *key = rgsw + ci * rgsw_stride;
@@ -244,14 +225,13 @@ __global__ void __launch_bounds__(kT64) rlwe_mult_rgsw64_split_kernel(const uint
         const uint64_t da = s.buf[0][px(k)], db = s.buf[1][px(k)];
         const ulonglong2 a0 = __ldg(k0 + k), b0 = __ldg(k0 + 2048 + k);
         const ulonglong2 a1 = __ldg(k1 + k), b1 = __ldg(k1 + 2048 + k);
-        out[k] = mul64_2<PM>(da, a0, db, a1, c);
-        out[2048 + k] = mul64_2<PM>(da, b0, db, b1, c);
+        out[k] = mul64<false>(da, a0, c) + mul64<false>(db, a1, c);
+        out[2048 + k] = mul64<false>(da, b0, c) + mul64<false>(db, b1, c);
     }
 }
 
 // acc_out[ci] = sum over h of partial[ci][h] mod Q (canonical); the sum of
 // digitG shares < 4Q stays below 2^64 (checked by the launcher).
-template <bool PM>
 __global__ void rlwe_split_sum64_kernel(const uint64_t *__restrict__ partial, uint64_t *__restrict__ acc_out,
                                         size_t count, int DG, const __grid_constant__ Ntt64Consts c)
 {
@@ -261,7 +241,7 @@ __global__ void rlwe_split_sum64_kernel(const uint64_t *__restrict__ partial, ui
         const uint64_t *p = partial + ci * (unsigned)DG * 4096 + e;
         uint64_t sum = 0;
         for (int h = 0; h < DG; h++) sum += p[(size_t)h * 4096];
-        acc_out[w] = canonical64<PM>(sum, c);
+        acc_out[w] = canonical64<false>(sum, c);
     }
 }
 
@@ -358,7 +338,7 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
                                                           const __grid_constant__ Ntt64Consts c)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint8_t *res = smem_raw + W * sizeof(Step64SmemT<true>);   // [group][n * digitR]
+    uint8_t *res = smem_raw + W * sizeof(Step64Smem);   // [group][n * digitR]
     __shared__ uint32_t bvals[kMaxGroup64 * W], b1s[kMaxGroup64 * W], b2s[kMaxGroup64 * W];
     __shared__ int done[kMaxGroup64 * W];
     __shared__ int plan[W][3];
@@ -367,7 +347,7 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
     __shared__ unsigned long long claim_first;
     __shared__ int claim_m;
     const int wk = threadIdx.x / kT64, tid = threadIdx.x - wk * kT64, bar = 1 + 3 * wk;
-    Step64SmemT<true> &s = reinterpret_cast<Step64SmemT<true> *>(smem_raw)[wk];
+    Step64Smem &s = reinterpret_cast<Step64Smem *>(smem_raw)[wk];
     const int S = A.n * (int)A.digitR;
     const size_t rgsw_pairs = (size_t)A.DG * 4 * 2048;
     const int mode = issue_mode(A.flags);
@@ -465,7 +445,7 @@ __global__ void __launch_bounds__(W * kT64, MINB) br64_kernel(const __grid_const
                 const uint64_t pol = l2_keep_policy();
                 for (int e = tid; e < 4096; e += kT64) s.acc[e >> 11][px(e & 2047)] = ld_keep64(acc + e, pol);
                 group_sync(bar, kT64);
-                step64<false, true, true>(s, A.btkey + ((size_t)st * A.Br + r) * rgsw_pairs, A.DG, A.bg_bits, tw, itw, c,
+                step64<true>(s, A.btkey + ((size_t)st * A.Br + r) * rgsw_pairs, A.DG, A.bg_bits, tw, itw, c,
                        A.derive_last ? acc : nullptr, tid, bar);
             }
             // the item again from the plan (not held in registers across the step;
@@ -710,15 +690,14 @@ int launch_derive_keys64(Context &c, uint64_t *d_keys, size_t count, const ulong
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "derive keys launch");
 }
 
-int launch_const_pairs64(Context &c, const uint64_t *d_in, ulonglong2 *d_out, size_t n, cudaStream_t st)
+int launch_shoup_pairs64(Context &c, const uint64_t *d_in, ulonglong2 *d_out, size_t n, cudaStream_t st)
 {
     if (!n) return FHEACC_OK;
     unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)sms_of(c) * 32);
-    auto kern = c.nc64.pm_c ? dev::const_pairs64_kernel<true> : dev::const_pairs64_kernel<false>;
-    kern<<<blocks, 256, 0, st>>>(d_in, d_out, n, c.nc64);
+    dev::shoup_pairs64_kernel<<<blocks, 256, 0, st>>>(d_in, d_out, n, c.p.Q);
     c.launches++;
     cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "constant pairs launch");
+    return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "Shoup pairs launch");
 }
 
 int launch_ntt64(Context &c, uint64_t *d_polys, size_t count, bool inverse, cudaStream_t st)
@@ -750,7 +729,7 @@ int launch_rlwe_mult_rgsw64(Context &c, const uint64_t *d_acc, const uint64_t *d
         A.out = d_out; A.out_per = 1; A.out_s1 = 4096; A.count = count;
         return launch_products64(c, A, st);
     }
-    // constant pairs of the RGSWs, after the last-digit identity when it applies
+    // Shoup pairs of the RGSWs, after the last-digit identity when it applies
     // (2 of the 2 digitG digit NTTs of a product saved); a call of a few
     // products keeps the plain RGSWs, whose derivation would cost it more
     // (PSI query: homo_expand 7.87 -> 7.51 ms, its 1-item CMUXes 0.79 -> 0.90 ms)
@@ -774,12 +753,12 @@ int launch_rlwe_mult_rgsw64(Context &c, const uint64_t *d_acc, const uint64_t *d
         if (rc) return rc;
         src = staged;
     }
-    rc = launch_const_pairs64(c, src, pairs, words, st);
+    rc = launch_shoup_pairs64(c, src, pairs, words, st);
     if (rc) return rc;
     if (split) {
         uint64_t *partial = reinterpret_cast<uint64_t *>(pairs + words);
-        const size_t smem = sizeof(dev::Step64SmemT<true>);
-        auto kern = c.nc64.pm_c ? dev::rlwe_mult_rgsw64_split_kernel<true> : dev::rlwe_mult_rgsw64_split_kernel<false>;
+        const size_t smem = sizeof(dev::Step64Smem);
+        auto kern = dev::rlwe_mult_rgsw64_split_kernel;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         kern<<<(unsigned)(count * DG), dev::kT64, smem, st>>>(
             d_acc, pairs, partial, stride, (int)DG, c.p.BG_bits, c.d_tw64, c.d_itw64, c.nc64);
@@ -787,14 +766,14 @@ int launch_rlwe_mult_rgsw64(Context &c, const uint64_t *d_acc, const uint64_t *d
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return c.cuda_fail(e, "rlwe_mult_rgsw64 split launch");
         const unsigned blocks = (unsigned)std::min<size_t>((count * 4096 + 255) / 256, (size_t)sms_of(c) * 4);
-        auto sum = c.nc64.pm_c ? dev::rlwe_split_sum64_kernel<true> : dev::rlwe_split_sum64_kernel<false>;
+        auto sum = dev::rlwe_split_sum64_kernel;
         sum<<<blocks, 256, 0, st>>>(partial, d_out, count, (int)DG, c.nc64);
         c.launches++;
         e = cudaGetLastError();
         return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "rlwe_mult_rgsw64 split sum launch");
     }
-    const size_t smem = sizeof(dev::Step64SmemT<true>);
-    auto kern = c.nc64.pm_c ? dev::rlwe_mult_rgsw64_kernel<true> : dev::rlwe_mult_rgsw64_kernel<false>;
+    const size_t smem = sizeof(dev::Step64Smem);
+    auto kern = dev::rlwe_mult_rgsw64_kernel;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     size_t blocks = std::min<size_t>(count, (size_t)sms_of(c) * 2);
     kern<<<(unsigned)blocks, dev::kT64, smem, st>>>(
@@ -823,12 +802,12 @@ static int launch_br64_shape(Context &c, dev::Br64Args A, int max_ctas, cudaStre
     const size_t steps = (size_t)c.p.n * c.p.digitR;
     // group cap: kMaxGroup64 (or the tuned cap) per worker, within the shared memory of one CTA
     int cap = W * (c.tune.br_group > 0 ? std::min(c.tune.br_group, dev::kMaxGroup64) : dev::kMaxGroup64);
-    const size_t fixed = W * sizeof(dev::Step64SmemT<true>) + 32;
+    const size_t fixed = W * sizeof(dev::Step64Smem) + 32;
     if (fixed + (size_t)cap * steps > kPipeSmemBudget)
         cap = fixed < kPipeSmemBudget ? (int)((kPipeSmemBudget - fixed) / steps) : 0;
     if (cap < 1) return c.fail(FHEACC_EINVAL, "n * digitR too large for the blind rotation's residue table");
     auto smem_of = [&](int group) {
-        return W * sizeof(dev::Step64SmemT<true>) + ((size_t)group * steps + 15) / 16 * 16;
+        return W * sizeof(dev::Step64Smem) + ((size_t)group * steps + 15) / 16 * 16;
     };
     size_t smem = smem_of(cap);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

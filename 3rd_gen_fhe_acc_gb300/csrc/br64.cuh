@@ -16,7 +16,7 @@ struct Br64Args {
     const uint32_t *idx1, *idx2;   // optional: gate g reads c1 + idx1[g] * (n+1) (else g)
     const int32_t *gates;
     size_t count;
-    const ulonglong2 *btkey;   // [(i*digitR + j)*Br + r][digitG][2][2][2048] constant pairs
+    const ulonglong2 *btkey;   // [(i*digitR + j)*Br + r][digitG][2][2][2048] Shoup pairs
     uint64_t *accs;            // scratch [count][2][2048], NTT domain, values < 2Q
     uint64_t *acc_out;         // optional canonical NTT accumulators [count][4096]
     uint64_t *extract;         // optional [count][kExtract64]

@@ -126,11 +126,11 @@ struct Context {
     ulonglong2 *d_tw64 = nullptr, *d_itw64 = nullptr;
     dev::Ntt64Consts nc64{};
     // the bootstrap key of a Q = 2^b - c in limb words (blind_rotate64.cu), or of
-    // any other Q in constant pairs (bootstrap64.cu), same order
+    // any other Q in Shoup pairs (bootstrap64.cu), same order
     uint2 *d_btkey64_limbs = nullptr;
-    ulonglong2 *d_btkey64 = nullptr;   // constant pairs, [(i*digitR + j)*Br + r][digitG][2][2][N]
+    ulonglong2 *d_btkey64 = nullptr;   // Shoup pairs, [(i*digitR + j)*Br + r][digitG][2][2][N]
     ulonglong2 *d_cf64 = nullptr;      // factors of the last-digit identity, digitG constant pairs
-    void *d_subs64 = nullptr;    // limb words or constant pairs, [logN][digitKS_R][2][N]
+    void *d_subs64 = nullptr;    // limb words or Shoup pairs, [logN][digitKS_R][2][N]
     // rotations, [logN][N]: NTT(-X^(N - 2^j)), rotate_vector_gen(false), and
     // NTT(X^(2^j)), rotate_vector_gen(true); wide: constant pairs
     uint64_t *d_rot = nullptr, *d_rot_fwd = nullptr;
@@ -227,7 +227,7 @@ int launch_extract_from_ntt32(Context &c, const uint64_t *d_rlwe, size_t count, 
                               cudaStream_t st);
 int launch_modswitch(Context &c, const uint64_t *d_in, size_t count, uint64_t *d_out, cudaStream_t st);
 // 64-bit path (bootstrap64.cu)
-int launch_const_pairs64(Context &c, const uint64_t *d_in, ulonglong2 *d_out, size_t n, cudaStream_t st);
+int launch_shoup_pairs64(Context &c, const uint64_t *d_in, ulonglong2 *d_out, size_t n, cudaStream_t st);
 // The last-digit identity applied in place to count RGSWs (d_cf: digitG constant pairs).
 int launch_derive_keys64(Context &c, uint64_t *d_keys, size_t count, const ulonglong2 *d_cf, cudaStream_t st);
 int launch_ntt64(Context &c, uint64_t *d_polys, size_t count, bool inverse, cudaStream_t st);

@@ -39,11 +39,11 @@ struct ExpArgs {
     uint32_t bits;           // Bks_R_bits
     uint32_t ipow;           // (N / 2^f + 1)^-1 mod 2N
     const uint32_t *ksk32;   // [L][2][N] u32 (narrow)
-    const ulonglong2 *ksk64; // [L][2][N] constant pairs (wide)
+    const ulonglong2 *ksk64; // [L][2][N] Shoup pairs (wide, other moduli)
     const uint2 *ksk_limbs;  // the same as limb words (wide, block form)
     uint32_t c54, power;     // 2^54 mod Q (block form); N / 2^f + 1 (KS: 1)
     const uint64_t *rot;     // [N] NTT(-X^(N - 2^f)) (EXPAND, narrow)
-    const ulonglong2 *rot64; // the same as constant pairs (wide)
+    const ulonglong2 *rot64; // rot as constant pairs (mul64 in ntt64.cuh; wide)
     uint64_t Q, mu64;
 };
 
@@ -202,11 +202,11 @@ __global__ void __launch_bounds__(256, 2) expand64_kernel(const __grid_constant_
                 const int poly = A.mode == kSubs ? tr : (tr == L ? 1 : 0);
                 // A.ipow = 1 is the identity (kKs)
                 if (A.mode != kSubs && tr < L) {
-                    ntt64_fwd_2048_load<false, 128, true, true>(
+                    ntt64_fwd_2048_load<false, 128, true>(
                         buf[grp], LoadSubs64{t[poly], Q, A.ipow, A.bits * (uint32_t)tr, (1u << A.bits) - 1}, tw, c, gtid,
                         1 + grp);
                 } else {
-                    ntt64_fwd_2048_load<false, 128, true, false>(buf[grp], LoadSubs64{t[poly], Q, A.ipow, 0, 0}, tw, c,
+                    ntt64_fwd_2048_load<false, 128, true>(buf[grp], LoadSubs64{t[poly], Q, A.ipow, 0, 0}, tw, c,
                                                                gtid, 1 + grp);
                 }
             }
@@ -300,10 +300,10 @@ __global__ void __launch_bounds__(256) expand64_split_kernel(const __grid_consta
     const int tr = 2 * p + grp;
     if (tr < nt) {
         if (tr < L)
-            ntt64_fwd_2048_load<false, 128, true, true>(
+            ntt64_fwd_2048_load<false, 128, true>(
                 buf[grp], LoadSubs64{t[0], Q, A.ipow, A.bits * (uint32_t)tr, (1u << A.bits) - 1}, tw, c, gtid, 1 + grp);
         else
-            ntt64_fwd_2048_load<false, 128, true, false>(buf[grp], LoadSubs64{t[1], Q, A.ipow, 0, 0}, tw, c, gtid,
+            ntt64_fwd_2048_load<false, 128, true>(buf[grp], LoadSubs64{t[1], Q, A.ipow, 0, 0}, tw, c, gtid,
                                                        1 + grp);
     }
     __syncthreads();
@@ -621,13 +621,11 @@ static int launch_expand_blocks(Context &c, const dev::ExpArgs &A, size_t items,
     if (!rc && !fits) rc = launch_expand_cluster<4, 1>(c, A, items, st, &fits);
     if (rc || fits) return rc;
     const size_t one = dev::ExpandLayout<4, 1>::bytes(A.L), most = 227 * 1024 - 512;   // 512: the kernel's static part
-    return 3 * one <= most   ? launch_expand_workers<3>(c, A, items, st)
-           : 2 * one <= most ? launch_expand_workers<2>(c, A, items, st)
-                             : launch_expand_workers<1>(c, A, items, st);
+    return 3 * one <= most ? launch_expand_workers<3>(c, A, items, st) : launch_expand_workers<2>(c, A, items, st);
 }
 
 // ksk: narrow, u32 [L][2][N] device words; wide, limb words (block form,
-// products64_apply) or constant pairs (mul64).
+// products64_apply) or Shoup pairs.
 int launch_expand(Context &c, int mode, const uint64_t *d_in, uint64_t *d_out, size_t count, int f,
                   const void *ksk, cudaStream_t st, size_t batches, size_t bstride)
 {

@@ -23,7 +23,9 @@
 //     x w = x0 w + x1 (w 2^30) below 2^(b+32), and the bits above 2^b fold
 //     back times c: five 32 x 32 -> 64 multiplies (20 issue slots of the
 //     multiply pipe's 16 lanes) where Shoup's form takes 33. A register-only
-//     butterfly loop: 34 cycles per warp against 42 with Shoup's.
+//     butterfly loop: 34 cycles per warp against 42 with Shoup's. The blind
+//     rotation, products and expansion of such a Q are in block form
+//     (block64.cuh); of the transforms here they use the whole-polynomial ones.
 //   PM = false: Shoup's multiplication, any Q < 2^58.
 #pragma once
 #include <cstdint>
@@ -50,17 +52,13 @@ struct Ntt64Consts {
     uint64_t iN, iNs;       // N^-1 as a constant pair (w, companion)
     uint64_t iw1N, iw1Ns;   // irou[1] * N^-1
     uint64_t mu64;          // floor(2^64 / Q)
-    uint64_t p30, p30s;     // PM: 2^30 mod Q as a constant pair
-    // PM: twiddles of a digit's first two stages times 2^pm_s (digit_radix4):
-    // w1, w2, w3, w2 w1, -w3 w1 mod Q
-    uint64_t dw1, dw2, dw3, dw21, dw31;
     uint32_t pm_c;          // 2^b - Q where the PM form applies (else 0)
     uint32_t pm_s;          // 64 - b
 };
 
 // 64 - b if Q = 2^b - c with 48 <= b <= 54 and c <= 2^(b-36), else 0. The
 // bounds make every product of mul64<true> less than (1 + 2^-4) 2^b < 2Q, and
-// b <= 54 leaves the forward transform's 23Q below the 2^59 of mul64_2<true>.
+// b <= 54 keeps a residue in two 27-bit limbs (mac27 in block64.cuh).
 inline int pm64_shift(uint64_t Q)
 {
     for (int b = 48; b <= 54; b++) {
@@ -112,26 +110,6 @@ __device__ __forceinline__ uint64_t mul64(uint64_t x, ulonglong2 w, const Ntt64C
     }
     const uint64_t t = __umul64hi(x, w.y);
     return x * w.x - t * c.Q;
-}
-
-// x v + y w mod Q for constant pairs v, w: below 2Q (PM: one fold for both
-// products, x and y < 2^59, sums below 2 (2^62 + 2^61) + 2^32) or 4Q (Shoup).
-template <bool PM>
-__device__ __forceinline__ uint64_t mul64_2(uint64_t x, ulonglong2 v, uint64_t y, ulonglong2 w, const Ntt64Consts &c)
-{
-    if (PM) {
-        const uint32_t x0 = (uint32_t)x & 0x3fffffffu, x1 = (uint32_t)(x >> 30);
-        const uint32_t y0 = (uint32_t)y & 0x3fffffffu, y1 = (uint32_t)(y >> 30);
-        uint64_t U = mul_wide64(x0, (uint32_t)v.x), V = mul_wide64(x0, (uint32_t)(v.x >> 32));
-        U = mad_wide64(x1, (uint32_t)v.y, U);
-        V = mad_wide64(x1, (uint32_t)(v.y >> 32), V);
-        U = mad_wide64(y0, (uint32_t)w.x, U);
-        V = mad_wide64(y0, (uint32_t)(w.x >> 32), V);
-        U = mad_wide64(y1, (uint32_t)w.y, U);
-        V = mad_wide64(y1, (uint32_t)(w.y >> 32), V);
-        return fold64(U, V, c);
-    }
-    return mul64<PM>(x, v, c) + mul64<PM>(y, w, c);
 }
 
 // Any 64-bit x to [0, 2Q). PM: x = x1 2^b + x0 folds to x0 + c x1 < 2^b + 2^34.
@@ -222,60 +200,19 @@ __device__ __forceinline__ void ntt64_fwd_2048(uint64_t *a, const ulonglong2 *__
     group_sync(bar, G);
 }
 
-// Stages t = 1024 and 512 of four digits (x0, x1, x2, x3) = words e, e + 512,
-// e + 1024, e + 1536 below 2^30, with w1 = psi^bitrev(1) (t = 1024), w2 and w3
-// (t = 512):
-//   x0 + w1 x2 + (w2 x1 + w2 w1 x3)     x0 + w1 x2 - (w2 x1 + w2 w1 x3)
-//   x0 - w1 x2 + (w3 x1 - w3 w1 x3)     x0 - w1 x2 - (w3 x1 - w3 w1 x3)
-// each below 4Q + BG. PM: a product with a digit takes two 32 x 32 -> 64
-// multiplies, so the four outputs take 10 and three folds where butterflies take
-// 20 and four. (Tables of the products in shared memory cost more: their
-// gathers at random digits conflict, and the shared-memory pipe was the busiest
-// unit of the blind rotation.)
-template <bool PM>
-__device__ __forceinline__ void digit_radix4(uint64_t &x0, uint64_t &x1, uint64_t &x2, uint64_t &x3,
-                                             const ulonglong2 *__restrict__ tw, const Ntt64Consts &c)
-{
-    if (PM) {
-        auto lo = [](uint64_t w) { return (uint32_t)w; };
-        auto hi = [](uint64_t w) { return (uint32_t)(w >> 32); };
-        const uint32_t d1 = (uint32_t)x1, d2 = (uint32_t)x2, d3 = (uint32_t)x3;
-        const uint64_t A = fold64(mul_wide64(d2, lo(c.dw1)), mul_wide64(d2, hi(c.dw1)), c);
-        const uint64_t B = fold64(mad_wide64(d1, lo(c.dw2), mul_wide64(d3, lo(c.dw21))),
-                                  mad_wide64(d1, hi(c.dw2), mul_wide64(d3, hi(c.dw21))), c);
-        const uint64_t D = fold64(mad_wide64(d1, lo(c.dw3), mul_wide64(d3, lo(c.dw31))),
-                                  mad_wide64(d1, hi(c.dw3), mul_wide64(d3, hi(c.dw31))), c);
-        const uint64_t u = x0 + A, v = x0 + c.twoQ - A;
-        x0 = u + B;
-        x1 = u + c.twoQ - B;
-        x2 = v + D;
-        x3 = v + c.twoQ - D;
-        return;
-    }
-    const ulonglong2 w1 = __ldg(tw + 1);
-    ct64<PM>(x0, x2, w1, c);
-    ct64<PM>(x1, x3, w1, c);
-    ct64<PM>(x0, x1, __ldg(tw + 2), c);
-    ct64<PM>(x2, x3, __ldg(tw + 3), c);
-}
-
-// First forward pass (stages t = 1024 .. 128) of the polynomial whose word e is
-// load(j, k), e = j + 128 k, into a (layout pi<P>): no pass of its own to write
-// the words first. DIGIT: words below 2^30 (digit_radix4).
-template <bool PM, int G, bool P, bool DIGIT, class Load>
-__device__ __forceinline__ void fwd_pass16_load(uint64_t *a, Load load, const ulonglong2 *__restrict__ tw,
-                                                const Ntt64Consts &c, int tid)
+// Forward NTT as ntt64_fwd_2048 of the polynomial whose word e is load(j, k),
+// e = j + 128 k, into a (layout pi<P>): the first pass (stages t = 1024 .. 128)
+// needs no pass of its own to write the words before it. Output < 23Q.
+template <bool PM, int G, bool P, class Load>
+__device__ __forceinline__ void ntt64_fwd_2048_load(uint64_t *a, Load load, const ulonglong2 *__restrict__ tw,
+                                                    const Ntt64Consts &c, int tid, int bar)
 {
     for (int j = tid; j < 128; j += G) {
         uint64_t x[16];
 #pragma unroll
         for (int k = 0; k < 16; k++) x[k] = load(j, k);
-        if (DIGIT) {
 #pragma unroll
-            for (int r = 0; r < 4; r++) digit_radix4<PM>(x[r], x[r + 4], x[r + 8], x[r + 12], tw, c);
-        }
-#pragma unroll
-        for (int st = DIGIT ? 2 : 0; st < 4; st++) {
+        for (int st = 0; st < 4; st++) {
             const int d = 16 >> (st + 1);
 #pragma unroll
             for (int k = 0; k < 16; k++) {
@@ -287,14 +224,6 @@ __device__ __forceinline__ void fwd_pass16_load(uint64_t *a, Load load, const ul
 #pragma unroll
         for (int k = 0; k < 16; k++) b[pi<P>(k * 128)] = x[k];
     }
-}
-
-// Forward NTT of such a polynomial as ntt64_fwd_2048; output < 23Q.
-template <bool PM, int G, bool P, bool DIGIT, class Load>
-__device__ __forceinline__ void ntt64_fwd_2048_load(uint64_t *a, Load load, const ulonglong2 *__restrict__ tw,
-                                                    const Ntt64Consts &c, int tid, int bar)
-{
-    fwd_pass16_load<PM, G, P, DIGIT>(a, load, tw, c, tid);   // t = 1024 .. 128
     group_sync(bar, G);
     fwd_passR<PM, G, 4, P>(a, tw, c, tid, 64, 16);    // t = 64 .. 8
     group_sync(bar, G);

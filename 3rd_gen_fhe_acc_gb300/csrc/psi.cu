@@ -23,13 +23,12 @@ namespace dev {
 enum { kEwSub = 0, kEwAdd = 1, kEwRot = 2 };
 
 // out[i] = a[i] * rot[e] mod Q (e = coefficient) for `words` words of N = 2048
-// RLWEs, canonical; rot: constant pairs (mul64).
-template <bool PM>
+// RLWEs, canonical; rot: Shoup pairs (mul64).
 __global__ void rlwe_rotate64_kernel(const uint64_t *__restrict__ a, const ulonglong2 *__restrict__ rot,
                                      uint64_t *__restrict__ out, size_t words, const __grid_constant__ Ntt64Consts c)
 {
     for (size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x; x < words; x += (size_t)gridDim.x * blockDim.x) {
-        const uint64_t v = mul64<PM>(a[x], __ldg(rot + (x & 2047)), c);
+        const uint64_t v = mul64<false>(a[x], __ldg(rot + (x & 2047)), c);
         out[x] = v >= c.Q ? v - c.Q : v;
     }
 }
@@ -83,8 +82,7 @@ static int launch_rotate64(Context &c, const uint64_t *a, const ulonglong2 *rot,
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
     const size_t words = count * 4096;
     const unsigned blocks = (unsigned)std::min<size_t>((words + 255) / 256, (size_t)std::max(sms, 1) * 8);
-    auto kern = c.nc64.pm_c ? dev::rlwe_rotate64_kernel<true> : dev::rlwe_rotate64_kernel<false>;
-    kern<<<blocks, 256, 0, st>>>(a, rot, out, words, c.nc64);
+    dev::rlwe_rotate64_kernel<<<blocks, 256, 0, st>>>(a, rot, out, words, c.nc64);
     c.launches++;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "rotation launch");
