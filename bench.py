@@ -243,11 +243,10 @@ def param_view(p):
 
 
 def profile_case(preset=0, gates=912, n=64):
-    """The case the committed ncu section captures use: the bench parameter
-    set with n = 64 (same per-step work), 912 random gates (6 per SM: the
-    3-pipeline shape of the 32-bit kernel, one wave of the 64-bit grid), two
-    batched launches, outputs checked by decryption. gates = 1, n = 500: a
-    lone gate of the bench set (the latency form of the 32-bit kernel)."""
+    """The case the committed ncu captures use: a parameter set with a small n
+    (same per-step work), `gates` random gates (912: 6 per SM), two batched
+    launches, outputs checked by decryption. The gate count picks the form of
+    the blind rotation; gates = 1, n = 500 is a lone gate of the bench set."""
     import torch
     import __graft_entry__
     __graft_entry__.build_product()
@@ -684,7 +683,7 @@ def run_psi(args, cache=None):
     n_mult = dG * N + (entries - 1) + logN
     work = items * expand_item + n_mult * mult + logN * 2 * N
     imad = ctx.measure_imad_rate()
-    slots = 16
+    slots = 10   # five 32 x 32 -> 64 multiplies, 2 issue slots each
     peak = imad / slots
     achieved = work / (statistics.mean(step_ms) / 1e3)
     roofline = {"bound": "int", "achieved": achieved / 1e9, "peak": peak / 1e9, "unit": "G modmul/s",
@@ -692,7 +691,7 @@ def run_psi(args, cache=None):
                 "work": "%d expand items x %d + %d RLWE x RGSW x %d + %d rotation multiplies = %.3g 64-bit modular "
                         "multiplies per query" % (items, expand_item, n_mult, mult, logN * 2 * N, work),
                 "peak_source": "IMAD rate measured in this run (%.1f T lane-op/s) / %d IMAD issue slots per 64-bit "
-                               "Shoup modular multiply" % (imad / 1e12, slots)}
+                               "modular multiply (five 32 x 32 -> 64 multiplies)" % (imad / 1e12, slots)}
 
     cpu = None
     if not args.no_cpu:
@@ -749,7 +748,7 @@ def fheacc_key_bytes(P):
     """Device bytes of the bootstrap + key-switch keys of a parameter set."""
     if P.N == 1024:
         return P.Br * P.digitR * P.n * P.digitG * 4 * P.N * 4 + P.Bks * P.digitKS * P.N * ((P.n + 32) // 32 * 32) * 4
-    return P.Br * P.digitR * P.n * P.digitG * 4 * P.N * 16 + P.Bks * P.digitKS * P.N * ((P.n + 32) // 32 * 32) * 8
+    return P.Br * P.digitR * P.n * P.digitG * 4 * P.N * 8 + P.Bks * P.digitKS * P.N * ((P.n + 32) // 32 * 32) * 8
 
 
 def config_of(P, batch):
@@ -966,10 +965,9 @@ def measure_batch(F, D, cache, preset, B, args, dev_id, n_steps, plain_sample, s
     modmul_per_step = (2 + 2 * dG) * (N // 2) * logN + 2 * (2 * dG) * N + 2 * N
     br_s = statistics.mean(br_ms) / 1e3
     achieved_modmul = total_steps * modmul_per_step / br_s
-    # IMAD issue slots per Shoup modular multiply: 32-bit words 4 (mul.hi counts
-    # 2); 64-bit words 16 (the 128-bit quotient estimate takes three wide and one
-    # high 32-bit product, each 2 slots, and the two low 64-bit products 4 each)
-    slots = 4.0 if N == 1024 else 16.0
+    # IMAD issue slots per modular multiply: 32-bit words (Shoup) 4 (mul.hi counts
+    # 2); 64-bit words, Q = 2^b - c, 10 (five 32 x 32 -> 64 multiplies, 2 each)
+    slots = 4.0 if N == 1024 else 10.0
     peak_modmul = imad / slots
     word = 4 if N == 1024 else 8
     rgsw_bytes = 2 * dG * 2 * N * word
@@ -981,7 +979,7 @@ def measure_batch(F, D, cache, preset, B, args, dev_id, n_steps, plain_sample, s
         if B == 4096 and preset == 0:
             traffic = tj.get("br32_pipe", {}).get("bytes_per_launch_4096")
         elif B == 2048 and preset == 1:
-            traffic = tj.get("br64", {}).get("bytes_per_launch_2048")
+            traffic = tj.get("br64_items", {}).get("bytes_per_launch_2048")
     hbm_peak = None
     peaks_src = "fallback 6800 GB/s"
     if os.path.exists(PEAKS_FILE):
@@ -999,10 +997,10 @@ def measure_batch(F, D, cache, preset, B, args, dev_id, n_steps, plain_sample, s
     roofline = {
         "bound": "int", "achieved": achieved_modmul / 1e9, "peak": peak_modmul / 1e9, "unit": "G modmul/s",
         "frac": achieved_modmul / peak_modmul, "traffic": traffic,
-        "kernel": "br32_pipe_kernel" if N == 1024 else "br64_kernel", "kernel_ms": statistics.mean(br_ms),
+        "kernel": "br32_pipe_kernel" if N == 1024 else "br64_items_kernel", "kernel_ms": statistics.mean(br_ms),
         "work": "%d RLWE x RGSW steps x %d modular multiplies (NTT butterflies, MAC products, N^-1 scaling)" % (
             total_steps, modmul_per_step),
-        "peak_source": "IMAD rate measured in this run (%.1f T lane-op/s) / %d IMAD issue slots per %d-bit Shoup "
+        "peak_source": "IMAD rate measured in this run (%.1f T lane-op/s) / %d IMAD issue slots per %d-bit "
                        "modular multiply" % (imad / 1e12, slots, 32 if N == 1024 else 64),
     }
     if comp:
