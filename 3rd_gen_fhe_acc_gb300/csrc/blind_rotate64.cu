@@ -27,8 +27,8 @@
 //      three 64-bit sums, reduced once per output.
 // The last digit's NTT is the accumulator itself (DevParams::last_digit_from_acc).
 //
-// Two kernels. br64_cluster_kernel (up to one ciphertext per SM) is for latency: per
-// step 8.5 us on 8 CTAs, 10.5 on 4, 17.6 on 2, 31.4 on one, where a 256-thread worker
+// Two kernels. br64_cluster_kernel (up to about 1.6 ciphertexts per SM) is for latency: per
+// step 8.7 us on 8 CTAs, 10.3 on 4, 17.1 on 2, 30.7 on one, where a 256-thread worker
 // took 75 us (40 with its register spills gone). br64_items_kernel is for batches: 27.5
 // us per step and SM (2048 gates: 446 ms; 582 before the moduli's fold form). Both are
 // bound by the multiply pipe: a loop of butterflies on registers alone keeps it 74 %
@@ -51,7 +51,11 @@ struct BlockArgs {
     uint32_t bg_bits, Br, flags;
     uint32_t c54;         // 2^54 mod Q
     unsigned *status;
-    unsigned wait_limit;
+    unsigned wait_limit;       // polls of a key wait (items form: of an item's wait)
+    // latency form over items: the cursor, the ciphertexts' done words, polls of their waits
+    unsigned long long *cursor;
+    int *done;
+    unsigned item_wait_limit;
 };
 
 __device__ __forceinline__ int next_issued(const uint8_t *res, int s, int S, int mode)
@@ -61,10 +65,47 @@ __device__ __forceinline__ int next_issued(const uint8_t *res, int s, int S, int
     return S;
 }
 
+// Polls of a worker waiting for another worker's item of the same ciphertext
+// (about 60 ns each) before it gives up and flags the launch.
+constexpr unsigned kItemWaitLimit = 1u << 26;
+
+// Item v of the step-major cursor as (item of the ciphertext, ciphertext) in plan, once
+// the item before it of that ciphertext is done: that one was taken earlier, by CTAs that
+// are running, so the wait ends whether or not the whole grid is resident. plan[0] = -1:
+// no item left, or the wait was given up.
+__device__ __forceinline__ void take_item(unsigned long long *cursor, const int *done, size_t count,
+                                          unsigned long long items, unsigned limit, unsigned *status, int (&plan)[2])
+{
+    const unsigned long long v = atomicAdd(cursor, 1ull);
+    plan[0] = v < items ? (int)(v / count) : -1;
+    plan[1] = v < items ? (int)(v % count) : 0;
+    if (plan[0] < 0) return;
+    const volatile int *d = done + plan[1];
+    const int before = plan[0] - 1;
+    unsigned polls = 0;
+    while (*d != before) {
+        if (++polls > limit) {
+            atomicOr(status, kStatusWaitLimit);
+            plan[0] = -1;
+            break;
+        }
+        __nanosleep(32);
+    }
+    __threadfence();
+}
+
+// Steps of an item of the latency form: its accumulator, the barriers and the first keys
+// of an item cost about a third of a step.
+constexpr int kClusterItemSteps = 16;
+
 // Latency form: one ciphertext per cluster of C CTAs at a time, its accumulator in
 // shared memory for all its steps, a block's keys by bulk copies issued as soon as
-// the products of the block before are done.
-template <int B, int C>
+// the products of the block before are done. ITEMS, for more ciphertexts than
+// clusters that run at once: the clusters take items of kClusterItemSteps steps of a
+// ciphertext from a cursor, the accumulators in global memory between items (100 gates on
+// 76 clusters of 2: 23 us per step of all, where one CTA each took 30.7; a runtime flag
+// instead of the instances cost the others 2 %).
+template <int B, int C, bool ITEMS>
 __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_constant__ BlockArgs A,
                                                              const ulonglong2 *__restrict__ tw,
                                                              const ulonglong2 *__restrict__ itw,
@@ -79,6 +120,7 @@ __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_const
     uint2 *const kbuf = reinterpret_cast<uint2 *>(smem_raw + L::key_off(A.DG));
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint64_t zeta[NB][B - 1];
+    __shared__ int plan[2];
     const int tid = threadIdx.x, DG = A.DG;
     const int rank = C > 1 ? (int)(blockIdx.x % C) : 0, first = rank * NW;
     const int mode = issue_mode(A.flags);
@@ -99,8 +141,35 @@ __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_const
     else __syncthreads();
     unsigned parity = 0;
     bool failed = false, pending = false;   // pending: a key copy not yet waited for
+    const unsigned long long items =
+        (unsigned long long)((A.S + kClusterItemSteps - 1) / kClusterItemSteps) * A.count;
 
-    for (size_t gid = blockIdx.x / C; gid < A.count; gid += gridDim.x / C) {
+    for (size_t at = blockIdx.x / C;; at += gridDim.x / C) {
+        size_t gid = at;
+        int it = 0, s = -1, end = A.S;
+        if (ITEMS) {
+            if (rank == 0 && tid == 0) {
+                int pl[2];
+                take_item(A.cursor, A.done, A.count, items, A.item_wait_limit, A.status, pl);
+                plan[0] = pl[0];
+                plan[1] = pl[1];
+#pragma unroll
+                for (int r = 1; r < C; r++) {
+                    int *const q = cg::this_cluster().map_shared_rank(plan, r);
+                    q[0] = pl[0];
+                    q[1] = pl[1];
+                }
+            }
+            if (C > 1) cg::this_cluster().sync();
+            else __syncthreads();
+            it = plan[0];
+            if (it < 0) break;
+            gid = (size_t)plan[1];
+            s = it * kClusterItemSteps - 1;
+            end = min(A.S, (it + 1) * kClusterItemSteps);
+        } else if (gid >= A.count) {
+            break;
+        }
         const uint8_t *res = A.res + gid * (size_t)A.S;
         uint64_t *ga = A.accs + gid * 4096;
         for (int u = tid; u < 2 * NW; u += T) {
@@ -116,13 +185,13 @@ __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_const
             const uint2 *src = A.btkey + ((size_t)s * A.Br + res[s]) * rgsw + first + lb * M;
             if (tid < DG * 4) bulk_copy_g2s(kbuf + tid * M, src + (size_t)tid * 2048, M * 8, &bar);
         };
-        int s = next_issued(res, -1, A.S, mode);
-        if (s < A.S) {
+        s = next_issued(res, s, end, mode);
+        if (s < end) {
             fetch(s, 0);
             pending = !failed;
         }
-        for (int buf = 0; s < A.S; buf ^= C > 1) {
-            const int next = next_issued(res, s, A.S, mode);
+        for (int buf = 0; s < end; buf ^= C > 1) {
+            const int next = next_issued(res, s, end, mode);
             BlockCta<B, C> cta{g + buf * 4096, acc, work, {}, zeta, rank};
 #pragma unroll
             for (int r = 0; r < C; r++) cta.peer[r] = peer[r] + buf * 4096;
@@ -143,7 +212,7 @@ __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_const
                 },
                 [&](int lb) {
                     if (lb + 1 < NB) fetch(s, lb + 1);
-                    else if (next < A.S) fetch(next, 0);
+                    else if (next < end) fetch(next, 0);
                     else pending = pending && failed;   // nothing in flight, but for a copy that was given up
                 });
             s = next;
@@ -152,16 +221,16 @@ __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_const
             const int p = u / NW, e = u - p * NW;
             ga[p * 2048 + first + e] = acc[p * px(NW) + px(e)];
         }
-        __syncthreads();
+        if (ITEMS) __threadfence();
+        // the whole cluster: the next ciphertext starts with the first g buffer again
+        if (C > 1) cg::this_cluster().sync();
+        else __syncthreads();
+        if (ITEMS && rank == 0 && tid == 0) atomicExch(A.done + gid, it);
     }
     // a copy that was given up must land before the CTA's shared memory goes
     if (failed && tid == 0) mbar_wait_bounded(&bar, parity, (int)kKeyWaitLimit);
     if (C > 1) cg::this_cluster().sync();
 }
-
-// Polls of a worker waiting for another worker's item of the same ciphertext
-// (about 60 ns each) before it gives up and flags the launch.
-constexpr unsigned kItemWaitLimit = 1u << 26;
 
 // Steps of an item: long enough that taking it, and the accumulator's way through L2
 // and back, cost little, short enough that the keys in use (9 MB a step) stay in L2 and
@@ -203,26 +272,7 @@ __global__ void __launch_bounds__(W * worker_threads64(W), 1) br64_items_kernel(
     __syncthreads();
     const unsigned long long items = (unsigned long long)((A.S + kItemSteps - 1) / kItemSteps) * A.count;
     for (;;) {
-        if (tid == 0) {
-            const unsigned long long v = atomicAdd(cursor, 1ull);
-            const int it = v < items ? (int)(v / A.count) : -1;
-            const size_t k = it < 0 ? 0 : (size_t)(v - (unsigned long long)it * A.count);
-            plan[0] = it;
-            plan[1] = (int)k;
-            if (it >= 0) {
-                const volatile int *d = done + k;
-                unsigned polls = 0;
-                while (*d != it - 1) {
-                    if (++polls > A.wait_limit) {
-                        atomicOr(A.status, kStatusWaitLimit);
-                        plan[0] = -1;
-                        break;
-                    }
-                    __nanosleep(32);
-                }
-                __threadfence();
-            }
-        }
+        if (tid == 0) take_item(cursor, done, A.count, items, A.wait_limit, A.status, plans[wk]);
         group_sync(bar, T);
         const int it = plan[0], k = plan[1];
         if (it < 0) break;
@@ -336,43 +386,100 @@ static int sm_count64(Context &c)
     return v > 0 ? v : 1;
 }
 
-template <int B, int C>
-static int launch_cluster(Context &c, const dev::BlockArgs &A, int max_ctas, cudaStream_t st, bool *fits)
+// Launch configuration of the latency form and the clusters that run at once (0: the form
+// does not fit).
+template <int B, int C, bool ITEMS>
+static int cluster_config(Context &c, const dev::BlockArgs &A, cudaStream_t st, cudaLaunchConfig_t &cfg,
+                          cudaLaunchAttribute (&attr)[1])
 {
-    auto kern = dev::br64_cluster_kernel<B, C>;
+    auto kern = dev::br64_cluster_kernel<B, C, ITEMS>;
     const size_t smem = dev::BlockLayout<B, C>::key_off(A.DG) + dev::BlockLayout<B, C>::key_bytes(A.DG);
-    *fits = false;
-    if (smem > 227 * 1024 || (max_ctas > 0 && max_ctas < C)) return FHEACC_OK;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return c.cuda_fail(e, "blind rotation smem attribute");
-    cudaLaunchConfig_t cfg = {};
+    if (smem > 227 * 1024) return 0;
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3(C);
     cfg.blockDim = dim3(dev::kTB);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = C;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = C > 1 ? 1 : 0;
-    size_t clusters = (size_t)sm_count64(c);
-    if (C > 1) {
-        int n = 0;
-        cfg.gridDim = dim3(C);
-        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            return FHEACC_OK;
-        }
-        clusters = (size_t)n;
-        if (A.count > clusters) return FHEACC_OK;   // more than one round: fewer CTAs per ciphertext
+    int n = sm_count64(c);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        (C > 1 && cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess)) {
+        cudaGetLastError();
+        return 0;
     }
+    return n;
+}
+
+template <int B, int C, bool ITEMS>
+static int launch_cluster(Context &c, const dev::BlockArgs &A, int max_ctas, cudaStream_t st)
+{
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    size_t clusters = (size_t)cluster_config<B, C, ITEMS>(c, A, st, cfg, attr);
     if (max_ctas > 0) clusters = std::min<size_t>(clusters, (size_t)(max_ctas / C));
-    *fits = true;
+    if (!clusters) return c.fail(FHEACC_EINVAL, "blind rotation latency form does not fit");
+    cudaError_t e;
+    if (ITEMS) {
+        e = cudaMemsetAsync(A.cursor, 0, sizeof(*A.cursor), st);
+        if (e != cudaSuccess) return c.cuda_fail(e, "blind rotation cursor reset");
+    }
     cfg.gridDim = dim3((unsigned)(std::min<size_t>(A.count, clusters) * C));
-    e = cudaLaunchKernelEx(&cfg, kern, A, (const ulonglong2 *)c.d_tw64, (const ulonglong2 *)c.d_itw64, c.nc64);
+    e = cudaLaunchKernelEx(&cfg, dev::br64_cluster_kernel<B, C, ITEMS>, A, (const ulonglong2 *)c.d_tw64,
+                           (const ulonglong2 *)c.d_itw64, c.nc64);
     c.launches++;
     if (e == cudaSuccess) e = cudaGetLastError();
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "blind rotation launch");
+}
+
+// The latency form in the CTAs per ciphertext (and over items or not) that give a step of
+// all ciphertexts the least time, unless the throughput form's is less (*taken = false).
+// The times, us, as a + b (digitG - 2), fitted at digitG = 2, 4 and 6: a step on 8, 4, 2
+// and 1 CTAs while all ciphertexts run at once; that times ciphertexts per cluster and 4 %
+// over items; the throughput form's, a worker's chain up to two ciphertexts per SM. At
+// digitG = 6: over items 4 CTAs from 39 to 60 gates, 2 from 77 to 131, 1 from 153 to 241.
+// Blind rotation of n = 200: 50 gates 6.57 ms on 2 CTAs, 5.57 over items on 4; 62 gates 6.55
+// and 6.59; 100 gates 11.8 on one, 8.8 over items on 2; 130 gates 11.7 and 11.6; 160 gates
+// 19.4 in the throughput form, 12.7 over items on one; 230 gates 20.2 and 18.0; 260 gates
+// 20.5 and 20.6.
+static int launch_latency(Context &c, const dev::BlockArgs &A, int max_ctas, cudaStream_t st, bool *taken)
+{
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    const size_t sms = (size_t)sm_count64(c), at_once = max_ctas > 0 ? (size_t)max_ctas : sms;
+    struct Form {
+        int (*launch)(Context &, const dev::BlockArgs &, int, cudaStream_t);
+        int C, n;
+        double step;
+        bool items;
+    };
+    const int n4 = cluster_config<4, 4, false>(c, A, st, cfg, attr), n2 = cluster_config<4, 2, false>(c, A, st, cfg, attr),
+              n1 = cluster_config<4, 1, false>(c, A, st, cfg, attr);
+    const double d = A.DG - 2;
+    const double t4 = 7.5 + 0.7 * d, t2 = 11.2 + 1.475 * d, t1 = 15.2 + 3.88 * d;
+    const Form forms[] = {
+        {launch_cluster<8, 8, false>, 8, c.p.BG_bits <= 29 ? cluster_config<8, 8, false>(c, A, st, cfg, attr) : 0,
+         6.8 + 0.47 * d, false},
+        {launch_cluster<4, 4, false>, 4, n4, t4, false}, {launch_cluster<4, 2, false>, 2, n2, t2, false},
+        {launch_cluster<4, 1, false>, 1, n1, t1, false}, {launch_cluster<4, 4, true>, 4, n4, t4, true},
+        {launch_cluster<4, 2, true>, 2, n2, t2, true},   {launch_cluster<4, 1, true>, 1, n1, t1, true}};
+    double least = std::max(31.0 + 5.0 * d, (14.5 + 3.25 * d) * (double)A.count / sms);
+    const Form *best = nullptr;
+    for (const Form &f : forms) {
+        if (f.n < 1 || at_once < (size_t)f.C) continue;
+        const bool fits = A.count <= (size_t)f.n;
+        if (f.items ? fits || max_ctas > 0 : !fits) continue;
+        const double t = f.items ? 1.04 * f.step * (double)A.count / f.n : f.step;
+        if (t < least) {
+            best = &f;
+            least = t;
+        }
+    }
+    *taken = best != nullptr;
+    return best ? best->launch(c, A, max_ctas, st) : FHEACC_OK;
 }
 
 template <int B, int W>
@@ -413,17 +520,13 @@ int launch_blind_rotate64_blocks(Context &c, const dev::Br64Args &R, int max_cta
     c.launches++;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return c.cuda_fail(e, "blind rotation begin launch");
-    // up to one ciphertext per SM the latency form, on as many CTAs per ciphertext as
-    // run at once; beyond that the items form (an explicit worker count asks for it)
-    bool fits = false;
-    int rc = FHEACC_OK;
-    if (c.tune.br_pipes == 0 && R.count <= (size_t)sm_count64(c)) {
-        if (c.p.BG_bits <= 29) rc = launch_cluster<8, 8>(c, A, max_ctas, st, &fits);
-        if (!rc && !fits) rc = launch_cluster<4, 4>(c, A, max_ctas, st, &fits);
-        if (!rc && !fits) rc = launch_cluster<4, 2>(c, A, max_ctas, st, &fits);
-        if (!rc && !fits) rc = launch_cluster<4, 1>(c, A, max_ctas, st, &fits);
-    }
-    if (!rc && !fits)   // digitG = 7 and 8: one worker's work area more than fills half an SM
+    A.cursor = cursor;
+    A.done = done;
+    A.item_wait_limit = c.tune.debug_wait_limit >= 0 ? (unsigned)c.tune.debug_wait_limit : dev::kItemWaitLimit;
+    // an explicit worker count asks for the throughput form
+    bool taken = false;
+    int rc = c.tune.br_pipes == 0 ? launch_latency(c, A, max_ctas, st, &taken) : FHEACC_OK;
+    if (!rc && !taken)   // digitG = 7 and 8: one worker's work area more than fills half an SM
         rc = 2 * dev::BlockLayout<4, 1>::key_off(A.DG) <= 227 * 1024 ? launch_items<4, 2>(c, A, cursor, done, max_ctas, st)
                                                                      : launch_items<4, 1>(c, A, cursor, done, max_ctas, st);
     if (rc) return rc;

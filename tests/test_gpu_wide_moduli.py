@@ -115,3 +115,40 @@ def test_forms_agree(F, cuda_ok, small_wide, count):
                 ctx.set_option(F.OPT_BR_PIPES, 0)
             got.append((acc, out))
         assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.fixture(scope="module")
+def longer_wide(F, cuda_ok):
+    P = F.params_preset(1)
+    P.n = 20   # 40 steps: three items of the latency form
+    F.derive(P)
+    lsk, rsk = F.LWE_secretkey(P, 1), F.RLWE_secretkey(P, 2)
+    with F.Context(P, 0) as ctx:
+        ctx.upload_bootstrap_key(F.bootstrap_key(P, 3, lsk, rsk))
+        ctx.upload_keyswitch_key(F.keyswitch_key(P, 4, rsk, lsk))
+        yield P, ctx, lsk
+
+
+@pytest.mark.parametrize("count", [38, 39, 61, 64, 77, 100, 131, 134, 153, 200])
+def test_cluster_items_agree(F, cuda_ok, longer_wide, count):
+    """More gates than clusters that run at once: clusters that take items of the gates
+    against the items form, in the three issue orders; twice, from the same scratch."""
+    torch = cuda_ok
+    P, ctx, lsk = longer_wide
+    rng = np.random.default_rng(count)
+    ct = F.LWE_encrypt(P, 70 + count, lsk, rng.integers(0, 2, 2 * count, dtype=np.uint8))
+    d1, d2 = dev(torch, ct[:count]), dev(torch, ct[count:])
+    dg = torch.from_numpy(rng.integers(0, 6, count).astype(np.int32)).cuda()
+    for flags in (0, F.FLAG_FPGA_COMPAT, F.FLAG_FPGA_X1):
+        got = []
+        for pipes in (0, 0, 2):
+            ctx.set_option(F.OPT_BR_PIPES, pipes)
+            try:
+                acc = torch.zeros((count, 2 * P.N), dtype=torch.int64, device="cuda")
+                ctx.blind_rotate_async(d1.data_ptr(), d2.data_ptr(), dg.data_ptr(), count, acc.data_ptr(), flags)
+                ctx.sync()
+                got.append(host(acc))
+            finally:
+                ctx.set_option(F.OPT_BR_PIPES, 0)
+        assert np.array_equal(got[0], got[2]) and np.array_equal(got[1], got[2]), flags
+    assert ctx.device_status() == 0
