@@ -594,6 +594,12 @@ static bool items32_pay(size_t count, size_t sms)
     return 2.42 * (double)count / (double)sms < 2.24 * (double)((count + sms - 1) / sms) + 0.4;
 }
 
+// Workers per CTA of the items form: one up to 1.8 gates per SM (a step 3.2 us with its
+// whole key brought to shared memory; blind rotation, one / two workers: 160 gates 3.18 /
+// 4.73 ms, 260 gates 5.10 / 5.36, 290 gates 5.69 / 5.53), 1.7 at digitG = 3 and 1.55 at 2
+// (n = 100, whole calls: 240 gates 0.951 / 1.026 and 0.785 / 0.788, 273 gates 1.074 / 1.060
+// and 0.887 / 0.826); two up to 2.5, else three (block32.cuh).
+//
 // Pipelines per CTA. By default from the gates per SM (one GB300, 4096-gate
 // key set): up to 2 a single pipeline per SM is fastest (its items do not
 // wait on other pipelines), up to 5 two pipelines, beyond that three.
@@ -611,7 +617,8 @@ static int launch_pipe_shape(Context &c, const dev::PipeArgs &A, int max_ctas, c
     }
     if (A.items_ok && c.tune.br_solo != 0 && c.tune.br_pipes == 0 && c.tune.debug_wait_limit < 0 &&
         items32_pay(A.count, sms))
-        return 2 * A.count <= 5 * sms ? launch_items32<DG, 2>(c, A, max_ctas, st)
+        return 20 * A.count <= (DG == 2 ? 31 : DG == 3 ? 34 : 36) * sms ? launch_items32<DG, 1>(c, A, max_ctas, st)
+               : 2 * A.count <= 5 * sms ? launch_items32<DG, 2>(c, A, max_ctas, st)
                                       : launch_items32<DG, 3>(c, A, max_ctas, st);
     const int np = c.tune.br_pipes > 0 ? c.tune.br_pipes : A.count <= 2 * sms ? 1 : A.count <= 5 * sms ? 2 : 3;
     if (np == 3) return launch_pipe_dg<DG, 3, 1>(c, A, max_ctas, st);

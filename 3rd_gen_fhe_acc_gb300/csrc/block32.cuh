@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(Block32Layout<DG, C>::T, 1)
     }
 }
 
-// ---- Items form (a few gates per SM): W workers of 768 / W threads per CTA, whose
+// ---- Items form (more than a gate per SM, to a few): W workers of 768 / W threads per CTA, whose
 // barriers and loads overlap, take items, consecutive steps of one ciphertext, from a
 // cursor that walks them step-major; the accumulator goes through L2 between items. So
 // the work spreads evenly over the SMs whatever the batch, where the pipelines give whole
@@ -435,13 +435,14 @@ __global__ void __launch_bounds__(Block32Layout<DG, C>::T, 1)
 // workers of 8 warps divide every phase evenly over the four schedulers and reach 2.5 us
 // per step and SM; with two of 12 the few ciphertexts of a small batch advance faster
 // (blind rotation, two / three workers: 304 gates 5.6 / 6.1 ms, 512 gates 9.1 / 8.2 ms).
-// Bound by the multiply pipe (61 % busy; a loop of butterflies alone reaches 82 %).
+// Bound by the multiply pipe (70 % busy; a loop of butterflies alone reaches 82 %).
 // Digit tables instead of multiplications did not pay here: 1000 gates 16.0 -> 16.1 ms.
-// With three workers the shared memory left holds the first 4 of a step's 16 key rows,
-// by one bulk copy that the transforms hide; the others come from L2 as they are
-// multiplied (1000 gates 15.95 -> 15.70 ms). With two workers 4 to 12 rows gained nothing.
+// A step's key rows in shared memory, by one bulk copy that the transforms hide: all of
+// them with one worker (160 gates 3.75 -> 3.18 ms), the first 4 of 16 with three (1000 gates
+// 15.95 -> 15.70 ms), the others from L2 as they are multiplied. With two workers 4 to 12
+// rows gained nothing.
 constexpr int kItem32Threads = 768;   // of a CTA
-__host__ __device__ constexpr int item32_key_rows(int W) { return W == 2 ? 0 : 4; }
+__host__ __device__ constexpr int item32_key_rows(int DG, int W) { return W == 1 ? 4 * DG : W == 2 ? 0 : 4; }
 constexpr int kItem32KeyWaitLimit = 1 << 22;   // polls before a key wait gives up
 __host__ __device__ constexpr int item32_steps(int W) { return W == 2 ? 8 : 16; }
 
@@ -453,7 +454,7 @@ template <int DG, int W>
 __host__ __device__ constexpr size_t item32_worker_bytes()
 {
     return 4 * (2 * kN32 + (size_t)2 * 2 * 4 * kB32E + (size_t)2 * (DG - 1) * 4 * kB32E +
-                (size_t)item32_key_rows(W) * kN32);
+                (size_t)item32_key_rows(DG, W) * kN32);
 }
 template <int DG, int W>
 constexpr size_t item32_bytes()
@@ -494,7 +495,7 @@ __global__ void __launch_bounds__(kItem32Threads, 1)
     const int wk = threadIdx.x / T, tid = threadIdx.x - wk * T, bar = 1 + wk;
     uint32_t *const g = reinterpret_cast<uint32_t *>(blk_smem + 2 * kN32 * sizeof(uint2) + wk * item32_worker_bytes<DG, W>());
     uint32_t *const acc = g + 2 * kN32, *const dbuf = acc + 2 * 2 * 4 * kB32E, *const head = dbuf + 2 * (DG - 1) * 4 * kB32E;
-    constexpr int KP = item32_key_rows(W);
+    constexpr int KP = item32_key_rows(DG, W);
     __shared__ __align__(8) uint64_t bars[W];
     unsigned parity = 0;
     bool failed = false;
