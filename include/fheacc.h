@@ -245,8 +245,8 @@ int fheacc_lwe_modswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t cou
  *                             8 for 64-bit); the launch fits equal groups to
  *                             the batch under the cap
  *  (64-bit words, Q = 2^b - c with 48 <= b <= 54 and c <= 2^(b-36): one kernel
- *  on clusters of CTAs up to one ciphertext per SM, else one that takes items
- *  of a few steps from a shared cursor; FHEACC_OPT_BR_PIPES other than 0 asks
+ *  on clusters of CTAs for up to 1.6 ciphertexts per SM, else one of workers
+ *  that take items of a few steps from a shared cursor; FHEACC_OPT_BR_PIPES other than 0 asks
  *  for the second at any count, and GROUP, WINDOW and POOL do not apply)
  *  FHEACC_OPT_BR_WINDOW     : 64-bit words: steps per bucket of the step
  *                             window that keeps the CTAs of a launch within
