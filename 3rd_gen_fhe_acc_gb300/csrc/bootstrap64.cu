@@ -531,11 +531,14 @@ __device__ __forceinline__ uint64_t scale_round64(uint64_t x, uint64_t new_mod, 
 // One CTA per ciphertext, one thread per two words of a key row (ks_row / 2
 // threads, one 128-bit load per row), eight rows in flight per iteration;
 // the 64-bit sums are folded mod Q every A.fold rows (fold * Q < 2^64).
+// Dig: the digits' type, the narrowest that holds Bks - 1 (ks_digit_bytes).
 constexpr int kKs64Unroll = 8;
 
+template <class Dig>
 __global__ void __launch_bounds__(512) lwe_ks64_kernel(const __grid_constant__ Ks64Args A)
 {
-    extern __shared__ uint8_t digits[];   // [N][digitKS]
+    extern __shared__ __align__(16) unsigned char ks_smem[];
+    Dig *const digits = reinterpret_cast<Dig *>(ks_smem);   // [N][digitKS]
     const int n = A.n, N = A.N, D = A.digitKS, t = threadIdx.x;
     const uint64_t Q = A.Q;
     const size_t rs2 = A.ks_row / 2;
@@ -545,7 +548,7 @@ __global__ void __launch_bounds__(512) lwe_ks64_kernel(const __grid_constant__ K
         for (int i = t; i < N; i += blockDim.x) {
             uint64_t a = ext[i];
             for (int j = 0; j < D; j++) {
-                digits[i * D + j] = (uint8_t)(a % A.Bks);
+                digits[i * D + j] = (Dig)(a % A.Bks);
                 a /= A.Bks;
             }
         }
@@ -609,10 +612,11 @@ __global__ void __launch_bounds__(512) lwe_ks64_kernel(const __grid_constant__ K
 // they were the kernel's time (100 gates, n = 630: 13.0 ms, now 1.07).
 constexpr int kKs64MaxFold = 256;
 
+template <class Dig>
 __global__ void __launch_bounds__(512) ks64_partial_kernel(const __grid_constant__ Ks64Args A,
                                                            unsigned long long *part, int slices, uint64_t magic)
 {
-    __shared__ uint8_t dig[kKs64MaxFold];
+    __shared__ Dig dig[kKs64MaxFold];
     const int N = A.N, D = A.digitKS, t = threadIdx.x;
     const uint64_t Q = A.Q;
     const size_t rs2 = A.ks_row / 2;
@@ -626,7 +630,7 @@ __global__ void __launch_bounds__(512) ks64_partial_kernel(const __grid_constant
         for (int j = 0; j < D; j++) {
             const uint64_t qt = magic ? __umul64hi(a, magic) : a / A.Bks;
             const int r = i * D + j;
-            if (r >= r0 && r < r1) dig[r - r0] = (uint8_t)(a - qt * A.Bks);
+            if (r >= r0 && r < r1) dig[r - r0] = (Dig)(a - qt * A.Bks);
             a = qt;
         }
     }
@@ -945,6 +949,7 @@ int launch_lwe_keyswitch64(Context &c, const uint64_t *d_extract, size_t count, 
     // below that each ciphertext's rows are split over CTAs (ks_tiled = 0: only below two
     // ciphertexts per SM), with at most `fold` rows per CTA and slices * Q < 2^64
     const int rows = c.p.N * (int)c.p.digitKS;
+    const size_t digit_bytes = ks_digit_bytes(c.p.Bks);
     const size_t max_slices = std::min<uint64_t>(UINT64_MAX / c.p.Q, 4096);
     const size_t slices = std::min<size_t>(max_slices, std::max<size_t>((size_t)(rows + A.fold - 1) / A.fold,
                                                                          sms * 8 / std::max<size_t>(count, 1)));
@@ -953,8 +958,10 @@ int launch_lwe_keyswitch64(Context &c, const uint64_t *d_extract, size_t count, 
         unsigned long long *part = reinterpret_cast<unsigned long long *>(d_scratch);
         cudaError_t e = cudaMemsetAsync(part, 0, count * c.dp.ks_row * sizeof(uint64_t), st);
         if (e != cudaSuccess) return c.cuda_fail(e, "key switch partials reset");
-        dev::ks64_partial_kernel<<<(unsigned)(count * slices), threads, 0, st>>>(A, part, (int)slices,
-                                                                                       ks64_digit_magic(c));
+        const auto kern = digit_bytes == 1   ? dev::ks64_partial_kernel<uint8_t>
+                          : digit_bytes == 2 ? dev::ks64_partial_kernel<uint16_t>
+                                             : dev::ks64_partial_kernel<uint32_t>;
+        kern<<<(unsigned)(count * slices), threads, 0, st>>>(A, part, (int)slices, ks64_digit_magic(c));
         c.launches++;
         e = cudaGetLastError();
         if (e != cudaSuccess) return c.cuda_fail(e, "key switch partial launch");
@@ -964,9 +971,12 @@ int launch_lwe_keyswitch64(Context &c, const uint64_t *d_extract, size_t count, 
         e = cudaGetLastError();
         return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "key switch final launch");
     }
-    const size_t smem = (size_t)c.p.N * c.p.digitKS;
+    const size_t smem = (size_t)c.p.N * c.p.digitKS * digit_bytes;
     size_t blocks = std::min<size_t>(count, sms * 6);
-    dev::lwe_ks64_kernel<<<(unsigned)blocks, threads, smem, st>>>(A);
+    const auto kern = digit_bytes == 1   ? dev::lwe_ks64_kernel<uint8_t>
+                      : digit_bytes == 2 ? dev::lwe_ks64_kernel<uint16_t>
+                                         : dev::lwe_ks64_kernel<uint32_t>;
+    kern<<<(unsigned)blocks, threads, smem, st>>>(A);
     c.launches++;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "lwe_ks64 launch");

@@ -55,6 +55,11 @@ constexpr size_t kPipeSmemBudget = 220 * 1024;   // dynamic shared memory of one
 // of up to n + 1 <= 1024 words.
 constexpr int kKsMaxThreads = 256;
 
+// Bytes of a base-Bks digit of the LWE key switch in shared memory: a digit reaches
+// Bks - 1. (The tiled forms take a Bks of at most 255.)
+constexpr size_t ks_digit_bytes(uint32_t Bks) { return Bks <= 256 ? 1 : Bks <= 65536 ? 2 : 4; }
+constexpr size_t kKsDigitSmem = 48 * 1024;   // digits of a split key-switch CTA
+
 constexpr size_t kClaimWords = 64;   // u32 words of claim counters after the blind-rotation accumulators
 // 64-bit blind rotation: most remainder gates of a batch that the CTAs share
 // item by item (their per-gate state follows the claim words)

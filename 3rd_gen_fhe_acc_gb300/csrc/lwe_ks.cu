@@ -59,11 +59,14 @@ __device__ __forceinline__ uint64_t scale_round_dev(uint64_t x, uint64_t new_mod
 // digits in shared memory, then walks the N * digitKS rows it selects
 // (kskey[d][j][i]), kKsUnroll rows per iteration so that each thread has that
 // many independent loads in flight, with 64-bit sums.
+// Dig: the digits' type, the narrowest that holds Bks - 1 (ks_digit_bytes).
 constexpr int kKsUnroll = 8;
 
+template <class Dig>
 __global__ void __launch_bounds__(kKsMaxThreads) lwe_ks32_kernel(const __grid_constant__ KsArgs A)
 {
-    extern __shared__ uint8_t digits[];   // [N][digitKS]
+    extern __shared__ __align__(16) unsigned char ks_smem[];
+    Dig *const digits = reinterpret_cast<Dig *>(ks_smem);   // [N][digitKS]
     const int n = A.n, N = A.N, D = A.digitKS, t = threadIdx.x;
     const uint32_t Q = (uint32_t)A.Q;
     const size_t rs4 = A.ks_row / 4;
@@ -73,7 +76,7 @@ __global__ void __launch_bounds__(kKsMaxThreads) lwe_ks32_kernel(const __grid_co
         for (int i = t; i < N; i += blockDim.x) {
             uint32_t a = ext[i];
             for (int j = 0; j < D; j++) {
-                digits[i * D + j] = (uint8_t)(a % A.Bks);
+                digits[i * D + j] = (Dig)(a % A.Bks);
                 a /= A.Bks;
             }
         }
@@ -128,10 +131,12 @@ __global__ void __launch_bounds__(kKsMaxThreads) lwe_ks32_kernel(const __grid_co
 // the grid (the ciphertexts' CTAs of one slice read its rows together, from L2), and
 // the CTA's digits are computed once into shared memory: computed by every thread for
 // every row, with up to digitKS - 1 divisions each, 96 gates took 0.42 ms.
+template <class Dig>
 __global__ void __launch_bounds__(kKsMaxThreads) ks_partial_kernel(const __grid_constant__ KsArgs A,
                                                                    unsigned long long *part, int slices)
 {
-    extern __shared__ uint8_t dig[];   // [per]
+    extern __shared__ __align__(16) unsigned char ks_smem[];
+    Dig *const dig = reinterpret_cast<Dig *>(ks_smem);   // [per]
     const int N = A.N, D = A.digitKS, t = threadIdx.x;
     const size_t rs4 = A.ks_row / 4;
     const uint4 *key4 = reinterpret_cast<const uint4 *>(A.kskey) + t;
@@ -143,7 +148,7 @@ __global__ void __launch_bounds__(kKsMaxThreads) ks_partial_kernel(const __grid_
         uint32_t a = ext[i];
         for (int j = 0; j < D; j++) {
             const int r = i * D + j;
-            if (r >= r0 && r < r1) dig[r - r0] = (uint8_t)(a % A.Bks);
+            if (r >= r0 && r < r1) dig[r - r0] = (Dig)(a % A.Bks);
             a /= A.Bks;
         }
     }
@@ -681,13 +686,19 @@ int launch_lwe_keyswitch32(Context &c, const uint32_t *d_extract, size_t count, 
         return launch_lwe_keyswitch32_indexed(c, d_extract, count, modswitch, d_out, d_out_idx, st);
     uint64_t *d_partials = (uint64_t *)d_scratch;
     const int rows = c.p.N * (int)c.p.digitKS;
+    const size_t digit_bytes = ks_digit_bytes(c.p.Bks);
     // 32 CTAs (of 4 warps) per SM, at least 8 per ciphertext, at least 48 rows each
-    // (1000 gates: 1.14 ms; 8 per SM 1.73, 16 per SM 1.29, 64 per SM 1.13)
+    // (1000 gates: 1.14 ms; 8 per SM 1.73, 16 per SM 1.29, 64 per SM 1.13), and at most
+    // 48 KB of digits each (only a digitKS of hundreds reaches that)
     const int slices = (int)std::max<size_t>(
-        1, std::min<size_t>((size_t)rows / 48, std::max<size_t>(8, (size_t)sms * 32 / count)));
+        {1, ((size_t)rows * digit_bytes + kKsDigitSmem - 1) / kKsDigitSmem,
+         std::min<size_t>((size_t)rows / 48, std::max<size_t>(8, (size_t)sms * 32 / count))});
     cudaError_t e = cudaMemsetAsync(d_partials, 0, count * c.dp.ks_row * sizeof(uint64_t), st);
     if (e != cudaSuccess) return c.cuda_fail(e, "key switch partials reset");
-    dev::ks_partial_kernel<<<(unsigned)(count * slices), c.dp.ks_row / 4, (size_t)(rows + slices - 1) / slices, st>>>(
+    const auto kern = digit_bytes == 1   ? dev::ks_partial_kernel<uint8_t>
+                      : digit_bytes == 2 ? dev::ks_partial_kernel<uint16_t>
+                                         : dev::ks_partial_kernel<uint32_t>;
+    kern<<<(unsigned)(count * slices), c.dp.ks_row / 4, (size_t)((rows + slices - 1) / slices) * digit_bytes, st>>>(
         A, reinterpret_cast<unsigned long long *>(d_partials), slices);
     c.launches++;
     e = cudaGetLastError();
@@ -710,12 +721,15 @@ int launch_lwe_keyswitch32_indexed(Context &c, const uint32_t *d_extract, size_t
     A.ext = d_extract; A.count = count; A.kskey = c.d_kskey; A.out = d_out; A.out_idx = d_out_idx;
     A.n = c.p.n; A.N = c.p.N; A.digitKS = (int)c.p.digitKS; A.Bks = c.p.Bks; A.ks_row = c.dp.ks_row;
     A.q = c.p.q; A.modswitch = modswitch ? 1u : 0u; A.Q = c.p.Q;
-    const size_t smem = (size_t)c.p.N * c.p.digitKS;
+    const size_t digit_bytes = ks_digit_bytes(c.p.Bks), smem = (size_t)c.p.N * c.p.digitKS * digit_bytes;
+    const auto kern = digit_bytes == 1   ? dev::lwe_ks32_kernel<uint8_t>
+                      : digit_bytes == 2 ? dev::lwe_ks32_kernel<uint16_t>
+                                         : dev::lwe_ks32_kernel<uint32_t>;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
     const unsigned threads = (unsigned)(c.dp.ks_row / 4);   // ks_row: multiple of 32 words, > n
     size_t blocks = std::min<size_t>(count, (size_t)std::max(sms, 1) * 16);
-    dev::lwe_ks32_kernel<<<(unsigned)blocks, threads, smem, st>>>(A);
+    kern<<<(unsigned)blocks, threads, smem, st>>>(A);
     c.launches++;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "lwe_ks32 launch");
