@@ -94,6 +94,26 @@ __device__ __forceinline__ void take_item(unsigned long long *cursor, const int 
     __threadfence();
 }
 
+// The give-up state of a CTA's key copies.
+struct KeyWaits {
+    int gave_up;   // a thread has given up a wait: no more copies are issued
+    int stopped;   // warp 0 has seen that
+    int owed;      // 1 + the phase of a copy that may still land (0: none)
+};
+
+// The rest of a key wait that the first of `limit` polls did not end: to the last, or until
+// another thread of the CTA has given up (its warp may not have issued the copy). Giving
+// up flags the launch.
+__device__ __noinline__ void wait_keys_slow(uint64_t *bar, unsigned parity, unsigned limit, volatile KeyWaits *w,
+                                            unsigned *status)
+{
+    for (unsigned i = 1; i < limit && !w->gave_up; i++)
+        if (mbar_try_wait(bar, parity)) return;
+    if (!w->gave_up) atomicOr(status, kStatusWaitLimit);
+    w->gave_up = 1;
+    if (threadIdx.x == 0 && !w->stopped) w->owed = 1 + (int)parity;
+}
+
 // Steps of an item of the latency form: its accumulator, the barriers and the first keys
 // of an item cost about a third of a step.
 constexpr int kClusterItemSteps = 16;
@@ -121,6 +141,7 @@ __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_const
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint64_t zeta[NB][B - 1];
     __shared__ int plan[2];
+    __shared__ volatile KeyWaits waits;
     const int tid = threadIdx.x, DG = A.DG;
     const int rank = C > 1 ? (int)(blockIdx.x % C) : 0, first = rank * NW;
     const int mode = issue_mode(A.flags);
@@ -134,13 +155,13 @@ __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_const
     }
     block_zeta<B, NB>(zeta, rank * NB, tw, c);
     if (tid == 0) {
+        waits.gave_up = waits.stopped = waits.owed = 0;
         mbar_init(&bar, 1);
         mbar_fence_init();
     }
     if (C > 1) cg::this_cluster().sync();
     else __syncthreads();
     unsigned parity = 0;
-    bool failed = false, pending = false;   // pending: a key copy not yet waited for
     const unsigned long long items =
         (unsigned long long)((A.S + kClusterItemSteps - 1) / kClusterItemSteps) * A.count;
 
@@ -177,19 +198,22 @@ __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_const
             acc[p * px(NW) + px(e)] = __ldcg(ga + p * 2048 + first + e);
         }
         __syncthreads();
-        // rows of block lb of step s into kbuf (warp 0)
+        // rows of block lb of step s into kbuf (warp 0; after a wait that was given up the
+        // warp issues no more, as one: a copy is issued whole or not at all, and the
+        // cluster runs to its end without keys, as its barriers need every CTA)
         auto fetch = [&](int s, int lb) {
-            if (tid >= 32 || failed) return;
+            if (tid >= 32) return;
+            if (__any_sync(~0u, waits.gave_up)) {
+                if (tid == 0) waits.stopped = 1;
+                return;
+            }
             if (tid == 0) mbar_expect_tx(&bar, (unsigned)L::key_bytes(DG));
             __syncwarp();
             const uint2 *src = A.btkey + ((size_t)s * A.Br + res[s]) * rgsw + first + lb * M;
             if (tid < DG * 4) bulk_copy_g2s(kbuf + tid * M, src + (size_t)tid * 2048, M * 8, &bar);
         };
         s = next_issued(res, s, end, mode);
-        if (s < end) {
-            fetch(s, 0);
-            pending = !failed;
-        }
+        if (s < end) fetch(s, 0);
         for (int buf = 0; s < end; buf ^= C > 1) {
             const int next = next_issued(res, s, end, mode);
             BlockCta<B, C> cta{g + buf * 4096, acc, work, {}, zeta, rank};
@@ -198,22 +222,14 @@ __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_const
             block_step<B, C, T, false>(
                 cta, A, tw, itw, c, M, tid, 0,
                 [&](int) {
-                    if (pending && !failed) {
-                        if (mbar_wait_bounded(&bar, parity, (int)A.wait_limit)) {
-                            parity ^= 1u;
-                        } else {
-                            // flag the launch and let the cluster run to its end without
-                            // keys: its barriers need every CTA
-                            failed = true;
-                            if (tid == 0) atomicOr(A.status, kStatusWaitLimit);
-                        }
-                    }
+                    if (!A.wait_limit || !mbar_try_wait(&bar, parity))
+                        wait_keys_slow(&bar, parity, A.wait_limit, &waits, A.status);
+                    parity ^= 1u;
                     return (const uint2 *)kbuf;
                 },
                 [&](int lb) {
                     if (lb + 1 < NB) fetch(s, lb + 1);
                     else if (next < end) fetch(next, 0);
-                    else pending = pending && failed;   // nothing in flight, but for a copy that was given up
                 });
             s = next;
         }
@@ -228,7 +244,7 @@ __global__ void __launch_bounds__(kTB, 1) br64_cluster_kernel(const __grid_const
         if (ITEMS && rank == 0 && tid == 0) atomicExch(A.done + gid, it);
     }
     // a copy that was given up must land before the CTA's shared memory goes
-    if (failed && tid == 0) mbar_wait_bounded(&bar, parity, (int)kKeyWaitLimit);
+    if (tid == 0 && waits.owed) mbar_wait_bounded(&bar, (unsigned)waits.owed - 1, (int)kKeyWaitLimit);
     if (C > 1) cg::this_cluster().sync();
 }
 
