@@ -571,8 +571,10 @@ static int launch_items32(Context &c, dev::PipeArgs A, int max_ctas, cudaStream_
     c.launches++;
     size_t blocks = std::min<size_t>((size_t)sm_count(c), A.count);
     if (max_ctas > 0) blocks = std::min<size_t>(blocks, (size_t)max_ctas);
-    kern<<<(unsigned)blocks, dev::kItem32Threads, smem, st>>>(A, c.nc, c.d_plain_tw, res, done,
-                                                                                    dev::kItem32WaitLimit);
+    const int limit = c.tune.debug_wait_limit;
+    kern<<<(unsigned)blocks, dev::kItem32Threads, smem, st>>>(
+        A, c.nc, c.d_plain_tw, res, done, limit >= 0 ? (unsigned)limit : dev::kItem32WaitLimit,
+        limit >= 0 ? limit : dev::kItem32KeyWaitLimit);
     c.launches++;
     dev::br32_end_kernel<<<(unsigned)A.count, 64, 0, st>>>(A, c.nc, c.d_inv_tw);
     c.launches++;
@@ -607,7 +609,8 @@ template <int DG>
 static int launch_pipe_shape(Context &c, const dev::PipeArgs &A, int max_ctas, cudaStream_t st)
 {
     const size_t sms = (size_t)sm_count(c);
-    // explicit pipeline shapes and the wait-limit tests keep the pipelines
+    // explicit pipeline shapes keep the pipelines, and so do the wait-limit tests unless
+    // they ask for these forms
     const int solo = c.tune.br_solo >= 0 ? c.tune.br_solo : kSoloGatesPerSm;
     if (solo > 0 && c.tune.br_pipes == 0 && c.tune.debug_wait_limit < 0 && A.count <= (size_t)solo * sms) {
         int rc = launch_block32<DG, 4>(c, A, max_ctas, st);
@@ -615,8 +618,8 @@ static int launch_pipe_shape(Context &c, const dev::PipeArgs &A, int max_ctas, c
         if (rc == 1) rc = launch_block32<DG, 1>(c, A, max_ctas, st);
         if (rc != 1) return rc;
     }
-    if (A.items_ok && c.tune.br_solo != 0 && c.tune.br_pipes == 0 && c.tune.debug_wait_limit < 0 &&
-        items32_pay(A.count, sms))
+    if (A.items_ok && c.tune.br_solo != 0 && c.tune.br_pipes == 0 &&
+        (c.tune.debug_wait_limit < 0 || c.tune.br_solo > 0) && items32_pay(A.count, sms))
         return 20 * A.count <= (DG == 2 ? 31 : DG == 3 ? 34 : 36) * sms ? launch_items32<DG, 1>(c, A, max_ctas, st)
                : 2 * A.count <= 5 * sms ? launch_items32<DG, 2>(c, A, max_ctas, st)
                                       : launch_items32<DG, 3>(c, A, max_ctas, st);

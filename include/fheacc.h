@@ -279,16 +279,18 @@ int fheacc_lwe_modswitch_async(fheacc_ctx *ctx, const uint64_t *d_in, size_t cou
  *                             to this many gates per SM; -1 (default) = 1,
  *                             0 = off, and so is the form for a few gates
  *                             per SM (workers that take items of a few
- *                             steps from a shared cursor). Not taken when
- *                             FHEACC_OPT_BR_PIPES or
- *                             FHEACC_OPT_DEBUG_WAIT_LIMIT is set.
+ *                             steps from a shared cursor). Neither is taken
+ *                             when FHEACC_OPT_BR_PIPES is set; with
+ *                             FHEACC_OPT_DEBUG_WAIT_LIMIT only the second,
+ *                             and only if this option is above 0.
  *  FHEACC_OPT_DEBUG_WAIT_LIMIT: for tests of the error path only. The
  *                             number of polls (64-bit workers, the step
- *                             window) or idle periods (32-bit pipelines) a
+ *                             window, key copies, gates worked on item by
+ *                             item) or idle periods (32-bit pipelines) a
  *                             bounded wait may take before it gives up;
  *                             -1 (default) = the built-in limits. With a
- *                             small value the waits between the workers of a
- *                             CTA expire: the kernel still returns, the
+ *                             small value such waits expire: the kernel
+ *                             still returns, the
  *                             launch's results are invalid,
  *                             FHEACC_STATUS_WAIT_LIMIT is set and
  *                             fheacc_sync / fheacc_bootstrap return

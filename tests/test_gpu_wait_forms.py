@@ -65,3 +65,23 @@ def expire(F, torch, P, ctx, lsk, count, limit, must):
 def test_wide_clusters(F, cuda_ok, wide, count, limit):
     """8, 4 and 2 CTAs a gate, and items of more gates than clusters that run at once."""
     expire(F, cuda_ok, *wide, count, limit, limit == 0)
+
+
+@pytest.fixture(scope="module")
+def narrow(F, cuda_ok):
+    P, ctx, lsk = make(F, 0, 20)   # 40 steps: three or five items of a gate
+    yield P, ctx, lsk
+    ctx.close()
+
+
+@pytest.mark.parametrize("limit", [0, 1, 2, 3])
+def test_narrow_items(F, cuda_ok, narrow, limit):
+    """One worker per CTA (whole keys copied), two (no copies; more workers than gates, so
+    the surplus ones wait for a gate's item before) and three (a part of the keys)."""
+    sms = cuda_ok.cuda.get_device_properties(0).multi_processor_count
+    narrow[1].set_option(F.OPT_BR_SOLO, 1)   # the items form, also with a limit
+    try:
+        for count in (sms + 8, 2 * sms - 20, 3 * sms):
+            expire(F, cuda_ok, *narrow, count, limit, limit == 0)
+    finally:
+        narrow[1].set_option(F.OPT_BR_SOLO, -1)
