@@ -566,8 +566,9 @@ class Context:
 
     def autotune(self, count, max_trials=64):
         """Times the blind rotation's launch options on a synthetic batch of
-        `count` gates and keeps the fastest (fheacc_autotune). Returns the
-        trials as dicts (regs_for_3, ctas_per_sm, group, ms)."""
+        `count` gates and keeps the fastest, the default shape (pipes = 0) if no
+        other is more than 1 % faster (fheacc_autotune). Returns the trials as
+        dicts (regs_for_3, ctas_per_sm, group, window, pipes, ms)."""
         arr = (TuneTrial * max_trials)()
         n = ctypes.c_int()
         self.check(lib().fheacc_autotune(self._h, count, arr, max_trials, ctypes.byref(n)))

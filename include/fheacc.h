@@ -333,7 +333,8 @@ int fheacc_measure_components(fheacc_ctx *ctx, double ns[4]);
 /* Picks the blind rotation's launch options (the FHEACC_OPT_BR_* above)
  * for batches of `count` gates: times every candidate on a synthetic batch of
  * that size (uniform LWE inputs mod q, the six gates in turn) with this
- * context's keys, and leaves the fastest set on the context. `trials` (may be
+ * context's keys, and leaves the fastest set on the context, the default
+ * (FHEACC_OPT_BR_PIPES = 0) if no other is more than 1 % faster. `trials` (may be
  * NULL) receives up to max_trials of the candidates with their times and
  * *n_trials (may be NULL) their number. Results are unchanged by the options;
  * only the launch shape differs. The reference has no counterpart (the FPGA
