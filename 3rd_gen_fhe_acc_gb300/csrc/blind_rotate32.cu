@@ -487,7 +487,7 @@ static int launch_pipe_dg(Context &c, dev::PipeArgs A, int max_ctas, cudaStream_
     if (cap < 1) return c.fail(FHEACC_EINVAL, "n * digitR too large for the blind rotation's residue table");
     // residency with the largest group allowed; the group is then fitted to the batch
     size_t smem = dev::pipe_tables_offset<GW, NP>(cap, steps) + tables;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(kern);
     if (e != cudaSuccess) return c.cuda_fail(e, "blind rotation smem attribute");
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
@@ -520,7 +520,7 @@ static int launch_block32(Context &c, const dev::PipeArgs &A, int max_ctas, cuda
     auto kern = dev::br32_block_kernel<DG, C>;
     const size_t smem = L::bytes((size_t)c.p.n * c.p.digitR);
     if (smem > kPipeSmemBudget || (max_ctas > 0 && max_ctas < C)) return 1;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(kern);
     if (e != cudaSuccess) return c.cuda_fail(e, "blind rotation (latency form) smem attribute");
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(L::T);
@@ -564,7 +564,7 @@ static int launch_items32(Context &c, dev::PipeArgs A, int max_ctas, cudaStream_
     A.claim_next = reinterpret_cast<unsigned long long *>(A.accs + A.count * 2048);
     int *done = reinterpret_cast<int *>(A.accs + A.count * 2048 + kClaimWords);
     uint8_t *res = reinterpret_cast<uint8_t *>(done + A.count);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(kern);
     if (e == cudaSuccess) e = cudaMemsetAsync(A.claim_next, 0, kClaimWords * sizeof(uint32_t), st);
     if (e != cudaSuccess) return c.cuda_fail(e, "blind rotation (items form) set-up");
     dev::br32_begin_kernel<<<(unsigned)A.count, 32, 0, st>>>(A, c.nc, c.d_fwd_tw, res, done, mu32);

@@ -410,7 +410,7 @@ static int cluster_config(Context &c, const dev::BlockArgs &A, cudaStream_t st, 
 {
     auto kern = dev::br64_cluster_kernel<B, C, ITEMS>;
     const size_t smem = dev::BlockLayout<B, C>::key_off(A.DG) + dev::BlockLayout<B, C>::key_bytes(A.DG);
-    if (smem > 227 * 1024) return 0;
+    if (smem > kMaxDynamicSmem) return 0;
     cfg = cudaLaunchConfig_t{};
     cfg.gridDim = dim3(C);
     cfg.blockDim = dim3(dev::kTB);
@@ -422,7 +422,7 @@ static int cluster_config(Context &c, const dev::BlockArgs &A, cudaStream_t st, 
     cfg.attrs = attr;
     cfg.numAttrs = C > 1 ? 1 : 0;
     int n = sm_count64(c);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (allow_dynamic_smem(kern) != cudaSuccess ||
         (C > 1 && cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess)) {
         cudaGetLastError();
         return 0;
@@ -504,7 +504,7 @@ static int launch_items(Context &c, dev::BlockArgs A, unsigned long long *cursor
 {
     auto kern = dev::br64_items_kernel<B, W>;
     const size_t smem = W * dev::BlockLayout<B, 1>::key_off(A.DG);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(kern);
     if (e != cudaSuccess) return c.cuda_fail(e, "blind rotation smem attribute");
     // an SM per ciphertext while there are enough: the surplus workers wait their turn
     size_t blocks = std::min<size_t>((size_t)sm_count64(c), A.count * std::max(c.tune.br_pipes, 1));
@@ -543,8 +543,9 @@ int launch_blind_rotate64_blocks(Context &c, const dev::Br64Args &R, int max_cta
     bool taken = false;
     int rc = c.tune.br_pipes == 0 ? launch_latency(c, A, max_ctas, st, &taken) : FHEACC_OK;
     if (!rc && !taken)   // digitG = 7 and 8: one worker's work area more than fills half an SM
-        rc = 2 * dev::BlockLayout<4, 1>::key_off(A.DG) <= 227 * 1024 ? launch_items<4, 2>(c, A, cursor, done, max_ctas, st)
-                                                                     : launch_items<4, 1>(c, A, cursor, done, max_ctas, st);
+        rc = 2 * dev::BlockLayout<4, 1>::key_off(A.DG) <= kMaxDynamicSmem
+                 ? launch_items<4, 2>(c, A, cursor, done, max_ctas, st)
+                 : launch_items<4, 1>(c, A, cursor, done, max_ctas, st);
     if (rc) return rc;
     dev::br64_end_kernel<<<(unsigned)R.count, dev::kT64, 0, st>>>(R, c.d_itw64, c.nc64);
     c.launches++;

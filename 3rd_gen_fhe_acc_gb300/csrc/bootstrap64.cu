@@ -814,7 +814,7 @@ static int launch_br64_shape(Context &c, dev::Br64Args A, int max_ctas, cudaStre
         return W * sizeof(dev::Step64Smem) + ((size_t)group * steps + 15) / 16 * 16;
     };
     size_t smem = smem_of(cap);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(kern);
     if (e != cudaSuccess) return c.cuda_fail(e, "br64 smem attribute");
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, W * dev::kT64, smem);

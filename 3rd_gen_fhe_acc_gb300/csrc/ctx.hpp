@@ -49,6 +49,17 @@ struct Tuning {
     int br_solo = -1;         // 32-bit path: latency form up to this many gates per SM (0: off; -1: default)
 };
 
+// Dynamic shared memory that a kernel is allowed, the same for every launch of it: the
+// attribute is the kernel's, not the launch's, so two contexts that ask for different
+// amounts from two threads would take each other's away between setting and launching.
+// 1 KB of a CTA's 227 is left to the kernels' static part.
+constexpr size_t kMaxDynamicSmem = 226 * 1024;
+template <class Kernel>
+inline cudaError_t allow_dynamic_smem(Kernel kern)
+{
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynamicSmem);
+}
+
 constexpr size_t kPipeSmemBudget = 220 * 1024;   // dynamic shared memory of one blind-rotation CTA
 
 // Threads of a 32-bit LWE key-switch CTA, four words of a key row each: rows

@@ -567,8 +567,8 @@ static int launch_expand_cluster(Context &c, const dev::ExpArgs &A, size_t items
     auto kern = dev::expand64_cluster_kernel<B, C>;
     const size_t smem = dev::ExpandLayout<B, C>::bytes(A.L);
     *fits = false;
-    if (smem > 227 * 1024 || items * C > (size_t)sms(c)) return FHEACC_OK;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > kMaxDynamicSmem || items * C > (size_t)sms(c)) return FHEACC_OK;
+    cudaError_t e = allow_dynamic_smem(kern);
     if (e != cudaSuccess) return c.cuda_fail(e, "expand smem attribute");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(items * C));
@@ -601,7 +601,7 @@ static int launch_expand_workers(Context &c, const dev::ExpArgs &A, size_t items
 {
     auto kern = dev::expand64_workers_kernel<4, W>;
     const int bytes = (int)dev::ExpandLayout<4, 1>::bytes(A.L);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, W * bytes);
+    cudaError_t e = allow_dynamic_smem(kern);
     if (e != cudaSuccess) return c.cuda_fail(e, "expand smem attribute");
     kern<<<(unsigned)std::min<size_t>(items, (size_t)sms(c)), W * dev::kTE, W * bytes, st>>>(
         A, items, bytes, c.d_tw64, c.d_itw64, c.nc64);
@@ -620,8 +620,8 @@ static int launch_expand_blocks(Context &c, const dev::ExpArgs &A, size_t items,
     if (!rc && !fits) rc = launch_expand_cluster<4, 2>(c, A, items, st, &fits);
     if (!rc && !fits) rc = launch_expand_cluster<4, 1>(c, A, items, st, &fits);
     if (rc || fits) return rc;
-    const size_t one = dev::ExpandLayout<4, 1>::bytes(A.L), most = 227 * 1024 - 512;   // 512: the kernel's static part
-    return 3 * one <= most ? launch_expand_workers<3>(c, A, items, st) : launch_expand_workers<2>(c, A, items, st);
+    return 3 * dev::ExpandLayout<4, 1>::bytes(A.L) <= kMaxDynamicSmem ? launch_expand_workers<3>(c, A, items, st)
+                                                                     : launch_expand_workers<2>(c, A, items, st);
 }
 
 // ksk: narrow, u32 [L][2][N] device words; wide, limb words (block form,

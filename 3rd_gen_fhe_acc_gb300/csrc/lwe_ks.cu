@@ -509,7 +509,7 @@ static int launch_ks_tiled_gw(Context &c, const dev::KsTiledArgs &T, size_t bloc
     void (*kern)(const dev::KsTiledArgs);
     if constexpr (WIDE) kern = dev::lwe_ks64_tiled_kernel<GW>;
     else kern = dev::lwe_ks32_tiled_kernel<GW>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(kern);
     if (e != cudaSuccess) return c.cuda_fail(e, "tiled key switch smem attribute");
     kern<<<(unsigned)blocks, dev::kKsTileWarps * 32, smem, st>>>(T);
     c.launches++;

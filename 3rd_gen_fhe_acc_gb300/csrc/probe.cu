@@ -240,7 +240,7 @@ int measure_components(Context &c, double ns[4])
     int rc = FHEACC_OK;
     auto k0 = dev::ntt_rate_kernel<0>, k1 = dev::ntt_rate_kernel<1>, k2 = dev::ntt_rate_kernel<2>;
     for (auto k : {k0, k1, k2})
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        if (allow_dynamic_smem(k) != cudaSuccess)
             return c.cuda_fail(cudaGetLastError(), "component probe smem attribute");
     rc = time_best(c, [&] { k0<<<blocks, 320, smem, c.stream>>>(nullptr, iters, c.nc, c.d_fwd_tw, c.d_inv_tw, bg); }, &ms[0]);
     if (!rc && tables)

@@ -132,8 +132,8 @@ static int launch_products_cluster(Context &c, const Products64 &A, cudaStream_t
     auto kern = dev::products64_cluster_kernel<B, C>;
     const size_t smem = dev::BlockLayout<B, C>::key_off(A.DG), sms = (size_t)sms_products(c);
     *fits = false;
-    if (smem > 227 * 1024 || A.count * C > sms) return FHEACC_OK;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > kMaxDynamicSmem || A.count * C > sms) return FHEACC_OK;
+    cudaError_t e = allow_dynamic_smem(kern);
     if (e != cudaSuccess) return c.cuda_fail(e, "products smem attribute");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(A.count * C));
@@ -166,7 +166,7 @@ static int launch_products_workers(Context &c, const Products64 &A, cudaStream_t
 {
     auto kern = dev::products64_workers_kernel<B, W>;
     const size_t smem = W * dev::BlockLayout<B, 1>::key_off(A.DG);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(kern);
     if (e != cudaSuccess) return c.cuda_fail(e, "products smem attribute");
     const size_t blocks = std::min<size_t>((size_t)sms_products(c), A.count);
     kern<<<(unsigned)blocks, W * dev::worker_threads64(W), smem, st>>>(A, c.d_tw64, c.d_itw64, c.nc64);
@@ -188,8 +188,8 @@ int launch_products64(Context &c, Products64 A, cudaStream_t st)
     if (!rc && !fits) rc = launch_products_cluster<4, 2>(c, A, st, &fits);
     if (!rc && !fits) rc = launch_products_cluster<4, 1>(c, A, st, &fits);
     if (rc || fits) return rc;
-    return 2 * dev::BlockLayout<4, 1>::key_off(A.DG) <= 227 * 1024 ? launch_products_workers<4, 2>(c, A, st)
-                                                                  : launch_products_workers<4, 1>(c, A, st);
+    return 2 * dev::BlockLayout<4, 1>::key_off(A.DG) <= kMaxDynamicSmem ? launch_products_workers<4, 2>(c, A, st)
+                                                                     : launch_products_workers<4, 1>(c, A, st);
 }
 
 }  // namespace fheacc
