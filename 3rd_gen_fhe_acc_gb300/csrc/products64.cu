@@ -175,9 +175,30 @@ static int launch_products_workers(Context &c, const Products64 &A, cudaStream_t
     return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "products launch");
 }
 
+// Whether the outputs (out_per = 1) overlap the inputs at `in` other than each its own: a
+// product reads its inputs before it writes, but not before the others write.
+static bool outputs_overlap(const Products64 &A, const uint64_t *in)
+{
+    if (!in || (in == A.out && (A.count == 1 || A.in_stride == A.out_s1))) return false;
+    const uint64_t *in_end = in + (A.count - 1) * A.in_stride + 4096, *out_end = A.out + (A.count - 1) * A.out_s1 + 4096;
+    return in < out_end && A.out < in_end;
+}
+
 int launch_products64(Context &c, Products64 A, cudaStream_t st)
 {
     if (!A.count) return FHEACC_OK;
+    if (A.out_per == 1 && (outputs_overlap(A, A.in0) || outputs_overlap(A, A.in1))) {
+        int rc = ensure_scratch(c, c.psi, A.count * 4096 * sizeof(uint64_t));
+        if (rc) return rc;
+        Products64 B = A;
+        B.out = (uint64_t *)c.psi.ptr;
+        B.out_s1 = 4096;
+        rc = launch_products64(c, B, st);
+        if (rc) return rc;
+        cudaError_t e = cudaMemcpy2DAsync(A.out, A.out_s1 * sizeof(uint64_t), B.out, 4096 * sizeof(uint64_t),
+                                          4096 * sizeof(uint64_t), A.count, cudaMemcpyDeviceToDevice, st);
+        return e == cudaSuccess ? FHEACC_OK : c.cuda_fail(e, "products copy");
+    }
     A.DG = (int)c.p.digitG;
     A.bg_bits = c.p.BG_bits;
     A.c54 = limb_c54(c);
