@@ -580,6 +580,8 @@ int fheacc_upload_bootstrap_key(fheacc_ctx *ctx, const uint64_t *btkey, size_t w
     if (!ctx) return FHEACC_EINVAL;
     Context &c = *reinterpret_cast<Context *>(ctx);
     if (!btkey || words != fheacc_bootstrap_key_words(&c.p)) return c.fail(FHEACC_EINVAL, "bootstrap key size mismatch");
+    // the blind rotations keep a residue, below Br and q, in a byte
+    if (std::min(c.p.Br, c.p.q) > 256) return c.fail(FHEACC_EINVAL, "refresh base above 256: gates are not supported");
     DeviceGuard g(c.device);
     return bootstrap_key_pass(c, btkey, words, false);
 }

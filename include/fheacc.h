@@ -156,7 +156,9 @@ size_t fheacc_device_bytes(const fheacc_ctx *ctx);
 /* Key upload, host words in the formats above; re-laid-out for the device
  * once, at upload. Replace dma_write_bootstrap_key (myfpga.cpp:596-656),
  * dma_write_subs_key (myfpga.cpp:658-712). The LWE key-switch key has no FPGA
- * counterpart (the FPGA runtime key-switches on the host, myfpga.cpp:1519). */
+ * counterpart (the FPGA runtime key-switches on the host, myfpga.cpp:1519). The
+ * bootstrap key's refresh residues must stay below 256 (Br or q at most 256;
+ * else FHEACC_EINVAL). */
 int fheacc_upload_bootstrap_key(fheacc_ctx *ctx, const uint64_t *btkey, size_t words);
 int fheacc_upload_lwe_ks_key(fheacc_ctx *ctx, const uint64_t *kskey, size_t words);
 int fheacc_upload_subs_key(fheacc_ctx *ctx, const uint64_t *subs_key, size_t words);
