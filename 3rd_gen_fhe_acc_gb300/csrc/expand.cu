@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256) expand32_kernel(const __grid_constant__ E
                                                       const uint2 *__restrict__ inv_tw, uint32_t mu32)
 {
     __shared__ __align__(16) uint32_t t[2][kPadN];
-    __shared__ __align__(16) uint32_t d[5][kPadN];
+    __shared__ __align__(16) uint32_t d[4][kPadN];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t Q = c.Q;
     const int L = A.L;
