@@ -406,7 +406,10 @@ def run_mixed(args, cache=None):
         S["trials"] = S["ctx"].autotune(S["total"])
         S["tuned_ms"] = alone(S)
         S["tuned_same"] = np.array_equal(S["dout"].cpu().numpy().view(np.uint64), S["ref_out"])
+        # the shape that the tuner keeps: the default (pipes = 0) unless another is 1 % faster
+        default = next(t for t in S["trials"] if t["pipes"] == 0)
         best = min(S["trials"], key=lambda t: t["ms"])
+        best = default if best["ms"] >= 0.99 * default["ms"] else best
         S["best"] = {k: best[k] for k in ("regs_for_3", "ctas_per_sm", "group", "window", "pipes")}
 
     graph = F.Graph()
@@ -670,28 +673,28 @@ def run_psi(args, cache=None):
             e2e.append(time.perf_counter() - t0)
     e2e_ok = decodes(h_out.numpy().view(np.uint64))
 
-    # integer roofline: 64-bit modular multiplies of the query, the reference's
-    # algorithm (an N = 2048 NTT is N/2 log2 N butterflies, an inverse NTT that
-    # plus N scalings): per expand item (one RLWE of one level) the inverse
-    # NTTs of a and b, digitKS_R + 1 forward NTTs, 2 digitKS_R N key products
-    # and 2N for the rotation; per RLWE x RGSW 210,944 as in the bootstrap
+    # integer roofline: the multiplies that the query's launches execute (fold_form_slots);
+    # beside it the 64-bit modular multiplies of the reference's algorithm (an N = 2048 NTT
+    # is N/2 log2 N butterflies, an inverse NTT that plus N scalings): per expand item (one
+    # RLWE of one level) the inverse NTTs of a and b, digitKS_R + 1 forward NTTs, 2 digitKS_R
+    # N key products and 2N for the rotation; per RLWE x RGSW 210,944 as in the bootstrap
     L = P.digitKS_R
     ntt = N // 2 * logN
     mult = 2 * (ntt + N) + 2 * dG * ntt + 4 * dG * N   # 210,944
     expand_item = 2 * (ntt + N) + (L + 1) * ntt + 2 * L * N + 2 * N
     items = dG * (N - 1)
     n_mult = dG * N + (entries - 1) + logN
-    work = items * expand_item + n_mult * mult + logN * 2 * N
+    ref_work = items * expand_item + n_mult * mult + logN * 2 * N
+    step_slots, expand_slots = fold_form_slots(P)
+    work = items * expand_slots + n_mult * step_slots + logN * 2 * N * 10
     imad = ctx.measure_imad_rate()
-    slots = 10   # five 32 x 32 -> 64 multiplies, 2 issue slots each
-    peak = imad / slots
-    achieved = work / (statistics.mean(step_ms) / 1e3)
-    roofline = {"bound": "int", "achieved": achieved / 1e9, "peak": peak / 1e9, "unit": "G modmul/s",
-                "frac": achieved / peak, "traffic": None, "kernel": "whole query",
-                "work": "%d expand items x %d + %d RLWE x RGSW x %d + %d rotation multiplies = %.3g 64-bit modular "
-                        "multiplies per query" % (items, expand_item, n_mult, mult, logN * 2 * N, work),
-                "peak_source": "IMAD rate measured in this run (%.1f T lane-op/s) / %d IMAD issue slots per 64-bit "
-                               "modular multiply (five 32 x 32 -> 64 multiplies)" % (imad / 1e12, slots)}
+    query_s = statistics.mean(step_ms) / 1e3
+    roofline = {"bound": "int", "achieved": work / query_s / 1e9, "peak": imad / 1e9, "unit": "G issue slots/s",
+                "frac": work / query_s / imad, "traffic": None, "kernel": "whole query",
+                "work": "%d expand items x %d + %d RLWE x RGSW x %d + %d rotation multiplies x 10 = %.3g IMAD issue "
+                        "slots per query" % (items, expand_slots, n_mult, step_slots, logN * 2 * N, work),
+                "reference_gmodmul_per_s": ref_work / query_s / 1e9,
+                "peak_source": "IMAD rate measured in this run"}
 
     cpu = None
     if not args.no_cpu:
@@ -742,6 +745,22 @@ def run_psi(args, cache=None):
         print(json.dumps(line))
         ctx.close()
     return line
+
+
+def fold_form_slots(P):
+    """IMAD issue slots of the multiplies that the block form executes (64-bit words,
+    Q = 2^b - c, four blocks; csrc/block64.cuh): of one RLWE x RGSW step and of one expand
+    item. A 32 x 32 -> 64 multiply is 2 slots: 5 of them a modular multiply by a constant,
+    3 a MAC product, 4 the reduction of a MAC sum, 1 each fold; a word of a digit's residue
+    takes 2 per other block and a fold."""
+    N, dG, L, B = P.N, P.digitG, P.digitKS_R, 4
+    logN = N.bit_length() - 1
+    mul, mac, mac_end, fold = 10, 6, 8, 2
+    inverse = (N // 2 * logN + N // 2) * mul + N // 2 * fold   # the last stage: two multiplies a pair
+    digit = N * ((B - 1) * 4 + fold) + N // 2 * (logN - 2) * mul
+    step = 2 * inverse + 2 * (dG - 1) * digit + 4 * dG * N * mac + 2 * N * mac_end
+    expand = inverse + L * digit + 2 * L * N * mac + 2 * N * mac_end + 2 * N * mul
+    return step, expand
 
 
 def fheacc_key_bytes(P):
@@ -965,9 +984,9 @@ def measure_batch(F, D, cache, preset, B, args, dev_id, n_steps, plain_sample, s
     modmul_per_step = (2 + 2 * dG) * (N // 2) * logN + 2 * (2 * dG) * N + 2 * N
     br_s = statistics.mean(br_ms) / 1e3
     achieved_modmul = total_steps * modmul_per_step / br_s
-    # IMAD issue slots per modular multiply: 32-bit words (Shoup) 4 (mul.hi counts
-    # 2); 64-bit words, Q = 2^b - c, 10 (five 32 x 32 -> 64 multiplies, 2 each)
-    slots = 4.0 if N == 1024 else 10.0
+    # 32-bit words: IMAD issue slots per (Shoup) modular multiply, 4 (mul.hi counts 2), and the
+    # reference's multiplies. 64-bit words, Q = 2^b - c: the slots of the multiplies executed
+    slots = 4.0
     peak_modmul = imad / slots
     word = 4 if N == 1024 else 8
     rgsw_bytes = 2 * dG * 2 * N * word
@@ -994,15 +1013,27 @@ def measure_batch(F, D, cache, preset, B, args, dev_id, n_steps, plain_sample, s
     ks_rows = P.N * P.digitKS
     plain_bytes = float(steps[:Pn].mean()) * rgsw_bytes + ks_rows * (P.n + 1) * word
     plain_gbs = plain_bytes / (statistics.mean(lat) / 1e3) / 1e9
-    roofline = {
-        "bound": "int", "achieved": achieved_modmul / 1e9, "peak": peak_modmul / 1e9, "unit": "G modmul/s",
-        "frac": achieved_modmul / peak_modmul, "traffic": traffic,
-        "kernel": "br32_pipe_kernel" if N == 1024 else "br64_items_kernel", "kernel_ms": statistics.mean(br_ms),
-        "work": "%d RLWE x RGSW steps x %d modular multiplies (NTT butterflies, MAC products, N^-1 scaling)" % (
-            total_steps, modmul_per_step),
-        "peak_source": "IMAD rate measured in this run (%.1f T lane-op/s) / %d IMAD issue slots per %d-bit "
-                       "modular multiply" % (imad / 1e12, slots, 32 if N == 1024 else 64),
-    }
+    if N == 1024:
+        roofline = {
+            "bound": "int", "achieved": achieved_modmul / 1e9, "peak": peak_modmul / 1e9, "unit": "G modmul/s",
+            "frac": achieved_modmul / peak_modmul, "traffic": traffic,
+            "kernel": "br32_pipe_kernel", "kernel_ms": statistics.mean(br_ms),
+            "work": "%d RLWE x RGSW steps x %d modular multiplies of the reference's algorithm (NTT butterflies, MAC "
+                    "products, N^-1 scaling)" % (total_steps, modmul_per_step),
+            "peak_source": "IMAD rate measured in this run (%.1f T lane-op/s) / %d IMAD issue slots per 32-bit "
+                           "modular multiply" % (imad / 1e12, slots),
+        }
+    else:
+        step_slots = fold_form_slots(P)[0]
+        achieved = total_steps * step_slots / br_s
+        roofline = {
+            "bound": "int", "achieved": achieved / 1e9, "peak": imad / 1e9, "unit": "G issue slots/s",
+            "frac": achieved / imad, "traffic": traffic,
+            "kernel": "br64_items_kernel", "kernel_ms": statistics.mean(br_ms),
+            "work": "%d RLWE x RGSW steps x %d IMAD issue slots of the multiplies executed" % (total_steps, step_slots),
+            "reference_gmodmul_per_s": achieved_modmul / 1e9,
+            "peak_source": "IMAD rate measured in this run",
+        }
     if comp:
         # SM time of one step's pieces run alone vs the pipeline's SM time per step
         sms = torch.cuda.get_device_properties(dev_id).multi_processor_count
