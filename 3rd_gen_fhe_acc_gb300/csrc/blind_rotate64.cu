@@ -448,9 +448,9 @@ static int launch_cluster(Context &c, const dev::BlockArgs &A, int max_ctas, cud
 // and 1 CTAs while all ciphertexts run at once; that times ciphertexts per cluster and 4 %
 // over items; the throughput form's, a worker's chain up to two ciphertexts per SM. At
 // digitG = 6: over items 4 CTAs from 39 to 60 gates, 2 from 77 to 131, 1 from 153 to 241.
-// Blind rotation of n = 200: 50 gates 6.57 ms on 2 CTAs, 5.57 over items on 4; 62 gates 6.55
-// and 6.59; 100 gates 11.8 on one, 8.8 over items on 2; 130 gates 11.7 and 11.6; 160 gates
-// 19.4 in the throughput form, 12.7 over items on one; 230 gates 20.2 and 18.0; 260 gates
+// Blind rotation of n = 200: 50 gates 6.57 ms on 2 CTAs, 5.63 over items on 4; 62 gates 6.55
+// and 6.59; 100 gates 11.9 on one, 8.8 over items on 2; 130 gates 11.7 and 11.6; 160 gates
+// 19.4 in the throughput form, 12.6 over items on one; 230 gates 20.2 and 17.9; 260 gates
 // 20.5 and 20.6.
 static int launch_latency(Context &c, const dev::BlockArgs &A, int max_ctas, cudaStream_t st, bool *taken)
 {

@@ -17,7 +17,8 @@
 //      of each digit, of which the CTA keeps its blocks' words;
 //   3. a warp per digit and block: forward stages t = 128 .. 1;
 //   4. multiply-accumulate of the CTA's words, keys from shared memory (copied
-//      a step ahead with cp.async, by the warps that have no part in 1).
+//      a step ahead with cp.async: on one CTA by the warps that have no part in 1, on more
+//      by those that have none in 3).
 // One GB300, per step: 2.0 us on 4 CTAs, 2.5 on 2, 3.4 on one; a CTA of 8 warps with one
 // transform each took 3.8 (one gate) to 4.3 (152). On 4 CTAs a step is 4160 cycles: 830
 // for 1 (two warps, a chain of eight stages), 685 for the cluster barrier, 865 for 2

@@ -12,7 +12,8 @@ namespace dev {
 namespace cg = cooperative_groups;
 
 // Threads of a CTA: the 10 digits' 512-word blocks are 640 octets (digitG = 6), all
-// at once in the latency form, half of them in the throughput form (two CTAs per SM).
+// at once in the latency form (kTB), half of them for each of the throughput form's two
+// workers in a CTA (kTP).
 constexpr int kTB = 640, kTP = 320;
 // A worker alone on its SM (digitG = 7 and 8, whose work areas fill more than half of the
 // shared memory) has kTB threads: 1000 products at digitG = 8 451 us with kTP, 344 so;
@@ -29,8 +30,8 @@ __device__ __forceinline__ void mac27(uint64_t (&s)[3], uint32_t x0, uint32_t x1
     s[2] += mul_wide64(x1, w.y);
 }
 
-// The value sums[0] + 2^27 (sums[1] - sums[0] - sums[2]) + 2^54 sums[2] mod Q, below 2Q: c54 (2^54 mod Q, below 2^19) folds the part
-// Y above 2^54 (Y < 2^64) twice.
+// The value sums[0] + 2^27 (sums[1] - sums[0] - sums[2]) + 2^54 sums[2] mod Q, below 2Q:
+// c54 (2^54 mod Q, below 2^19) folds the part Y above 2^54 (Y < 2^64) twice.
 __device__ __forceinline__ uint64_t mac27_reduce(const uint64_t (&s)[3], uint32_t c54, const Ntt64Consts &c)
 {
     constexpr uint64_t m27 = (1u << 27) - 1;

@@ -320,7 +320,7 @@ __device__ __forceinline__ bool pool_take(const Br64Args &A, int S, int mode, un
 }
 
 // W workers of 256 threads per CTA (W = 1: a lone gate per SM, 128 registers
-// without spills; 49 ms for one gate where 80 registers took 95 ms). Each
+// without spills). Each
 // CTA claims groups of consecutive ciphertexts; its workers share the group's
 // (step, ciphertext) items through a cursor that walks them step-major, and a
 // worker issues an item once the previous item of its ciphertext (its last

@@ -226,8 +226,8 @@ int launch_lwe_keyswitch32_indexed(Context &c, const uint32_t *d_extract, size_t
                                    uint64_t *d_out, const uint32_t *d_out_idx, cudaStream_t st);
 // LWE key switch (+ optional modulus switch) from extracted RLWEs
 // (lwe_ks.cu). d_scratch (optional, scratch_bytes of free device memory, 16-byte
-// aligned; the blind rotation's accumulators once it is done) lets a few
-// ciphertexts' rows be split over many CTAs (count * ks_row u64 words of
+// aligned; the blind rotation's accumulators once it is done) lets each
+// ciphertext's rows be split over CTAs (count * ks_row u64 words of
 // partial sums) and large batches take the tiled form (their digits,
 // N * digitKS bytes per gate).
 int launch_lwe_keyswitch32(Context &c, const uint32_t *d_extract, size_t count, bool modswitch, uint64_t *d_out,
@@ -268,9 +268,9 @@ uint64_t ks64_digit_magic(const Context &c);
 bool ks64_tiled_applies(const Context &c, size_t count, int sms, size_t scratch_bytes);
 int launch_ks64_tiled(Context &c, const uint64_t *d_extract, size_t count, bool modswitch, uint64_t *d_out,
                       const uint32_t *d_out_idx, void *scratch, int sms, cudaStream_t st);
-// d_scratch (optional, scratch_bytes of free device memory): from two gates
-// per SM holds the tiled form's digits; below, lets a few ciphertexts' rows be
-// split over many CTAs (count * ks_row u64 partial sums).
+// d_scratch (optional, scratch_bytes of free device memory): from
+// kKs64TiledGatesPerSm gates per SM holds the tiled form's digits; below, lets each
+// ciphertext's rows be split over CTAs (count * ks_row u64 partial sums).
 int launch_lwe_keyswitch64(Context &c, const uint64_t *d_extract, size_t count, bool modswitch, uint64_t *d_out,
                            cudaStream_t st, const uint32_t *d_out_idx = nullptr, void *d_scratch = nullptr,
                            size_t scratch_bytes = 0);

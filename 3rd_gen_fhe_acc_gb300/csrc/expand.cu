@@ -7,13 +7,15 @@
 // (app.cpp:26-76); on the FPGA the RLWESUBS instruction (subs_module.sv +
 // the NTT/MAC chain) and fpga_expand_RLWE (myfpga.cpp:1662-1790).
 //
-// One CTA handles one RLWE (an "item"). The substitution is applied while the
+// An RLWE is an "item": of one CTA (32-bit words, and 64-bit moduli without a fold form),
+// or of a cluster of CTAs or a worker (block form). The substitution is applied while the
 // time-domain coefficients are read: out[e] = in[i'] when i' < N, else
 // -in[i' - N], with i' = e * power^-1 mod 2N and power = N / 2^f + 1 (odd) --
 // the inverse of poly_substitute's scatter out[i * power mod N] = +-in[i]. The
 // key switch then decomposes sigma(a) in base 2^Bks_R_bits, transforms each
-// digit and multiply-accumulates with the key rows; sigma(b) is transformed
-// once. Modes:
+// digit and multiply-accumulates with the key rows. Of sigma(b) only the NTT is needed,
+// whose words the automorphism permutes (subs_ntt_src; the moduli without a fold form
+// transform it). Modes:
 //   SUBS      out = RLWE_substitute(c, f)
 //   KS        out = RLWE_keyswitch(c, ksk)                (f = 0 is the identity)
 //   SUBS_KS   out = RLWE_keyswitch(RLWE_substitute(c, f), ksk)

@@ -10,7 +10,9 @@
 // Every operation is composed of the library's batched RLWE x RGSW kernels
 // (bootstrap32.cu / bootstrap64.cu, which take one RGSW per item or one shared
 // RGSW), expand_RLWE (expand.cu) and one elementwise kernel (RLWE subtraction,
-// addition, and the NTT-domain rotation RLWE_rotate_freq, RLWE.cpp:411-430).
+// addition, and the NTT-domain rotation RLWE_rotate_freq, RLWE.cpp:411-430); for
+// 64-bit moduli Q = 2^b - c the products take these into their loads and stores
+// (products64.cu).
 // Ciphertexts are canonical NTT-domain RLWEs, [count][2N] u64, as in the
 // reference; results are bit-identical to it.
 #include "br64.cuh"
